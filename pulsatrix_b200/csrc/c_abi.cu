@@ -21,6 +21,7 @@
 #include "scan_rows.cuh"
 #include "shard_records.cuh"
 #include "topk_rows.cuh"
+#include "whole_rows.cuh"
 
 namespace {
 
@@ -317,16 +318,48 @@ psx_status psx_b200_sample_rows(psx_ctx* ctx, void* stream_ptr, const float* log
                                      plan, sp, /*alternate=*/true)) {
         return s;
     }
-    if (psx_status s = configure_merge(ctx, plan, plan.parts)) return s;
-
-    psx::MergeParams mp{};
-    psx::fill_merge_params(mp, sp, plan, config, rows, vocab, uniforms, tokens, log_probs, row_status, diag, logits, row_stride);
-
     cudaEvent_t marks[3] = {nullptr, nullptr, nullptr};
     if (ctx->timing) {
         for (cudaEvent_t& e : marks) PSX_CUDA(cudaEventCreate(&e));
         PSX_CUDA(cudaEventRecord(marks[0], stream));
     }
+    if (plan.lists_cannot_bound && plan.nucleus) {  // no filter at all: two kernels of their own (whole_rows.cu)
+        psx::WholeRowParams wp{};
+        wp.logits = logits;
+        wp.row_stride = row_stride;
+        wp.rows = rows;
+        wp.vocab = vocab;
+        wp.history_ids = sp.apply_penalty ? history_ids : nullptr;
+        wp.history_offsets = history_offsets;
+        wp.banned_ids = sp.banned_ids;
+        wp.num_banned = sp.num_banned;
+        wp.penalty = sp.penalty;
+        wp.apply_temperature = sp.apply_temperature;
+        wp.temperature = sp.temperature;
+        wp.segments = (int32_t)psx::whole_row_segments(vocab);
+        wp.inputs_ready = sp.inputs_ready;
+        wp.wait_before_writes = sp.wait_before_writes;
+        Buffer& records = ctx->stats[ctx->scratch_set];
+        if (psx_status s = reserve(records, (size_t)rows * wp.segments * sizeof(psx::SegmentStats))) return s;
+        wp.stats = static_cast<psx::SegmentStats*>(records.ptr);
+        wp.uniforms = uniforms;
+        wp.tokens = tokens;
+        wp.log_probs = log_probs;
+        wp.row_status = row_status;
+        wp.diag = diag;
+        if (ctx->timing) PSX_CUDA(cudaEventRecord(marks[1], stream));  // (one stage: its time is the second's)
+        PSX_CUDA(psx::launch_whole_rows(wp, stream));
+        ctx->launches += 2;
+        if (ctx->timing) {
+            PSX_CUDA(cudaEventRecord(marks[2], stream));
+            ctx->timing_events.insert(ctx->timing_events.end(), marks, marks + 3);
+        }
+        return PSX_OK;
+    }
+    if (psx_status s = configure_merge(ctx, plan, plan.parts)) return s;
+
+    psx::MergeParams mp{};
+    psx::fill_merge_params(mp, sp, plan, config, rows, vocab, uniforms, tokens, log_probs, row_status, diag, logits, row_stride);
     if (!plan.lists_cannot_bound) {
         PSX_CUDA(psx::launch_scan_rows(sp, plan.nucleus, stream));
         ++ctx->launches;

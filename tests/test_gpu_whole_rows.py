@@ -1,0 +1,48 @@
+"""Sampling with no filter (whole_rows.cu): segments of 512 columns, a run of several segments per thread of the
+drawing kernel beyond 131,072 columns, rows off the 16-byte grid, everything banned in a segment.  Token ids, statuses
+and survivor counts as the reference's; the distance of the draw from its bucket's edges, which both sides form from
+sums over the whole row, agrees to what the reference's sequential double sums may be off by: 3 sums of `vocab` terms
+of at most 1 in all, each addition rounded at 2^-53."""
+import numpy as np
+import pytest
+
+import gpu_harness as gh
+import oracle_lib as ol
+import pulsatrix_b200 as psx
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(vocab, rows, settings, **kw):
+    logits, hist = ol.synth_rows(np.arange(rows) + 7 * vocab, vocab, 2.0, 0.7, 40)
+    hist[:, 3] = hist[:, 5]  # an id twice
+    cfg = ol.make_config(max_new_tokens=4, do_sample=True, **settings)
+    (_, _, _, diag), want = gh.check_rows_against_oracle(logits, hist, np.arange(rows + 1, dtype=np.int64) * 40, cfg,
+                                                         np.arange(rows, dtype=np.uint64) + vocab, **kw)
+    assert np.abs(diag["draw_margin"] - want["draw_margin"]).max() <= 3 * vocab * 2.0**-53
+
+
+@pytest.mark.parametrize("vocab", [1025, 1537, 4095, 4097, 20011, 131072, 131073, 262144, 300007])
+@pytest.mark.parametrize("settings", [dict(), dict(temperature=0.9, repetition_penalty=1.2)], ids=["plain", "processed"])
+def test_edges_of_segments(vocab, settings):
+    _run(vocab, 5, settings)
+
+
+def test_rows_off_the_vector_grid():
+    for shift in (1, 2, 3):
+        _run(5003, 6, dict(temperature=1.4, repetition_penalty=0.8), pad_columns=shift, shift=shift)
+
+
+def test_many_rows_share_a_warp():
+    _run(12289, 300, dict(temperature=0.7, repetition_penalty=1.1))
+
+
+def test_banned_segments_and_failed_rows():
+    vocab, rows = 2048, 4
+    logits = np.full((rows, vocab), -3.0, dtype=np.float32)
+    logits[:, 700] = 1000.0  # everything else has no mass in double precision
+    logits[1, 2047] = np.inf
+    cfg = ol.make_config(max_new_tokens=2, do_sample=True, min_new_tokens=1, eos_token_ids=list(range(512)))
+    hist, offsets = np.zeros((rows, 1), dtype=np.int64), np.arange(rows + 1, dtype=np.int64)
+    (tokens, _, status, _), _ = gh.check_rows_against_oracle(logits, hist, offsets, cfg, np.arange(rows, dtype=np.uint64), expect_ok=False)
+    assert status[1] == psx.ROW_NON_FINITE and (tokens[[0, 2, 3]] == 700).all()
