@@ -338,7 +338,6 @@ psx_status psx_b200_sample_rows(psx_ctx* ctx, void* stream_ptr, const float* log
         wp.temperature = sp.temperature;
         wp.segments = (int32_t)psx::whole_row_segments(vocab);
         wp.inputs_ready = sp.inputs_ready;
-        wp.wait_before_writes = sp.wait_before_writes;
         Buffer& records = ctx->stats[ctx->scratch_set];
         if (psx_status s = reserve(records, (size_t)rows * wp.segments * sizeof(psx::SegmentStats))) return s;
         wp.stats = static_cast<psx::SegmentStats*>(records.ptr);

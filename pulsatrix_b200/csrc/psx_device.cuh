@@ -105,6 +105,12 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     return r;
 }
 
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -146,10 +152,10 @@ __device__ __forceinline__ void grid_dependents_may_launch() { asm volatile("gri
 
 // ---- warp / block helpers ------------------------------------------------------------------------
 
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
+__device__ __forceinline__ float warp_max(float v) {  // (NaN operands are skipped, as by fmaxf)
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

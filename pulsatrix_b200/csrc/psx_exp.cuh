@@ -1,58 +1,52 @@
 // exp() of a difference of two floats in double precision, for sweeps that take it of every logit of a row.
 //
 // Tang's table method ("Table-driven implementation of the exponential function in IEEE floating-point
-// arithmetic", ACM TOMS 15, 1989): d = n * ln2/512 + r, exp(d) = 2^(n / 512) * 2^((n % 512) / 512) * exp(r).  With
-// |r| <= ln2/1024 (and a little, n is rounded in single precision) the Taylor series to r^4 / 24 ends below
-// 2e-18; the rounding of ln2/512, n times, adds at most |d| * 2^-53 -- what the rounding of the reference's own
-// argument (double)x - (double)max (src/generation.cpp:46) may do as well.  Relative error (4 + |d|) * 2^-53 at most.
-// Nine double-precision operations, against the twenty-odd of the general function, which has to take any argument.
+// arithmetic", ACM TOMS 15, 1989): d = n * ln2/32 + r, exp(d) = 2^(n / 32) * 2^((n % 32) / 32) * exp(r).  With
+// |r| <= ln2/64 the Taylor series to r^6 / 720 ends below 4e-18; the rounding of ln2/32, n times, adds at most
+// |d| * 2^-53 -- what the rounding of the reference's own argument (double)x - (double)max (src/generation.cpp:46)
+// may do as well.  Relative error (4 + |d|) * 2^-53 at most.  Twelve double-precision operations, against the
+// twenty-odd of the general function, which has to take any argument.
+//
+// The table's 32 powers lie one in each lane, and a look-up is two shuffles: nothing to load ahead of the sweep, no
+// shared memory, no two lanes in one another's way.  (A table of 512 in shared memory saves two operations of the
+// series, but its random look-ups queue six deep at the banks; sixteen copies of 64 entries do not, but every CTA then
+// writes 8 KB before it starts.)
 #pragma once
 
 #include <stdint.h>
 
 namespace psx {
 
-constexpr int kExpTable = 512;
-
-struct ExpTable {
-    double power[kExpTable];  // 2^(j / 512)
-    constexpr ExpTable() : power() {
-        for (int j = 0; j < kExpTable; ++j) {
-            const double x = (double)j / kExpTable * 0.693147180559945309417232121458;  // 2^t = e^(t ln 2), t in [0, 1)
+struct ExpPowers {
+    double power[32];  // 2^(j / 32)
+    constexpr ExpPowers() : power() {
+        for (int j = 0; j < 32; ++j) {
+            const double x = (double)j / 32 * 0.693147180559945309417232121458;  // 2^t = e^(t ln 2), t in [0, 1)
             double sum = 1.0;
             for (int k = 24; k >= 1; --k) sum = 1.0 + sum * x / k;
             power[j] = sum;
         }
     }
 };
-static __device__ constexpr ExpTable kExpPowers{};
+static __device__ constexpr ExpPowers kExpPowers{};
+__device__ __forceinline__ double exp_power_of_lane() { return kExpPowers.power[threadIdx.x & 31]; }
 
-// The table in shared memory (4 KB): every thread of the block calls this, and the block meets before the first use.
-__device__ __forceinline__ void load_exp_table(double* table) {
-    for (int j = threadIdx.x; j < kExpTable; j += blockDim.x) table[j] = kExpPowers.power[j];
-}
-
-// A float as a double by its bits (the conversion instruction runs at a quarter of the double-precision rate).  A zero or
-// subnormal comes out below 2^-126 in magnitude, which moves no exponential here.  Finite x only.
-__device__ __forceinline__ double double_of_float(float x) {
-    const uint32_t u = __float_as_uint(x);
-    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(u << 29));
+// exp(d) for -705 <= d <= 0, by a whole warp; `power` is exp_power_of_lane().
+__device__ __forceinline__ double exp_of_gap(double d, double power) {
+    const double shifted = fma(d, 46.166241308446828, 6755399441055744.0);  // 32 / ln2; + 1.5 * 2^52: n in the low word
+    const int n = __double2loint(shifted);
+    const double r = fma(shifted - 6755399441055744.0, -0.021660849392498290919288503568, d);  // ln2 / 32
+    const double r2 = r * r;
+    const double high = fma(r2, 1.0 / 720.0, fma(r, 1.0 / 120.0, 1.0 / 24.0));
+    const double tail = fma(r2, fma(r2, high, fma(r, 1.0 / 6.0, 0.5)), r);
+    const double p = __hiloint2double(__shfl_sync(0xFFFFFFFFu, __double2hiint(power), n), __shfl_sync(0xFFFFFFFFu, __double2loint(power), n));
+    const double y = fma(p, tail, p);
+    return __hiloint2double(__double2hiint(y) + ((n & ~31) << 15), __double2loint(y));
 }
 
 constexpr float kExpFloor = -700.0f;  // exp(-700) = 1e-304: what lies below counts as nothing
 
-// exp(x - top) for finite x <= top (x_d, top_d: the same two as doubles); 0 below kExpFloor and for x = -inf.
-__device__ __forceinline__ double exp_below(float x, double x_d, float top, double top_d, const double* table) {
-    const float gap = __fsub_rn(x, top);
-    const float rounded = __fmaf_rn(fmaxf(gap, kExpFloor), 738.65986f, 12582912.0f);  // + 1.5 * 2^23: n in the low bits
-    const int n = (int)(__float_as_uint(rounded) - 0x4B400000u);
-    const double whole = __hiloint2double(0x43300000, n ^ (int)0x80000000) - 4503601774854144.0;  // n: 2^52 + 2^31 + n, less the offset
-    const double r = fma(whole, -0.001353803087031143182455531, x_d - top_d);                              // - ln2 / 512
-    const double tail = fma(r * r, fma(r, fma(r, 1.0 / 24.0, 1.0 / 6.0), 0.5), r);
-    const double p = table[n & (kExpTable - 1)];
-    const double y = fma(p, tail, p);
-    const double scaled = __hiloint2double(__double2hiint(y) + ((n >> 9) << 20), __double2loint(y));
-    return gap >= kExpFloor ? scaled : 0.0;
-}
+// exp(x - top) for finite x <= top by a thread of its own; 0 below kExpFloor and for x = -inf.
+__device__ __forceinline__ double exp_below(float x, float top) { return x - top >= kExpFloor ? exp((double)x - (double)top) : 0.0; }
 
 }  // namespace psx

@@ -2,21 +2,23 @@
 // off -- the penalty, the EOS ban and the temperature may be on).  Every token can be drawn, so there is no short
 // list of candidates; what the draw needs is the mass of every run of columns, then the columns of one run.
 //
-//   1. weigh_segments_kernel reads every logit once.  A warp takes a segment of 512 columns into registers, finds its
-//      two maxima (raw and processed) and sums exp() of both in double precision; it reports 32 bytes.  The warps of a
-//      CTA share a bitmap of the history and a table of powers, nothing else.
-//   2. draw_token_kernel, one CTA per row: the segments' masses brought to the row's maximum, their running sum
-//      against u times the whole (the inverse-CDF walk of :140-152 in steps of a segment), then the logits of the one
-//      segment that holds the crossing, column by column.
+//   1. weigh_segments_kernel: a warp takes a segment of 512 columns into registers, finds its two maxima (raw and processed), sums exp() of
+//      both in double precision and reports 32 bytes.  The warps of a CTA share a bitmap of the history, nothing else.
+//   2. draw_token_kernel, one CTA per row: the segments' masses brought to the row's maximum, their running sum against
+//      u times the whole (the inverse-CDF walk of :140-152 in steps of a segment), then the logits of the one segment that
+//      holds the crossing, column by column.  (Drawing in the CTA that finishes a row's last segment saves the launch,
+//      but costs a fence and an atomic per CTA and runs under the arithmetic of other rows: 5 to 10 % slower from a few rows on.)
 //
 // Sums are in double precision in a fixed order (the same input gives the same bits); they differ from the
 // reference's sequential sums by rounding only, and a draw closer than that to an edge shows in draw_margin.
 //
 // Bound: 4 bytes per logit from HBM, and two double-precision exponentials per logit (one when the processed row is
-// the raw one).  The double-precision pipe (64 lanes per SM) is the longer of the two -- about 17 operations per logit
-// against 4 bytes are 1.35 : 1 -- which is why the exponential is the table one (psx_exp.cuh).  A segment is a warp's:
-// 512 columns keep 16 logits per lane in registers, so that the maximum is known before the first exponential and
-// nothing is rescaled, and one row of 50 K columns still gives 98 warps to spread over the SMs.
+// the raw one).  The double-precision pipe (64 lanes per SM) and the issue slots beside it are the longer of the two,
+// which is why the exponential is the table one (psx_exp.cuh) and the temperature a product.  A segment is a warp's: 512
+// columns keep 16 logits per lane in registers, so that the maximum is known before the first exponential and nothing is
+// rescaled, and one row of 50 K columns still gives 98 warps to spread over the SMs.
+// 100 rows x 50,021, T = 0.9: 865 us per call when one CTA per row did this in the survivor stage, 20.5 now (17 us for the
+// first kernel in two rounds of CTAs, double-precision pipe 43 % and issue slots 53 % busy); 330 rows x 50,257: 32 us.
 #include "whole_rows.cuh"
 
 #include <algorithm>
@@ -28,7 +30,7 @@ namespace psx {
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;   // eight CTAs to an SM (64 registers): the loads of some run under the arithmetic of others
 constexpr int kWarps = kThreads / 32;
 constexpr int kSegmentCols = kSegmentVecs * 4;
 constexpr int kVecs = kSegmentVecs / 32;  // float4 per lane
@@ -49,13 +51,19 @@ __device__ __forceinline__ RowWindow row_window(const WholeRowParams& p, int64_t
 }
 
 // Marks, in a bitmap of `slots` bits that starts at column `first`, the columns that `ids` names (:62: ids outside the
-// vocabulary are ignored -- their bits stand for no column of the row).  By the whole block.
+// vocabulary are ignored -- their bits stand for no column of the row).  By the whole block; four ids per thread are
+// asked for together, one trip to memory for 512 of them.
 __device__ __forceinline__ void mark_columns(const int64_t* ids, int64_t begin, int64_t end, int64_t first, int slots, int64_t vocab,
                                              uint32_t* bits) {
-    for (int64_t i = begin + threadIdx.x; i < end; i += kThreads) {
-        const int64_t id = ids[i];
-        const uint64_t at = (uint64_t)(id - first);
-        if (at < (uint64_t)slots && (uint64_t)id < (uint64_t)vocab) atomicOr(&bits[at >> 5], 1u << (at & 31));
+    for (int64_t i = begin + threadIdx.x; i < end; i += 4 * kThreads) {
+        int64_t id[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) id[q] = i + q * kThreads < end ? ids[i + q * kThreads] : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t at = (uint64_t)(id[q] - first);
+            if (at < (uint64_t)slots && (uint64_t)id[q] < (uint64_t)vocab) atomicOr(&bits[at >> 5], 1u << (at & 31));
+        }
     }
 }
 
@@ -67,137 +75,55 @@ __device__ __forceinline__ float processed(float l, bool flagged, bool banned, c
     return temper(y, p.apply_temperature != 0, p.temperature);
 }
 
-// kPlain: the processed row is the raw row (no penalty, no ban, no temperature).
-template <bool kPlain>
-__global__ void __launch_bounds__(kThreads) weigh_segments_kernel(const WholeRowParams p) {
-    __shared__ double s_table[kExpTable];
-    __shared__ uint32_t s_flag[kMostPerWarp * kWarps * kSegmentCols / 32], s_ban[kMostPerWarp * kWarps * kSegmentCols / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t row = (int64_t)blockIdx.z * 65535 + blockIdx.y;
-    const bool ends_the_grid = !p.wait_before_writes && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1;
-    grid_dependents_may_launch();
-    if (!p.inputs_ready) grid_dependency_wait();
-    if (row >= p.rows) {
-        if (ends_the_grid) grid_dependency_wait();
-        return;
-    }
-    const RowWindow w = row_window(p, row);
-    const int per_warp = p.segments_per_warp, first_segment = blockIdx.x * kWarps * per_warp;
-    float4 d[kVecs];
-    auto load = [&](int segment) {
-#pragma unroll
-        for (int k = 0; k < kVecs; ++k) {
-            const int v = segment * kSegmentVecs + k * 32 + lane;
-            d[k] = v < w.vectors ? w.base[v] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-        }
-    };
-    load(first_segment + warp);  // (under the table and the bitmap)
-    load_exp_table(s_table);
-    const bool penalise = !kPlain && p.history_ids != nullptr, flags = penalise || (!kPlain && p.num_banned > 0);
-    const int64_t first_col = (int64_t)first_segment * kSegmentCols - w.misalign;
-    const int slots = per_warp * kWarps * kSegmentCols;
-    if (flags) {
-        for (int i = threadIdx.x; i < slots / 32; i += kThreads) s_flag[i] = s_ban[i] = 0u;
-        __syncthreads();
-        if (penalise) mark_columns(p.history_ids, p.history_offsets[row], p.history_offsets[row + 1], first_col, slots, p.vocab, s_flag);
-        mark_columns(p.banned_ids, 0, p.num_banned, first_col, slots, p.vocab, s_ban);
-    }
-    __syncthreads();
-    if (p.inputs_ready && p.wait_before_writes) grid_dependency_wait();
-#pragma unroll 1
-    for (int turn = 0; turn < per_warp; ++turn) {
-        const int local = turn * kWarps + warp, segment = first_segment + local;
-        if (segment >= p.segments) break;
-        if (turn > 0) load(segment);
-        float raw_max = -INFINITY, y_max = -INFINITY;
-        bool bad = false;
-        uint32_t alive = 0;
-        float l[kVecs * 4], y[kVecs * 4];
-#pragma unroll
-        for (int k = 0; k < kVecs; ++k) {
-            const float c4[4] = {d[k].x, d[k].y, d[k].z, d[k].w};
-            const int v = k * 32 + lane;  // within the segment
-            uint32_t flag4 = 0, ban4 = 0;
-            if (flags) {
-                const int word = (local * kSegmentVecs + v) >> 3, shift = (v & 7) * 4;
-                flag4 = s_flag[word] >> shift;
-                ban4 = s_ban[word] >> shift;
-            }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int col = (segment * kSegmentVecs + v) * 4 + c - w.misalign;
-                const bool here = (uint32_t)col < (uint32_t)p.vocab;
-                bad = bad || (here && !(fabsf(c4[c]) < INFINITY));
-                l[4 * k + c] = here ? c4[c] : -INFINITY;
-                raw_max = fmaxf(raw_max, l[4 * k + c]);
-                if (!kPlain) {
-                    y[4 * k + c] = processed(l[4 * k + c], (flag4 >> c) & 1u, (ban4 >> c) & 1u, p);
-                    y_max = fmaxf(y_max, y[4 * k + c]);
-                    alive += y[4 * k + c] > -INFINITY ? 1u : 0u;
-                } else {
-                    alive += here ? 1u : 0u;
-                }
-            }
-        }
-        raw_max = warp_max(raw_max);
-        y_max = kPlain ? raw_max : warp_max(y_max);
-        const double raw_top = double_of_float(raw_max), y_top = double_of_float(y_max);
-        double raw_sum = 0.0, mass = 0.0;
-#pragma unroll
-        for (int i = 0; i < kVecs * 4; ++i) {
-            raw_sum += exp_below(l[i], double_of_float(l[i]), raw_max, raw_top, s_table);
-            if (!kPlain) mass += exp_below(y[i], double_of_float(y[i]), y_max, y_top, s_table);
-        }
-        raw_sum = warp_sum(raw_sum);
-        mass = kPlain ? raw_sum : warp_sum(mass);
-        alive = __reduce_add_sync(0xFFFFFFFFu, alive);
-        const bool any_bad = __any_sync(0xFFFFFFFFu, bad);
-        if (lane == 0) {
-            SegmentStats s;
-            s.raw_sum = raw_sum;  // (a segment past the end of its row: maxima of -inf, sums of nothing)
-            s.mass = mass;
-            s.raw_max = raw_max;
-            s.y_max = y_max;
-            s.alive = alive;
-            s.nonfinite = any_bad ? 1u : 0u;
-            p.stats[row * p.segments + segment] = s;
-        }
-    }
-    if (ends_the_grid) grid_dependency_wait();
-}
-
-// Inclusive running sum over the block in thread order; `total` is the whole.
-__device__ __forceinline__ double block_running_sum(double v, double* scratch, double& total) {
+// Running sums over the block in thread order: up to this thread, up to and with it, over all.  A thread's `before` is
+// the thread before it's `upto` bit for bit.
+struct RunningSum {
+    double before, upto, total;
+};
+__device__ __forceinline__ RunningSum block_running_sum(double v, double* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double up = __shfl_up_sync(0xFFFFFFFFu, v, o);
         if (lane >= o) v += up;
     }
-    __syncthreads();
+    double earlier = __shfl_up_sync(0xFFFFFFFFu, v, 1);
+    if (lane == 0) earlier = 0.0;
     if (lane == 31) scratch[warp] = v;
     __syncthreads();
-    double before = 0.0;
-    total = 0.0;
+    RunningSum r;
+    double base = 0.0;
+    r.total = 0.0;
 #pragma unroll
     for (int i = 0; i < kWarps; ++i) {
-        if (i < warp) before += scratch[i];
-        total += scratch[i];
+        if (i == warp) base = r.total;
+        r.total += scratch[i];
     }
-    return before + v;
+    r.before = base + earlier;
+    r.upto = base + v;
+    return r;
 }
 
-__global__ void __launch_bounds__(kThreads) draw_token_kernel(const WholeRowParams p) {
-    __shared__ double s_table[kExpTable], s_scratch[kWarps];
-    __shared__ double s_before;
-    __shared__ int s_segment, s_last, s_chosen, s_hit, s_any_alive;
+// The last thread of the block whose value is positive.
+__device__ __forceinline__ int block_last_positive(double v, uint32_t* scratch) {
+    const uint32_t votes = __ballot_sync(0xFFFFFFFFu, v > 0.0);
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = votes;
+    __syncthreads();
+    int last = -1;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) {
+        if (scratch[i] != 0) last = 32 * i + 31 - __clz(scratch[i]);
+    }
+    return last;
+}
+
+__global__ void __launch_bounds__(kThreads) draw_token_kernel(const __grid_constant__ WholeRowParams p) {
+    __shared__ double s_mass[kWarps], s_z[kWarps], s_own[kWarps], s_before;
+    __shared__ int s_hit, s_alive;
     __shared__ float s_max[2][kWarps];
-    __shared__ uint32_t s_flag[kSegmentCols / 32], s_ban[kSegmentCols / 32];
+    __shared__ uint32_t s_votes[2][kWarps], s_flag[kSegmentCols / 32], s_ban[kSegmentCols / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t row = blockIdx.x;
-    load_exp_table(s_table);
-    if (tid == 0) { s_segment = 0x7FFFFFFF; s_last = -1; s_chosen = 0x7FFFFFFF; s_hit = -1; }
-    if (tid < kSegmentCols / 32) s_flag[tid] = s_ban[tid] = 0u;
     grid_dependency_wait();
     grid_dependents_may_launch();
     const SegmentStats* stats = p.stats + row * p.segments;
@@ -209,12 +135,19 @@ __global__ void __launch_bounds__(kThreads) draw_token_kernel(const WholeRowPara
     mine.raw_max = mine.y_max = -INFINITY;
     mine.alive = mine.nonfinite = 0;
     if (begin < end) mine = stats[begin];
+    // (asked for now, needed below)
+    const double u = p.uniforms[row];
+    int64_t h_begin = 0, h_end = 0;
+    if (p.history_ids != nullptr) { h_begin = p.history_offsets[row]; h_end = p.history_offsets[row + 1]; }
+    if (tid == 0) s_alive = 0;
+    if (tid < kSegmentCols / 32) s_flag[tid] = s_ban[tid] = 0u;
     float raw_max = mine.raw_max, y_max = mine.y_max;
     uint32_t bad = mine.nonfinite;
     for (int s = begin + 1; s < end; ++s) {
-        raw_max = fmaxf(raw_max, stats[s].raw_max);
-        y_max = fmaxf(y_max, stats[s].y_max);
-        bad |= stats[s].nonfinite;
+        const SegmentStats other = stats[s];
+        raw_max = fmaxf(raw_max, other.raw_max);
+        y_max = fmaxf(y_max, other.y_max);
+        bad |= other.nonfinite;
     }
     raw_max = warp_max(raw_max);
     y_max = warp_max(y_max);
@@ -231,103 +164,250 @@ __global__ void __launch_bounds__(kThreads) draw_token_kernel(const WholeRowPara
         }
         return;
     }
-    const double y_top = double_of_float(y_max), raw_top = double_of_float(raw_max);
-    auto share = [&](double sum, float top, float row_top, double row_top_d) {
-        return sum > 0.0 ? sum * exp_below(top, double_of_float(top), row_top, row_top_d, s_table) : 0.0;
-    };
+    auto share = [&](double sum, float top, float row_top) { return sum > 0.0 ? sum * exp_below(top, row_top) : 0.0; };
     double mass = 0.0, z = 0.0;
-    int alive = 0;
+    uint32_t alive = 0;
     for (int s = begin; s < end; ++s) {
         if (s > begin) mine = stats[s];
-        mass += share(mine.mass, mine.y_max, y_max, y_top);
-        z += share(mine.raw_sum, mine.raw_max, raw_max, raw_top);
-        alive += (int)mine.alive;
+        mass += share(mine.mass, mine.y_max, y_max);
+        z += share(mine.raw_sum, mine.raw_max, raw_max);
+        alive += mine.alive;
     }
-    double total, z_total;
-    const double upto = block_running_sum(mass, s_scratch, total);
-    block_running_sum(z, s_scratch, z_total);
-    const double u = p.uniforms[row], target = u * total;
-    // ---- the segment that holds the crossing: the first whose running sum rises above the target (:140-152); if
-    // rounding leaves none, the last that holds mass -----------------------------------------------------------------
-    if (mass > 0.0) {
-        if (upto > target) atomicMin(&s_segment, begin);
-        atomicMax(&s_last, begin);
-    }
-    __syncthreads();
-    const int owner_begin = s_segment != 0x7FFFFFFF ? s_segment : s_last;
-    if (begin == owner_begin && mass > 0.0) {
-        double at = upto - mass, before = at;
+    z = warp_sum(z);
+    if (lane == 0) s_z[warp] = z;
+    const RunningSum run = block_running_sum(mass, s_mass);
+    const double total = run.total, target = u * total;
+    // ---- the segment that holds the crossing: the running sum rises above the target there (:140-152); if rounding
+    // leaves none, the last that holds mass ----------------------------------------------------------------------------
+    bool holds = run.before <= target && target < run.upto;
+    if (!(target < total)) holds = tid == block_last_positive(mass, s_votes[0]);
+    if (holds) {
+        double at = run.before, before = at;
         int found = begin;
         for (int s = begin; s < end; ++s) {
             if (end - begin > 1) mine = stats[s];
-            const double share_of = end - begin > 1 ? share(mine.mass, mine.y_max, y_max, y_top) : mass;
-            if (share_of > 0.0) { found = s; before = at; }
-            at += share_of;
-            if (share_of > 0.0 && at > target) break;
+            const double here = end - begin > 1 ? share(mine.mass, mine.y_max, y_max) : mass;
+            if (here > 0.0) { found = s; before = at; }
+            at += here;
+            if (here > 0.0 && at > target) break;
         }
         s_hit = found;
         s_before = before;
     }
     __syncthreads();
+    // ---- its columns, in order: thread t has vector t of the segment ------------------------------------------------------
     const int segment = s_hit;
-    const double before_segment = s_before;
-    // ---- its columns, in order: thread t has columns 2t and 2t + 1 of the segment --------------------------------------
     const RowWindow w = row_window(p, row);
     const int64_t first_col = (int64_t)segment * kSegmentCols - w.misalign;
-    static_assert(kSegmentCols == 2 * kThreads, "two columns per thread");
-    float l[2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const int64_t col = first_col + 2 * tid + c;
-        l[c] = col >= 0 && col < p.vocab ? p.logits[row * p.row_stride + col] : -INFINITY;
+    static_assert(kSegmentVecs == kThreads, "one vector per thread");
+    float l[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    if (segment * kSegmentVecs + tid < w.vectors) {
+        const float4 d = w.base[segment * kSegmentVecs + tid];
+        l[0] = d.x; l[1] = d.y; l[2] = d.z; l[3] = d.w;
     }
-    if (p.history_ids != nullptr) {
-        mark_columns(p.history_ids, p.history_offsets[row], p.history_offsets[row + 1], first_col, kSegmentCols, p.vocab, s_flag);
-    }
+    if (p.history_ids != nullptr) mark_columns(p.history_ids, h_begin, h_end, first_col, kSegmentCols, p.vocab, s_flag);
     mark_columns(p.banned_ids, 0, p.num_banned, first_col, kSegmentCols, p.vocab, s_ban);
-    __syncthreads();
-    double e[2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const int at = 2 * tid + c;
-        const float y = processed(l[c], (s_flag[at >> 5] >> (at & 31)) & 1u, (s_ban[at >> 5] >> (at & 31)) & 1u, p);
-        e[c] = y > -INFINITY ? exp_below(y, double_of_float(y), y_max, y_top, s_table) : 0.0;
-    }
-    double unused;
-    const double run = before_segment + block_running_sum(e[0] + e[1], s_scratch, unused);
-    const double run_first = run - e[1];  // up to this thread's first column
-    if (tid == 0) s_last = -1;
-    __syncthreads();
-    if (e[1] > 0.0) {
-        if (run > target) atomicMin(&s_chosen, 2 * tid + 1);
-        atomicMax(&s_last, 2 * tid + 1);
-    }
-    if (e[0] > 0.0) {
-        if (run_first > target) atomicMin(&s_chosen, 2 * tid);
-        atomicMax(&s_last, 2 * tid);
-    }
-    __syncthreads();
-    const int chosen = s_chosen != 0x7FFFFFFF ? s_chosen : s_last;
     if (p.diag) {
-        alive = (int)__reduce_add_sync(0xFFFFFFFFu, (uint32_t)alive);
-        __syncthreads();
-        if (tid == 0) s_any_alive = 0;
-        __syncthreads();
-        if (lane == 0) atomicAdd(&s_any_alive, alive);
-        __syncthreads();
+        alive = __reduce_add_sync(0xFFFFFFFFu, alive);
+        if (lane == 0) atomicAdd(&s_alive, (int)alive);
     }
-    if (chosen >> 1 == tid) {
-        const int c = chosen & 1;
+    __syncthreads();
+    const uint32_t flag4 = s_flag[tid >> 3] >> ((tid & 7) * 4), ban4 = s_ban[tid >> 3] >> ((tid & 7) * 4);
+    double e[4], own = 0.0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const bool here = (uint64_t)(first_col + 4 * tid + c) < (uint64_t)p.vocab;
+        e[c] = here ? exp_below(processed(l[c], (flag4 >> c) & 1u, (ban4 >> c) & 1u, p), y_max) : 0.0;
+        own += e[c];
+    }
+    const RunningSum cols = block_running_sum(own, s_own);
+    // the target within the segment; its columns' sum may fall short of it by the rounding of the segment's
+    const double rest = target - s_before;
+    holds = cols.before <= rest && rest < cols.upto;
+    if (!(rest < cols.total)) holds = tid == block_last_positive(own, s_votes[1]);
+    if (holds) {
+        double at = cols.before, before = at, upto = at;
+        int chosen = -1;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (e[c] > 0.0 && !(chosen >= 0 && upto > rest)) {
+                before = at;
+                upto = at + e[c];
+                chosen = c;
+            }
+            at += e[c];
+        }
+        double z_total = s_z[0];
+#pragma unroll
+        for (int i = 1; i < kWarps; ++i) z_total += s_z[i];
+        const float x = chosen == 0 ? l[0] : chosen == 1 ? l[1] : chosen == 2 ? l[2] : l[3];
         p.row_status[row] = PSX_ROW_OK;
-        p.tokens[row] = first_col + chosen;
+        p.tokens[row] = first_col + 4 * tid + chosen;
         // the unprocessed log-softmax (:133,156)
-        p.log_probs[row] = (float)log(exp((double)l[c] - (double)raw_max) / z_total);
+        p.log_probs[row] = (float)log(exp((double)x - (double)raw_max) / z_total);
         if (p.diag) {
-            const double hi = (c ? run : run_first) / total, lo = ((c ? run_first : run_first - e[0])) / total;
-            const double margin = lo <= 0.0 ? fabs(u - hi) : fmin(fabs(u - lo), fabs(u - hi));
-            p.diag[row] = psx_row_diag{(int)p.vocab, s_any_alive, margin, INFINITY};
+            const double lo = (s_before + before) / total, hi = (s_before + upto) / total;
+            p.diag[row] = psx_row_diag{(int)p.vocab, s_alive, lo <= 0.0 ? fabs(u - hi) : fmin(fabs(u - lo), fabs(u - hi)), INFINITY};
         }
     }
+}
+
+// x / T as the float divide rounds it (:78), from the reciprocal in double precision: the product is off by 2^-52 of
+// the quotient at most, and the quotient of two floats is never closer than 2^-49 of itself to a point halfway between two
+// floats (that point times T is an integer of at most 49 bits in units that x is a whole number of, and never x itself),
+// so rounding the product to 24 bits -- Dekker's splitting with 2^29 + 1, two additions and a product -- gives the same.
+// (Quotients below 2^-126 keep more bits than a float has: no exponential notices.)
+__device__ __forceinline__ double tempered(double x, double reciprocal) {
+    const double q = __dmul_rn(x, reciprocal), c = __dmul_rn(q, 536870913.0);  // (never contracted)
+    return __dsub_rn(c, __dsub_rn(c, q));
+}
+
+// kProcessed: penalty, ban or temperature make the processed row another than the raw one.  kFlags: a penalty or a ban.
+template <bool kProcessed, bool kFlags>
+__global__ void __launch_bounds__(kThreads, 8) weigh_segments_kernel(const __grid_constant__ WholeRowParams p) {
+    __shared__ uint32_t s_flag[kMostPerWarp * kWarps * kSegmentCols / 32], s_ban[kMostPerWarp * kWarps * kSegmentCols / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t row = (int64_t)blockIdx.z * 65535 + blockIdx.y;
+    // (see ScanParams::wait_before_writes: the last CTA of the grid keeps the kernel from finishing early)
+    const bool ends_the_grid = p.inputs_ready && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1;
+    grid_dependents_may_launch();
+    if (!p.inputs_ready) grid_dependency_wait();
+    if (row >= p.rows) {
+        if (ends_the_grid) grid_dependency_wait();
+        return;
+    }
+    const RowWindow w = row_window(p, row);
+    const int per_warp = p.segments_per_warp, first_segment = blockIdx.x * kWarps * per_warp;
+    float4 d[kVecs];
+    auto load = [&](int segment) {
+#pragma unroll
+        for (int k = 0; k < kVecs; ++k) {
+            const int v = segment * kSegmentVecs + k * 32 + lane;
+            d[k] = v < w.vectors ? w.base[v] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        }
+    };
+    load(first_segment + warp);  // (lands under the bitmap)
+    const int64_t first_col = (int64_t)first_segment * kSegmentCols - w.misalign;
+    if (kFlags) {
+        const int slots = per_warp * kWarps * kSegmentCols;
+        for (int i = threadIdx.x; i < slots / 32; i += kThreads) s_flag[i] = s_ban[i] = 0u;
+        __syncthreads();
+        if (p.history_ids != nullptr) {
+            mark_columns(p.history_ids, p.history_offsets[row], p.history_offsets[row + 1], first_col, slots, p.vocab, s_flag);
+        }
+        mark_columns(p.banned_ids, 0, p.num_banned, first_col, slots, p.vocab, s_ban);
+        __syncthreads();
+    }
+    const double power = exp_power_of_lane();
+    const double reciprocal = p.apply_temperature ? 1.0 / (double)p.temperature : 1.0;
+#pragma unroll 1
+    for (int turn = 0; turn < per_warp; ++turn) {
+        const int local = turn * kWarps + warp, segment = first_segment + local;
+        if (segment >= p.segments) break;
+        if (turn > 0) load(segment);
+        const int lane_col = (segment * kSegmentVecs + lane) * 4 - w.misalign;  // the column of d[0].x; d[k] lies 128 k further
+        float l[kVecs * 4];
+        uint32_t marked = 0, banned = 0;  // bit 4 k + c: component c of d[k]
+#pragma unroll
+        for (int k = 0; k < kVecs; ++k) {
+            l[4 * k] = d[k].x; l[4 * k + 1] = d[k].y; l[4 * k + 2] = d[k].z; l[4 * k + 3] = d[k].w;
+            if (kFlags) {
+                const int v = local * kSegmentVecs + k * 32 + lane, shift = (v & 7) * 4;
+                banned |= ((s_ban[v >> 3] >> shift) & 15u) << (4 * k);
+                marked |= ((s_flag[v >> 3] >> shift) & 15u) << (4 * k);
+            }
+        }
+        marked |= banned;
+        // The first and the last vector of a row may reach past it.
+        uint32_t here = 0xFFFFu;
+        const bool edge = segment == 0 || segment * kSegmentVecs + kSegmentVecs >= w.vectors;
+        if (edge) {
+#pragma unroll
+            for (int i = 0; i < kVecs * 4; ++i) {
+                const int col = lane_col + (i >> 2) * 128 + (i & 3);
+                if (!((uint32_t)col < (uint32_t)p.vocab)) {
+                    here &= ~(1u << i);
+                    l[i] = -FLT_MAX;  // (finite; never the maximum)
+                }
+            }
+        }
+        bool finite = true;
+        float raw_max = -INFINITY, raw_min = INFINITY, clear_max = -INFINITY;  // clear: neither penalised nor banned
+#pragma unroll
+        for (int i = 0; i < kVecs * 4; i += 2) {
+            finite = finite && fabsf(l[i]) < INFINITY && fabsf(l[i + 1]) < INFINITY;
+            raw_max = fmax3(raw_max, l[i], l[i + 1]);
+            if (kFlags) clear_max = fmax3(clear_max, ((marked >> i) & 1u) ? -FLT_MAX : l[i], ((marked >> i) & 2u) ? -FLT_MAX : l[i + 1]);
+        }
+        raw_max = warp_max(raw_max);
+        if (kFlags) clear_max = warp_max(clear_max);
+        if (!__any_sync(0xFFFFFFFFu, here != 0)) raw_max = -INFINITY;  // (past the end of the row)
+        if (edge) {  // what is not there weighs next to nothing: exp(-690) in both sums, exp(-690 T) in the raw one if T < 1
+            const float nothing = __fmaf_rn(-690.0f, fminf(1.0f, p.apply_temperature ? p.temperature : 1.0f), raw_max);
+#pragma unroll
+            for (int i = 0; i < kVecs * 4; ++i) l[i] = ((here >> i) & 1u) ? l[i] : nothing;
+        }
+#pragma unroll
+        for (int i = 0; i < kVecs * 4; i += 2) raw_min = fmin3(raw_min, l[i], l[i + 1]);
+        raw_min = -warp_max(-raw_min);
+        if (kFlags && !__any_sync(0xFFFFFFFFu, (here & ~marked) != 0)) clear_max = -INFINITY;
+        // the processed value of a marked logit, which is read again from the row (a lane usually has none)
+        auto marked_value = [&](int i) {
+            const int col = lane_col + (i >> 2) * 128 + (i & 3);
+            return processed(p.logits[row * p.row_stride + col], true, (banned >> i) & 1u, p);
+        };
+        float y_max = raw_max;
+        if (kProcessed) y_max = temper(kFlags ? clear_max : raw_max, p.apply_temperature != 0, p.temperature);
+        if (kFlags) {
+            float most = -INFINITY;
+            for (uint32_t bits = marked & here; bits; bits &= bits - 1) most = fmaxf(most, marked_value(__ffs(bits) - 1));
+            y_max = fmaxf(y_max, warp_max(most));
+        }
+        double raw_sum = 0.0, mass = 0.0;
+        const bool within = !(edge && p.apply_temperature && p.temperature < 0.1f) && raw_max - raw_min <= 700.0f && (!kProcessed || y_max - temper(raw_min, p.apply_temperature != 0, p.temperature) <= 700.0f);
+        if (within) {  // no exponential needs looking after
+            const double raw_top = (double)raw_max, y_top = (double)y_max;
+#pragma unroll
+            for (int i = 0; i < kVecs * 4; ++i) {
+                const double x = (double)l[i];
+                raw_sum += exp_of_gap(x - raw_top, power);
+                if (kProcessed) {
+                    const double e = exp_of_gap(tempered(x, reciprocal) - y_top, power);
+                    // a marked logit's term is next to nothing here: its upper half is taken away
+                    mass += kFlags ? __hiloint2double(((marked >> i) & 1u) ? 0 : __double2hiint(e), __double2loint(e)) : e;
+                }
+            }
+        } else {  // logits further apart than an exponential reaches; the ends of a row at a very low temperature
+#pragma unroll 1
+            for (int i = 0; i < kVecs * 4; ++i) {
+                if (!((here >> i) & 1u)) continue;
+                const float x = p.logits[row * p.row_stride + lane_col + (i >> 2) * 128 + (i & 3)];
+                raw_sum += exp_below(x, raw_max);
+                if (kProcessed && !((marked >> i) & 1u)) mass += exp_below(temper(x, p.apply_temperature != 0, p.temperature), y_max);
+            }
+        }
+        if (kFlags) {
+            for (uint32_t bits = marked & here; bits; bits &= bits - 1) {
+                const float y = marked_value(__ffs(bits) - 1);
+                if (y > -INFINITY) mass += exp_below(y, y_max);
+            }
+        }
+        raw_sum = warp_sum(raw_sum);
+        mass = kProcessed ? warp_sum(mass) : raw_sum;
+        const uint32_t alive = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(here & ~banned));
+        const bool all_finite = __all_sync(0xFFFFFFFFu, finite);
+        if (lane == 0) {
+            SegmentStats s;
+            s.raw_sum = raw_sum;  // (a segment past the end of its row: maxima of -inf, sums of nothing)
+            s.mass = mass;
+            s.raw_max = raw_max;
+            s.y_max = y_max;
+            s.alive = alive;
+            s.nonfinite = all_finite ? 0u : 1u;
+            p.stats[row * p.segments + segment] = s;
+        }
+    }
+    if (ends_the_grid) grid_dependency_wait();
 }
 
 }  // namespace
@@ -337,15 +417,14 @@ cudaError_t launch_whole_rows(const WholeRowParams& p, cudaStream_t stream) {
     if (p.rows > 65535ll * 65535ll || p.rows > 0x7FFFFFFFll) return cudaErrorInvalidConfiguration;
     // One segment per warp while that leaves the GPU short of warps; up to four, which share a CTA's table and
     // bitmap, once there are some six thousand warps' worth (148 SMs x 40 warps).
-    const int64_t warps = p.rows * p.segments;
     WholeRowParams q = p;
-    q.segments_per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(kMostPerWarp, warps / 6000));
+    q.segments_per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(kMostPerWarp, p.rows * p.segments / 12000));
     const int64_t per_cta = (int64_t)kWarps * q.segments_per_warp;
     const dim3 grid((unsigned)((p.segments + per_cta - 1) / per_cta), (unsigned)std::min<int64_t>(p.rows, 65535),
                     (unsigned)((p.rows + 65534) / 65535));
-    const bool plain = p.history_ids == nullptr && p.num_banned == 0 && !p.apply_temperature;
-    const cudaError_t e = launch_overlapping(plain ? weigh_segments_kernel<true> : weigh_segments_kernel<false>, grid, dim3(kThreads), 0,
-                                           stream, q);
+    const bool flags = p.history_ids != nullptr || p.num_banned > 0;
+    const auto kernel = flags ? weigh_segments_kernel<true, true> : p.apply_temperature ? weigh_segments_kernel<true, false> : weigh_segments_kernel<false, false>;
+    const cudaError_t e = launch_overlapping(kernel, grid, dim3(kThreads), 0, stream, q);
     if (e != cudaSuccess) return e;
     return launch_overlapping(draw_token_kernel, dim3((unsigned)p.rows), dim3(kThreads), 0, stream, q);
 }

@@ -34,8 +34,7 @@ struct WholeRowParams {
     int32_t segments;                // per row
     int32_t segments_per_warp;       // filled in by launch_whole_rows
     int32_t inputs_ready;            // as in ScanParams
-    int32_t wait_before_writes;
-    SegmentStats* stats;             // rows * segments
+    SegmentStats* stats;             // rows * segments; another set than the call before, as ScanParams::wait_before_writes = 0 wants
     const double* uniforms;
     int64_t* tokens;
     float* log_probs;
