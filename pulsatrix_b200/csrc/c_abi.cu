@@ -867,7 +867,7 @@ psx_status psx_b200_lm_head_logits(psx_ctx* ctx, void* stream_ptr, const float* 
     if (!logits || row_stride < vocab) return fail(PSX_ERR_BAD_ARGUMENT, "psx_b200: logits is null or row_stride is smaller than the row");
     PSX_CUDA(cudaSetDevice(ctx->device));
     PSX_CUDA(psx::launch_lm_head(hidden, rows, d, weight, vocab, weight_layout == PSX_HEAD_VOCAB_BY_D, logits, row_stride,
-                                 static_cast<cudaStream_t>(stream_ptr)));
+                                 ctx->sm_count, static_cast<cudaStream_t>(stream_ptr)));
     ctx->launches += (uint64_t)((rows + 63) / 64);
     return PSX_OK;
 }
@@ -885,7 +885,7 @@ psx_status psx_b200_lm_head_sample_rows(psx_ctx* ctx, void* stream_ptr, const fl
     if (psx_status s = reserve(ctx->head_logits, (size_t)rows * stride * sizeof(float))) return s;
     float* logits = static_cast<float*>(ctx->head_logits.ptr);
     PSX_CUDA(psx::launch_lm_head(hidden, rows, d, weight, vocab, weight_layout == PSX_HEAD_VOCAB_BY_D, logits, stride,
-                                 static_cast<cudaStream_t>(stream_ptr)));
+                                 ctx->sm_count, static_cast<cudaStream_t>(stream_ptr)));
     ctx->launches += (uint64_t)((rows + 63) / 64);
     // The logits were written by the kernel just enqueued: the row pass must wait for it whatever the
     // caller promised about its own inputs.

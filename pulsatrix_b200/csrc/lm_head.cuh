@@ -11,6 +11,6 @@ namespace psx {
 // (token_major: the tied embedding) or d x vocab (an untied Linear's weight).  logits: row m at
 // logits + m * row_stride.
 cudaError_t launch_lm_head(const float* hidden, int64_t rows, int64_t d, const float* weight, int64_t vocab, bool token_major,
-                           float* logits, int64_t row_stride, cudaStream_t stream);
+                           float* logits, int64_t row_stride, int sm_count, cudaStream_t stream);
 
 }  // namespace psx

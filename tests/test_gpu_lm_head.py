@@ -76,6 +76,14 @@ def test_head_equals_the_references_loop_bit_for_bit(rows, d, vocab, vocab_by_d)
     assert got.cpu().numpy().view(np.uint32).tolist() == want.view(np.uint32).tolist()
 
 
+@pytest.mark.parametrize("rows,d,vocab", [(1, 36, 75_800), (2, 33, 113_000), (4, 32, 132_003), (7, 18, 113_700), (16, 20, 150_001),
+                                          (31, 17, 190_002), (64, 16, 95_003), (65, 35, 151_936)])
+@pytest.mark.parametrize("vocab_by_d", [True, False])
+def test_rounds_of_whole_tiles_and_the_tiles_after_them(rows, d, vocab, vocab_by_d):
+    """One size per number of rows a thread takes, wide enough for a full round of CTAs and a rest; bit for bit."""
+    test_head_equals_the_references_loop_bit_for_bit(rows, d, vocab, vocab_by_d)
+
+
 def test_head_and_sampling_in_one_call_match_sampling_the_references_logits():
     import torch
     rng = np.random.RandomState(4)
