@@ -70,6 +70,7 @@ ROW_DIAG_DTYPE = np.dtype({"names": ["candidates", "survivors", "draw_margin", "
                            "formats": ["<i4", "<i4", "<f8", "<f8"], "itemsize": C.sizeof(RowDiag)})
 
 _lib = None
+_native = None  # the per-step calls without ctypes (host/python_calls.cpp); bound to the same library
 
 
 def library_path() -> Path:
@@ -82,7 +83,7 @@ def library_path() -> Path:
 
 def library():
     """Loads libpsx_b200.so.  Raises when it has not been built: there is nothing to fall back to."""
-    global _lib
+    global _lib, _native
     if _lib is None:
         path = library_path()
         if not path.exists():
@@ -135,8 +136,24 @@ def library():
                                                   i64, ptr]
         lib.psx_uniforms_mt19937_64.argtypes = [ptr, i64, ptr]
         lib.psx_uniforms_portable.argtypes = [ptr, i64, ptr]
+        from . import _native as native
+        native.load(str(path))
+        _native = native
         _lib = lib
     return _lib
+
+
+def _stream_of(tensor):
+    """The raw handle of torch's current stream on the tensor's device."""
+    from torch._C import _cuda_getCurrentRawStream
+    device = tensor.get_device()
+    if device < 0:
+        raise ValueError(f"Expected a cuda tensor, but got one on {tensor.device}")
+    return _cuda_getCurrentRawStream(device)
+
+
+def _ptr(t):
+    return None if t is None else t.data_ptr()
 
 
 def _check(status):
@@ -180,12 +197,13 @@ def sample_rows_static(logits, history_ids, history_offsets, config, uniforms, t
     log_probs (float32), status (int32).  Asynchronous on `stream` (default: torch's current)."""
     rows = logits.shape[0]
     vocab = logits.shape[1] if vocab is None else vocab
-    if stream is None:
-        import torch
-        stream = torch.cuda.current_stream(logits.device).cuda_stream
-    _check(library().psx_b200_sample_rows_static(
-        C.c_void_p(stream), _dptr(logits), rows, vocab, logits.stride(0) if rows else vocab, _dptr(history_ids),
-        _dptr(history_offsets), C.addressof(config), _dptr(uniforms), _dptr(tokens), _dptr(log_probs), _dptr(status)))
+    if _native is None:
+        library()
+    status_code = _native.sample_rows_static(
+        _stream_of(logits) if stream is None else stream, logits.data_ptr(), rows, vocab, logits.stride(0) if rows else vocab,
+        _ptr(history_ids), _ptr(history_offsets), config, _ptr(uniforms), _ptr(tokens), _ptr(log_probs), _ptr(status))
+    if status_code:
+        _check(status_code)
 
 
 class Context:
@@ -195,12 +213,15 @@ class Context:
         self._lib = library()
         self._ctx = C.c_void_p()
         _check(self._lib.psx_b200_ctx_create(C.c_int(device), C.byref(self._ctx)))
+        self._handle = self._ctx.value  # (what the native calls take)
+        self._zero_words = []
         self.device = device
 
     def close(self):
         if self._ctx:
             self._lib.psx_b200_ctx_destroy(self._ctx)
             self._ctx = C.c_void_p()
+            self._handle = None
 
     def __del__(self):
         try:
@@ -257,17 +278,17 @@ class Context:
     def sample_rows(self, logits, history_ids, history_offsets, config, uniforms, out=None, stream=None, vocab=None):
         """logits: cuda float32 (rows, >=vocab) with unit column stride; history/uniforms: cuda
         tensors (int64 / float64) or None.  Asynchronous; returns the dict of output tensors."""
-        rows = logits.shape[0]
-        vocab = logits.shape[1] if vocab is None else vocab
-        assert logits.stride(1) == 1 or rows == 0
+        rows, cols = logits.shape
+        row_stride, column_stride = logits.stride()
+        assert column_stride == 1 or rows == 0
+        vocab = cols if vocab is None else vocab
         out = out or self.alloc_outputs(rows)
-        if stream is None:
-            import torch
-            stream = torch.cuda.current_stream(logits.device).cuda_stream
-        _check(self._lib.psx_b200_sample_rows(
-            self._ctx, C.c_void_p(stream), _dptr(logits), rows, vocab, logits.stride(0) if rows else vocab,
-            _dptr(history_ids), _dptr(history_offsets), C.addressof(config), _dptr(uniforms), _dptr(out["tokens"]),
-            _dptr(out["log_probs"]), _dptr(out["status"]), _dptr(out["diag"])))
+        status = _native.sample_rows(
+            self._handle, _stream_of(logits) if stream is None else stream, logits.data_ptr(), rows, vocab,
+            row_stride if rows else vocab, _ptr(history_ids), _ptr(history_offsets), config, _ptr(uniforms),
+            out["tokens"].data_ptr(), out["log_probs"].data_ptr(), out["status"].data_ptr(), _ptr(out["diag"]))
+        if status:
+            _check(status)
         return out
 
     def bind_sample_rows(self, logits, history_ids, history_offsets, config, uniforms, out=None, stream=None,
@@ -279,14 +300,10 @@ class Context:
         vocab = logits.shape[1] if vocab is None else vocab
         assert logits.stride(1) == 1 or rows == 0
         out = out or self.alloc_outputs(rows)
-        if stream is None:
-            import torch
-            stream = torch.cuda.current_stream(logits.device).cuda_stream
-        args = (self._ctx, C.c_void_p(stream), _dptr(logits), C.c_int64(rows), C.c_int64(vocab),
-                C.c_int64(logits.stride(0) if rows else vocab), _dptr(history_ids), _dptr(history_offsets),
-                C.c_void_p(C.addressof(config)), _dptr(uniforms), _dptr(out["tokens"]), _dptr(out["log_probs"]),
-                _dptr(out["status"]), _dptr(out["diag"]))
-        fn = self._lib.psx_b200_sample_rows
+        args = (self._handle, _stream_of(logits) if stream is None else stream, logits.data_ptr(), rows, vocab,
+                logits.stride(0) if rows else vocab, _ptr(history_ids), _ptr(history_offsets), C.addressof(config), _ptr(uniforms),
+                _ptr(out["tokens"]), _ptr(out["log_probs"]), _ptr(out["status"]), _ptr(out["diag"]))
+        fn = _native.sample_rows
         keep = (logits, history_ids, history_offsets, config, uniforms, out)  # the buffers live as long as the call
 
         def call(fn=fn, args=args, out=out, keep=keep):
@@ -321,12 +338,8 @@ class Context:
         rows, vocab = logits.shape
         status = np.zeros(rows, dtype=np.int32)
 
-        def hptr(a):
-            return None if a is None else C.c_void_p(a.ctypes.data)
-
-        _check(self._lib.psx_b200_process_logits_host(self._ctx, hptr(logits), rows, vocab, logits.strides[0] // 4,
-                                                      hptr(history_ids), hptr(history_offsets), C.addressof(config),
-                                                      hptr(status)))
+        _check(_native.process_logits_host(self._handle, logits, rows, vocab, logits.strides[0] // 4, history_ids, history_offsets,
+                                           config, status))
         return status
 
     def row_pass_only(self, logits, history_ids, history_offsets, config, stream=None, vocab=None):
@@ -357,14 +370,11 @@ class Context:
         status = np.zeros(rows, dtype=np.int32)
         diag = np.zeros(rows, dtype=ROW_DIAG_DTYPE)
 
-        def hptr(a):
-            if a is None:
-                return None
-            return C.c_void_p(a.ctypes.data if hasattr(a, "ctypes") else a.data_ptr())
+        def host(a):  # numpy arrays give their address themselves
+            return a.data_ptr() if hasattr(a, "data_ptr") else a
 
-        rc = self._lib.psx_b200_sample_rows_host(self._ctx, hptr(logits), rows, vocab, row_stride, hptr(history_ids),
-                                                 hptr(history_offsets), C.addressof(config), hptr(uniforms),
-                                                 hptr(tokens), hptr(logp), hptr(status), hptr(diag))
+        rc = _native.sample_rows_host(self._handle, host(logits), rows, vocab, row_stride, host(history_ids), host(history_offsets),
+                                      config, host(uniforms), tokens, logp, status, diag)
         if rc != OK and (rc != ERR_ROW_FAILED or raise_on_row_failure):
             _check(rc)
         return tokens, logp, status, diag
@@ -376,10 +386,8 @@ class Context:
         rows, cols = x.shape
         values = torch.empty((rows, max(k, 0)), dtype=torch.float32, device=x.device)
         indices = torch.empty((rows, max(k, 0)), dtype=torch.float32, device=x.device)
-        if stream is None:
-            stream = torch.cuda.current_stream(x.device).cuda_stream
-        _check(self._lib.psx_b200_top_k_rows(self._ctx, C.c_void_p(stream), _dptr(x), _dptr(values), _dptr(indices),
-                                             rows, cols, k if k >= 0 else 0, int(largest)))
+        _check(_native.top_k_rows(self._handle, _stream_of(x) if stream is None else stream, x.data_ptr(), values.data_ptr(),
+                                  indices.data_ptr(), rows, cols, k if k >= 0 else 0, int(largest)))
         return values, indices
 
     # ---- the language-model head -------------------------------------------------------------------------
@@ -389,25 +397,20 @@ class Context:
         rows, d = hidden.shape
         vocab = weight.shape[0] if vocab_by_d else weight.shape[1]
         out = torch.empty((rows, vocab), dtype=torch.float32, device=hidden.device) if out is None else out
-        if stream is None:
-            stream = torch.cuda.current_stream(hidden.device).cuda_stream
-        _check(self._lib.psx_b200_lm_head_logits(self._ctx, C.c_void_p(stream), _dptr(hidden), rows, d, _dptr(weight), vocab,
-                                                 0 if vocab_by_d else 1, _dptr(out), out.stride(0)))
+        _check(_native.lm_head_logits(self._handle, _stream_of(hidden) if stream is None else stream, hidden.data_ptr(), rows, d,
+                                      weight.data_ptr(), vocab, 0 if vocab_by_d else 1, out.data_ptr(), out.stride(0)))
         return out
 
     def lm_head_sample_rows(self, hidden, weight, history_ids, history_offsets, config, uniforms, vocab_by_d=True, out=None,
                             stream=None):
         """The head and the sampling step in one call: the logits stay in the context's scratch."""
-        import torch
         rows, d = hidden.shape
         vocab = weight.shape[0] if vocab_by_d else weight.shape[1]
         out = out or self.alloc_outputs(rows)
-        if stream is None:
-            stream = torch.cuda.current_stream(hidden.device).cuda_stream
-        _check(self._lib.psx_b200_lm_head_sample_rows(
-            self._ctx, C.c_void_p(stream), _dptr(hidden), rows, d, _dptr(weight), vocab, 0 if vocab_by_d else 1,
-            _dptr(history_ids), _dptr(history_offsets), C.addressof(config), _dptr(uniforms), _dptr(out["tokens"]),
-            _dptr(out["log_probs"]), _dptr(out["status"]), _dptr(out["diag"])))
+        _check(_native.lm_head_sample_rows(
+            self._handle, _stream_of(hidden) if stream is None else stream, hidden.data_ptr(), rows, d, weight.data_ptr(), vocab,
+            0 if vocab_by_d else 1, _ptr(history_ids), _ptr(history_offsets), config, _ptr(uniforms), _ptr(out["tokens"]),
+            _ptr(out["log_probs"]), _ptr(out["status"]), _ptr(out["diag"])))
         return out
 
     # ---- row primitives ---------------------------------------------------------------------------------
@@ -415,28 +418,31 @@ class Context:
         """x: cuda float32 contiguous (rows, cols); out may be x itself."""
         import torch
         out = torch.empty_like(x) if out is None else out
-        if stream is None:
-            stream = torch.cuda.current_stream(x.device).cuda_stream
-        _check(self._lib.psx_b200_softmax_rows(self._ctx, C.c_void_p(stream), _dptr(x), _dptr(out), x.shape[0], x.shape[1]))
+        rows, cols = x.shape
+        _check(_native.softmax_rows(self._handle, _stream_of(x) if stream is None else stream, x.data_ptr(), out.data_ptr(), rows, cols))
         return out
 
     def logsumexp_rows(self, x, stream=None):
         import torch
-        out = torch.empty(x.shape[0], dtype=torch.float32, device=x.device)
-        if stream is None:
-            stream = torch.cuda.current_stream(x.device).cuda_stream
-        _check(self._lib.psx_b200_logsumexp_rows(self._ctx, C.c_void_p(stream), _dptr(x), _dptr(out), x.shape[0], x.shape[1]))
+        rows, cols = x.shape
+        out = torch.empty(rows, dtype=torch.float32, device=x.device)
+        _check(_native.logsumexp_rows(self._handle, _stream_of(x) if stream is None else stream, x.data_ptr(), out.data_ptr(), rows, cols))
         return out
 
     def gather_rows(self, table, indices, stream=None):
         """table: cuda float32 (n, dim); indices: cuda float32 whole numbers (count,)."""
         import torch
         out = torch.empty((indices.shape[0], table.shape[1]), dtype=torch.float32, device=table.device)
-        if stream is None:
-            stream = torch.cuda.current_stream(table.device).cuda_stream
-        _check(self._lib.psx_b200_gather_rows(self._ctx, C.c_void_p(stream), _dptr(table), _dptr(indices), _dptr(out),
-                                              indices.shape[0], table.shape[1]))
+        _check(_native.gather_rows(self._handle, _stream_of(table) if stream is None else stream, table.data_ptr(), indices.data_ptr(),
+                                   out.data_ptr(), indices.shape[0], table.shape[1]))
         return out
+
+    def _zero_word(self, device):
+        """A one-element int32 tensor that holds zero: the next of a block that was zeroed with one launch."""
+        if not self._zero_words or self._zero_words[-1].device != device:
+            import torch
+            self._zero_words = list(torch.zeros(256, dtype=torch.int32, device=device).split(1))
+        return self._zero_words.pop()
 
     def decode_attention(self, q, keys, values, cached, scale=None, causal=True, window=0, key_keep=None, stream=None):
         """Attention of the new positions over the KV cache (psx_b200_decode_attention).  q: cuda float32
@@ -449,13 +455,10 @@ class Context:
         if scale is None:
             scale = 1.0 / float(np.sqrt(np.float32(head_dim)))
         context = torch.empty_like(q)
-        status = torch.zeros(1, dtype=torch.int32, device=q.device)
-        if stream is None:
-            stream = torch.cuda.current_stream(q.device).cuda_stream
-        _check(self._lib.psx_b200_decode_attention(self._ctx, C.c_void_p(stream), _dptr(q), _dptr(keys), _dptr(values),
-                                                   _dptr(key_keep) if key_keep is not None else None, _dptr(context), batch, heads,
-                                                   kv_heads, q_len, head_dim, cached, max_len, C.c_float(scale), int(bool(causal)),
-                                                   window, _dptr(status)))
+        status = self._zero_word(q.device)
+        _check(_native.decode_attention(self._handle, _stream_of(q) if stream is None else stream, q.data_ptr(), keys.data_ptr(),
+                                        values.data_ptr(), _ptr(key_keep), context.data_ptr(), batch, heads, kv_heads, q_len, head_dim,
+                                        cached, max_len, float(scale), int(bool(causal)), window, status.data_ptr()))
         return context, status
 
     # ---- vocabulary-sharded -----------------------------------------------------------------------------
@@ -463,27 +466,20 @@ class Context:
         return int(self._lib.psx_b200_shard_record_bytes(C.addressof(config)))
 
     def shard_scan(self, shard_logits, shard_begin, vocab, history_ids, history_offsets, config, records, stream=None):
-        import torch
         rows, cols = shard_logits.shape
-        if stream is None:
-            stream = torch.cuda.current_stream(shard_logits.device).cuda_stream
-        _check(self._lib.psx_b200_shard_scan(self._ctx, C.c_void_p(stream), _dptr(shard_logits), rows, cols,
-                                             shard_logits.stride(0), shard_begin, vocab, _dptr(history_ids),
-                                             _dptr(history_offsets), C.addressof(config), _dptr(records)))
+        _check(_native.shard_scan(self._handle, _stream_of(shard_logits) if stream is None else stream, shard_logits.data_ptr(), rows,
+                                  cols, shard_logits.stride(0), shard_begin, vocab, _ptr(history_ids), _ptr(history_offsets), config,
+                                  _ptr(records)))
 
     def shard_merge(self, gathered, num_shards, rows, vocab, config, uniforms, out=None, stream=None, row_begin=0,
                     row_count=None):
         """Merges rows row_begin .. row_begin + row_count - 1 (all of them by default); `out` holds
         the merged rows only, the first of them at index 0."""
-        import torch
         row_count = rows - row_begin if row_count is None else row_count
         out = out or self.alloc_outputs(row_count)
-        if stream is None:
-            stream = torch.cuda.current_stream(gathered.device).cuda_stream
-        _check(self._lib.psx_b200_shard_merge_rows(self._ctx, C.c_void_p(stream), _dptr(gathered), num_shards, rows,
-                                                   row_begin, row_count, vocab, C.addressof(config), _dptr(uniforms),
-                                                   _dptr(out["tokens"]), _dptr(out["log_probs"]), _dptr(out["status"]),
-                                                   _dptr(out.get("diag"))))
+        _check(_native.shard_merge_rows(self._handle, _stream_of(gathered) if stream is None else stream, gathered.data_ptr(), num_shards,
+                                        rows, row_begin, row_count, vocab, config, _ptr(uniforms), _ptr(out["tokens"]),
+                                        _ptr(out["log_probs"]), _ptr(out["status"]), _ptr(out.get("diag"))))
         return out
 
     def exchange(self, world, rank, rows, config):
@@ -519,15 +515,12 @@ class Exchange:
         _check(self._lib.psx_b200_exchange_open(self._ex, handles))
 
     def sample(self, shard_logits, shard_begin, vocab, history_ids, history_offsets, config, uniforms, stream=None):
-        import torch
         rows, cols = shard_logits.shape
         if rows != self.rows:
             raise ValueError(f"the exchange was created for {self.rows} rows, got {rows}")
-        if stream is None:
-            stream = torch.cuda.current_stream(shard_logits.device).cuda_stream
-        _check(self._lib.psx_b200_exchange_sample(self._ex, C.c_void_p(stream), _dptr(shard_logits), cols,
-                                                  shard_logits.stride(0), shard_begin, vocab, _dptr(history_ids),
-                                                  _dptr(history_offsets), C.addressof(config), _dptr(uniforms)))
+        _check(_native.exchange_sample(self._ex.value, _stream_of(shard_logits) if stream is None else stream, shard_logits.data_ptr(),
+                                       cols, shard_logits.stride(0), shard_begin, vocab, _ptr(history_ids), _ptr(history_offsets), config,
+                                       _ptr(uniforms)))
         return self.results(shard_logits.device)
 
     def results(self, device):

@@ -10,6 +10,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PACKAGE = Path(__file__).resolve().parent
@@ -17,6 +18,7 @@ CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libpsx_b200.so"
 SOURCES = ["c_abi.cu", "scan_rows.cu", "merge_rows.cu", "whole_rows.cu", "topk_rows.cu", "shard_records.cu", "peer_exchange.cu", "no_alloc.cu", "read_floor.cu", "process_rows.cu", "row_ops.cu", "lm_head.cu", "decode_attention.cu"]
 HOST_SOURCES = ["determinism.cpp", "sampler.cpp", "backend.cpp", "generation.cpp"]  # the C++ API over the C ABI
+PYTHON_CALLS = PACKAGE / "_native.so"  # the per-step calls as a CPython extension module (host/python_calls.cpp)
 CPP_TEST = PACKAGE.parent / "tests" / "cpp" / "host_api_test"
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--fmad=true",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
@@ -30,9 +32,9 @@ def _profiling() -> bool:
 
 
 def _stale() -> bool:
-    if not LIBRARY.exists():
+    if not LIBRARY.exists() or not PYTHON_CALLS.exists():
         return True
-    built = LIBRARY.stat().st_mtime
+    built = min(LIBRARY.stat().st_mtime, PYTHON_CALLS.stat().st_mtime)
     deps = (list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list((PACKAGE / "host").glob("*.cpp")) +
             list((PACKAGE.parent / "include").rglob("*.h*")))
     return any(p.stat().st_mtime > built for p in deps)
@@ -74,8 +76,16 @@ def build(force: bool = False, verbose: bool = False, defines=(), output: Path |
             raise RuntimeError(f"nvcc failed on {src}")
     subprocess.run(["nvcc", "-arch=sm_100a", "-shared", "-o", str(library), *objects, "-lcudart"], check=True)
     if not profiling and not variant:
+        build_python_calls()
         build_cpp_test()
     return library
+
+
+def build_python_calls() -> Path:
+    subprocess.run(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"],
+                    "-I", str(PACKAGE.parent / "include"), str(PACKAGE / "host" / "python_calls.cpp"), "-o", str(PYTHON_CALLS), "-ldl"],
+                   check=True)
+    return PYTHON_CALLS
 
 
 def build_cpp_test() -> Path:

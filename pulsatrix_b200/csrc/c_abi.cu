@@ -47,6 +47,10 @@ struct Buffer {
     size_t bytes = 0;
 };
 
+// Page-locked staging for rows that lie in ordinary host memory: eight slots of 256 KB.
+constexpr int kRingSlots = 8;
+constexpr size_t kRingSlotBytes = 256 << 10;
+
 }  // namespace
 
 // For the library's other translation units: record an error where psx_b200_last_error() finds it.
@@ -69,8 +73,11 @@ struct psx_ctx {
     Buffer banned, sort_keys, head_logits, attention_partial;
     // ProcessLogits: the surviving set between the survivor stage and the write-back, dummy draw outputs
     Buffer surv_cols, surv_vals, surv_counts, pl_tokens, pl_log_probs, pl_status;
-    // staging of the host entry point
-    Buffer h_logits, h_history, h_offsets, h_uniforms, h_tokens, h_log_probs, h_status, h_diag;
+    // staging of the host entry points: the rows, the small inputs and the results, each in one piece on the device, and
+    // page-locked memory on the host that the copies go through
+    Buffer h_logits, h_inputs, h_results;
+    Buffer pinned_inputs, pinned_results, pinned_ring;
+    cudaEvent_t ring_done[kRingSlots] = {};  // the copy out of (or into) a slot has finished
     // staging of the sharded path
     Buffer shard_uniform_scratch;
     // optional per-kernel timing: (before row pass, between, after survivor stage) per call
@@ -91,6 +98,112 @@ psx_status reserve(Buffer& b, size_t bytes) {
     const size_t want = bytes + bytes / 4 + 256;
     PSX_CUDA(cudaMalloc(&b.ptr, want));
     b.bytes = want;
+    return PSX_OK;
+}
+
+// The same for page-locked host memory.  (Nothing is in flight in it: the host entry points end with a synchronisation.)
+psx_status reserve_pinned(Buffer& b, size_t bytes) {
+    if (bytes <= b.bytes) return PSX_OK;
+    if (b.ptr) PSX_CUDA(cudaFreeHost(b.ptr));
+    b.ptr = nullptr;
+    b.bytes = 0;
+    const size_t want = bytes + bytes / 4 + 256;
+    PSX_CUDA(cudaHostAlloc(&b.ptr, want, cudaHostAllocDefault));
+    b.bytes = want;
+    return PSX_OK;
+}
+
+// Whether the copy engine can take (or put) these bytes itself.
+bool copy_engine_reaches(const void* host) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type != cudaMemoryTypeUnregistered;
+}
+
+// Rows between host and device, packed on the device (stride = vocab) whatever the host stride is.  Page-locked rows are
+// one copy.  From ordinary memory the driver would copy through a staging buffer of its own, the call waiting for it, and
+// only then start; here the copy into page-locked memory runs in pieces, each on its way to the device while the next one is
+// made: one row of 128,256 logits 94 -> 45 us.  Pieces of a quarter of the rows, 64 to 256 KB: smaller ones cost more calls
+// than they overlap.  The caller synchronises the stream before the ring is used again.
+psx_status copy_rows(psx_ctx* ctx, cudaStream_t stream, float* device, float* host, int64_t rows, int64_t vocab, int64_t row_stride,
+                     bool to_device) {
+    const size_t row_bytes = (size_t)vocab * sizeof(float), total = (size_t)rows * row_bytes;
+    const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+    if (copy_engine_reaches(host)) {
+        void* dst = to_device ? (void*)device : host;
+        const void* src = to_device ? (const void*)host : device;
+        const size_t stride = (size_t)row_stride * sizeof(float);
+        if (row_stride == vocab) {
+            PSX_CUDA(cudaMemcpyAsync(dst, src, total, kind, stream));
+        } else {
+            PSX_CUDA(cudaMemcpy2DAsync(dst, to_device ? row_bytes : stride, src, to_device ? stride : row_bytes, row_bytes, (size_t)rows, kind, stream));
+        }
+        return PSX_OK;
+    }
+    if (psx_status s = reserve_pinned(ctx->pinned_ring, kRingSlots * kRingSlotBytes)) return s;
+    for (cudaEvent_t& e : ctx->ring_done) {
+        if (e == nullptr) PSX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    const size_t piece = std::min(kRingSlotBytes, std::max<size_t>(64 << 10, (total / 4 + 4095) / 4096 * 4096));
+    const size_t pieces = (total + piece - 1) / piece;
+    char* const ring = static_cast<char*>(ctx->pinned_ring.ptr);
+    auto between_host_and_slot = [&](size_t i) {  // piece i of the packed rows, row by row where the host's are apart
+        char* slot = ring + (i % kRingSlots) * kRingSlotBytes;
+        for (size_t at = i * piece, end = std::min(total, at + piece); at < end;) {
+            const size_t row = row_stride == vocab ? 0 : at / row_bytes, in_row = at - row * row_bytes;
+            const size_t n = row_stride == vocab ? end - at : std::min(end - at, row_bytes - in_row);
+            char* there = reinterpret_cast<char*>(host + row * row_stride) + in_row;
+            if (to_device) std::memcpy(slot, there, n); else std::memcpy(there, slot, n);
+            slot += n;
+            at += n;
+        }
+    };
+    // to the device: fill a slot, send it off; from the device: ask for up to all slots ahead, empty them in turn
+    for (size_t i = 0; i < pieces + (to_device ? 0 : kRingSlots); ++i) {
+        if (i >= kRingSlots && (to_device || i - kRingSlots < pieces)) PSX_CUDA(cudaEventSynchronize(ctx->ring_done[i % kRingSlots]));
+        if (!to_device && i >= kRingSlots && i - kRingSlots < pieces) between_host_and_slot(i - kRingSlots);
+        if (i >= pieces) continue;
+        if (to_device) between_host_and_slot(i);
+        char* slot = ring + (i % kRingSlots) * kRingSlotBytes;
+        char* there = reinterpret_cast<char*>(device) + i * piece;
+        const size_t n = std::min(piece, total - i * piece);
+        PSX_CUDA(cudaMemcpyAsync(to_device ? there : slot, to_device ? slot : there, n, kind, stream));
+        if (!to_device || pieces > kRingSlots) PSX_CUDA(cudaEventRecord(ctx->ring_done[i % kRingSlots], stream));
+    }
+    return PSX_OK;
+}
+
+// The small inputs of a host entry point (history offsets and ids, uniforms), packed into one copy.
+struct HostInputs {
+    const int64_t* offsets = nullptr;  // on the device
+    const int64_t* history = nullptr;
+    const double* uniforms = nullptr;
+};
+psx_status upload_inputs(psx_ctx* ctx, cudaStream_t stream, int64_t rows, const int64_t* history_ids, const int64_t* history_offsets,
+                         const double* uniforms, HostInputs& out) {
+    const bool with_history = history_ids && history_offsets;
+    const size_t history = with_history ? (size_t)std::max<int64_t>(history_offsets[rows], 0) : 0;
+    const size_t offset_words = with_history ? (size_t)rows + 1 : 0, uniform_words = uniforms ? (size_t)rows : 0;
+    const size_t words = offset_words + history + uniform_words;
+    if (words == 0) return PSX_OK;
+    if (psx_status s = reserve(ctx->h_inputs, words * 8)) return s;
+    if (psx_status s = reserve_pinned(ctx->pinned_inputs, words * 8)) return s;
+    int64_t* packed = static_cast<int64_t*>(ctx->pinned_inputs.ptr);
+    if (with_history) {
+        std::memcpy(packed, history_offsets, offset_words * 8);
+        std::memcpy(packed + offset_words, history_ids, history * 8);
+    }
+    if (uniforms) std::memcpy(packed + offset_words + history, uniforms, uniform_words * 8);
+    PSX_CUDA(cudaMemcpyAsync(ctx->h_inputs.ptr, packed, words * 8, cudaMemcpyHostToDevice, stream));
+    const int64_t* device = static_cast<const int64_t*>(ctx->h_inputs.ptr);
+    if (with_history) {
+        out.offsets = device;
+        out.history = device + offset_words;
+    }
+    if (uniforms) out.uniforms = reinterpret_cast<const double*>(device + offset_words + history);
     return PSX_OK;
 }
 
@@ -230,10 +343,15 @@ void psx_b200_ctx_destroy(psx_ctx* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     for (Buffer* b : {&ctx->stats[0], &ctx->stats[1], &ctx->part_counts[0], &ctx->part_counts[1], &ctx->candidates[0], &ctx->candidates[1], &ctx->banned, &ctx->sort_keys, &ctx->head_logits, &ctx->attention_partial, &ctx->surv_cols, &ctx->surv_vals,
-                      &ctx->surv_counts, &ctx->pl_tokens, &ctx->pl_log_probs, &ctx->pl_status, &ctx->h_logits, &ctx->h_history,
-                      &ctx->h_offsets, &ctx->h_uniforms, &ctx->h_tokens, &ctx->h_log_probs, &ctx->h_status,
-                      &ctx->h_diag, &ctx->shard_uniform_scratch}) {
+                      &ctx->surv_counts, &ctx->pl_tokens, &ctx->pl_log_probs, &ctx->pl_status, &ctx->h_logits, &ctx->h_inputs,
+                      &ctx->h_results, &ctx->shard_uniform_scratch}) {
         if (b->ptr) cudaFree(b->ptr);
+    }
+    for (Buffer* b : {&ctx->pinned_inputs, &ctx->pinned_results, &ctx->pinned_ring}) {
+        if (b->ptr) cudaFreeHost(b->ptr);
+    }
+    for (cudaEvent_t e : ctx->ring_done) {
+        if (e) cudaEventDestroy(e);
     }
     for (cudaEvent_t e : ctx->timing_events) cudaEventDestroy(e);
     cudaStreamDestroy(ctx->stream);
@@ -452,40 +570,29 @@ psx_status psx_b200_process_logits_host(psx_ctx* ctx, float* logits, int64_t row
     if (rows == 0) return PSX_OK;
     PSX_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t stream = ctx->stream;
-    const bool with_history = history_ids && history_offsets;
-    const int64_t history_total = with_history ? history_offsets[rows] : 0;
     if (psx_status s = reserve(ctx->h_logits, (size_t)rows * vocab * sizeof(float))) return s;
-    if (psx_status s = reserve(ctx->h_history, (size_t)std::max<int64_t>(history_total, 1) * sizeof(int64_t))) return s;
-    if (psx_status s = reserve(ctx->h_offsets, (size_t)(rows + 1) * sizeof(int64_t))) return s;
-    if (psx_status s = reserve(ctx->h_status, (size_t)rows * sizeof(int32_t))) return s;
-    PSX_CUDA(cudaMemcpy2DAsync(ctx->h_logits.ptr, (size_t)vocab * sizeof(float), logits, (size_t)row_stride * sizeof(float),
-                               (size_t)vocab * sizeof(float), (size_t)rows, cudaMemcpyHostToDevice, stream));
-    if (with_history) {
-        if (history_total > 0) {
-            PSX_CUDA(cudaMemcpyAsync(ctx->h_history.ptr, history_ids, (size_t)history_total * sizeof(int64_t),
-                                     cudaMemcpyHostToDevice, stream));
-        }
-        PSX_CUDA(cudaMemcpyAsync(ctx->h_offsets.ptr, history_offsets, (size_t)(rows + 1) * sizeof(int64_t),
-                                 cudaMemcpyHostToDevice, stream));
-    }
+    if (psx_status s = reserve(ctx->h_results, (size_t)rows * sizeof(int32_t))) return s;
+    if (psx_status s = reserve_pinned(ctx->pinned_results, (size_t)rows * sizeof(int32_t))) return s;
+    float* const device_rows = static_cast<float*>(ctx->h_logits.ptr);
+    HostInputs in;
+    if (psx_status s = upload_inputs(ctx, stream, rows, history_ids, history_offsets, nullptr, in)) return s;
+    if (psx_status s = copy_rows(ctx, stream, device_rows, logits, rows, vocab, row_stride, /*to_device=*/true)) return s;
     struct RestorePromise {  // the staged inputs are being copied in by the transfers just enqueued
         psx_ctx* ctx;
         bool saved;
         ~RestorePromise() { ctx->inputs_ready = saved; }
     } restore{ctx, ctx->inputs_ready};
     ctx->inputs_ready = false;
-    if (psx_status s = psx_b200_process_logits(ctx, stream, static_cast<float*>(ctx->h_logits.ptr), rows, vocab, vocab,
-                                               with_history ? static_cast<const int64_t*>(ctx->h_history.ptr) : nullptr,
-                                               with_history ? static_cast<const int64_t*>(ctx->h_offsets.ptr) : nullptr,
-                                               config, static_cast<int32_t*>(ctx->h_status.ptr))) {
+    if (psx_status s = psx_b200_process_logits(ctx, stream, device_rows, rows, vocab, vocab, in.history, in.offsets, config,
+                                               static_cast<int32_t*>(ctx->h_results.ptr))) {
         return s;
     }
-    PSX_CUDA(cudaMemcpy2DAsync(logits, (size_t)row_stride * sizeof(float), ctx->h_logits.ptr, (size_t)vocab * sizeof(float),
-                               (size_t)vocab * sizeof(float), (size_t)rows, cudaMemcpyDeviceToHost, stream));
-    std::vector<int32_t> local((size_t)rows);
-    int32_t* out_status = row_status ? row_status : local.data();
-    PSX_CUDA(cudaMemcpyAsync(out_status, ctx->h_status.ptr, (size_t)rows * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+    const int32_t* out_status = static_cast<const int32_t*>(ctx->pinned_results.ptr);
+    PSX_CUDA(cudaMemcpyAsync(ctx->pinned_results.ptr, ctx->h_results.ptr, (size_t)rows * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+    PSX_CUDA(cudaStreamSynchronize(stream));  // (the ring is free again)
+    if (psx_status s = copy_rows(ctx, stream, device_rows, logits, rows, vocab, row_stride, /*to_device=*/false)) return s;
     PSX_CUDA(cudaStreamSynchronize(stream));
+    if (row_status) std::memcpy(row_status, out_status, (size_t)rows * sizeof(int32_t));
     for (int64_t r = 0; r < rows; ++r) {
         if (out_status[r] != PSX_ROW_OK && out_status[r] != PSX_ROW_ALL_REMOVED) {
             return fail(PSX_ERR_ROW_FAILED, std::string(row_failure_text(out_status[r])) + " (row " + std::to_string(r) + ")");
@@ -557,36 +664,15 @@ psx_status psx_b200_sample_rows_host(psx_ctx* ctx, const float* logits, int64_t 
     const int64_t history_total = with_history ? history_offsets[rows] : 0;
     if (with_history && history_total < 0) return fail(PSX_ERR_BAD_ARGUMENT, "psx_b200: history_offsets must ascend");
 
-    if (psx_status s = reserve(ctx->h_logits, (size_t)rows * vocab * sizeof(float))) return s;
-    if (psx_status s = reserve(ctx->h_history, (size_t)std::max<int64_t>(history_total, 1) * sizeof(int64_t))) return s;
-    if (psx_status s = reserve(ctx->h_offsets, (size_t)(rows + 1) * sizeof(int64_t))) return s;
-    if (psx_status s = reserve(ctx->h_uniforms, (size_t)rows * sizeof(double))) return s;
-    if (psx_status s = reserve(ctx->h_tokens, (size_t)rows * sizeof(int64_t))) return s;
-    if (psx_status s = reserve(ctx->h_log_probs, (size_t)rows * sizeof(float))) return s;
-    if (psx_status s = reserve(ctx->h_status, (size_t)rows * sizeof(int32_t))) return s;
-    if (psx_status s = reserve(ctx->h_diag, (size_t)rows * sizeof(psx_row_diag))) return s;
-
-    // Rows are packed on the device (stride = vocab) whatever the host stride is.
-    if (row_stride == vocab) {
-        PSX_CUDA(cudaMemcpyAsync(ctx->h_logits.ptr, logits, (size_t)rows * vocab * sizeof(float), cudaMemcpyHostToDevice,
-                                 stream));
-    } else {
-        PSX_CUDA(cudaMemcpy2DAsync(ctx->h_logits.ptr, (size_t)vocab * sizeof(float), logits,
-                                   (size_t)row_stride * sizeof(float), (size_t)vocab * sizeof(float), (size_t)rows,
-                                   cudaMemcpyHostToDevice, stream));
-    }
-    if (with_history) {
-        if (history_total > 0) {
-            PSX_CUDA(cudaMemcpyAsync(ctx->h_history.ptr, history_ids, (size_t)history_total * sizeof(int64_t),
-                                     cudaMemcpyHostToDevice, stream));
-        }
-        PSX_CUDA(cudaMemcpyAsync(ctx->h_offsets.ptr, history_offsets, (size_t)(rows + 1) * sizeof(int64_t),
-                                 cudaMemcpyHostToDevice, stream));
-    }
-    if (config->do_sample) {
-        PSX_CUDA(cudaMemcpyAsync(ctx->h_uniforms.ptr, uniforms, (size_t)rows * sizeof(double), cudaMemcpyHostToDevice,
-                                 stream));
-    }
+    // The results in one piece: tokens, diagnostics, log-probs, statuses.
+    const size_t n = (size_t)rows, diag_bytes = diag ? n * sizeof(psx_row_diag) : 0, result_bytes = 8 * n + diag_bytes + 8 * n;
+    if (psx_status s = reserve(ctx->h_logits, n * vocab * sizeof(float))) return s;
+    if (psx_status s = reserve(ctx->h_results, result_bytes)) return s;
+    if (psx_status s = reserve_pinned(ctx->pinned_results, result_bytes)) return s;
+    float* const device_rows = static_cast<float*>(ctx->h_logits.ptr);
+    HostInputs in;
+    if (psx_status s = upload_inputs(ctx, stream, rows, history_ids, history_offsets, config->do_sample ? uniforms : nullptr, in)) return s;
+    if (psx_status s = copy_rows(ctx, stream, device_rows, const_cast<float*>(logits), rows, vocab, row_stride, /*to_device=*/true)) return s;
     // The staged inputs are being copied in by the transfers just enqueued: no promise holds for them.
     struct RestorePromise {
         psx_ctx* ctx;
@@ -594,25 +680,23 @@ psx_status psx_b200_sample_rows_host(psx_ctx* ctx, const float* logits, int64_t 
         ~RestorePromise() { ctx->inputs_ready = saved; }
     } restore{ctx, ctx->inputs_ready};
     ctx->inputs_ready = false;
-    if (psx_status s = psx_b200_sample_rows(
-            ctx, stream, static_cast<const float*>(ctx->h_logits.ptr), rows, vocab, vocab,
-            with_history ? static_cast<const int64_t*>(ctx->h_history.ptr) : nullptr,
-            with_history ? static_cast<const int64_t*>(ctx->h_offsets.ptr) : nullptr, config,
-            static_cast<const double*>(ctx->h_uniforms.ptr), static_cast<int64_t*>(ctx->h_tokens.ptr),
-            static_cast<float*>(ctx->h_log_probs.ptr), static_cast<int32_t*>(ctx->h_status.ptr),
-            diag ? static_cast<psx_row_diag*>(ctx->h_diag.ptr) : nullptr)) {
+    char* const results = static_cast<char*>(ctx->h_results.ptr);
+    auto tokens_in = [](char* block) { return reinterpret_cast<int64_t*>(block); };
+    auto diag_in = [&](char* block) { return reinterpret_cast<psx_row_diag*>(block + 8 * n); };
+    auto log_probs_in = [&](char* block) { return reinterpret_cast<float*>(block + 8 * n + diag_bytes); };
+    auto status_in = [&](char* block) { return reinterpret_cast<int32_t*>(block + 8 * n + diag_bytes + 4 * n); };
+    if (psx_status s = psx_b200_sample_rows(ctx, stream, device_rows, rows, vocab, vocab, in.history, in.offsets, config, in.uniforms,
+                                            tokens_in(results), log_probs_in(results), status_in(results),
+                                            diag ? diag_in(results) : nullptr)) {
         return s;
     }
-    PSX_CUDA(cudaMemcpyAsync(tokens, ctx->h_tokens.ptr, (size_t)rows * sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
-    PSX_CUDA(cudaMemcpyAsync(log_probs, ctx->h_log_probs.ptr, (size_t)rows * sizeof(float), cudaMemcpyDeviceToHost,
-                             stream));
-    PSX_CUDA(cudaMemcpyAsync(row_status, ctx->h_status.ptr, (size_t)rows * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                             stream));
-    if (diag) {
-        PSX_CUDA(cudaMemcpyAsync(diag, ctx->h_diag.ptr, (size_t)rows * sizeof(psx_row_diag), cudaMemcpyDeviceToHost,
-                                 stream));
-    }
+    char* const arrived = static_cast<char*>(ctx->pinned_results.ptr);
+    PSX_CUDA(cudaMemcpyAsync(arrived, results, result_bytes, cudaMemcpyDeviceToHost, stream));
     PSX_CUDA(cudaStreamSynchronize(stream));
+    std::memcpy(tokens, tokens_in(arrived), 8 * n);
+    std::memcpy(log_probs, log_probs_in(arrived), 4 * n);
+    std::memcpy(row_status, status_in(arrived), 4 * n);
+    if (diag) std::memcpy(diag, diag_in(arrived), diag_bytes);
     for (int64_t r = 0; r < rows; ++r) {
         if (row_status[r] != PSX_ROW_OK) {
             const char* what = row_failure_text(row_status[r]);
