@@ -31,6 +31,7 @@ __device__ unsigned long long g_merge_times[1024 * 4];
 #endif
 #include "general_row_impl.cuh"
 #include "merge_rows_impl.cuh"
+#include "merge_rows_list_impl.cuh"
 #include "merge_rows_warp_impl.cuh"
 #include "peer_exchange.cuh"
 
@@ -38,8 +39,13 @@ namespace psx {
 
 namespace {
 
+template <int kKind>
 __device__ __forceinline__ void decide_row(const MergeParams& p, const int64_t row, unsigned long long* dyn) {
-    if (p.general != 2) survivor::merge_row(p, row, dyn);
+    if (p.general != 2) {
+        if (survivor::list_row<kKind>(p, row, dyn)) return;
+        __syncthreads();
+        survivor::merge_row(p, row, dyn);  // too many for the list, or a decision too close to its level
+    }
     if (p.general != 0 && p.logits != nullptr) {
         // A row the candidate lists could not decide is decided from the row itself.
         __syncthreads();
@@ -47,8 +53,9 @@ __device__ __forceinline__ void decide_row(const MergeParams& p, const int64_t r
     }
 }
 
-__global__ void __launch_bounds__(kMergeThreads, 3) merge_rows_kernel(const MergeParams p) {
-    extern __shared__ unsigned long long dyn[];
+template <int kKind>
+__global__ void __launch_bounds__(kMergeThreads, kKind == survivor::kListNucleus ? 2 : 3) merge_rows_kernel(const __grid_constant__ MergeParams p) {
+    extern __shared__ __align__(16) unsigned long long dyn[];
     PSX_MERGE_TIME(0);
     if (p.only_undecided) {
         // After a launch by warps: a few CTAs look through the rows for what the warps left undecided
@@ -69,7 +76,7 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_rows_kernel(const Merg
             for (int i = 0; i < found; ++i) {  // (in any order: rows do not depend on one another)
                 const int64_t row = r0 + s_found[i];
                 __syncthreads();
-                decide_row(p, row, dyn);
+                decide_row<kKind>(p, row, dyn);
                 __syncthreads();
             }
         }
@@ -85,7 +92,7 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_rows_kernel(const Merg
         if (threadIdx.x == 0) s_arrived = wait_until_at_least(p.arrivals + row, p.arrivals_target, p.arrivals_wait_ns) ? 1 : 0;
         __syncthreads();
         if (s_arrived) {
-            decide_row(p, row, dyn);
+            decide_row<kKind>(p, row, dyn);
         } else if (threadIdx.x == 0) {
             p.tokens[row] = -1;
             p.log_probs[row] = 0.0f;
@@ -108,13 +115,13 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_rows_kernel(const Merg
     grid_dependency_wait();        // everything this kernel reads was written by the kernel before it
     grid_dependents_may_launch();  // a row pass that follows reads none of this kernel's results
     PSX_MERGE_TIME(1);
-    decide_row(p, p.row_begin + blockIdx.x, dyn);
+    decide_row<kKind>(p, p.row_begin + blockIdx.x, dyn);
     PSX_MERGE_TIME(2);
 }
 
 template <int N>
 __global__ void __launch_bounds__(kMergeThreads) merge_rows_warp_kernel(const MergeParams p) {
-    extern __shared__ unsigned long long dyn[];
+    extern __shared__ __align__(16) unsigned long long dyn[];
     grid_dependency_wait();        // everything this kernel reads was written by the kernel before it
     grid_dependents_may_launch();
     const int warp = threadIdx.x >> 5;
@@ -148,7 +155,19 @@ int merge_slot_shift(int parts, int part_cap, int expected) {
     return shift;
 }
 
-cudaError_t configure_merge_rows() { return allow_all_dynamic_shared(merge_rows_kernel); }
+cudaError_t configure_merge_rows() {
+    cudaError_t e = allow_all_dynamic_shared(merge_rows_kernel<survivor::kListGreedy>);
+    if (e == cudaSuccess) e = allow_all_dynamic_shared(merge_rows_kernel<survivor::kListTopK>);
+    if (e == cudaSuccess) e = allow_all_dynamic_shared(merge_rows_kernel<survivor::kListNucleus>);
+    return e;
+}
+
+namespace {
+auto kernel_for(const MergeParams& p) {
+    if (!p.do_sample) return merge_rows_kernel<survivor::kListGreedy>;
+    return p.top_k > 0 && p.top_k < p.vocab ? merge_rows_kernel<survivor::kListTopK> : merge_rows_kernel<survivor::kListNucleus>;
+}
+}  // namespace
 
 bool plan_merge_by_warp(MergeParams& p, int k_need, bool greedy, int expected) {
     p.by_warp = 0;
@@ -177,7 +196,7 @@ cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_
     const bool by_warp = p.by_warp != 0 && p.general != 2 && p.survivor_cols == nullptr && p.arrivals == nullptr && p.rows >= kRowsByWarpFrom;
     if (launched != nullptr) *launched += by_warp ? 2 : 1;
     if (!by_warp) {
-        return launch_overlapping(merge_rows_kernel, dim3((unsigned)p.rows), dim3(kMergeThreads), shared, stream, with_size);
+        return launch_overlapping(kernel_for(p), dim3((unsigned)p.rows), dim3(kMergeThreads), shared, stream, with_size);
     }
     // One warp per row, eight rows per CTA; then the block-per-row kernel over what the warps left undecided.
     const int fetches = (int)((((long long)p.parts << p.warp_slot_shift) + 31) / 32);
@@ -192,7 +211,7 @@ cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_
     if (e != cudaSuccess) return e;
     with_size.only_undecided = 1;
     const unsigned ctas = (unsigned)(p.rows < 32 ? p.rows : 32);
-    return launch_overlapping(merge_rows_kernel, dim3(ctas), dim3(kMergeThreads), shared, stream, with_size);
+    return launch_overlapping(kernel_for(p), dim3(ctas), dim3(kMergeThreads), shared, stream, with_size);
 }
 
 }  // namespace psx

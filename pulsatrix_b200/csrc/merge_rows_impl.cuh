@@ -868,7 +868,7 @@ __device__ __forceinline__ Joined join_and_gather(const MergeParams& p, const ch
 
 // One row of the survivor stage, by a whole block of kMergeThreads threads; `dyn` is the block's
 // dynamic shared memory (merge_rows_shared_bytes(...) bytes, 8-byte aligned).
-__device__ __forceinline__ void merge_row(const MergeParams& p, const int64_t row, u64* dyn) {
+__device__ __noinline__ void merge_row(const MergeParams& p, const int64_t row, u64* dyn) {
     const int cap = p.sort_capacity, gcap = p.gather_capacity;
     u64* keyA = dyn;
     u64* keyB = keyA + cap;
