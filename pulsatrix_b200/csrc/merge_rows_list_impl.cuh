@@ -28,13 +28,37 @@ constexpr int kWideCap = 2048;       // candidates at or above the threshold, be
 constexpr int kNucleusCap = 4096;    // the same without a top-k
 constexpr double kDoubt = 1e-11;     // of the whole mass: well above 512 units of 2^-52
 constexpr double kNucleusDoubt = 4e-9;  // the same for kNucleusCap units of 2^-40
+constexpr uint32_t kRemoved = 0x80000000u;
 constexpr int kTopKArena = kListCap * (16 + 8 + 4) + kWideCap * 12;
-constexpr int kNucleusArena = kListCap * (16 + 4) + kNucleusCap * 12 + 4 * 256 * 4;
+constexpr int kNucleusArena = kListCap * (16 + 4) + kNucleusCap * 20 + 4 * 256 * 4;
 
-// sum over the warp of integers below 2^59, by two of the 32-bit reductions
-__device__ __forceinline__ u64 warp_sum_units(u64 v) {
-    const uint32_t lo = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)v & 0x7FFFFFFu), hi = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)(v >> 27));
-    return (u64)lo + ((u64)hi << 27);
+// Where one row's inputs lie and where its results go.
+struct RowView {
+    const char *stats, *counts, *lists;
+    int64_t stats_stride, count_stride, list_stride;  // from part to part
+    int32_t cap;                                      // slots of a part's list
+    double u;
+    int64_t* token;
+    float* log_prob;
+    int32_t* status;
+    psx_row_diag* diag;
+};
+
+__device__ __forceinline__ RowView view_of_row(const MergeParams& p, const int64_t row) {
+    RowView v;
+    v.stats = static_cast<const char*>(p.stats) + row * p.stats_row_stride;
+    v.counts = static_cast<const char*>(p.part_counts) + row * p.count_row_stride;
+    v.lists = static_cast<const char*>(p.candidates) + row * p.cand_row_stride;
+    v.stats_stride = p.stats_part_stride;
+    v.count_stride = p.count_part_stride;
+    v.list_stride = p.cand_part_stride;
+    v.cap = p.part_cap;
+    v.u = p.do_sample && p.uniforms ? p.uniforms[row] : 0.5;
+    v.token = p.tokens + row;
+    v.log_prob = p.log_probs + row;
+    v.status = p.row_status + row;
+    v.diag = p.diag ? p.diag + row : nullptr;
+    return v;
 }
 
 // What every warp knows of the row's parts; lane L keeps part L's record.
@@ -50,9 +74,8 @@ struct ChunkWalk {
     int64_t stride;
     int parts, cap, lane, part, chunk, step_part, step_chunk;
 
-    __device__ __forceinline__ ChunkWalk(const MergeParams& p, const int64_t row)
-        : lists(static_cast<const char*>(p.candidates) + row * p.cand_row_stride), stride(p.cand_part_stride), parts(p.parts), cap(p.part_cap),
-          lane(threadIdx.x & 31) {
+    __device__ __forceinline__ ChunkWalk(const MergeParams& p, const RowView& v)
+        : lists(v.lists), stride(v.list_stride), parts(p.parts), cap(v.cap), lane(threadIdx.x & 31) {
         const int warp = threadIdx.x >> 5;
         chunk = warp / parts;
         part = warp - chunk * parts;
@@ -74,21 +97,21 @@ struct ChunkWalk {
     __device__ __forceinline__ bool beyond(uint32_t longest) const { return (uint32_t)(chunk * 32) >= longest; }
 };
 
-__device__ __forceinline__ void load_parts(const MergeParams& p, const int64_t row, PartsJoined& j) {
+__device__ __forceinline__ void load_parts(const MergeParams& p, const RowView& v, PartsJoined& j) {
     const int lane = threadIdx.x & 31;
     j.mine.raw_tail = 0.0; j.mine.proc_tail = 0.0;
     j.mine.raw_max = -FLT_MAX; j.mine.y_max = -INFINITY; j.mine.thr = -INFINITY;
     j.mine.nonfinite = 0; j.mine.alive_tail = 0; j.mine.overflow = 0;
     j.count = 0;
     if (lane < p.parts) {
-        j.mine = *reinterpret_cast<const PartStats*>(static_cast<const char*>(p.stats) + row * p.stats_row_stride + lane * p.stats_part_stride);
-        j.count = *reinterpret_cast<const uint32_t*>(static_cast<const char*>(p.part_counts) + row * p.count_row_stride + lane * p.count_part_stride);
+        j.mine = *reinterpret_cast<const PartStats*>(v.stats + lane * v.stats_stride);
+        j.count = *reinterpret_cast<const uint32_t*>(v.counts + lane * v.count_stride);
     }
 }
 
 // false: the row is not for this way (a list that ran out of slots)
-__device__ __forceinline__ bool join_parts(const MergeParams& p, PartsJoined& j) {
-    j.count = min(j.count, (uint32_t)p.part_cap);
+__device__ __forceinline__ bool join_parts(const RowView& v, PartsJoined& j) {
+    j.count = min(j.count, (uint32_t)v.cap);
     j.raw_max = warp_max(j.mine.raw_max);
     j.y_max = warp_max(j.mine.y_max);
     j.thr = warp_max(j.mine.thr);
@@ -99,15 +122,21 @@ __device__ __forceinline__ bool join_parts(const MergeParams& p, PartsJoined& j)
 }
 
 // true: the row has a non-finite logit, a copy that did not arrive, or nothing left; its status is written
-__device__ __forceinline__ bool settle_bad_row(const MergeParams& p, const int64_t row, const PartsJoined& j) {
+__device__ __forceinline__ bool settle_bad_row(const RowView& v, const PartsJoined& j) {
     if (j.bad == 0 && j.y_max > -INFINITY) return false;
     if (threadIdx.x == 0) {
-        p.tokens[row] = -1;
-        p.log_probs[row] = 0.0f;
-        p.row_status[row] = (j.bad & 2u) ? PSX_ROW_DEVICE_TIMEOUT : (j.bad & 1u) ? PSX_ROW_NON_FINITE : PSX_ROW_ALL_REMOVED;
-        if (p.diag) p.diag[row] = psx_row_diag{0, 0, INFINITY, INFINITY};
+        *v.token = -1;
+        *v.log_prob = 0.0f;
+        *v.status = (j.bad & 2u) ? PSX_ROW_DEVICE_TIMEOUT : (j.bad & 1u) ? PSX_ROW_NON_FINITE : PSX_ROW_ALL_REMOVED;
+        if (v.diag) *v.diag = psx_row_diag{0, 0, INFINITY, INFINITY};
     }
     return true;
+}
+
+// sum over the warp of integers below 2^59, by two of the 32-bit reductions
+__device__ __forceinline__ u64 warp_sum_units(u64 v) {
+    const uint32_t lo = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)v & 0x7FFFFFFu), hi = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)(v >> 27));
+    return (u64)lo + ((u64)hi << 27);
 }
 
 // The raw sum-exp: what the row pass left behind (the parts' tails, joined by one warp), and float exponentials of the candidates
@@ -122,7 +151,9 @@ struct RawSum {
         c_res = __fmaf_rn(raw_max, kLog2e, -c_l2);
     }
     __device__ __forceinline__ void add_low(float l) { low += ex2_approx(__fmaf_rn(l, kLog2e, -c_l2)); }
-    __device__ __forceinline__ double of_warp() const { return warp_sum(high + (double)low * exp2_of_minus_small(c_res)); }
+    // The warp's sum, in units of 2^-40 of the largest term: integer reductions, a fraction of the time of five additions in double
+    // one after another.  (A lane has at most a few dozen terms of at most one.)
+    __device__ __forceinline__ u64 of_warp() const { return warp_sum_units((u64)__double2ull_rn((high + (double)low * exp2_of_minus_small(c_res)) * 0x1p40)); }
 };
 
 __device__ __forceinline__ double tails_of_parts(const PartsJoined& j) {  // by one warp; the sum in every lane
@@ -138,21 +169,31 @@ __device__ __forceinline__ double exp_to(float v, float top, bool there, double 
     return small ? 0.0 : e;
 }
 
-__device__ __forceinline__ void barrier_of_half() { asm volatile("bar.sync 1, 128;" ::: "memory"); }  // the first four warps
+// The sum over the lanes before this one, and over all, by a whole warp.
+__device__ __forceinline__ u64 lanes_before(u64 v, int lane, u64& all) {
+    u64 incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += up;
+    }
+    all = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    return incl - v;
+}
 
 // ---- greedy ----------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool list_greedy(const MergeParams& p, const int64_t row) {
-    __shared__ double s_z[kListWarps];
-    __shared__ u64 s_best[kListWarps];
+__device__ __forceinline__ bool list_greedy(const MergeParams& p, const RowView& v) {
+    __shared__ u64 s_z[kListWarps], s_best[kListWarps];
+    __shared__ double s_tails;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     PartsJoined j;
     uint2 c[4];
     uint32_t where[4];
-    ChunkWalk walk(p, row);
-    load_parts(p, row, j);
+    ChunkWalk walk(p, v);
+    load_parts(p, v, j);
     walk.fetch(c, where);
-    if (!join_parts(p, j)) return false;
-    if (settle_bad_row(p, row, j)) return true;
+    if (!join_parts(v, j)) return false;
+    if (settle_bad_row(v, j)) return true;
     PSX_MERGE_STAGE(3);
     const float keep_from = fmaxf(j.y_max, -FLT_MAX);
     RawSum z(j.raw_max);
@@ -175,40 +216,44 @@ __device__ __forceinline__ bool list_greedy(const MergeParams& p, const int64_t 
         if (walk.beyond(j.longest)) break;
         walk.fetch(c, where);
     }
-    double sum = z.of_warp();
-    if (warp == 0) sum += tails_of_parts(j);
+    const u64 of_warp = z.of_warp();
+    if (warp == kListWarps - 1) {
+        const double tails = tails_of_parts(j);
+        if (lane == 0) s_tails = tails;
+    }
     const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(best >> 32));
     if ((uint32_t)(best >> 32) == top && (top != 0 || lane == 0)) s_best[warp] = best;  // (columns differ: one lane)
-    if (lane == 0) s_z[warp] = sum;
+    if (lane == 0) s_z[warp] = of_warp;
     __syncthreads();
     PSX_MERGE_STAGE(4);
     if (threadIdx.x == 0) {
         best = s_best[0];
-        sum = s_z[0];
+        u64 sum = s_z[0];
 #pragma unroll
         for (int w = 1; w < kListWarps; ++w) {
             best = s_best[w] > best ? s_best[w] : best;
             sum += s_z[w];
         }
-        p.row_status[row] = PSX_ROW_OK;
-        p.tokens[row] = (int64_t)(uint32_t)~(uint32_t)(best >> 32);
-        p.log_probs[row] = (float)(((double)__uint_as_float((uint32_t)best) - (double)j.raw_max) - log(sum));  // src/generation.cpp:156
-        if (p.diag) p.diag[row] = psx_row_diag{1, 1, INFINITY, INFINITY};
+        *v.status = PSX_ROW_OK;
+        *v.token = (int64_t)(uint32_t)~(uint32_t)(best >> 32);
+        *v.log_prob = (float)(((double)__uint_as_float((uint32_t)best) - (double)j.raw_max) - log((double)sum * 0x1p-40 + s_tails));  // src/generation.cpp:156
+        if (v.diag) *v.diag = psx_row_diag{1, 1, INFINITY, INFINITY};
     }
     PSX_MERGE_STAGE(9);
     return true;
 }
 
 // ---- sampling under a top-k ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t row, u64* dyn) {
+__device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn) {
     ulonglong2* const s_list = reinterpret_cast<ulonglong2*>(dyn);       // (ordered value << 32) | column; units of 2^-52
-    u64* const s_after = reinterpret_cast<u64*>(s_list + kListCap);
-    float* const s_raw = reinterpret_cast<float*>(s_after + kListCap);
+    uint32_t* const s_by_value = reinterpret_cast<uint32_t*>(s_list + kListCap);  // place by column << 16 | entry
+    uint32_t* const s_by_column = s_by_value + kListCap;                          // entry, kRemoved
+    float* const s_raw = reinterpret_cast<float*>(s_by_column + kListCap);
     u64* const s_wide = reinterpret_cast<u64*>(s_raw + kListCap);        // raw logit, column | flags
     float* const s_wide_y = reinterpret_cast<float*>(s_wide + kWideCap);
     __shared__ uint32_t s_hist[32];
-    __shared__ double s_z[kListWarps], s_log_z;
-    __shared__ u64 s_part[4], s_margin;
+    __shared__ u64 s_z[kListWarps];
+    __shared__ double s_log_z;
     __shared__ int s_wide_n, s_n, s_doubt, s_won, s_survivors;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t below = (1u << lane) - 1u;
@@ -216,16 +261,16 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
     PartsJoined j;
     uint2 c[4];
     uint32_t where[4];
-    ChunkWalk walk(p, row);
-    load_parts(p, row, j);
+    ChunkWalk walk(p, v);
+    load_parts(p, v, j);
     walk.fetch(c, where);
-    const double u = p.uniforms ? p.uniforms[row] : 0.5;
+    const double u = v.u;
     if (tid < 32) s_hist[tid] = 0;
-    if (tid == 0) { s_wide_n = 0; s_n = 0; s_doubt = 0; s_won = 0; s_survivors = 0; s_margin = ~0ull; }
+    if (tid == 0) { s_wide_n = 0; s_n = 0; s_doubt = 0; s_won = 0; s_survivors = 0; }
     const double power = exp_power_of_lane();
     __syncthreads();
-    if (!join_parts(p, j)) return false;
-    if (settle_bad_row(p, row, j)) return true;
+    if (!join_parts(v, j)) return false;
+    if (settle_bad_row(v, j)) return true;
     PSX_MERGE_STAGE(3);
     // ---- 1. what reaches the largest part threshold (that part alone has k logits which reach it), and its histogram -------
     const float keep_from = relax_threshold(j.thr, apply_t, p.temperature);
@@ -308,112 +353,114 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
         }
     }
     {
-        const double sum = z.of_warp();
+        const u64 sum = z.of_warp();
         if (lane == 0) s_z[warp] = sum;
     }
     __syncthreads();
     PSX_MERGE_STAGE(5);
     const int n = s_n;
     if (n > kListCap || n == 0) return false;
-    bool won = false;
-    int won_entry = 0;
-    double won_margin = 0.0;
-    if (warp == kListWarps - 1) {
-        // the logarithm for the log-probability, meanwhile
-        double sum = tails_of_parts(j);
-#pragma unroll
-        for (int w = 0; w < kListWarps; ++w) sum += s_z[w];
-        if (lane == 0) s_log_z = log(sum);
-    } else if (warp < 4) {
-        // ---- 3. every entry against all the others; T neighbouring threads share one -----------------------------------------
+    // ---- 3. every entry's place by value and by column: it looks at all the others; T neighbouring threads share one ------------
+    {
         int n_pad = 8;
-        while (n_pad < n && n_pad < 128) n_pad <<= 1;
-        const int shift = 7 - (31 - __clz(n_pad)), T = 1 << shift, slice = tid & (T - 1);
-        u64 sum = 0;
+        while (n_pad < n && n_pad < kMergeThreads) n_pad <<= 1;
+        const int shift = 8 - (31 - __clz(n_pad)), T = 1 << shift, slice = tid & (T - 1);
         for (int e0 = 0; e0 < n; e0 += n_pad) {
             const int e = e0 + (tid >> shift);
-            const ulonglong2 me = e < n ? s_list[e] : make_ulonglong2(~0ull, 0);
-            uint32_t greater = 0;
-            u64 after = 0;
+            const u64 me = e < n ? s_list[e].x : 0;
+            uint32_t places = 0;  // by value, descending (equal values: the higher column first); by column, above it
 #pragma unroll 4
             for (int i = slice; i < n; i += T) {
-                const ulonglong2 other = s_list[i];
-                greater += (uint32_t)(other.x >> 32) > (uint32_t)(me.x >> 32) ? 1u : 0u;
-                after += other.x > me.x ? other.y : 0;  // later in the top-p walk: a larger value, or the same at a higher column
+                const u64 other = s_list[i].x;
+                places += other > me ? 1u : 0u;
+                places += (uint32_t)other < (uint32_t)me ? 0x10000u : 0u;
             }
-            for (int o = T >> 1; o > 0; o >>= 1) {
-                greater += __shfl_xor_sync(0xFFFFFFFFu, greater, o);
-                after += __shfl_xor_sync(0xFFFFFFFFu, after, o);
-            }
-            const bool stays = e < n && (int64_t)greater < p.top_k;  // :80-88: the k-th value and its ties stay
-            if (slice == 0 && e < n) {
-                s_after[e] = stays ? after : ~0ull;
-                sum += stays ? me.y : 0;
-            }
+            for (int o = T >> 1; o > 0; o >>= 1) places += __shfl_xor_sync(0xFFFFFFFFu, places, o);
+            if (slice == 0 && e < n) s_by_value[places & 0xFFFFu] = (places & 0xFFFF0000u) | (uint32_t)e;
         }
-        sum = warp_sum_units(sum);
-        if (lane == 0) s_part[warp] = sum;
-        barrier_of_half();
-        PSX_MERGE_STAGE(6);
-        sum = s_part[0] + s_part[1] + s_part[2] + s_part[3];
-        const double limit = 1.0 - (double)p.top_p, whole = (double)sum * 0x1p-52, min_p = (double)p.min_p;
-        bool doubt = false;
-        for (int e = tid; e < n; e += 128) {
-            const u64 after = s_after[e], unit = s_list[e].y;
-            bool stays = after != ~0ull;
+    }
+    __syncthreads();
+    PSX_MERGE_STAGE(6);
+    bool won = false, doubt = false;
+    int won_entry = 0, survivors = 0;
+    double won_margin = 0.0, top_p_margin = INFINITY;
+    if (warp == kListWarps - 1) {
+        // the logarithm for the log-probability, meanwhile
+        u64 sum = 0;
+#pragma unroll
+        for (int w = 0; w < kListWarps; ++w) sum += s_z[w];
+        const double log_z = log(tails_of_parts(j) + (double)sum * 0x1p-40);
+        if (lane == 0) s_log_z = log_z;
+    } else if (warp == 0) {
+        // ---- 4. who stays, by one warp: a lane takes `each` entries one after another in the order of the values ------------------
+        const int each = (n + 31) >> 5, begin = lane * each, end = min(begin + each, n);
+        const uint32_t kth = n >= p.top_k ? (uint32_t)(s_list[s_by_value[p.top_k - 1] & 0xFFFFu].x >> 32) : 0u;
+        u64 sum = 0;
+        for (int i = begin; i < end; ++i) {
+            const ulonglong2 it = s_list[s_by_value[i] & 0xFFFFu];
+            sum += (uint32_t)(it.x >> 32) >= kth ? it.y : 0;  // :80-88: the k-th value and its ties stay
+        }
+        u64 all, after = lanes_before(sum, lane, all);
+        const double limit = 1.0 - (double)p.top_p, whole = (double)all * 0x1p-52, min_p = (double)p.min_p;
+        for (int i = begin; i < end; ++i) {
+            const uint32_t at = s_by_value[i];
+            const ulonglong2 it = s_list[at & 0xFFFFu];
+            bool stays = (uint32_t)(it.x >> 32) >= kth;
             if (stays && p.top_p < 1.0f && after != 0) {  // :89-103; the last of the walk always stays
-                const double beyond = (double)(sum - after) * 0x1p-52 - limit * whole;
+                const double beyond = (double)(all - after) * 0x1p-52 - limit * whole;
                 stays = beyond > 0.0;
                 doubt = doubt || fabs(beyond) < kDoubt * whole;
-                if (p.diag) atomicMin(&s_margin, (u64)__double_as_longlong(fabs(beyond) / whole));
+                top_p_margin = fmin(top_p_margin, fabs(beyond));
             }
-            if (stays && min_p > 0.0 && unit < (1ull << 52)) {  // :104-111, against the first maximum's exp(0)
-                const double mass = (double)unit * 0x1p-52;
+            after += it.y;
+            if (stays && min_p > 0.0 && it.y < (1ull << 52)) {  // :104-111, against the first maximum's exp(0)
+                const double mass = (double)it.y * 0x1p-52;
                 stays = mass >= min_p;
                 doubt = doubt || fabs(mass - min_p) < kDoubt;
             }
-            s_after[e] = stays ? 1 : 0;
-            if (p.diag && p.survivor_cols == nullptr && stays) atomicAdd(&s_survivors, 1);
+            s_by_column[at >> 16] = (at & 0xFFFFu) | (stays ? 0u : kRemoved);
+            survivors += stays ? 1 : 0;
         }
-        if (doubt) s_doubt = 1;
-        barrier_of_half();
+        doubt = __any_sync(0xFFFFFFFFu, doubt);
+        __syncwarp();
         PSX_MERGE_STAGE(7);
-        // ---- 4. the draw (:140-152): the entry whose share of the running sum, by ascending column, holds u --------------------
-        if (p.survivor_cols == nullptr && s_doubt == 0) {
-            for (int e0 = 0; e0 < n; e0 += n_pad) {
-                const int e = e0 + (tid >> shift);
-                const ulonglong2 me = e < n ? s_list[e] : make_ulonglong2(~0ull, 0);
-                u64 before = 0, total = 0;
-#pragma unroll 4
-                for (int i = slice; i < n; i += T) {
-                    const ulonglong2 other = s_list[i];
-                    const u64 mass = s_after[i] != 0 ? other.y : 0;
-                    total += mass;
-                    before += (uint32_t)other.x < (uint32_t)me.x ? mass : 0;
-                }
-                for (int o = T >> 1; o > 0; o >>= 1) {
-                    total += __shfl_xor_sync(0xFFFFFFFFu, total, o);
-                    before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
-                }
-                const double target = u * (double)total, lo = target - (double)before, hi = (double)(before + me.y) - target;
-                if (e < n && slice == 0 && s_after[e] != 0 && lo >= 0.0 && hi > 0.0) {
-                    const double margin = before == 0 ? hi : fmin(lo, hi);
-                    if (margin >= kDoubt * (double)total) {  // (nobody takes it otherwise: replayed)
-                        won = true;
-                        won_entry = e;
-                        won_margin = margin / (double)total;
-                        s_won = 1;
-                    }
-                }
+        // ---- 5. the draw (:140-152): the entry whose share of the running sum, by ascending column, holds u -----------------------
+        sum = 0;
+        for (int i = begin; i < end; ++i) {
+            const uint32_t at = s_by_column[i];
+            sum += (at & kRemoved) ? 0 : s_list[at].y;
+        }
+        u64 before = lanes_before(sum, lane, all);
+        const double target = u * (double)all;
+        for (int i = begin; i < end && !doubt; ++i) {
+            const uint32_t at = s_by_column[i];
+            if (at & kRemoved) continue;
+            const u64 mass = s_list[at].y;
+            const double lo = target - (double)before, hi = (double)(before + mass) - target;
+            if (lo >= 0.0 && hi > 0.0) {
+                won_margin = before == 0 ? hi : fmin(lo, hi);
+                won_entry = (int)at;
+                won = won_margin >= kDoubt * (double)all;  // (nobody takes it otherwise: replayed)
             }
+            before += mass;
+        }
+        if (won) s_won = 1;
+        if (doubt && lane == 0) s_doubt = 1;
+        if (v.diag) {
+            won_margin /= (double)all;
+            top_p_margin /= whole;
+            survivors = (int)__reduce_add_sync(0xFFFFFFFFu, (uint32_t)survivors);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) top_p_margin = fmin(top_p_margin, __shfl_xor_sync(0xFFFFFFFFu, top_p_margin, o));
         }
     }
     __syncthreads();
     PSX_MERGE_STAGE(8);
     if (p.survivor_cols != nullptr) {  // the surviving set itself (ProcessLogits)
         if (s_doubt != 0 || n > p.survivor_cap) return false;
-        for (int e = tid; e < n; e += kMergeThreads) {
-            if (s_after[e] == 0) continue;
+        for (int i = tid; i < n; i += kMergeThreads) {
+            const uint32_t e = s_by_column[i];
+            if (e & kRemoved) continue;
             const int64_t at = row * p.survivor_cap + atomicAdd(&s_survivors, 1);
             p.survivor_cols[at] = (uint32_t)s_list[e].x;
             p.survivor_vals[at] = from_ordered_key((uint32_t)(s_list[e].x >> 32));
@@ -421,18 +468,15 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
         __syncthreads();
         if (tid == 0) {
             p.survivor_counts[row] = (uint32_t)s_survivors;
-            p.row_status[row] = PSX_ROW_OK;
+            *v.status = PSX_ROW_OK;
         }
         return true;
     }
     if (won) {
-        p.row_status[row] = PSX_ROW_OK;
-        p.tokens[row] = (int64_t)(uint32_t)s_list[won_entry].x;
-        p.log_probs[row] = (float)(((double)s_raw[won_entry] - (double)j.raw_max) - s_log_z);  // :133,156
-        if (p.diag) {
-            const double top_p_margin = s_margin == ~0ull ? (double)INFINITY : __longlong_as_double((long long)s_margin);
-            p.diag[row] = psx_row_diag{n, s_survivors, won_margin, top_p_margin};
-        }
+        *v.status = PSX_ROW_OK;
+        *v.token = (int64_t)(uint32_t)s_list[won_entry].x;
+        *v.log_prob = (float)(((double)s_raw[won_entry] - (double)j.raw_max) - s_log_z);  // :133,156
+        if (v.diag) *v.diag = psx_row_diag{n, survivors, won_margin, top_p_margin};
     }
     PSX_MERGE_STAGE(9);
     return s_won != 0;
@@ -444,53 +488,51 @@ __device__ __forceinline__ void add_units(uint32_t* hist, uint32_t bin, u64 unit
     atomicAdd(&hist[bin], (uint32_t)units & 0xFFFFFu);
     atomicAdd(&hist[256 + bin], (uint32_t)(units >> 20));
 }
-// The range in which the running sum over the ranges reaches `level` (a level of 0 and below: the first), by a whole warp: its
-// index (256: none does), the sum before it and with it; and the sum of all.
-__device__ __forceinline__ uint32_t find_range(const uint32_t* hist, double level, bool beyond, u64& before, u64& upto, u64& all) {
-    const int lane = threadIdx.x & 31;
-    u64 run[8], sum = 0;
+// The running sums over the ranges, by a whole warp; lane L holds ranges 8L to 8L + 7.
+struct RangeSums {
+    u64 run[8], lead, all;
+    int lane;
+    __device__ __forceinline__ explicit RangeSums(const uint32_t* hist) : lane(threadIdx.x & 31) {
+        u64 sum = 0;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const uint4 lo = reinterpret_cast<const uint4*>(hist)[2 * lane + half], hi = reinterpret_cast<const uint4*>(hist + 256)[2 * lane + half];
-        run[4 * half + 0] = sum += lo.x + ((u64)hi.x << 20);
-        run[4 * half + 1] = sum += lo.y + ((u64)hi.y << 20);
-        run[4 * half + 2] = sum += lo.z + ((u64)hi.z << 20);
-        run[4 * half + 3] = sum += lo.w + ((u64)hi.w << 20);
+        for (int half = 0; half < 2; ++half) {
+            const uint4 lo = reinterpret_cast<const uint4*>(hist)[2 * lane + half], hi = reinterpret_cast<const uint4*>(hist + 256)[2 * lane + half];
+            run[4 * half + 0] = sum += lo.x + ((u64)hi.x << 20);
+            run[4 * half + 1] = sum += lo.y + ((u64)hi.y << 20);
+            run[4 * half + 2] = sum += lo.z + ((u64)hi.z << 20);
+            run[4 * half + 3] = sum += lo.w + ((u64)hi.w << 20);
+        }
+        lead = lanes_before(sum, lane, all);
     }
-    u64 incl = sum;
+    // The first range whose running sum reaches `level` (kBeyond: goes past it), 256 when none does; the sum before it.
+    template <bool kBeyond>
+    __device__ __forceinline__ uint32_t find(double level, u64& before) const {
+        uint32_t short_of = 0;
+        u64 last = lead;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const u64 up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += up;
+        for (int q = 0; q < 8; ++q) {
+            const double reach = (double)(lead + run[q]);
+            if (!(kBeyond ? reach > level : reach >= level)) { ++short_of; last = lead + run[q]; }
+        }
+        const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, short_of < 8);
+        if (lanes == 0) { before = all; return 256u; }
+        const int src = __ffs(lanes) - 1;
+        before = __shfl_sync(0xFFFFFFFFu, last, src);
+        return 8u * src + __shfl_sync(0xFFFFFFFFu, short_of, src);
     }
-    all = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    const u64 lead = incl - sum;
-    uint32_t short_of = 0;
-    u64 last = lead, hit = 0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const double reach = (double)(lead + run[q]);
-        const bool reached = beyond ? reach > level : reach >= level;  // (`beyond`: has to go past it)
-        if (!reached) { ++short_of; last = lead + run[q]; }
-        if (reached && hit == 0) hit = lead + run[q] + 1;
-    }
-    const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, short_of < 8);
-    if (lanes == 0) { before = upto = all; return 256u; }
-    const int src = __ffs(lanes) - 1;
-    before = __shfl_sync(0xFFFFFFFFu, last, src);
-    upto = __shfl_sync(0xFFFFFFFFu, hit, src) - 1;
-    return 8u * src + __shfl_sync(0xFFFFFFFFu, short_of, src);
-}
+};
 
-__device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t row, u64* dyn) {
+__device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn) {
     ulonglong2* const s_list = reinterpret_cast<ulonglong2*>(dyn);
     float* const s_raw = reinterpret_cast<float*>(s_list + kListCap);
     uint32_t* const s_by_value = reinterpret_cast<uint32_t*>(s_raw + kListCap);  // masses over 256 ranges of the value
     uint32_t* const s_by_column = s_by_value + 512;                              // ... and of the column
-    float* const s_l = reinterpret_cast<float*>(s_by_column + 512);
+    u64* const s_unit = reinterpret_cast<u64*>(s_by_column + 512);               // a candidate's mass in units of 2^-40 of the largest
+    float* const s_l = reinterpret_cast<float*>(s_unit + kNucleusCap);
     float* const s_x = s_l + kNucleusCap;
     uint32_t* const s_col = reinterpret_cast<uint32_t*>(s_x + kNucleusCap);
-    __shared__ double s_z[kListWarps], s_rest[kListWarps];
+    __shared__ u64 s_z[kListWarps], s_rest[kListWarps];
+    __shared__ double s_tails, s_proc_tails;
     __shared__ u64 s_cut_key, s_margin;
     __shared__ uint32_t s_dropped[kListWarps];
     __shared__ int s_n, s_cut_n, s_draw_n, s_decided, s_survivors, s_doubt;
@@ -500,16 +542,16 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
     PartsJoined j;
     uint2 c[4];
     uint32_t where[4];
-    ChunkWalk walk(p, row);
-    load_parts(p, row, j);
+    ChunkWalk walk(p, v);
+    load_parts(p, v, j);
     walk.fetch(c, where);
-    const double u = p.uniforms ? p.uniforms[row] : 0.5;
+    const double u = v.u;
     reinterpret_cast<uint4*>(s_by_value)[tid] = make_uint4(0, 0, 0, 0);  // both histograms
     if (tid == 0) { s_n = 0; s_cut_n = 0; s_draw_n = 0; s_decided = 0; s_survivors = 0; s_doubt = 0; s_cut_key = ~0ull; s_margin = ~0ull; }
     const double power = exp_power_of_lane();
     __syncthreads();
-    if (!join_parts(p, j)) return false;
-    if (settle_bad_row(p, row, j)) return true;
+    if (!join_parts(v, j)) return false;
+    if (settle_bad_row(v, j)) return true;
     PSX_MERGE_STAGE(3);
     // ---- 1. candidates at or above the largest part threshold into shared memory, their masses by value; what lies below it
     // belongs to the rest of the vocabulary, which the candidates do not cover ---------------------------------------------------
@@ -528,30 +570,39 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
         uint32_t where_next[4];
         const bool last = walk.beyond(j.longest);
         if (!last) walk.fetch(next, where_next);
+        // (four candidates in straight line: their chains of dependent operations run side by side)
         float x[4];
-        uint32_t votes[4];
+        u64 units[4];
+        uint32_t votes[4], there = 0;
         int all = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const uint32_t here = __shfl_sync(0xFFFFFFFFu, j.count, where[q] & 255u);
-            const bool there = (where[q] >> 8) + lane < here;
-            const float l = __uint_as_float(c[q].x);
-            float y = there ? l : -INFINITY;
-            if (there && (c[q].y & ~kColumnMask) != 0) y = processed_before_temperature(l, c[q].y, p.penalty);
-            x[q] = temper(y, apply_t, p.temperature);
-            const bool on = y >= keep_from;
-            votes[q] = __ballot_sync(0xFFFFFFFFu, on);
-            if (!__any_sync(0xFFFFFFFFu, there)) continue;
-            const double mass = exp_to(x[q], x_max, y > -INFINITY, power);
-            if (there && !on) {
-                z.add_low(l);
-                rest += mass;
-                dropped += y > -INFINITY ? 1u : 0u;
-            }
-            if (votes[q] == 0) continue;
-            z.high += exp_to(l, j.raw_max, on, power);
-            if (on) add_units(s_by_value, bin_of(x[q]), (u64)__double2ull_rn(mass * 0x1p40));
+            const bool in = (where[q] >> 8) + lane < here;
+            there |= in ? 1u << q : 0u;
+            x[q] = in ? __uint_as_float(c[q].x) : -INFINITY;
+            if (in && (c[q].y & ~kColumnMask) != 0) x[q] = processed_before_temperature(x[q], c[q].y, p.penalty);
+            votes[q] = __ballot_sync(0xFFFFFFFFu, x[q] >= keep_from);
             all += __popc(votes[q]);
+        }
+        if (apply_t) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) x[q] = __fdiv_rn(x[q], p.temperature);
+        }
+        double mass[4], raw[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mass[q] = exp_to(x[q], x_max, x[q] > -INFINITY, power);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) raw[q] = exp_to(__uint_as_float(c[q].x), j.raw_max, (votes[q] >> lane) & 1u, power);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool on = (votes[q] >> lane) & 1u, in = (there >> q) & 1u;
+            units[q] = (u64)__double2ull_rn(mass[q] * 0x1p40);
+            z.high += raw[q];  // (zero unless listed)
+            if (on) add_units(s_by_value, bin_of(x[q]), units[q]);
+            rest += on ? 0.0 : mass[q];
+            dropped += !on && x[q] > -INFINITY ? 1u : 0u;
+            if (in && !on) z.add_low(__uint_as_float(c[q].x));
         }
         if (all != 0) {
             int at = 0;
@@ -561,6 +612,7 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
             for (int q = 0; q < 4; ++q) {
                 const int mine = at + __popc(votes[q] & below);
                 if (((votes[q] >> lane) & 1u) && mine < kNucleusCap) {
+                    s_unit[mine] = units[q];
                     s_l[mine] = __uint_as_float(c[q].x);
                     s_x[mine] = x[q];
                     s_col[mine] = c[q].y & kColumnMask;
@@ -573,26 +625,29 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
         for (int q = 0; q < 4; ++q) { c[q] = next[q]; where[q] = where_next[q]; }
     }
     {
-        double sum = z.of_warp();
-        if (warp == 0) {
-            sum += tails_of_parts(j);
+        const u64 sum = z.of_warp(), rest_of_warp = warp_sum_units((u64)__double2ull_rn(rest * 0x1p40));
+        if (warp == kListWarps - 1) {
+            const double tails = tails_of_parts(j);
+            if (lane == 0) s_tails = tails;
+        } else if (warp == kListWarps - 2) {
+            double tails = 0.0;
             if (j.mine.y_max > -INFINITY && j.mine.proc_tail > 0.0) {
-                rest += j.mine.proc_tail * exp((double)temper(j.mine.y_max, apply_t, p.temperature) - (double)x_max);
+                tails = j.mine.proc_tail * exp((double)temper(j.mine.y_max, apply_t, p.temperature) - (double)x_max);
             }
+            tails = warp_sum(tails);
+            if (lane == 0) s_proc_tails = tails;
         }
-        rest = warp_sum(rest);
         dropped = __reduce_add_sync(0xFFFFFFFFu, dropped);
-        if (lane == 0) { s_z[warp] = sum; s_rest[warp] = rest; s_dropped[warp] = dropped; }
+        if (lane == 0) { s_z[warp] = sum; s_rest[warp] = rest_of_warp; s_dropped[warp] = dropped; }
     }
     __syncthreads();
     PSX_MERGE_STAGE(4);
     const int n = s_n;
     if (n > kNucleusCap || n == 0) return false;
-    rest = s_rest[0];
-    double sum_exp = s_z[0];
-    u64 outside = j.tail_alive + s_dropped[0];
+    u64 rest_units = 0, sum_units = 0, outside = j.tail_alive;
 #pragma unroll
-    for (int w = 1; w < kListWarps; ++w) { rest += s_rest[w]; outside += s_dropped[w]; sum_exp += s_z[w]; }
+    for (int w = 0; w < kListWarps; ++w) { rest_units += s_rest[w]; sum_units += s_z[w]; outside += s_dropped[w]; }
+    rest = (double)rest_units * 0x1p-40 + s_proc_tails;
     // ---- 2. the top-p (:89-103): the range that its level falls into ---------------------------------------------------------
     const double limit = 1.0 - (double)p.top_p, min_p = (double)p.min_p;
     const bool top_p_on = p.top_p < 1.0f, rest_alive = outside != 0;
@@ -600,17 +655,16 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
     double top_p_margin = INFINITY;
     u64 cut_key = 0;
     if (top_p_on) {
-        u64 before, upto, all = 0;
-        for (int i = lane; i < 256; i += 32) all += s_by_value[i] + ((u64)s_by_value[256 + i] << 20);
-        all = warp_sum_units(all);
-        const double listed = (double)all * 0x1p-40, whole = listed + (rest_alive ? rest : 0.0);
+        u64 before;
+        const RangeSums ranges(s_by_value);
+        const double listed = (double)ranges.all * 0x1p-40, whole = listed + (rest_alive ? rest : 0.0);
         const double need = (whole - limit * whole) * 0x1p40;  // an entry stays while what comes after it is less
         // Everything outside the list leads the ascending walk and has to fall as a whole.
         if (rest_alive) {
             if (!(rest <= (limit - kNucleusDoubt) * whole)) return false;
             top_p_margin = fabs(rest / whole - limit);
         }
-        cut_bin = find_range(s_by_value, need, false, before, upto, all);
+        cut_bin = ranges.find<false>(need, before);
         if (cut_bin > 255u) return false;
         // ---- 3. its entries look at one another ---------------------------------------------------------------------------------
         for (int first = warp * 32; first < n; first += kMergeThreads) {
@@ -620,10 +674,8 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
             if (takers == 0) continue;
             int at = 0;
             if (lane == 0) at = atomicAdd(&s_cut_n, __popc(takers));
-            const float x = on ? s_x[e] : 0.0f;
-            const u64 units = (u64)__double2ull_rn(exp_to(x, x_max, on, power) * 0x1p40);
             at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(takers & below);
-            if (on && at < kListCap) s_list[at] = make_ulonglong2(((u64)ordered_key(x) << 32) | s_col[e], units);
+            if (on && at < kListCap) s_list[at] = make_ulonglong2(((u64)ordered_key(s_x[e]) << 32) | s_col[e], s_unit[e]);
         }
         __syncthreads();
         PSX_MERGE_STAGE(5);
@@ -657,36 +709,30 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
     }
     // ---- 4. the masses of those that stay, by column --------------------------------------------------------------------------
     const int col_shift = max(0, 24 - __clz((uint32_t)(p.vocab - 1)));
-    auto stays_of = [&](int e, u64& units) {  // by a whole warp; s_doubt where the min-p cannot tell
-        const float x = e < n ? s_x[e] : -INFINITY;
-        bool stays = e < n;
-        if (top_p_on && stays) {
+    auto stays = [&](int e) {  // (s_doubt where the min-p cannot tell)
+        if (top_p_on) {
+            const float x = s_x[e];
             const uint32_t b = bin_of(x);
-            stays = b < cut_bin || (b == cut_bin && (((u64)ordered_key(x) << 32) | s_col[e]) >= cut_key);
+            if (b > cut_bin || (b == cut_bin && (((u64)ordered_key(x) << 32) | s_col[e]) < cut_key)) return false;
         }
-        const double mass = exp_to(x, x_max, stays, power);
-        if (min_p > 0.0 && stays && x < x_max) {  // :104-111, against the first maximum's exp(0)
+        if (min_p > 0.0 && s_unit[e] < (1ull << 40)) {  // :104-111, against the first maximum's exp(0)
+            const double mass = (double)s_unit[e] * 0x1p-40;
             if (fabs(mass - min_p) < kDoubt) s_doubt = 1;
-            stays = mass >= min_p;
+            return mass >= min_p;
         }
-        units = stays ? (u64)__double2ull_rn(mass * 0x1p40) : 0;
-        return stays;
+        return true;
     };
-    for (int first = warp * 32; first < n; first += kMergeThreads) {
-        const int e = first + lane;
-        u64 units;
-        const bool stays = stays_of(e, units);
+    for (int e = tid; e < n; e += kMergeThreads) {
+        if (!stays(e)) continue;
         if (p.survivor_cols != nullptr) {
-            if (stays) {
-                const int at = atomicAdd(&s_survivors, 1);
-                if (at < p.survivor_cap) {
-                    p.survivor_cols[row * p.survivor_cap + at] = s_col[e];
-                    p.survivor_vals[row * p.survivor_cap + at] = s_x[e];
-                }
+            const int at = atomicAdd(&s_survivors, 1);
+            if (at < p.survivor_cap) {
+                p.survivor_cols[row * p.survivor_cap + at] = s_col[e];
+                p.survivor_vals[row * p.survivor_cap + at] = s_x[e];
             }
         } else {
-            if (units != 0) add_units(s_by_column, s_col[e] >> col_shift, units);
-            if (p.diag && stays) atomicAdd(&s_survivors, 1);
+            add_units(s_by_column, s_col[e] >> col_shift, s_unit[e]);
+            if (v.diag) atomicAdd(&s_survivors, 1);
         }
     }
     __syncthreads();
@@ -696,30 +742,21 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
         if (s_survivors > p.survivor_cap) return false;
         if (tid == 0) {
             p.survivor_counts[row] = (uint32_t)s_survivors;
-            p.row_status[row] = PSX_ROW_OK;
+            *v.status = PSX_ROW_OK;
         }
         return true;
     }
     // ---- 5. the draw (:140-152): the range of columns that holds u, then its entries one by one --------------------------------
-    u64 before, upto, total = 0;
-    for (int i = lane; i < 256; i += 32) total += s_by_column[i] + ((u64)s_by_column[256 + i] << 20);
-    total = warp_sum_units(total);
-    const double target = u * (double)total;
-    const uint32_t range = find_range(s_by_column, target, true, before, upto, total);
+    u64 before;
+    const RangeSums columns(s_by_column);
+    const double total = (double)columns.all, target = u * total;
+    const uint32_t range = columns.find<true>(target, before);
     if (range > 255u) return false;
-    for (int first = warp * 32; first < n; first += kMergeThreads) {
-        const int e = first + lane;
-        const bool near = e < n && (s_col[e] >> col_shift) == range;
-        if (!__any_sync(0xFFFFFFFFu, near)) continue;
-        u64 units;
-        const bool stays = stays_of(near ? e : n, units);
-        const uint32_t takers = __ballot_sync(0xFFFFFFFFu, stays);
-        if (takers == 0) continue;
-        int at = 0;
-        if (lane == 0) at = atomicAdd(&s_draw_n, __popc(takers));
-        at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(takers & below);
-        if (stays && at < kListCap) {
-            s_list[at] = make_ulonglong2(s_col[e], units);
+    for (int e = tid; e < n; e += kMergeThreads) {
+        if ((s_col[e] >> col_shift) != range || !stays(e)) continue;
+        const int at = atomicAdd(&s_draw_n, 1);
+        if (at < kListCap) {
+            s_list[at] = make_ulonglong2(s_col[e], s_unit[e]);
             s_raw[at] = s_l[e];
         }
     }
@@ -738,11 +775,11 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
         const double lo = target - (double)mine, hi = (double)(mine + me.y) - target;
         if (lo < 0.0 || hi <= 0.0) continue;
         const double margin = mine == 0 ? hi : fmin(lo, hi);
-        if (margin < kNucleusDoubt * (double)total) continue;  // (nobody takes it: replayed)
-        p.row_status[row] = PSX_ROW_OK;
-        p.tokens[row] = (int64_t)me.x;
-        p.log_probs[row] = (float)(((double)s_raw[e] - (double)j.raw_max) - log(sum_exp));  // :133,156
-        if (p.diag) p.diag[row] = psx_row_diag{n, s_survivors, margin / (double)total, top_p_margin};
+        if (margin < kNucleusDoubt * total) continue;  // (nobody takes it: replayed)
+        *v.status = PSX_ROW_OK;
+        *v.token = (int64_t)me.x;
+        *v.log_prob = (float)(((double)s_raw[e] - (double)j.raw_max) - log((double)sum_units * 0x1p-40 + s_tails));  // :133,156
+        if (v.diag) *v.diag = psx_row_diag{n, s_survivors, margin / total, top_p_margin};
         s_decided = 1;
     }
     __syncthreads();
@@ -753,11 +790,11 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
 enum ListKind { kListGreedy, kListTopK, kListNucleus };
 
 template <int kKind>
-__device__ __forceinline__ bool list_row(const MergeParams& p, const int64_t row, u64* dyn) {
+__device__ __forceinline__ bool list_row(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn) {
     if (p.parts > 32) return false;  // (a record per lane)
-    if (kKind == kListGreedy) return p.survivor_cols == nullptr && list_greedy(p, row);
-    if (kKind == kListTopK) return p.dyn_bytes >= kTopKArena && list_top_k(p, row, dyn);
-    return p.dyn_bytes >= kNucleusArena && list_nucleus(p, row, dyn);
+    if (kKind == kListGreedy) return p.survivor_cols == nullptr && list_greedy(p, v);
+    if (kKind == kListTopK) return p.dyn_bytes >= kTopKArena && list_top_k(p, row, v, dyn);
+    return p.dyn_bytes >= kNucleusArena && list_nucleus(p, row, v, dyn);
 }
 
 }  // namespace survivor
