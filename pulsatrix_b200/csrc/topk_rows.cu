@@ -4,12 +4,14 @@
 // row per CTA.  Entries are compared as order-preserving keys: NaN above every number,
 // -0.0 == +0.0, `largest == 0` mirrors the order.
 //
-// The short way (k <= 256): two sweeps over the slice as floats, straight from global memory, the
-// second one out of L2.  Sweep one notes every thread's best entry; the smallest over the warps of
+// The short way (k <= 256): two sweeps over the slice as floats, out of shared memory where a slice of
+// up to 16,384 entries fits (bulk copies; longer ones are read from global memory twice, the second time out of L2).
+// Bound by instructions more than by HBM: 4096 x 16,384, k 64: 79.7 us with 256 threads reading twice from global memory,
+// 75.3 now; 8192 x 4096, k 16: 63.5 -> 36.9 us.  Sweep one notes every thread's best entry; the smallest over the warps of
 // the kp-th best of those (kp = ceil(k / 8)) is a bound that k entries of the slice reach.  Sweep
 // two lists what reaches the bound, usually k and a few; the list is put in rank order by
 // counting, and with several CTAs per row the best k of each meet in the first CTA's shared memory
-// (distributed shared memory, two cluster barriers), where they are sorted and written out.
+// (distributed shared memory, two cluster barriers), where each finds its place in the others' lists by bisection.
 //
 // The long way (larger k, or a list that overflowed: thousands of ties): the slice becomes keys in
 // shared memory (or is swept from global memory when it does not fit), and
@@ -27,6 +29,8 @@
 // reference bit for bit.
 #include <cooperative_groups.h>
 
+#include "psx_async.cuh"
+#include "scan_rows.cuh"
 #include "topk_rows.cuh"
 
 namespace cg = cooperative_groups;
@@ -36,8 +40,10 @@ namespace psx {
 namespace {
 
 using u64 = unsigned long long;
-constexpr int kThreads = 256;
+constexpr int kWidest = 256;  // threads of a CTA at most
 constexpr int kSliceMax = 48 * 1024;  // keys one CTA keeps in shared memory (192 KB)
+constexpr uint32_t kHeldMax = 16 * 1024;  // entries the short way keeps in shared memory: 64 KB, three CTAs per SM
+constexpr uint32_t kHeldCopies = 4, kHeldChunk = kHeldMax / 4 / kHeldCopies;  // bulk copies, vectors of each
 
 __device__ __forceinline__ uint32_t rank_key(float x, bool largest) {
     const uint32_t k = (x != x) ? 0xFFFFFFFFu : ordered_key(x);
@@ -92,6 +98,7 @@ struct TopKParams {
     int in_shared;   // the slice's keys are kept in shared memory
     uint32_t k_pad;  // power of two >= k: slots of the collecting array
     uint32_t list_cap;  // entries of a CTA's short list (0: no lists)
+    unsigned long long wait_limit_ns;  // longest wait for a copy in flight
 };
 
 // The cluster's histograms of one pass, added up and scanned from the top by warp 0 of every CTA:
@@ -142,14 +149,20 @@ __device__ __forceinline__ Found find_digit(cg::cluster_group& cluster, uint32_t
     return f;
 }
 
-template <bool kLargest>
-__global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams p) {
+// kHeld: the short way keeps its slice (at most kHeldMax entries) in shared memory, where four bulk copies bring it, each on a barrier of its
+// own; the sweeps read it from there.
+// kThreads: most of a CTA's instructions are a warp's own (its bound, its entries, their places), whatever its share of the
+// slice: few warps where each still has at most 32 vectors per lane and k is at most half of the threads.
+template <bool kLargest, bool kHeld, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(const __grid_constant__ TopKParams p) {
     extern __shared__ __align__(16) unsigned char dyn[];
     // layout: [k_pad collected entries][list_cap listed entries][cluster * k_pad gathered entries], 8 bytes
     //         each, then [slice keys, 4 bytes each (when in_shared)]
     u64* collected = reinterpret_cast<u64*>(dyn);
     u64* list = collected + p.k_pad;
-    u64* gathered = list + p.list_cap;
+    uint32_t* list_key = reinterpret_cast<uint32_t*>(list + p.list_cap);  // the listed entries' keys by themselves
+    uint32_t* claimed = list_key + p.list_cap;                            // entries that found themselves at a place
+    u64* gathered = reinterpret_cast<u64*>(claimed + p.list_cap);
     uint32_t* keys = reinterpret_cast<uint32_t*>(gathered + (size_t)p.k_pad * (p.cluster > 1 && p.list_cap != 0 ? p.cluster : 0));
     // histograms of the long way, used in turn by its passes; a pass clears the one before it once the
     // cluster has met again (nobody reads it any more)
@@ -167,12 +180,30 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
     const uint32_t begin = min(n, (uint32_t)rank * p.slice), end = min(n, begin + p.slice);
     const uint32_t mine = end - begin;
     const bool in_shared = p.in_shared != 0;
+    // the slice from its first 16-byte boundary on, as vectors; up to three entries before them and after them
+    const float* src = row + begin;
+    const uint32_t head = min(mine, (uint32_t)((4 - ((reinterpret_cast<uintptr_t>(src) >> 2) & 3)) & 3));
+    const uint32_t vectors = (mine - head) / 4;
+    const float4* src4 = reinterpret_cast<const float4*>(src + head);
+    float4* held4 = reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(keys) + 15) & ~uintptr_t(15));
+    __shared__ __align__(8) uint64_t s_bar[kHeldCopies];
+    if (kHeld && tid < kHeldCopies) {
+        const uint32_t first = tid * kHeldChunk;
+        if (first < vectors) {
+            const uint32_t bytes = min(vectors - first, kHeldChunk) * 16;
+            barrier_init(&s_bar[tid], 1);
+            barrier_init_fence();
+            barrier_expect_bytes(&s_bar[tid], bytes);
+            bulk_copy_to_shared(held4 + first, src4 + first, bytes, &s_bar[tid]);
+        }
+    }
     // The cluster's barrier costs about a microsecond; one CTA on its own meets with the block barrier.
     auto meet = [&]() {
         if (ranks > 1) cluster.sync(); else __syncthreads();
     };
 
     for (int i = tid; i < 2 * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
+    for (uint32_t i = tid; i < 2 * p.list_cap; i += kThreads) list_key[i] = 0;
     if (tid == 0) {
         s_collected = 0;
         s_listed = 0;
@@ -188,11 +219,8 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
     //      is put in rank order by counting, and the best k of every CTA meet in the first CTA. ----------
     if (p.list_cap != 0) {  // uniform over the cluster
         __shared__ uint32_t s_warp_bound[kThreads / 32];
-        const float* src = row + begin;
-        const uint32_t head = min(mine, (uint32_t)((4 - ((reinterpret_cast<uintptr_t>(src) >> 2) & 3)) & 3));
-        const uint32_t vectors = (mine - head) / 4;
-        const float4* src4 = reinterpret_cast<const float4*>(src + head);
         constexpr int kBatch = 8;  // loads in flight per thread
+        bool landed = true;
         // sweep one: the extreme entry this thread sees.  With the largest wanted a NaN is the best
         // there is, and the maximum that returns NaN for a NaN operand finds it; with the smallest
         // wanted a NaN is the worst, and the plain minimum passes it by.
@@ -202,15 +230,27 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
             extreme = largest ? max3_nan(max3_nan(d.x, d.y, d.z), d.w, extreme) : min3(min3(d.x, d.y, d.z), d.w, extreme);
         };
         for (uint32_t i = tid; i < head; i += kThreads) note(src[i]);
-        for (uint32_t v0 = tid; v0 < vectors; v0 += kBatch * kThreads) {
-            float4 d[kBatch];
+        if (kHeld) {
+            for (uint32_t c = 0; c * kHeldChunk < vectors; ++c) {
+                landed = barrier_wait_bounded(&s_bar[c], 0, p.wait_limit_ns) && landed;
+                const uint32_t stop = min(vectors, (c + 1) * kHeldChunk);
 #pragma unroll
-            for (int q = 0; q < kBatch; ++q) {
-                const uint32_t v = v0 + q * kThreads;
-                d[q] = v < vectors ? __ldg(src4 + v) : make_float4(extreme, extreme, extreme, extreme);
+                for (uint32_t q = 0; q < kHeldChunk / kThreads; ++q) {
+                    const uint32_t v = c * kHeldChunk + q * kThreads + tid;
+                    if (v < stop) note4(held4[v]);
+                }
             }
+        } else {
+            for (uint32_t v0 = tid; v0 < vectors; v0 += kBatch * kThreads) {
+                float4 d[kBatch];
 #pragma unroll
-            for (int q = 0; q < kBatch; ++q) note4(d[q]);
+                for (int q = 0; q < kBatch; ++q) {
+                    const uint32_t v = v0 + q * kThreads;
+                    d[q] = v < vectors ? __ldg(src4 + v) : make_float4(extreme, extreme, extreme, extreme);
+                }
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) note4(d[q]);
+            }
         }
         for (uint32_t i = head + 4 * vectors + tid; i < mine; i += kThreads) note(src[i]);
         // The thread's best key, never overstated: a thread that saw nothing offers 0, and so does one
@@ -234,12 +274,21 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
         // sweep two: key >= bound, decided on the float itself: with the largest wanted, x is NaN or
         // x >= the bound's float; with the smallest wanted, x <= the mirrored bound's float.  A bound of
         // 0 lists everything; a bound that only NaN reaches is left to the long way.
-        const bool everything = bound == 0, only_nan = largest && bound == 0xFFFFFFFFu;
+        if (kHeld && __syncthreads_or(landed ? 0 : 1) != 0) {
+            // a copy did not arrive in time: one more bounded wait (nothing may land after the CTA has left), then the long way
+            for (uint32_t c = 0; c * kHeldChunk < vectors; ++c) barrier_wait_bounded(&s_bar[c], 0, p.wait_limit_ns);
+            landed = false;
+        }
+        const bool everything = bound == 0 && landed, only_nan = (largest && bound == 0xFFFFFFFFu) || !landed;
         const float edge = largest ? from_ordered_key(bound) : from_ordered_key(~bound);
         auto reaches = [&](float x) { return largest ? !(x < edge) : x <= edge; };
         auto put = [&](float x, uint32_t col) {
             const uint32_t slot = atomicAdd(&s_listed, 1u);
-            if (slot < p.list_cap) list[slot] = ((u64)rank_key(x, largest) << 32) | (uint32_t)~col;
+            if (slot < p.list_cap) {
+                const uint32_t key = rank_key(x, largest);
+                list[slot] = ((u64)key << 32) | (uint32_t)~col;
+                list_key[slot] = key;
+            }
         };
         if (everything) {
             if (mine <= p.list_cap) {
@@ -253,6 +302,45 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
             for (uint32_t i = tid; i < head; i += kThreads) {
                 if (reaches(src[i])) put(src[i], begin + i);
             }
+            if (kHeld) {
+                // branch-free over the vectors, one bit for each that reaches the bound; then a warp's slots at once
+                uint32_t noted = 0, count = 0;
+#pragma unroll 4
+                for (uint32_t t = 0; t * kThreads < vectors; ++t) {
+                    const uint32_t v = t * kThreads + tid;
+                    const float4 d = held4[min(v, vectors - 1)];
+                    const float best4 = largest ? max3_nan(max3_nan(d.x, d.y, d.z), d.w, d.w) : min3(min3(d.x, d.y, d.z), d.w, d.w);
+                    if (reaches(best4) && v < vectors) noted |= 1u << t;
+                }
+                auto hits_of = [&](const float4& d) {
+                    return (reaches(d.x) ? 1u : 0u) | (reaches(d.y) ? 2u : 0u) | (reaches(d.z) ? 4u : 0u) | (reaches(d.w) ? 8u : 0u);
+                };
+                for (uint32_t m = noted; m != 0; m &= m - 1) count += __popc(hits_of(held4[(__ffs(m) - 1) * kThreads + tid]));
+                uint32_t incl = count;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl += up;
+                }
+                uint32_t slot = 0;
+                if (lane == 31 && incl != 0) slot = atomicAdd(&s_listed, incl);
+                slot = __shfl_sync(0xFFFFFFFFu, slot, 31) + incl - count;
+                for (uint32_t m = noted; m != 0; m &= m - 1) {
+                    const uint32_t v = (__ffs(m) - 1) * kThreads + tid, col = begin + head + 4 * v;
+                    const float4 d = held4[v];
+                    const float x[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) {
+                        if (!reaches(x[q])) continue;
+                        if (slot < p.list_cap) {
+                            const uint32_t key = rank_key(x[q], largest);
+                            list[slot] = ((u64)key << 32) | (uint32_t)~(col + q);
+                            list_key[slot] = key;
+                        }
+                        ++slot;
+                    }
+                }
+            } else
             for (uint32_t v0 = tid; v0 < vectors; v0 += kBatch * kThreads) {
                 float4 d[kBatch];
 #pragma unroll
@@ -288,28 +376,44 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
         // first CTA's array.  An entry's place is the number of entries that rank before it.
         u64* gathered0 = ranks > 1 ? cluster.map_shared_rank(gathered, 0) + (size_t)rank * p.k_pad : nullptr;
         if (fits) {
-            if (on_list > (uint32_t)kThreads) {  // a long list: sort it
-                uint32_t n_pad = 2;
-                while (n_pad < on_list) n_pad <<= 1;
-                for (uint32_t i = on_list + tid; i < n_pad; i += kThreads) list[i] = 0;
-                __syncthreads();
-                block_bitonic_sort(list, (int)n_pad, /*descending=*/true);
-            }
-            for (uint32_t i = tid; i < on_list; i += kThreads) {
-                const u64 entry = list[i];
-                uint32_t place = i;
-                if (on_list <= (uint32_t)kThreads) {
-                    place = 0;
-                    for (uint32_t j = 0; j < on_list; ++j) place += list[j] > entry ? 1u : 0u;
+            auto place_entry = [&](u64 entry, uint32_t place) {
+                if (place >= best) return;
+                if (ranks == 1) {
+                    const uint32_t col = ~(uint32_t)entry, at = col - begin - head;
+                    out_v[place] = kHeld && at < 4 * vectors ? reinterpret_cast<const float*>(held4)[at] : row[col];
+                    out_i[place] = (float)col;
+                } else {
+                    gathered0[place] = entry;
                 }
-                if (place < best) {
-                    if (ranks == 1) {
-                        const uint32_t col = ~(uint32_t)entry;
-                        out_v[place] = row[col];
-                        out_i[place] = (float)col;
-                    } else {
-                        gathered0[place] = entry;
-                    }
+            };
+            // An entry's place by looking at all the others' keys, four at a time; neighbouring threads share an entry when there are
+            // threads left over.  Entries with equal keys find themselves at the same place: then (rare) the columns are looked at too.
+            uint32_t n_pad = 8;
+            while (n_pad < on_list && n_pad < (uint32_t)kThreads) n_pad <<= 1;
+            const uint32_t share = (uint32_t)kThreads / n_pad < 32u ? (uint32_t)kThreads / n_pad : 32u, slice = tid & (share - 1);
+            const uint32_t quads = (on_list + 3) / 4, per_round = (uint32_t)kThreads / share;  // (zeros behind the list)
+            bool tied = false;
+            for (uint32_t first = 0; first < on_list; first += per_round) {
+                const uint32_t i = first + (uint32_t)tid / share;
+                const uint32_t key = i < on_list ? list_key[i] : ~0u;
+                uint32_t place = 0;
+#pragma unroll 4
+                for (uint32_t j = slice; j < quads; j += share) {
+                    const uint4 other = reinterpret_cast<const uint4*>(list_key)[j];
+                    place += (other.x > key ? 1u : 0u) + (other.y > key ? 1u : 0u) + (other.z > key ? 1u : 0u) + (other.w > key ? 1u : 0u);
+                }
+                for (uint32_t o = share >> 1; o > 0; o >>= 1) place += __shfl_xor_sync(0xFFFFFFFFu, place, o);
+                if (slice == 0 && i < on_list && place < best) {
+                    if (atomicAdd(&claimed[place], 1u) != 0) tied = true;
+                    place_entry(list[i], place);
+                }
+            }
+            if (__syncthreads_or(tied ? 1 : 0) != 0) {
+                for (uint32_t i = tid; i < on_list; i += kThreads) {
+                    const u64 entry = list[i];
+                    uint32_t place = 0;
+                    for (uint32_t j = 0; j < on_list; ++j) place += list[j] > entry ? 1u : 0u;
+                    place_entry(entry, place);
                 }
             }
             if (ranks == 1) return;
@@ -323,11 +427,27 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
             if (overflow == 0) {  // uniform over the cluster
                 cluster.sync();   // everybody has read everybody's verdict: CTAs may leave
                 if (rank != 0) return;
-                block_bitonic_sort(gathered, (int)(p.k_pad * (uint32_t)ranks), /*descending=*/true);
-                for (uint32_t j = tid; j < (uint32_t)p.k; j += kThreads) {
-                    const uint32_t col = ~(uint32_t)gathered[j];
-                    out_v[j] = row[col];
-                    out_i[j] = (float)col;
+                // The CTAs' lists are in rank order (zeros fill them up): an entry's place is its place in its own list and, by
+                // bisection, the number of entries of each other list that rank before it.
+                for (uint32_t i = tid; i < p.k_pad * (uint32_t)ranks; i += kThreads) {
+                    const u64 entry = gathered[i];
+                    const uint32_t own = i / p.k_pad;
+                    uint32_t place = i - own * p.k_pad;
+                    if (entry == 0 || place >= (uint32_t)p.k) continue;
+                    for (uint32_t r = 0; r < (uint32_t)ranks; ++r) {
+                        if (r == own) continue;
+                        const u64* other = gathered + r * p.k_pad;
+                        uint32_t before = 0;
+                        for (uint32_t step = p.k_pad; step > 0; step >>= 1) {
+                            if (before + step <= p.k_pad && other[before + step - 1] > entry) before += step;
+                        }
+                        place += before;
+                    }
+                    if (place < (uint32_t)p.k) {
+                        const uint32_t col = ~(uint32_t)entry;
+                        out_v[place] = row[col];
+                        out_i[place] = (float)col;
+                    }
                 }
                 return;
             }
@@ -338,13 +458,9 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
 
     // ---- the slice as keys in shared memory, for the long way ----------------------------------------------
     if (in_shared) {
-        const float* src = row + begin;
-        const uint32_t head = min(mine, (uint32_t)((4 - ((reinterpret_cast<uintptr_t>(src) >> 2) & 3)) & 3));
         // keys[head] on a 16-byte boundary, like src[head]: the array starts up to three words in
         keys = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(keys) + 15) & ~uintptr_t(15)) + ((4 - head) & 3);
         for (uint32_t i = tid; i < head; i += kThreads) keys[i] = rank_key(src[i], largest);
-        const uint32_t vectors = (mine - head) / 4;
-        const float4* src4 = reinterpret_cast<const float4*>(src + head);
         uint4* keys4 = reinterpret_cast<uint4*>(keys + head);
         constexpr int kBatch = 8;  // loads in flight per thread
         for (uint32_t v0 = tid; v0 < vectors; v0 += kBatch * kThreads) {
@@ -385,7 +501,9 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
             if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
         }
         meet();
-        if (pass > 0) s_hist[(pass - 1) & 1][tid] = 0;  // kThreads == 256 bins
+        if (pass > 0) {
+            for (int i = tid; i < 256; i += kThreads) s_hist[(pass - 1) & 1][i] = 0;
+        }
         if (tid < 32) {
             const Found f = find_digit(cluster, hist, first_rank, ranks, remaining, lane);
             if (lane == 0) {
@@ -416,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, 4) topk_rows_kernel(const TopKParams
                 if ((inverted & cmask) == cprefix) atomicAdd(&hist[(inverted >> shift) & 255u], 1u);
             }
             meet();
-            s_hist[(pass + 1) & 1][tid] = 0;
+            for (int i = tid; i < 256; i += kThreads) s_hist[(pass + 1) & 1][i] = 0;
             if (tid < 32) {
                 const Found f = find_digit(cluster, hist, first_rank, ranks, cremaining, lane);
                 if (lane == 0) {
@@ -588,33 +706,38 @@ cudaError_t launch_topk_rows(const float* in, float* values, float* indices, siz
     p.largest = largest ? 1 : 0;
     p.cluster = cols <= 16384 ? 1 : cols <= 32768 ? 2 : cols <= 65536 ? 4 : 8;
     p.slice = (uint32_t)(((cols + p.cluster - 1) / p.cluster + 3) / 4 * 4);
-    p.k_pad = 1;
+    p.k_pad = 2;  // (an even number of slots: what follows them starts on 16 bytes)
     while (p.k_pad < k) p.k_pad <<= 1;
     // The short way (k <= 256) needs no keys in shared memory; if one of its lists overflows, the
     // long way sweeps global memory.  Otherwise the keys are kept when they fit.
-    p.list_cap = k <= (size_t)kThreads ? 4 * (p.k_pad < 64 ? 64 : p.k_pad) : 0;
-    const size_t entries = p.k_pad + p.list_cap + (p.cluster > 1 && p.list_cap != 0 ? (size_t)p.cluster * p.k_pad : 0);
+    p.list_cap = k <= (size_t)kWidest ? 4 * (p.k_pad < 64 ? 64 : p.k_pad) : 0;
+    const size_t entries = p.k_pad + 2 * p.list_cap + (p.cluster > 1 && p.list_cap != 0 ? (size_t)p.cluster * p.k_pad : 0);
     p.in_shared = p.list_cap == 0 && p.slice <= (uint32_t)kSliceMax &&
                   entries * 8 + (size_t)p.slice * 4 + 4096 <= 227 * 1024 ? 1 : 0;
-    const size_t shared = entries * 8 + (p.in_shared ? (size_t)p.slice * 4 + 32 : 0);
+    p.wait_limit_ns = kDefaultWaitLimitNs;
+    const bool held = p.list_cap != 0 && p.slice <= kHeldMax;
+    const int threads = !held || k > 64 ? kWidest : p.slice <= 4096 && k <= 32 ? 64 : 128;
+    auto kernel = largest ? topk_rows_kernel<true, false, kWidest> : topk_rows_kernel<false, false, kWidest>;
+    if (held && threads == 64) kernel = largest ? topk_rows_kernel<true, true, 64> : topk_rows_kernel<false, true, 64>;
+    else if (held && threads == 128) kernel = largest ? topk_rows_kernel<true, true, 128> : topk_rows_kernel<false, true, 128>;
+    else if (held) kernel = largest ? topk_rows_kernel<true, true, kWidest> : topk_rows_kernel<false, true, kWidest>;
+    const size_t shared = entries * 8 + (p.in_shared || held ? (size_t)p.slice * 4 + 32 : 0);
     if (rows * (size_t)p.cluster > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
     if (shared > 48 * 1024) {
-        // Once per device and direction (the call sets the same value every time, so two host threads
+        // Once per device and kernel (the call sets the same value every time, so two host threads
         // that both find the flag clear do no harm).
-        static bool lifted[2][64] = {};
+        static bool lifted[8][64] = {};
         int device = 0;
         if (cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return e;
-        bool& done = lifted[largest ? 1 : 0][device & 63];
+        bool& done = lifted[(largest ? 1 : 0) + (!held ? 0 : threads == 64 ? 2 : threads == 128 ? 4 : 6)][device & 63];
         if (!done) {
-            const cudaError_t e = largest ? allow_all_dynamic_shared(topk_rows_kernel<true>)
-                                          : allow_all_dynamic_shared(topk_rows_kernel<false>);
-            if (e != cudaSuccess) return e;
+            if (const cudaError_t e = allow_all_dynamic_shared(kernel); e != cudaSuccess) return e;
             done = true;
         }
     }
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)(rows * p.cluster));
-    config.blockDim = dim3(kThreads);
+    config.blockDim = dim3((unsigned)threads);
     config.dynamicSmemBytes = shared;
     config.stream = stream;
     cudaLaunchAttribute attribute[1];
@@ -624,7 +747,7 @@ cudaError_t launch_topk_rows(const float* in, float* values, float* indices, siz
     attribute[0].val.clusterDim.z = 1;
     config.attrs = attribute;
     config.numAttrs = p.cluster > 1 ? 1 : 0;  // a row of one CTA is an ordinary launch
-    return largest ? cudaLaunchKernelEx(&config, topk_rows_kernel<true>, p) : cudaLaunchKernelEx(&config, topk_rows_kernel<false>, p);
+    return cudaLaunchKernelEx(&config, kernel, p);
 }
 
 }  // namespace psx
