@@ -10,19 +10,22 @@
 // HBM bound: K and V of every (batch, kv head) are read once, 8 * total * D bytes each.
 // One CTA of six warps takes one (batch, kv head) and one slice of the cached positions; the query
 // rows of the whole group -- group heads x L new positions, at most 8 -- are answered together, so
-// grouped-query heads share one pass over their K/V head.  A warp works through its positions 32 at a
+// grouped-query heads share one pass over their K/V head.  A warp works through its positions 32 (or 16) at a
 // time:
-//   - the K rows of a tile arrive in shared memory by bulk asynchronous copies (one 4*D-byte row per
-//     lane, completing on an mbarrier, no multicast), padded to D + 4 floats so that lanes reading
-//     different rows at the same offset fall into different banks; the next tile's rows are asked for as
-//     soon as this tile's scores are formed, and land under the softmax and the context;
-//   - lane t forms the dot products of position t with every query row (the query rows are read as
-//     broadcasts), scales and masks them;
-//   - the running maximum and sum of every query row are brought up to date (online softmax: what has
-//     been accumulated is rescaled when the maximum moves), the tile's probabilities go to shared memory;
+//   - the K rows of a tile arrive in shared memory by one bulk asynchronous copy (they are one contiguous run;
+//     it completes on an mbarrier, no multicast); the next tile's rows are asked for as soon as this tile's
+//     scores are formed, and land under the softmax and the context;
+//   - eight lanes (16 beyond a head dimension of 128) share a position: each holds its part of every query row in
+//     registers, multiplies it with its part of the K row, and an exchange that halves the number of rows a
+//     lane carries at every step adds the parts up.  (One lane per position, the query rows read as broadcasts, spent half of the
+//     shared-memory pipe on them: a 128-bit read takes four cycles also where all lanes read one address.)
+//   - lane t scales and masks position t's scores; the running maximum of every query row is brought up to date
+//     (online softmax: what has been accumulated is rescaled when the maximum moves), every lane keeps the sum of its own
+//     positions, the tile's probabilities go to shared memory;
 //   - lane c accumulates floats 4c .. 4c+3 of the context rows from the V rows (one contiguous run per
 //     tile, one bulk copy, asked for when the tile starts: it lands while the scores are formed).
-// One K tile and one V tile per warp (34 KB for a head dimension of 128) leave room for six warps per SM.
+// 64 x 8 kv heads of 128, four query rows each, 4001 positions: 420 us so, 363 now (5.8 TB/s).
+// One K tile and one V tile per warp (33 KB for a head dimension of 128) leave room for six warps per SM.
 // The warps' partial results (maximum, sum, unnormalised context) meet in shared memory; with several
 // slices per (batch, kv head) they go to scratch and a second kernel joins them.
 //
@@ -41,10 +44,10 @@ namespace psx {
 
 namespace {
 
-constexpr int kAttnWarps = 6;      // warps of a CTA up to a head dimension of 128 (34 KB of tiles each)
-constexpr int kAttnWarpsWide = 3;  // beyond it (67 KB each at 256)
-inline int attention_warps(int head_dim) { return head_dim > 128 ? kAttnWarpsWide : kAttnWarps; }
-constexpr int kTile = 32;          // positions per warp and tile: one per lane
+constexpr int kAttnWarps = 6;  // warps of a CTA: 33 KB of tiles each
+// Positions per warp and tile: one per lane up to a head dimension of 128, half as many beyond it (the tiles take the same room then;
+// three warps with whole tiles left the chip idle: 32 x 4 kv heads of 256, two query rows: 261 us).
+__host__ __device__ constexpr int attention_tile(bool wide) { return wide ? 16 : 32; }
 constexpr float kMasked = -FLT_MAX;  // std::numeric_limits<float>::lowest()
 
 // src/row_math.hpp:117-127 (i: new position, j: cached position, offset: positions cached before).
@@ -55,21 +58,23 @@ __device__ __forceinline__ bool masked(const float* keep_row, int64_t i, int64_t
 }
 
 // R: query rows answered together (group x L, padded to 1, 2, 4 or 8); C: float4 chunks of a
-// context row per lane (D <= 128 C); W: warps of a CTA.
-template <int R, int C, int W>
-__global__ void __launch_bounds__(W * 32) decode_attention_kernel(const AttentionParams p) {
-    constexpr int kAttnWarps = W, kAttnThreads = W * 32;
+// context row per lane (D <= 128 C).
+template <int R, int C>
+__global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(const AttentionParams p) {
+    constexpr int kAttnThreads = kAttnWarps * 32, kTile = attention_tile(C == 2);
+    constexpr int G = C == 1 ? 8 : 16, kParts = 4;  // lanes that share a position; float4 chunks of a row that each has at most
+    static_assert(G * kParts * 4 == 128 * C, "the lanes of a group cover a row");
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int D = p.head_dim, pitch = D + 4;
+    const int D = p.head_dim;
     const int rows = p.group * p.q_len;  // query rows of this kv head (<= R)
     // shared memory: the query rows; per warp a K tile, a V tile and the tile's probabilities; the warps'
     // maxima and sums.  (At the end a warp's partial context rows lie over its own K tile.)
-    const size_t per_warp = (size_t)kTile * pitch + (size_t)kTile * D + (size_t)kTile * R;
+    const size_t per_warp = (size_t)kTile * D * 2 + (size_t)kTile * R;
     float* s_q = reinterpret_cast<float*>(smem);                        // R x D
-    float* s_k = s_q + R * D + warp * per_warp;                         // 32 x (D + 4)
-    float* s_v = s_k + kTile * pitch;                                   // 32 x D
-    float* s_p = s_v + kTile * D;                                       // 32 x R
+    float* s_k = s_q + R * D + warp * per_warp;                         // kTile x D
+    float* s_v = s_k + kTile * D;                                  // kTile x D
+    float* s_p = s_v + kTile * D;                                       // kTile x R
     float* s_ml = s_q + R * D + kAttnWarps * per_warp;                  // warps x R x 2
     auto ctx_of_warp = [&](int w) { return s_q + R * D + w * per_warp; };  // R x D, over warp w's K tile
     __shared__ __align__(8) uint64_t s_bar[kAttnWarps][2];              // K, V
@@ -98,9 +103,24 @@ __global__ void __launch_bounds__(W * 32) decode_attention_kernel(const Attentio
     }
     __syncthreads();
 
+    // Positions before the oldest query's window are masked for every query, and a masked score's weight is exactly zero -- unless
+    // a query has nothing left at all: then its weights are equal over all positions.  With key padding that is ruled out by a
+    // position that is kept and lies in every query's window.  (32 x 8 kv heads, 8001 positions, a window of 1024: 420 -> 64 us.)
+    int64_t oldest = 0;
+    if (p.causal != 0 && p.window > 0) {
+        oldest = max((int64_t)0, p.offset - p.window + 1);
+        if (keep_row != nullptr && oldest > 0) {
+            bool kept = false;
+            for (int64_t j = max((int64_t)0, p.offset + p.q_len - p.window) + threadIdx.x; j <= p.offset; j += kAttnThreads) {
+                kept = kept || keep_row[j] != 0.0f;
+            }
+            if (__syncthreads_or(kept ? 1 : 0) == 0) oldest = 0;
+        }
+    }
+
     // this warp's positions: the split's share, cut into the warps' shares, in whole tiles
-    const int64_t per_split = (p.total + p.splits - 1) / p.splits;
-    const int64_t s0 = split * per_split, s1 = min(s0 + per_split, p.total);
+    const int64_t per_split = (p.total - oldest + p.splits - 1) / p.splits;
+    const int64_t s0 = oldest + split * per_split, s1 = min(s0 + per_split, p.total);
     const int64_t tiles_in_split = s1 > s0 ? (s1 - s0 + kTile - 1) / kTile : 0;
     const int64_t tiles_per_warp = (tiles_in_split + kAttnWarps - 1) / kAttnWarps;
     const int64_t t_begin = s0 + warp * tiles_per_warp * kTile, t_end = min(t_begin + tiles_per_warp * kTile, s1);
@@ -114,15 +134,26 @@ __global__ void __launch_bounds__(W * 32) decode_attention_kernel(const Attentio
             bulk_copy_to_shared(s_v, values + first * D, (uint32_t)count * (uint32_t)D * 4u, &s_bar[warp][1]);
         }
     };
-    auto fetch_tile = [&](int64_t tile) {  // lane t asks for the K row of position t
+    auto fetch_tile = [&](int64_t tile) {  // ... and so are the K rows
         const int64_t first = t_begin + tile * kTile;
         const int count = (int)min((int64_t)kTile, t_end - first);
-        if (lane == 0) barrier_expect_bytes(&s_bar[warp][0], (uint32_t)count * (uint32_t)D * 4u);
-        __syncwarp();
-        if (lane < count) {
-            bulk_copy_to_shared(s_k + (size_t)lane * pitch, keys + (first + lane) * D, (uint32_t)D * 4u, &s_bar[warp][0]);
+        if (lane == 0) {
+            barrier_expect_bytes(&s_bar[warp][0], (uint32_t)count * (uint32_t)D * 4u);
+            bulk_copy_to_shared(s_k, keys + first * D, (uint32_t)count * (uint32_t)D * 4u, &s_bar[warp][0]);
         }
     };
+
+    // this lane's chunks of the query rows: chunks g, g + G, ... (what lies beyond D is zero)
+    const int g = lane & (G - 1);
+    float4 q[R][kParts];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int c = 0; c < kParts; ++c) {
+            const int d = 4 * (g + G * c);
+            q[r][c] = d < D ? *reinterpret_cast<const float4*>(s_q + r * D + d) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
 
     float m_run[R], l_run[R];
     float4 ctx[R][C];
@@ -150,22 +181,45 @@ __global__ void __launch_bounds__(W * 32) decode_attention_kernel(const Attentio
         const int count = (int)min((int64_t)kTile, t_end - first);
         const int64_t pos = first + lane;
 
-        // ---- scores of position `pos` against every query row -----------------------------------------
-        float s[R];
+        // ---- scores: 32 / G positions at a time ---------------------------------------------------------------
+#pragma unroll 2
+        for (int it = 0; it < kTile * G / 32; ++it) {
+            const int t = it * (32 / G) + lane / G;
+            float even[R], odd[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) s[r] = 0.0f;
-        const float* krow = s_k + (size_t)lane * pitch;
-#pragma unroll 4
-        for (int d = 0; d < D; d += 4) {
-            const float4 k4 = *reinterpret_cast<const float4*>(krow + d);
+            for (int r = 0; r < R; ++r) even[r] = odd[r] = 0.0f;
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float4 q4 = *reinterpret_cast<const float4*>(s_q + r * D + d);  // the same address in every lane
-                s[r] = __fmaf_rn(q4.x, k4.x, s[r]);
-                s[r] = __fmaf_rn(q4.y, k4.y, s[r]);
-                s[r] = __fmaf_rn(q4.z, k4.z, s[r]);
-                s[r] = __fmaf_rn(q4.w, k4.w, s[r]);
+            for (int c = 0; c < kParts; ++c) {
+                const int d = 4 * (g + G * c);
+                if (d >= D) break;
+                const float4 k4 = *reinterpret_cast<const float4*>(s_k + (size_t)t * D + d);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    fma_pair(even[r], odd[r], q[r][c].x, q[r][c].y, k4.x, k4.y, even[r], odd[r]);
+                    fma_pair(even[r], odd[r], q[r][c].z, q[r][c].w, k4.z, k4.w, even[r], odd[r]);
+                }
             }
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < R; ++r) even[r] += odd[r];
+            int carried = R;  // rows whose sums this lane still carries
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) {
+                if (carried > 1) {
+                    carried /= 2;
+                    const bool upper = (lane & o) != 0;
+#pragma unroll
+                    for (int i = 0; i < R / 2; ++i) {
+                        if (i < carried) {
+                            const float given = upper ? even[i] : even[i + carried], kept = upper ? even[i + carried] : even[i];
+                            even[i] = kept + __shfl_xor_sync(0xFFFFFFFFu, given, o);
+                        }
+                    }
+                } else {
+                    even[0] += __shfl_xor_sync(0xFFFFFFFFu, even[0], o);
+                }
+            }
+            if (g % (G / R) == 0) s_p[t * R + g / (G / R)] = even[0];
         }
         // The K tile is done with: the next tile's rows can land under the rest of this tile's work.
         __syncwarp();
@@ -175,6 +229,9 @@ __global__ void __launch_bounds__(W * 32) decode_attention_kernel(const Attentio
             issued = tile + 1;
         }
         // ---- scale, mask, and the running softmax of every query row ------------------------------------
+        float s[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) s[r] = lane < kTile ? s_p[lane * R + r] : 0.0f;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             float x = kMasked;
@@ -186,17 +243,17 @@ __global__ void __launch_bounds__(W * 32) decode_attention_kernel(const Attentio
             const float tile_max = warp_max(counts ? x : kMasked);
             const float m_new = fmaxf(m_run[r], tile_max);
             const float e = counts ? __expf(x - m_new) : 0.0f;
-            float e_sum = e;
+            if (m_new > m_run[r]) {  // (the same in every lane)
+                const float rescale = __expf(m_run[r] - m_new);  // 0 from the very first tile
+                l_run[r] *= rescale;
+                m_run[r] = m_new;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) e_sum += __shfl_xor_sync(0xFFFFFFFFu, e_sum, o);
-            const float rescale = __expf(m_run[r] - m_new);  // 1 when the maximum stays; 0 from the very first tile
-            l_run[r] = __fmaf_rn(l_run[r], rescale, e_sum);
-            m_run[r] = m_new;
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                ctx[r][c].x *= rescale; ctx[r][c].y *= rescale; ctx[r][c].z *= rescale; ctx[r][c].w *= rescale;
+                for (int c = 0; c < C; ++c) {
+                    ctx[r][c].x *= rescale; ctx[r][c].y *= rescale; ctx[r][c].z *= rescale; ctx[r][c].w *= rescale;
+                }
             }
-            s_p[lane * R + r] = e;
+            l_run[r] += e;
+            if (lane < kTile) s_p[lane * R + r] = e;
         }
         __syncwarp();
         // ---- context: lane c owns floats 4c .. 4c + 3 of every row; the V tile has had the scores' time to land ----
@@ -216,10 +273,8 @@ __global__ void __launch_bounds__(W * 32) decode_attention_kernel(const Attentio
                 const float pr = s_p[t * R + r];  // the same address in every lane
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
-                    ctx[r][c].x = __fmaf_rn(pr, v4[c].x, ctx[r][c].x);
-                    ctx[r][c].y = __fmaf_rn(pr, v4[c].y, ctx[r][c].y);
-                    ctx[r][c].z = __fmaf_rn(pr, v4[c].z, ctx[r][c].z);
-                    ctx[r][c].w = __fmaf_rn(pr, v4[c].w, ctx[r][c].w);
+                    fma_pair(ctx[r][c].x, ctx[r][c].y, pr, pr, v4[c].x, v4[c].y, ctx[r][c].x, ctx[r][c].y);
+                    fma_pair(ctx[r][c].z, ctx[r][c].w, pr, pr, v4[c].z, v4[c].w, ctx[r][c].z, ctx[r][c].w);
                 }
             }
         }
@@ -236,9 +291,12 @@ __global__ void __launch_bounds__(W * 32) decode_attention_kernel(const Attentio
             const int d = 4 * (lane + 32 * c);
             if (warp_landed && d < D) *reinterpret_cast<float4*>(ctx_of_warp(warp) + (size_t)r * D + d) = ctx[r][c];
         }
+        float l = l_run[r];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, o);
         if (lane == 0) {
             s_ml[(warp * R + r) * 2] = m_run[r];
-            s_ml[(warp * R + r) * 2 + 1] = l_run[r];
+            s_ml[(warp * R + r) * 2 + 1] = l;
         }
     }
     const int timed_out = __syncthreads_or(landed ? 0 : 1);
@@ -250,7 +308,7 @@ __global__ void __launch_bounds__(W * 32) decode_attention_kernel(const Attentio
         }
         return;
     }
-    // thread (r, d): joins the four warps' row r at column d
+    // thread (r, d): joins the warps' row r at column d
     for (int i = threadIdx.x; i < rows * D; i += kAttnThreads) {
         const int r = i / D, d = i % D;
         float m = kMasked;
@@ -304,15 +362,15 @@ __global__ void join_attention_splits_kernel(const AttentionParams p) {
     p.context[i] = l > 0.0f ? __fdiv_rn(acc, l) : 0.0f;
 }
 
-template <int R, int C, int W>
+template <int R, int C>
 cudaError_t launch_one(const AttentionParams& p, size_t shared, cudaStream_t stream) {
     static bool configured = false;  // (per instantiation; raising the limit twice is harmless)
     if (!configured) {
-        const cudaError_t e = allow_all_dynamic_shared(decode_attention_kernel<R, C, W>);
+        const cudaError_t e = allow_all_dynamic_shared(decode_attention_kernel<R, C>);
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    decode_attention_kernel<R, C, W><<<dim3((unsigned)(p.batch * p.kv_heads), (unsigned)p.splits), W * 32, shared, stream>>>(p);
+    decode_attention_kernel<R, C><<<dim3((unsigned)(p.batch * p.kv_heads), (unsigned)p.splits), kAttnWarps * 32, shared, stream>>>(p);
     return cudaGetLastError();
 }
 
@@ -321,9 +379,8 @@ cudaError_t launch_one(const AttentionParams& p, size_t shared, cudaStream_t str
 int attention_rows_padded(int rows) { return rows <= 1 ? 1 : rows <= 2 ? 2 : rows <= 4 ? 4 : 8; }
 
 size_t attention_shared_bytes(int rows_padded, int head_dim) {
-    const size_t per_warp = (size_t)kTile * (head_dim + 4) + (size_t)kTile * head_dim + (size_t)kTile * rows_padded;
-    const size_t warps = (size_t)attention_warps(head_dim);
-    const size_t floats = (size_t)rows_padded * head_dim + warps * per_warp + warps * rows_padded * 2;
+    const size_t tile = (size_t)attention_tile(head_dim > 128), per_warp = tile * head_dim * 2 + tile * rows_padded;
+    const size_t floats = (size_t)rows_padded * head_dim + kAttnWarps * per_warp + kAttnWarps * rows_padded * 2;
     return floats * sizeof(float);
 }
 
@@ -332,7 +389,7 @@ int attention_splits(int64_t batch_kv, int64_t total, int sm_count, int head_dim
     // is as full as the others (512 CTAs on 148 SMs are 3.46 rounds, i.e. four, an eighth of the time idle;
     // 1024 are 6.92), with at least two tiles per warp in a slice, and only when that wins a few per cent (the
     // slices cost a second kernel).
-    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(128, total / (2 * attention_warps(head_dim) * kTile)));
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(128, total / (2 * kAttnWarps * attention_tile(head_dim > 128))));
     auto filled = [&](int64_t ctas) { return (double)ctas / (double)(((ctas + sm_count - 1) / sm_count) * sm_count); };
     int best = 1;
     double best_fill = filled(batch_kv);
@@ -353,13 +410,13 @@ cudaError_t launch_decode_attention(const AttentionParams& p, cudaStream_t strea
     if (rows < 1 || rows > 8 || p.head_dim % 4 != 0 || p.head_dim > 256 || p.head_dim < 4) return cudaErrorInvalidValue;
     const int R = attention_rows_padded(rows);
     const size_t shared = attention_shared_bytes(R, p.head_dim);
-    const bool wide = p.head_dim > 128;  // two chunks of a context row per lane, three warps per CTA
+    const bool wide = p.head_dim > 128;  // two chunks of a context row per lane, tiles of 16 positions
     cudaError_t e;
     switch (R) {
-        case 1: e = wide ? launch_one<1, 2, kAttnWarpsWide>(p, shared, stream) : launch_one<1, 1, kAttnWarps>(p, shared, stream); break;
-        case 2: e = wide ? launch_one<2, 2, kAttnWarpsWide>(p, shared, stream) : launch_one<2, 1, kAttnWarps>(p, shared, stream); break;
-        case 4: e = wide ? launch_one<4, 2, kAttnWarpsWide>(p, shared, stream) : launch_one<4, 1, kAttnWarps>(p, shared, stream); break;
-        default: e = wide ? launch_one<8, 2, kAttnWarpsWide>(p, shared, stream) : launch_one<8, 1, kAttnWarps>(p, shared, stream); break;
+        case 1: e = wide ? launch_one<1, 2>(p, shared, stream) : launch_one<1, 1>(p, shared, stream); break;
+        case 2: e = wide ? launch_one<2, 2>(p, shared, stream) : launch_one<2, 1>(p, shared, stream); break;
+        case 4: e = wide ? launch_one<4, 2>(p, shared, stream) : launch_one<4, 1>(p, shared, stream); break;
+        default: e = wide ? launch_one<8, 2>(p, shared, stream) : launch_one<8, 1>(p, shared, stream); break;
     }
     if (e != cudaSuccess || p.splits == 1) return e;
     const int64_t elements = p.batch * p.heads * p.q_len * p.head_dim;
