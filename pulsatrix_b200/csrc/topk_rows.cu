@@ -197,13 +197,21 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
             bulk_copy_to_shared(held4 + first, src4 + first, bytes, &s_bar[tid]);
         }
     }
+    // The held slice is padded to whole trips of the block with what nothing ranks below, so that the sweeps need no bounds.
+    const uint32_t trips = (vectors + kThreads - 1) / kThreads;
+    if (kHeld && vectors != trips * kThreads && (trips - 1) * kThreads + tid >= vectors) {
+        const float worst = kLargest ? -INFINITY : INFINITY;
+        held4[(trips - 1) * kThreads + tid] = make_float4(worst, worst, worst, worst);
+    }
     // The cluster's barrier costs about a microsecond; one CTA on its own meets with the block barrier.
     auto meet = [&]() {
         if (ranks > 1) cluster.sync(); else __syncthreads();
     };
 
-    for (int i = tid; i < 2 * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
-    for (uint32_t i = tid; i < 2 * p.list_cap; i += kThreads) list_key[i] = 0;
+    for (uint32_t i = tid; i < p.list_cap / 2; i += kThreads) reinterpret_cast<uint4*>(list_key)[i] = make_uint4(0, 0, 0, 0);  // (claimed, too)
+    if (p.list_cap == 0) {
+        for (int i = tid; i < 2 * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
+    }
     if (tid == 0) {
         s_collected = 0;
         s_listed = 0;
@@ -231,13 +239,15 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
         };
         for (uint32_t i = tid; i < head; i += kThreads) note(src[i]);
         if (kHeld) {
+            constexpr uint32_t kTripsOfChunk = kHeldChunk / kThreads;
             for (uint32_t c = 0; c * kHeldChunk < vectors; ++c) {
                 landed = barrier_wait_bounded(&s_bar[c], 0, p.wait_limit_ns) && landed;
-                const uint32_t stop = min(vectors, (c + 1) * kHeldChunk);
+                const float4* const mine4 = held4 + c * kHeldChunk + tid;
+                if ((c + 1) * kTripsOfChunk <= trips) {
 #pragma unroll
-                for (uint32_t q = 0; q < kHeldChunk / kThreads; ++q) {
-                    const uint32_t v = c * kHeldChunk + q * kThreads + tid;
-                    if (v < stop) note4(held4[v]);
+                    for (uint32_t q = 0; q < kTripsOfChunk; ++q) note4(mine4[q * kThreads]);
+                } else {
+                    for (uint32_t q = 0; c * kTripsOfChunk + q < trips; ++q) note4(mine4[q * kThreads]);
                 }
             }
         } else {
@@ -303,42 +313,23 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
                 if (reaches(src[i])) put(src[i], begin + i);
             }
             if (kHeld) {
-                // branch-free over the vectors, one bit for each that reaches the bound; then a warp's slots at once
-                uint32_t noted = 0, count = 0;
-#pragma unroll 4
-                for (uint32_t t = 0; t * kThreads < vectors; ++t) {
-                    const uint32_t v = t * kThreads + tid;
-                    const float4 d = held4[min(v, vectors - 1)];
+                // branch-free over the vectors, one bit for each that reaches the bound
+                uint32_t noted = 0;
+                const float4* const mine4 = held4 + tid;
+#pragma unroll 8
+                for (uint32_t t = 0; t < trips; ++t) {
+                    const float4 d = mine4[t * kThreads];
                     const float best4 = largest ? max3_nan(max3_nan(d.x, d.y, d.z), d.w, d.w) : min3(min3(d.x, d.y, d.z), d.w, d.w);
-                    if (reaches(best4) && v < vectors) noted |= 1u << t;
+                    if (reaches(best4)) noted |= 1u << t;
                 }
-                auto hits_of = [&](const float4& d) {
-                    return (reaches(d.x) ? 1u : 0u) | (reaches(d.y) ? 2u : 0u) | (reaches(d.z) ? 4u : 0u) | (reaches(d.w) ? 8u : 0u);
-                };
-                for (uint32_t m = noted; m != 0; m &= m - 1) count += __popc(hits_of(held4[(__ffs(m) - 1) * kThreads + tid]));
-                uint32_t incl = count;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                    if (lane >= o) incl += up;
-                }
-                uint32_t slot = 0;
-                if (lane == 31 && incl != 0) slot = atomicAdd(&s_listed, incl);
-                slot = __shfl_sync(0xFFFFFFFFu, slot, 31) + incl - count;
+                if (trips * kThreads - kThreads + tid >= vectors) noted &= ~(1u << ((trips - 1) & 31));  // padding
                 for (uint32_t m = noted; m != 0; m &= m - 1) {
                     const uint32_t v = (__ffs(m) - 1) * kThreads + tid, col = begin + head + 4 * v;
                     const float4 d = held4[v];
-                    const float x[4] = {d.x, d.y, d.z, d.w};
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q) {
-                        if (!reaches(x[q])) continue;
-                        if (slot < p.list_cap) {
-                            const uint32_t key = rank_key(x[q], largest);
-                            list[slot] = ((u64)key << 32) | (uint32_t)~(col + q);
-                            list_key[slot] = key;
-                        }
-                        ++slot;
-                    }
+                    if (reaches(d.x)) put(d.x, col);
+                    if (reaches(d.y)) put(d.y, col + 1);
+                    if (reaches(d.z)) put(d.z, col + 2);
+                    if (reaches(d.w)) put(d.w, col + 3);
                 }
             } else
             for (uint32_t v0 = tid; v0 < vectors; v0 += kBatch * kThreads) {
@@ -395,6 +386,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
             bool tied = false;
             for (uint32_t first = 0; first < on_list; first += per_round) {
                 const uint32_t i = first + (uint32_t)tid / share;
+                if (first + (uint32_t)(tid & ~31) / share >= on_list) break;  // (nothing for this warp)
                 const uint32_t key = i < on_list ? list_key[i] : ~0u;
                 uint32_t place = 0;
 #pragma unroll 4
@@ -453,7 +445,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
             }
         }
         if (tid == 0) s_listed = 0;
-        __syncthreads();
+        for (int i = tid; i < 2 * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
+        meet();  // (the cluster adds its histograms up)
     }
 
     // ---- the slice as keys in shared memory, for the long way ----------------------------------------------
@@ -716,12 +709,12 @@ cudaError_t launch_topk_rows(const float* in, float* values, float* indices, siz
                   entries * 8 + (size_t)p.slice * 4 + 4096 <= 227 * 1024 ? 1 : 0;
     p.wait_limit_ns = kDefaultWaitLimitNs;
     const bool held = p.list_cap != 0 && p.slice <= kHeldMax;
-    const int threads = !held || k > 64 ? kWidest : p.slice <= 4096 && k <= 32 ? 64 : 128;
+    const int threads = !held || k > 32 ? kWidest : p.slice <= 4096 && k <= 32 ? 64 : 128;
     auto kernel = largest ? topk_rows_kernel<true, false, kWidest> : topk_rows_kernel<false, false, kWidest>;
     if (held && threads == 64) kernel = largest ? topk_rows_kernel<true, true, 64> : topk_rows_kernel<false, true, 64>;
     else if (held && threads == 128) kernel = largest ? topk_rows_kernel<true, true, 128> : topk_rows_kernel<false, true, 128>;
     else if (held) kernel = largest ? topk_rows_kernel<true, true, kWidest> : topk_rows_kernel<false, true, kWidest>;
-    const size_t shared = entries * 8 + (p.in_shared || held ? (size_t)p.slice * 4 + 32 : 0);
+    const size_t shared = entries * 8 + (p.in_shared ? (size_t)p.slice * 4 + 32 : held ? (p.slice / 4 + threads - 1) / threads * threads * 16 + 32 : 0);
     if (rows * (size_t)p.cluster > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
     if (shared > 48 * 1024) {
         // Once per device and kernel (the call sets the same value every time, so two host threads
