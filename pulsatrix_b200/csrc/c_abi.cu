@@ -50,6 +50,8 @@ struct Buffer {
 // Page-locked staging for rows that lie in ordinary host memory: eight slots of 256 KB.
 constexpr int kRingSlots = 8;
 constexpr size_t kRingSlotBytes = 256 << 10;
+constexpr size_t kLeadBytes = 16 << 10;      // small inputs that travel with the first piece
+constexpr size_t kResultsInPlace = 16 << 10;  // results up to this size are written straight to page-locked host memory
 
 }  // namespace
 
@@ -126,10 +128,13 @@ bool copy_engine_reaches(const void* host) {
 // Rows between host and device, packed on the device (stride = vocab) whatever the host stride is.  Page-locked rows are
 // one copy.  From ordinary memory the driver would copy through a staging buffer of its own, the call waiting for it, and
 // only then start; here the copy into page-locked memory runs in pieces, each on its way to the device while the next one is
-// made: one row of 128,256 logits 94 -> 45 us.  Pieces of a quarter of the rows, 64 to 256 KB: smaller ones cost more calls
-// than they overlap.  The caller synchronises the stream before the ring is used again.
+// made.  Pieces of half the rows, 64 to 256 KB: smaller ones cost more calls than they overlap (one row of 128,256 logits to its
+// token: 67.7 us in quarters, 62.8 in halves; a kernel that reads the page-locked memory across the bus takes as long as the
+// copy engine).  The caller synchronises the stream before the ring is used again.
+// lead: bytes that travel ahead of the rows in the first piece (from lead_from, to the `lead` bytes before `device`); ordinary
+// memory to the device only, at most kLeadBytes.
 psx_status copy_rows(psx_ctx* ctx, cudaStream_t stream, float* device, float* host, int64_t rows, int64_t vocab, int64_t row_stride,
-                     bool to_device) {
+                     bool to_device, const void* lead_from = nullptr, size_t lead = 0) {
     const size_t row_bytes = (size_t)vocab * sizeof(float), total = (size_t)rows * row_bytes;
     const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
     if (copy_engine_reaches(host)) {
@@ -143,13 +148,13 @@ psx_status copy_rows(psx_ctx* ctx, cudaStream_t stream, float* device, float* ho
         }
         return PSX_OK;
     }
-    if (psx_status s = reserve_pinned(ctx->pinned_ring, kRingSlots * kRingSlotBytes)) return s;
+    if (psx_status s = reserve_pinned(ctx->pinned_ring, kLeadBytes + kRingSlots * kRingSlotBytes)) return s;
     for (cudaEvent_t& e : ctx->ring_done) {
         if (e == nullptr) PSX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
-    const size_t piece = std::min(kRingSlotBytes, std::max<size_t>(64 << 10, (total / 4 + 4095) / 4096 * 4096));
+    const size_t piece = std::min(kRingSlotBytes, std::max<size_t>(64 << 10, (total / 2 + 4095) / 4096 * 4096));
     const size_t pieces = (total + piece - 1) / piece;
-    char* const ring = static_cast<char*>(ctx->pinned_ring.ptr);
+    char* const ring = static_cast<char*>(ctx->pinned_ring.ptr) + kLeadBytes;
     auto between_host_and_slot = [&](size_t i) {  // piece i of the packed rows, row by row where the host's are apart
         char* slot = ring + (i % kRingSlots) * kRingSlotBytes;
         for (size_t at = i * piece, end = std::min(total, at + piece); at < end;) {
@@ -169,7 +174,13 @@ psx_status copy_rows(psx_ctx* ctx, cudaStream_t stream, float* device, float* ho
         if (to_device) between_host_and_slot(i);
         char* slot = ring + (i % kRingSlots) * kRingSlotBytes;
         char* there = reinterpret_cast<char*>(device) + i * piece;
-        const size_t n = std::min(piece, total - i * piece);
+        size_t n = std::min(piece, total - i * piece);
+        if (i == 0 && lead != 0) {  // (a slot has this room before it)
+            slot -= lead;
+            there -= lead;
+            n += lead;
+            std::memcpy(slot, lead_from, lead);
+        }
         PSX_CUDA(cudaMemcpyAsync(to_device ? there : slot, to_device ? slot : there, n, kind, stream));
         if (!to_device || pieces > kRingSlots) PSX_CUDA(cudaEventRecord(ctx->ring_done[i % kRingSlots], stream));
     }
@@ -182,23 +193,34 @@ struct HostInputs {
     const int64_t* history = nullptr;
     const double* uniforms = nullptr;
 };
+// lead given: the inputs will travel ahead of the rows (copy_rows' lead) when they fit kLeadBytes; `lead` says how many bytes of
+// pinned_inputs do (0: they have been sent on their way here), and the device's copy lies that far before device_rows.
 psx_status upload_inputs(psx_ctx* ctx, cudaStream_t stream, int64_t rows, const int64_t* history_ids, const int64_t* history_offsets,
-                         const double* uniforms, HostInputs& out) {
+                         const double* uniforms, HostInputs& out, const void* device_rows = nullptr, size_t* lead = nullptr) {
     const bool with_history = history_ids && history_offsets;
     const size_t history = with_history ? (size_t)std::max<int64_t>(history_offsets[rows], 0) : 0;
     const size_t offset_words = with_history ? (size_t)rows + 1 : 0, uniform_words = uniforms ? (size_t)rows : 0;
     const size_t words = offset_words + history + uniform_words;
     if (words == 0) return PSX_OK;
-    if (psx_status s = reserve(ctx->h_inputs, words * 8)) return s;
-    if (psx_status s = reserve_pinned(ctx->pinned_inputs, words * 8)) return s;
+    const size_t padded = (words * 8 + 255) / 256 * 256;
+    const bool leads = lead != nullptr && padded <= kLeadBytes;
+    if (!leads) {
+        if (psx_status s = reserve(ctx->h_inputs, words * 8)) return s;
+    }
+    if (psx_status s = reserve_pinned(ctx->pinned_inputs, padded)) return s;
     int64_t* packed = static_cast<int64_t*>(ctx->pinned_inputs.ptr);
     if (with_history) {
         std::memcpy(packed, history_offsets, offset_words * 8);
         std::memcpy(packed + offset_words, history_ids, history * 8);
     }
     if (uniforms) std::memcpy(packed + offset_words + history, uniforms, uniform_words * 8);
-    PSX_CUDA(cudaMemcpyAsync(ctx->h_inputs.ptr, packed, words * 8, cudaMemcpyHostToDevice, stream));
     const int64_t* device = static_cast<const int64_t*>(ctx->h_inputs.ptr);
+    if (leads) {
+        *lead = padded;
+        device = reinterpret_cast<const int64_t*>(static_cast<const char*>(device_rows) - padded);
+    } else {
+        PSX_CUDA(cudaMemcpyAsync(ctx->h_inputs.ptr, packed, words * 8, cudaMemcpyHostToDevice, stream));
+    }
     if (with_history) {
         out.offsets = device;
         out.history = device + offset_words;
@@ -666,13 +688,21 @@ psx_status psx_b200_sample_rows_host(psx_ctx* ctx, const float* logits, int64_t 
 
     // The results in one piece: tokens, diagnostics, log-probs, statuses.
     const size_t n = (size_t)rows, diag_bytes = diag ? n * sizeof(psx_row_diag) : 0, result_bytes = 8 * n + diag_bytes + 8 * n;
-    if (psx_status s = reserve(ctx->h_logits, n * vocab * sizeof(float))) return s;
+    if (psx_status s = reserve(ctx->h_logits, kLeadBytes + n * vocab * sizeof(float))) return s;
     if (psx_status s = reserve(ctx->h_results, result_bytes)) return s;
     if (psx_status s = reserve_pinned(ctx->pinned_results, result_bytes)) return s;
-    float* const device_rows = static_cast<float*>(ctx->h_logits.ptr);
+    float* const device_rows = reinterpret_cast<float*>(static_cast<char*>(ctx->h_logits.ptr) + kLeadBytes);
     HostInputs in;
-    if (psx_status s = upload_inputs(ctx, stream, rows, history_ids, history_offsets, config->do_sample ? uniforms : nullptr, in)) return s;
-    if (psx_status s = copy_rows(ctx, stream, device_rows, const_cast<float*>(logits), rows, vocab, row_stride, /*to_device=*/true)) return s;
+    size_t lead = 0;
+    const bool staged = !copy_engine_reaches(logits);
+    if (psx_status s = upload_inputs(ctx, stream, rows, history_ids, history_offsets, config->do_sample ? uniforms : nullptr, in, device_rows,
+                                     staged ? &lead : nullptr)) {
+        return s;
+    }
+    if (psx_status s = copy_rows(ctx, stream, device_rows, const_cast<float*>(logits), rows, vocab, row_stride, /*to_device=*/true,
+                                 ctx->pinned_inputs.ptr, lead)) {
+        return s;
+    }
     // The staged inputs are being copied in by the transfers just enqueued: no promise holds for them.
     struct RestorePromise {
         psx_ctx* ctx;
@@ -680,7 +710,11 @@ psx_status psx_b200_sample_rows_host(psx_ctx* ctx, const float* logits, int64_t 
         ~RestorePromise() { ctx->inputs_ready = saved; }
     } restore{ctx, ctx->inputs_ready};
     ctx->inputs_ready = false;
-    char* const results = static_cast<char*>(ctx->h_results.ptr);
+    // A few results: the kernels write them to the page-locked host memory themselves (it has the same address on the device), which saves
+    // a copy behind them.
+    char* const arrived = static_cast<char*>(ctx->pinned_results.ptr);
+    const bool in_place = result_bytes <= kResultsInPlace;
+    char* const results = in_place ? arrived : static_cast<char*>(ctx->h_results.ptr);
     auto tokens_in = [](char* block) { return reinterpret_cast<int64_t*>(block); };
     auto diag_in = [&](char* block) { return reinterpret_cast<psx_row_diag*>(block + 8 * n); };
     auto log_probs_in = [&](char* block) { return reinterpret_cast<float*>(block + 8 * n + diag_bytes); };
@@ -690,8 +724,7 @@ psx_status psx_b200_sample_rows_host(psx_ctx* ctx, const float* logits, int64_t 
                                             diag ? diag_in(results) : nullptr)) {
         return s;
     }
-    char* const arrived = static_cast<char*>(ctx->pinned_results.ptr);
-    PSX_CUDA(cudaMemcpyAsync(arrived, results, result_bytes, cudaMemcpyDeviceToHost, stream));
+    if (!in_place) PSX_CUDA(cudaMemcpyAsync(arrived, results, result_bytes, cudaMemcpyDeviceToHost, stream));
     PSX_CUDA(cudaStreamSynchronize(stream));
     std::memcpy(tokens, tokens_in(arrived), 8 * n);
     std::memcpy(log_probs, log_probs_in(arrived), 4 * n);
