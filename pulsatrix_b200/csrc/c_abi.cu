@@ -399,7 +399,7 @@ psx_status plan_row_pass(psx_ctx* ctx, cudaStream_t stream, const float* logits,
                          int64_t row_stride, const int64_t* history_ids, const int64_t* history_offsets,
                          const psx_sampling_config* config, Plan& plan, psx::ScanParams& sp, bool alternate = false) {
     PSX_CUDA(cudaSetDevice(ctx->device));
-    plan = psx::make_plan(logits, vocab, row_stride, vocab, config);
+    plan = psx::make_plan(logits, rows, vocab, row_stride, vocab, config, ctx->sm_count);
     sp = psx::ScanParams{};
     sp.logits = logits;
     sp.row_stride = row_stride;
@@ -780,7 +780,7 @@ psx_status shard_scan_impl(psx_ctx* ctx, void* stream_ptr, const float* shard_lo
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     PSX_CUDA(cudaSetDevice(ctx->device));
 
-    const Plan plan = psx::make_plan(shard_logits, shard_cols, row_stride, vocab, config);
+    const Plan plan = psx::make_plan(shard_logits, rows, shard_cols, row_stride, vocab, config, ctx->sm_count);
     psx::ScanParams sp{};
     sp.logits = shard_logits;
     sp.row_stride = row_stride;

@@ -53,11 +53,14 @@ __global__ void __launch_bounds__(kMergeThreads, kKind == survivor::kListNucleus
         if (threadIdx.x == 0) s_arrived = wait_until_at_least(p.arrivals + row, p.arrivals_target, p.arrivals_wait_ns) ? 1 : 0;
         __syncthreads();
         arrived = s_arrived != 0;
-    } else {
+    }
+    auto ready = [&]() {
+        if (p.arrivals != nullptr) return;
         grid_dependency_wait();        // everything this kernel reads was written by the kernel before it
         grid_dependents_may_launch();  // a row pass that follows reads none of this kernel's results
         PSX_MERGE_TIME(1);
-    }
+    };
+    if (p.general == 2) ready();
     if (!arrived) {
         if (threadIdx.x == 0) {
             p.tokens[row] = -1;
@@ -65,7 +68,7 @@ __global__ void __launch_bounds__(kMergeThreads, kKind == survivor::kListNucleus
             p.row_status[row] = PSX_ROW_DEVICE_TIMEOUT;
             if (p.diag) p.diag[row] = psx_row_diag{0, 0, INFINITY, INFINITY};
         }
-    } else if (p.general == 2 || !survivor::list_row<kKind>(p, row, survivor::view_of_row(p, row), dyn)) {
+    } else if (p.general == 2 || !survivor::list_row<kKind>(p, row, survivor::view_of_row(p, row), dyn, ready)) {
         __syncthreads();
         if (p.general != 2) survivor::merge_row(p, row, dyn);  // too many for the list, or a decision too close to its level
         if (p.general != 0 && p.logits != nullptr) {

@@ -37,7 +37,7 @@ struct RowView {
     const char *stats, *counts, *lists;
     int64_t stats_stride, count_stride, list_stride;  // from part to part
     int32_t cap;                                      // slots of a part's list
-    double u;
+    const double* u;
     int64_t* token;
     float* log_prob;
     int32_t* status;
@@ -53,7 +53,7 @@ __device__ __forceinline__ RowView view_of_row(const MergeParams& p, const int64
     v.count_stride = p.count_part_stride;
     v.list_stride = p.cand_part_stride;
     v.cap = p.part_cap;
-    v.u = p.do_sample && p.uniforms ? p.uniforms[row] : 0.5;
+    v.u = p.uniforms ? p.uniforms + row : nullptr;
     v.token = p.tokens + row;
     v.log_prob = p.log_probs + row;
     v.status = p.row_status + row;
@@ -76,10 +76,10 @@ struct ChunkWalk {
 
     __device__ __forceinline__ ChunkWalk(const MergeParams& p, const RowView& v)
         : lists(v.lists), stride(v.list_stride), parts(p.parts), cap(v.cap), lane(threadIdx.x & 31) {
-        const int warp = threadIdx.x >> 5;
-        chunk = warp / parts;
-        part = warp - chunk * parts;
-        step_chunk = kListWarps / parts;
+        const uint32_t warp = threadIdx.x >> 5, per_part = (0x10000u + parts - 1) / (uint32_t)parts;  // (x * per_part) >> 16 == x / parts for x <= 8
+        chunk = (int)((warp * per_part) >> 16);
+        part = (int)warp - chunk * parts;
+        step_chunk = (int)((kListWarps * per_part) >> 16);
         step_part = kListWarps - step_chunk * parts;
     }
     // where[q]: part | first slot << 8 (slots beyond the list's count are fetched as well, and not looked at)
@@ -182,7 +182,8 @@ __device__ __forceinline__ u64 lanes_before(u64 v, int lane, u64& all) {
 }
 
 // ---- greedy ----------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool list_greedy(const MergeParams& p, const RowView& v) {
+template <class Ready>
+__device__ __forceinline__ bool list_greedy(const MergeParams& p, const RowView& v, Ready ready) {
     __shared__ u64 s_z[kListWarps], s_best[kListWarps];
     __shared__ double s_tails;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -190,6 +191,7 @@ __device__ __forceinline__ bool list_greedy(const MergeParams& p, const RowView&
     uint2 c[4];
     uint32_t where[4];
     ChunkWalk walk(p, v);
+    ready();
     load_parts(p, v, j);
     walk.fetch(c, where);
     if (!join_parts(v, j)) return false;
@@ -244,7 +246,8 @@ __device__ __forceinline__ bool list_greedy(const MergeParams& p, const RowView&
 }
 
 // ---- sampling under a top-k ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn) {
+template <class Ready>
+__device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn, Ready ready) {
     ulonglong2* const s_list = reinterpret_cast<ulonglong2*>(dyn);       // (ordered value << 32) | column; units of 2^-52
     uint32_t* const s_by_value = reinterpret_cast<uint32_t*>(s_list + kListCap);  // place by column << 16 | entry
     uint32_t* const s_by_column = s_by_value + kListCap;                          // entry, kRemoved
@@ -262,12 +265,13 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
     uint2 c[4];
     uint32_t where[4];
     ChunkWalk walk(p, v);
-    load_parts(p, v, j);
-    walk.fetch(c, where);
-    const double u = v.u;
+    const double power = exp_power_of_lane();
     if (tid < 32) s_hist[tid] = 0;
     if (tid == 0) { s_wide_n = 0; s_n = 0; s_doubt = 0; s_won = 0; s_survivors = 0; }
-    const double power = exp_power_of_lane();
+    ready();
+    load_parts(p, v, j);
+    walk.fetch(c, where);
+    const double u = v.u ? *v.u : 0.5;
     __syncthreads();
     if (!join_parts(v, j)) return false;
     if (settle_bad_row(v, j)) return true;
@@ -522,7 +526,8 @@ struct RangeSums {
     }
 };
 
-__device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn) {
+template <class Ready>
+__device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn, Ready ready) {
     ulonglong2* const s_list = reinterpret_cast<ulonglong2*>(dyn);
     float* const s_raw = reinterpret_cast<float*>(s_list + kListCap);
     uint32_t* const s_by_value = reinterpret_cast<uint32_t*>(s_raw + kListCap);  // masses over 256 ranges of the value
@@ -543,12 +548,13 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
     uint2 c[4];
     uint32_t where[4];
     ChunkWalk walk(p, v);
-    load_parts(p, v, j);
-    walk.fetch(c, where);
-    const double u = v.u;
+    const double power = exp_power_of_lane();
     reinterpret_cast<uint4*>(s_by_value)[tid] = make_uint4(0, 0, 0, 0);  // both histograms
     if (tid == 0) { s_n = 0; s_cut_n = 0; s_draw_n = 0; s_decided = 0; s_survivors = 0; s_doubt = 0; s_cut_key = ~0ull; s_margin = ~0ull; }
-    const double power = exp_power_of_lane();
+    ready();
+    load_parts(p, v, j);
+    walk.fetch(c, where);
+    const double u = v.u ? *v.u : 0.5;
     __syncthreads();
     if (!join_parts(v, j)) return false;
     if (settle_bad_row(v, j)) return true;
@@ -789,12 +795,17 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
 
 enum ListKind { kListGreedy, kListTopK, kListNucleus };
 
-template <int kKind>
-__device__ __forceinline__ bool list_row(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn) {
-    if (p.parts > 32) return false;  // (a record per lane)
-    if (kKind == kListGreedy) return p.survivor_cols == nullptr && list_greedy(p, v);
-    if (kKind == kListTopK) return p.dyn_bytes >= kTopKArena && list_top_k(p, row, v, dyn);
-    return p.dyn_bytes >= kNucleusArena && list_nucleus(p, row, v, dyn);
+// ready(): waits until the row's inputs are complete; what does not need them is done before.
+template <int kKind, class Ready>
+__device__ __forceinline__ bool list_row(const MergeParams& p, const int64_t row, const RowView& v, u64* dyn, Ready ready) {
+    const int arena = kKind == kListTopK ? kTopKArena : kKind == kListNucleus ? kNucleusArena : 0;
+    if (p.parts > 32 || p.dyn_bytes < arena || (kKind == kListGreedy && p.survivor_cols != nullptr)) {  // (a record per lane)
+        ready();
+        return false;
+    }
+    if (kKind == kListGreedy) return list_greedy(p, v, ready);
+    if (kKind == kListTopK) return list_top_k(p, row, v, dyn, ready);
+    return list_nucleus(p, row, v, dyn, ready);
 }
 
 }  // namespace survivor

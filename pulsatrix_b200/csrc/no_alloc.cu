@@ -132,7 +132,7 @@ extern "C" psx_status psx_b200_sample_rows_static(void* stream_ptr, const float*
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
 
     // ---- the same plan as psx_b200_sample_rows, within the fixed limits ----------------------------------------
-    const psx::Plan plan = psx::make_plan(logits, vocab, row_stride, vocab, c);
+    const psx::Plan plan = psx::make_plan(logits, rows, vocab, row_stride, vocab, c, /*sm_count=*/0);
     if (rows * plan.parts > kStaticParts) {
         return set_error(PSX_ERR_UNSUPPORTED,
                          "psx_b200_sample_rows_static: the batch needs " + std::to_string(rows * plan.parts) +

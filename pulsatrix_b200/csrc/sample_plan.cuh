@@ -27,7 +27,7 @@ struct Plan {
 constexpr int kNucleusNeed = 160;  // logits every part hands on when no top-k bounds the survivors
 
 // rows x cols logits on this GPU (cols == vocab unless the vocabulary is sharded).
-inline Plan make_plan(const float* logits, int64_t cols, int64_t row_stride, int64_t vocab, const psx_sampling_config* c) {
+inline Plan make_plan(const float* logits, int64_t rows, int64_t cols, int64_t row_stride, int64_t vocab, const psx_sampling_config* c, int sm_count) {
     Plan plan;
     const bool aligned = (reinterpret_cast<uintptr_t>(logits) % 16 == 0) && (row_stride % 4 == 0);
     const int64_t vectors = (cols + 3 + (aligned ? 0 : 3)) / 4;  // most float4 a row can span
@@ -36,6 +36,14 @@ inline Plan make_plan(const float* logits, int64_t cols, int64_t row_stride, int
         return env ? std::max(256, std::min(kPartVecs, std::atoi(env))) : kPartVecs;
     }();
     plan.parts = (int)((vectors + part_vecs - 1) / part_vecs);
+    // A few rows leave most SMs idle: smaller parts, as long as every CTA still has an SM to itself.  Under a top-k each part hands on k
+    // logits, so that more than eight cost the survivor stage what they save (one row of 49,152, top-k 50: 3 parts 12.5 us,
+    // 6 parts 11.7; of 128,256: 8 parts 13.1, 16 parts 14.2); greedy has a few per part (8 parts 7.7, 32 parts 7.0).
+    // Without a top-k, fewer and longer lists reach further down.
+    if (c->do_sample == 0 || (c->top_k > 0 && c->top_k < vocab)) {
+        const int most = c->do_sample == 0 ? 32 : 8;
+        while (plan.parts * 2 <= most && (int64_t)plan.parts * 2 * rows <= sm_count && vectors / (plan.parts * 2) >= 1024) plan.parts *= 2;
+    }
     plan.vecs_per_part = (int)((vectors + plan.parts - 1) / plan.parts);
     const bool sample = c->do_sample != 0;
     const bool top_k_on = sample && c->top_k > 0 && c->top_k < vocab;

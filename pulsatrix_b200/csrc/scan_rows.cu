@@ -177,6 +177,19 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanPa
     // its caller's inputs until it has something to hand on: when the caller has promised that they
     // are complete, it runs ahead of the kernel before it in the stream until its first write.
     grid_dependents_may_launch();
+    // What needs no inputs: the copies' barriers (copy i is set up and issued by the first thread of warp i).
+    const bool use_flags = p.apply_penalty || p.num_banned > 0;
+    const int copies = nvec > 0 ? (nvec * 16 + (int)kCopyChunk - 1) / (int)kCopyChunk : 0;
+    const bool copies_here = lane == 0 && warp < copies;
+    const uint32_t copy_from = (uint32_t)warp * kCopyChunk, copy_bytes = copies_here ? min(kCopyChunk, (uint32_t)nvec * 16u - copy_from) : 0u;
+    if (copies_here) {
+        static_assert(kCopies <= kScanWarps, "one warp per copy");
+        barrier_init(&s_bar[warp], 1);
+        barrier_init_fence();
+        // (test hook: announcing more bytes than the copy delivers leaves the barrier open with
+        // nothing in flight, which is how the bounded wait is exercised)
+        barrier_expect_bytes(&s_bar[warp], copy_bytes + (p.test_short_copy ? 16u : 0u));
+    }
     if (!p.inputs_ready) grid_dependency_wait();
     if (nvec <= 0) {  // a part past the end of a row that starts on a 16-byte boundary: nothing to report
         if (p.wait_before_writes || ends_the_grid) grid_dependency_wait();
@@ -192,20 +205,8 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanPa
     }
 
     // ---- start the copy at once, and build the history bitmaps while it is in flight ---------------
-    const bool use_flags = p.apply_penalty || p.num_banned > 0;
-    const int copies = (nvec * 16 + (int)kCopyChunk - 1) / (int)kCopyChunk;
-    if (lane == 0 && warp < copies) {  // copy i is set up and issued by the first thread of warp i
-        static_assert(kCopies <= kScanWarps, "one warp per copy");
-        const uint32_t bytes = (uint32_t)nvec * 16u, off = (uint32_t)warp * kCopyChunk;
-        const uint32_t piece = min(kCopyChunk, bytes - off);
-        barrier_init(&s_bar[warp], 1);
-        barrier_init_fence();
-        // (test hook: announcing more bytes than the copy delivers leaves the barrier open with
-        // nothing in flight, which is how the bounded wait is exercised)
-        barrier_expect_bytes(&s_bar[warp], piece + (p.test_short_copy ? 16u : 0u));
-        bulk_copy_to_shared(dyn_smem + off, reinterpret_cast<const char*>(vbase + v0) + off, piece, &s_bar[warp]);
-    }
-    // The history's bounds and every thread's first id are asked for now, ahead of the barrier below.
+    if (copies_here) bulk_copy_to_shared(dyn_smem + copy_from, reinterpret_cast<const char*>(vbase + v0) + copy_from, copy_bytes, &s_bar[warp]);
+    // The history's bounds and every thread's first id, asked for all at once.
     int64_t h_begin = 0, h_end = 0, h_first = 0, b_first = 0;
     if (p.apply_penalty) {
         h_begin = p.history_offsets[row];
