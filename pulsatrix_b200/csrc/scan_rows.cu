@@ -96,6 +96,8 @@ __device__ __forceinline__ void mark_ids(const int64_t* ids, int64_t begin, int6
     }
 }
 
+constexpr uint32_t kNotedCap = 96;  // vectors of a warp that are dealt out over its lanes
+constexpr uint32_t kStageCap = 64;  // logits of a warp that wait in shared memory to be handed on
 constexpr int kPool = 64 / kScanWarps;  // per-thread maxima a warp can offer to the pooled threshold (64 in all)
 constexpr uint32_t kKeyMinusInf = 0x007FFFFFu;  // monotone_key(-inf): the lowest key a threshold can have
 constexpr uint32_t kKeyNone = 0xFFFFFFFFu;      // "no entry" in the pool (above every key of a number)
@@ -123,7 +125,8 @@ __device__ unsigned long long g_stage_clocks[4096 * 24];
 //          reaches it raw as well, and the rest belong to the raw tail with their raw value.
 // kAnnounce: raise ScanParams::row_ready when a part is written (a build of its own, so that the usual one
 //   carries nothing for it).
-template <bool kNucleus, bool kRestore, bool kAnnounce = false>
+// kGreedy: the part's maximum and its ties are all that is handed on (k_need == 1).
+template <bool kNucleus, bool kRestore, bool kAnnounce = false, bool kGreedy = false>
 __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanParams p) {
     static_assert(!(kNucleus && kRestore), "the processed tail needs the flagged logits out of the sums");
 #ifdef PSX_STAGE_CLOCKS
@@ -146,6 +149,10 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanPa
     __shared__ double s_wtail[kScanWarps], s_wproc[kScanWarps];
     __shared__ uint32_t s_wfill[kScanWarps], s_wflag[kScanWarps], s_wban[kScanWarps];
     __shared__ uint32_t s_banned_here;
+    __shared__ uint16_t s_noted[kScanWarps][kGreedy ? 1 : kNotedCap];
+    // what a warp hands on, until its place in the list is known; without kRestore over the bitmaps, which are done with by then
+    __shared__ uint2 s_stage_own[kRestore ? kScanWarps * kStageCap : 1];
+    static_assert(kScanWarps * kStageCap * sizeof(uint2) <= sizeof(s_bits), "the stage fits the bitmaps");
 
     const int part = blockIdx.x;  // grid: (parts, rows in chunks of 65535, chunks)
     const int64_t row = (int64_t)blockIdx.z * 65535 + blockIdx.y;
@@ -384,7 +391,7 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanPa
     // only offer less, i.e. lower the threshold.  (A thread without logits offers the padding value:
     // such a part has fewer than 1024 logits and hands all of them on.)  Beyond 8 per warp a warp
     // offers its kp-th largest only, and beyond 32 there is no threshold.
-    const bool single = p.k_need == 1;
+    const bool single = kGreedy || p.k_need == 1;
     const int kp = (int)min(((int64_t)p.k_need + kScanWarps - 1) / kScanWarps, (int64_t)33);
     const bool pooled = kp <= kPool;
     {
@@ -543,40 +550,108 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanPa
         noted |= hit ? (1u << t) : 0u;
     }
     STAGE(8);
-    // What reaches the threshold is counted now and handed on after the block has met (below): a
-    // warp's run in the part's list starts where the runs of the warps before it end.  It leaves
-    // the sums (its exp is taken in double by the survivor stage); its neighbours in the vector stay.
-    uint32_t count = 0, before_mine = 0, warp_count = 0, banned_hits = 0;
+    // What reaches the threshold leaves the sums (its exp is taken in double by the survivor stage; its neighbours in the vector
+    // stay) and waits in shared memory until the block has met: a warp's run in the part's list starts where the runs of the
+    // warps before it end.  The noted vectors are dealt out over the lanes -- a warp has some ten (top-k) to fifty (nucleus), a single lane
+    // often three or four, one after the other.
+    uint2* const stage = (kRestore ? s_stage_own : reinterpret_cast<uint2*>(s_bits)) + warp * kStageCap;
     const bool any_noted = __ballot_sync(0xFFFFFFFFu, noted != 0) != 0;
-    if (any_noted) {
+    uint32_t noted_total = 0, banned_hits = 0, warp_count = 0;
+    // Goes through the warp's noted vectors, a batch of at most one per lane at a time, in a fixed order; what reaches the threshold
+    // goes to out[0..], up to `room`.  Returns how many there are.
+    auto deal = [&](uint2* out, uint32_t room, bool sums) {
+        const bool dealt_out = !kGreedy && noted_total <= kNotedCap;
+        const uint32_t batches = dealt_out ? (noted_total + 31) / 32 : (uint32_t)trips;
+        uint32_t filled = 0;
+        for (uint32_t i = 0; i < batches; ++i) {
+            const bool mine = dealt_out ? i * 32 + lane < noted_total : ((noted >> i) & 1u) != 0;
+            if (!dealt_out && __ballot_sync(0xFFFFFFFFu, mine) == 0) continue;
+            const int v = !mine ? tid : dealt_out ? (int)s_noted[warp][i * 32 + lane] : (int)i * kScanThreads + tid;
+            const float4 d = data4[v];
+            const float l[4] = {d.x, d.y, d.z, d.w};
+            if (sums) {
+                float e0, e1, e2, e3, q0, q1, q2, q3;
+                exps_of(d, e0, e1, e2, e3, q0, q1, q2, q3);
+                const float e[4] = {e0, e1, e2, e3}, q[4] = {q0, q1, q2, q3};
+                float st = 0.0f, sp = 0.0f;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const bool stays = mine && !(l[c] >= tprime);
+                    st += stays ? e[c] : 0.0f;
+                    if (second_exp) sp += stays ? q[c] : 0.0f;
+                }
+                tail += st;
+                if (second_exp) proc += sp;
+            }
+            const uint32_t col = (uint32_t)(col_base + v * 4);
+            uint32_t flag_nib = 0, ban_nib = 0;  // this vector's four bits of the bitmaps
+            if (kRestore && use_flags) {
+                flag_nib = (s_flag[v >> 3] >> ((v & 7) * 4)) & 15u;
+                ban_nib = (s_ban[v >> 3] >> ((v & 7) * 4)) & 15u;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const bool hit = mine && l[c] >= tprime;
+                const uint32_t votes = __ballot_sync(0xFFFFFFFFu, hit);
+                const uint32_t at = filled + __popc(votes & ((1u << lane) - 1u));
+                if (hit && at < room) {
+                    const uint32_t flags = ((ban_nib >> c) & 1u) ? kFlagBanned : ((flag_nib >> c) & 1u) ? kFlagPenalized : 0u;
+                    out[at] = make_uint2(__float_as_uint(l[c]), (col + c) | flags);
+                }
+                if (kRestore && hit) banned_hits += (ban_nib >> c) & 1u;  // (the others that are banned are not alive)
+                filled += __popc(votes);
+            }
+        }
+        return filled;
+    };
+    if (kGreedy && any_noted) {
+        // As a rule one logit of the whole part; a lane takes its own.
+        uint32_t hits = 0, held_col = 0;
+        float held = 0.0f;
         for (uint32_t m2 = noted; m2; m2 &= m2 - 1) {
             const int v = (__ffs(m2) - 1) * kScanThreads + tid;
             const float4 d = data4[v];
             float e0, e1, e2, e3, q0, q1, q2, q3;
             exps_of(d, e0, e1, e2, e3, q0, q1, q2, q3);
-            const bool h0 = d.x >= tprime, h1 = d.y >= tprime, h2 = d.z >= tprime, h3 = d.w >= tprime;
-            count += (h0 ? 1u : 0u) + (h1 ? 1u : 0u) + (h2 ? 1u : 0u) + (h3 ? 1u : 0u);
-            tail += ((h0 ? 0.0f : e0) + (h1 ? 0.0f : e1)) + ((h2 ? 0.0f : e2) + (h3 ? 0.0f : e3));
-            if (second_exp) proc += ((h0 ? 0.0f : q0) + (h1 ? 0.0f : q1)) + ((h2 ? 0.0f : q2) + (h3 ? 0.0f : q3));
-            if (kRestore && p.num_banned > 0) {  // banned logits that are handed on (the others are not alive)
-                const uint32_t nib = (s_ban[v >> 3] >> ((v & 7) * 4)) & 15u;
-                banned_hits += ((h0 ? nib : 0u) & 1u) + ((h1 ? nib >> 1 : 0u) & 1u) + ((h2 ? nib >> 2 : 0u) & 1u) + ((h3 ? nib >> 3 : 0u) & 1u);
-            }
-        }
-        // Slots in lane order.  Usually a lane hands on one logit; otherwise scan the counts.
-        const uint32_t voters = __ballot_sync(0xFFFFFFFFu, count != 0);
-        before_mine = __popc(voters & ((1u << lane) - 1u));
-        warp_count = __popc(voters);
-        if (__ballot_sync(0xFFFFFFFFu, count > 1) != 0) {
-            uint32_t incl = count;
+            const float l[4] = {d.x, d.y, d.z, d.w}, e[4] = {e0, e1, e2, e3};
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                if (lane >= o) incl += up;
+            for (int c = 0; c < 4; ++c) {
+                const bool hit = l[c] >= tprime;
+                tail += hit ? 0.0f : e[c];
+                if (hit) { ++hits; held = l[c]; held_col = (uint32_t)(v * 4 + c); }
             }
-            before_mine = incl - count;
-            warp_count = __shfl_sync(0xFFFFFFFFu, incl, 31);
         }
+        __syncwarp();
+        const uint32_t voters = __ballot_sync(0xFFFFFFFFu, hits != 0);
+        if (__ballot_sync(0xFFFFFFFFu, hits > 1) != 0) {
+            warp_count = deal(stage, kStageCap, false);
+        } else {
+            if (hits != 0) {
+                uint32_t flags = 0;
+                if (kRestore && use_flags) {
+                    const uint32_t bit = held_col & 31u;
+                    flags = (s_ban[held_col >> 5] >> bit & 1u) ? kFlagBanned : (s_flag[held_col >> 5] >> bit & 1u) ? kFlagPenalized : 0u;
+                    banned_hits += flags == kFlagBanned ? 1u : 0u;
+                }
+                stage[__popc(voters & ((1u << lane) - 1u))] = make_uint2(__float_as_uint(held), ((uint32_t)col_base + held_col) | flags);
+            }
+            warp_count = __popc(voters);
+        }
+        __syncwarp();
+    } else if (!kGreedy && any_noted) {
+        uint32_t upto = __popc(noted);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+            if (lane >= o) upto += up;
+        }
+        noted_total = __shfl_sync(0xFFFFFFFFu, upto, 31);
+        if (noted_total <= kNotedCap) {
+            uint32_t at = upto - __popc(noted);
+            for (uint32_t m2 = noted; m2; m2 &= m2 - 1) s_noted[warp][at++] = (uint16_t)((__ffs(m2) - 1) * kScanThreads + tid);
+        }
+        __syncwarp();
+        warp_count = deal(stage, kStageCap, true);
     }
 
     STAGE(9);
@@ -649,26 +724,13 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanPa
         }
     }
     STAGE(19);
-    if (any_noted) {  // slots in warp order, then lane, trip, component -- a fixed order
-        uint32_t slot = flagged_total + before_mine + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? s_wfill[lane] : 0u);
-        for (uint32_t m2 = noted; m2; m2 &= m2 - 1) {
-            const int v = (__ffs(m2) - 1) * kScanThreads + tid;
-            const float4 d = data4[v];
-            const float l[4] = {d.x, d.y, d.z, d.w};
-            const uint32_t col = (uint32_t)(col_base + v * 4);
-            uint32_t flag_nib = 0, ban_nib = 0;  // this vector's four bits of the bitmaps
-            if (kRestore && use_flags) {
-                flag_nib = (s_flag[v >> 3] >> ((v & 7) * 4)) & 15u;
-                ban_nib = (s_ban[v >> 3] >> ((v & 7) * 4)) & 15u;
-            }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                if (l[c] >= tprime) {
-                    const uint32_t flags = ((ban_nib >> c) & 1u) ? kFlagBanned : ((flag_nib >> c) & 1u) ? kFlagPenalized : 0u;
-                    if (slot < (uint32_t)kPartCap) part_out[slot] = make_uint2(__float_as_uint(l[c]), (col + c) | flags);
-                    ++slot;
-                }
-            }
+    if (any_noted) {  // slots in warp order, then in the order of the dealing -- a fixed order
+        const uint32_t slot = flagged_total + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? s_wfill[lane] : 0u);
+        const uint32_t room = slot < (uint32_t)kPartCap ? (uint32_t)kPartCap - slot : 0u;
+        if (warp_count <= kStageCap) {
+            for (uint32_t i = lane; i < min(warp_count, room); i += 32) part_out[slot + i] = stage[i];
+        } else {
+            deal(part_out + slot, room, false);
         }
     }
     announce_part();
@@ -694,6 +756,8 @@ cudaError_t configure_scan_rows() {
     cudaError_t e = allow_all_dynamic_shared(scan_rows_kernel<true, false>);
     if (e == cudaSuccess) e = allow_all_dynamic_shared(scan_rows_kernel<false, false>);
     if (e == cudaSuccess) e = allow_all_dynamic_shared(scan_rows_kernel<false, true>);
+    if (e == cudaSuccess) e = allow_all_dynamic_shared(scan_rows_kernel<false, false, false, true>);
+    if (e == cudaSuccess) e = allow_all_dynamic_shared(scan_rows_kernel<false, true, false, true>);
     if (e == cudaSuccess) e = allow_all_dynamic_shared(scan_rows_kernel<false, false, true>);
     if (e == cudaSuccess) e = allow_all_dynamic_shared(scan_rows_kernel<false, true, true>);
     return e;
@@ -707,6 +771,7 @@ cudaError_t launch_scan_rows(const ScanParams& p, bool nucleus, cudaStream_t str
     // A flag can only lower a logit unless the penalty is below one (then l / p > l for l > 0).
     const bool flags_only_lower = !p.apply_penalty || p.penalty >= 1.0f;
     auto kernel = nucleus ? scan_rows_kernel<true, false> : flags_only_lower ? scan_rows_kernel<false, true> : scan_rows_kernel<false, false>;
+    if (!nucleus && p.k_need == 1) kernel = flags_only_lower ? scan_rows_kernel<false, true, false, true> : scan_rows_kernel<false, false, false, true>;
     if (p.row_ready != nullptr) {  // (asked for by the vocabulary-sharded step, which has a top-k or is greedy)
         if (nucleus) return cudaErrorInvalidConfiguration;
         kernel = flags_only_lower ? scan_rows_kernel<false, true, true> : scan_rows_kernel<false, false, true>;
