@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(const
     auto ctx_of_warp = [&](int w) { return s_q + R * D + w * per_warp; };  // R x D, over warp w's K tile
     __shared__ __align__(8) uint64_t s_bar[kAttnWarps][2];              // K, V
 
+    if (p.splits > 1) grid_dependents_may_launch();  // (the kernel that joins the slices is set up meanwhile; it waits for this one)
     const int64_t nkv = blockIdx.x;  // (batch, kv head)
     const int64_t n = nkv / p.kv_heads, kvh = nkv % p.kv_heads;
     const int split = blockIdx.y;
@@ -339,6 +340,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(const
 
 // Joins the slices of every query row: thread per (row, column).
 __global__ void join_attention_splits_kernel(const AttentionParams p) {
+    grid_dependency_wait();
     const int D = p.head_dim;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t out_rows = p.batch * p.heads * p.q_len;
@@ -420,8 +422,7 @@ cudaError_t launch_decode_attention(const AttentionParams& p, cudaStream_t strea
     }
     if (e != cudaSuccess || p.splits == 1) return e;
     const int64_t elements = p.batch * p.heads * p.q_len * p.head_dim;
-    join_attention_splits_kernel<<<(unsigned)((elements + 255) / 256), 256, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapping(join_attention_splits_kernel, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, stream, p);
 }
 
 }  // namespace psx
