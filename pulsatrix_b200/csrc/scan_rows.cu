@@ -531,8 +531,8 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanPa
         e_bound = __fmul_rn(t0, 1.0f - 0x1p-19f);
         if (!(e_bound >= 0x1p-120f)) e_bound = 0.0f;
     }
-#pragma unroll 4
-    for (int t = 0; t < trips; ++t) {
+    // (four trips at a time: a hit is a predicated constant, its bits move to their place once per four)
+    auto look = [&](int t, uint32_t bit, uint32_t& hits) {
         const float4 d = data4[t * kScanThreads + tid];
         float e0, e1, e2, e3, q0, q1, q2, q3;
         exps_of(d, e0, e1, e2, e3, q0, q1, q2, q3);
@@ -540,15 +540,23 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_rows_kernel(const ScanPa
         add_pair(s01, s23, e0, e2, e1, e3);  // (e0 + e1), (e2 + e3)
         const float s = s01 + s23;
         const bool hit = s >= e_bound;
-        tail += hit ? 0.0f : s;
+        if (hit) hits |= bit; else tail += s;
         if (second_exp) {
             float q01, q23;
             add_pair(q01, q23, q0, q2, q1, q3);
             const float q = q01 + q23;
-            proc += hit ? 0.0f : q;
+            if (!hit) proc += q;
         }
-        noted |= hit ? (1u << t) : 0u;
+    };
+    int t4 = 0;
+#pragma unroll 1
+    for (; t4 + 4 <= trips; t4 += 4) {
+        uint32_t hits = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) look(t4 + q, 1u << q, hits);
+        noted |= hits << t4;
     }
+    for (; t4 < trips; ++t4) look(t4, 1u << t4, noted);
     STAGE(8);
     // What reaches the threshold leaves the sums (its exp is taken in double by the survivor stage; its neighbours in the vector
     // stay) and waits in shared memory until the block has met: a warp's run in the part's list starts where the runs of the
