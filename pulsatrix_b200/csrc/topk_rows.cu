@@ -7,7 +7,7 @@
 // The short way (k <= 256): two sweeps over the slice as floats, out of shared memory where a slice of
 // up to 16,384 entries fits (bulk copies; longer ones are read from global memory twice, the second time out of L2).
 // Bound by instructions more than by HBM: 4096 x 16,384, k 64: 79.7 us with 256 threads reading twice from global memory,
-// 75.3 now; 8192 x 4096, k 16: 63.5 -> 36.9 us.  Sweep one notes every thread's best entry; the smallest over the warps of
+// 67.9 now; 8192 x 4096, k 16: 63.5 -> 34.8 us.  Sweep one notes every thread's best entry; the smallest over the warps of
 // the kp-th best of those (kp = ceil(k / 8)) is a bound that k entries of the slice reach.  Sweep
 // two lists what reaches the bound, usually k and a few; the list is put in rank order by
 // counting, and with several CTAs per row the best k of each meet in the first CTA's shared memory
@@ -63,16 +63,18 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
     return r;
 }
 
-// The kp-th largest (1-based, kp <= 32) of the 32 lanes' keys: for small kp the maximum is taken
-// away kp - 1 times, else a bitonic sort across the lanes.
+// A key that at least kp (1-based, kp <= 32) of the 32 lanes' keys reach, the kp-th largest or up to 31 below it: for small kp the
+// maximum is taken away kp - 1 times, the low five bits of a key giving way to its lane so that all are distinct; else a
+// bitonic sort across the lanes.
 __device__ __forceinline__ uint32_t warp_kth_largest_key(uint32_t key, int kp, int lane) {
-    if (kp <= 6) {
+    if (kp <= 10) {
+        key = (key & ~31u) | (uint32_t)lane;
+        uint32_t top = __reduce_max_sync(0xFFFFFFFFu, key);
         for (int i = 1; i < kp; ++i) {
-            const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, key);
-            const uint32_t holders = __ballot_sync(0xFFFFFFFFu, key == top);
-            if (lane == __ffs(holders) - 1) key = 0;
+            key = key == top ? 0u : key;
+            top = __reduce_max_sync(0xFFFFFFFFu, key);
         }
-        return __reduce_max_sync(0xFFFFFFFFu, key);
+        return top & ~31u;
     }
 #pragma unroll
     for (int k = 2; k <= 32; k <<= 1) {
@@ -289,8 +291,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
             for (uint32_t c = 0; c * kHeldChunk < vectors; ++c) barrier_wait_bounded(&s_bar[c], 0, p.wait_limit_ns);
             landed = false;
         }
-        const bool everything = bound == 0 && landed, only_nan = (largest && bound == 0xFFFFFFFFu) || !landed;
         const float edge = largest ? from_ordered_key(bound) : from_ordered_key(~bound);
+        const bool everything = bound == 0 && landed, only_nan = edge != edge || !landed;  // (or only what no number lies below)
         auto reaches = [&](float x) { return largest ? !(x < edge) : x <= edge; };
         auto put = [&](float x, uint32_t col) {
             const uint32_t slot = atomicAdd(&s_listed, 1u);
