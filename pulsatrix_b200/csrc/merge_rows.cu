@@ -5,12 +5,12 @@
 //   1. joins the parts' partial log-sum-exp (raw, and processed when a full-vocabulary top-p or
 //      min-p needs it): M = max m_i, Z = sum z_i * exp(m_i - M) + sum over candidates, in double;
 //   2. keeps the candidates at or above the largest part threshold (only those can survive any
-//      filter), applies penalty and temperature with the reference's float operations, and sorts
-//      them by (value descending, column ascending) in shared memory;
-//   3. replays src/generation.cpp:80-152 on that short list in the reference's own order and
-//      precision -- the k-th value with its ties, softmax sums in column order, the top-p walk in
-//      ascending (value, column) order against 1 - (double)top_p, min-p against the first
-//      maximum, the inverse-CDF walk in column order against the row's uniform -- all in double;
+//      filter) and applies penalty and temperature with the reference's float operations;
+//   3. decides src/generation.cpp:80-152 on that short list: as a rule with integer sums over the entries that come
+//      before an entry (merge_rows_list_impl.cuh), and where a list does not fit or a decision is too close to its level by
+//      replaying the reference's own order and precision -- the k-th value with its ties, softmax sums in column order,
+//      the top-p walk in ascending (value, column) order against 1 - (double)top_p, min-p against the first
+//      maximum, the inverse-CDF walk in column order against the row's uniform -- all in double (merge_rows_impl.cuh);
 //   4. writes the token, float(log(exp(l - M) / Z)) of the raw logits (src/generation.cpp:156),
 //      a row status and the distances of the two decisions from their boundaries.
 // Reads a few KB per row and never touches the logits -- except for a row that does not fit the
