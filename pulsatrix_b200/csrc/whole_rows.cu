@@ -342,8 +342,14 @@ __global__ void __launch_bounds__(kThreads, 8) weigh_segments_kernel(const __gri
         raw_max = warp_max(raw_max);
         if (kFlags) clear_max = warp_max(clear_max);
         if (!__any_sync(0xFFFFFFFFu, here != 0)) raw_max = -INFINITY;  // (past the end of the row)
-        if (edge) {  // what is not there weighs next to nothing: exp(-690) in both sums, exp(-690 T) in the raw one if T < 1
-            const float nothing = __fmaf_rn(-690.0f, fminf(1.0f, p.apply_temperature ? p.temperature : 1.0f), raw_max);
+        // What is not there weighs next to nothing: exp(-690), in the raw sum exp(-690 T) if T < 1, in the other one exp(-690 / T) if T > 1.
+        // 511 slots of exp(-60) are 5e-24; where it could be more (very low or high temperatures, maxima so large that 690
+        // rounds away), and in a segment that is not there at all, the sums leave the slots out one by one.
+        bool absent_weighs = false;
+        if (edge) {
+            const float nothing = __fmaf_rn(-690.0f, fminf(1.0f, p.apply_temperature ? p.temperature : 1.0f), raw_max), gap = raw_max - nothing;
+            // (with flags the other sum leaves them out anyway)
+            absent_weighs = !(gap >= 60.0f && (kFlags || !p.apply_temperature || gap >= 60.0f * p.temperature));
 #pragma unroll
             for (int i = 0; i < kVecs * 4; ++i) l[i] = ((here >> i) & 1u) ? l[i] : nothing;
         }
@@ -364,20 +370,21 @@ __global__ void __launch_bounds__(kThreads, 8) weigh_segments_kernel(const __gri
             y_max = fmaxf(y_max, warp_max(most));
         }
         double raw_sum = 0.0, mass = 0.0;
-        const bool within = !(edge && p.apply_temperature && p.temperature < 0.1f) && raw_max - raw_min <= 700.0f && (!kProcessed || y_max - temper(raw_min, p.apply_temperature != 0, p.temperature) <= 700.0f);
+        const bool within = !absent_weighs && raw_max - raw_min <= 700.0f && (!kProcessed || y_max - temper(raw_min, p.apply_temperature != 0, p.temperature) <= 700.0f);
         if (within) {  // no exponential needs looking after
             const double raw_top = (double)raw_max, y_top = (double)y_max;
+            const uint32_t apart = marked | ~here;  // marked logits are added below, absent ones (they may lie above y_top) never
 #pragma unroll
             for (int i = 0; i < kVecs * 4; ++i) {
                 const double x = (double)l[i];
                 raw_sum += exp_of_gap(x - raw_top, power);
                 if (kProcessed) {
                     const double e = exp_of_gap(tempered(x, reciprocal) - y_top, power);
-                    // a marked logit's term is next to nothing here: its upper half is taken away
-                    mass += kFlags ? __hiloint2double(((marked >> i) & 1u) ? 0 : __double2hiint(e), __double2loint(e)) : e;
+                    // (what is left of a term without its upper half is next to nothing)
+                    mass += kFlags ? __hiloint2double(((apart >> i) & 1u) ? 0 : __double2hiint(e), __double2loint(e)) : e;
                 }
             }
-        } else {  // logits further apart than an exponential reaches; the ends of a row at a very low temperature
+        } else {  // logits further apart than an exponential reaches; ends of a row whose absent slots would weigh
 #pragma unroll 1
             for (int i = 0; i < kVecs * 4; ++i) {
                 if (!((here >> i) & 1u)) continue;

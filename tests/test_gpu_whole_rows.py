@@ -46,3 +46,31 @@ def test_banned_segments_and_failed_rows():
     hist, offsets = np.zeros((rows, 1), dtype=np.int64), np.arange(rows + 1, dtype=np.int64)
     (tokens, _, status, _), _ = gh.check_rows_against_oracle(logits, hist, offsets, cfg, np.arange(rows, dtype=np.uint64), expect_ok=False)
     assert status[1] == psx.ROW_NON_FINITE and (tokens[[0, 2, 3]] == 700).all()
+
+
+# The first and the last segment of a row have slots that lie outside it; none of them may weigh anything.
+@pytest.mark.parametrize("vocab", [1025, 50021])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+@pytest.mark.parametrize("settings", [dict(temperature=50.0), dict(temperature=100.0), dict(temperature=1000.0),
+                                      dict(temperature=100.0, repetition_penalty=1.2), dict(temperature=0.05)], ids=str)
+def test_slots_outside_the_row_weigh_nothing(vocab, shift, settings):
+    _run(vocab, 5, settings, pad_columns=shift, shift=shift)
+
+
+def test_slots_outside_the_row_beside_a_banned_maximum():
+    # the last segment's largest logit is banned and lies 200 above the others: at T = 0.2 anything derived from it outweighs the row
+    vocab, rows = 1500, 4
+    logits, hist = ol.synth_rows(np.arange(rows) + 31, vocab, 2.0, 0.7, 4)
+    logits[:, 1490] = 200.0
+    cfg = ol.make_config(max_new_tokens=2, do_sample=True, temperature=0.2, min_new_tokens=1, eos_token_ids=[1490])
+    (_, _, _, diag), want = gh.check_rows_against_oracle(logits, hist, np.arange(rows + 1, dtype=np.int64) * 4, cfg, np.arange(rows, dtype=np.uint64))
+    assert np.abs(diag["draw_margin"] - want["draw_margin"]).max() <= 3 * vocab * 2.0**-53
+
+
+def test_slots_outside_the_row_beside_a_maximum_that_690_does_not_move():
+    vocab, rows = 1025, 3  # the last segment: this one column
+    logits, hist = ol.synth_rows(np.arange(rows) + 5, vocab, 2.0, 0.7, 4)
+    logits[:, -1] = 1e11
+    for settings in (dict(), dict(temperature=0.9, repetition_penalty=1.2)):
+        cfg = ol.make_config(max_new_tokens=1, do_sample=True, **settings)
+        gh.check_rows_against_oracle(logits, hist, np.arange(rows + 1, dtype=np.int64) * 4, cfg, np.arange(rows, dtype=np.uint64))
