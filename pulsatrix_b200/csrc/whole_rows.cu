@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(kThreads, 8) weigh_segments_kernel(const __gri
             y_max = fmaxf(y_max, warp_max(most));
         }
         double raw_sum = 0.0, mass = 0.0;
+        uint32_t gone = banned;  // not alive
         const bool within = !absent_weighs && raw_max - raw_min <= 700.0f && (!kProcessed || y_max - temper(raw_min, p.apply_temperature != 0, p.temperature) <= 700.0f);
         if (within) {  // no exponential needs looking after
             const double raw_top = (double)raw_max, y_top = (double)y_max;
@@ -390,18 +391,23 @@ __global__ void __launch_bounds__(kThreads, 8) weigh_segments_kernel(const __gri
                 if (!((here >> i) & 1u)) continue;
                 const float x = p.logits[row * p.row_stride + lane_col + (i >> 2) * 128 + (i & 3)];
                 raw_sum += exp_below(x, raw_max);
-                if (kProcessed && !((marked >> i) & 1u)) mass += exp_below(temper(x, p.apply_temperature != 0, p.temperature), y_max);
+                if (kProcessed && !((marked >> i) & 1u)) {
+                    const float y = temper(x, p.apply_temperature != 0, p.temperature);
+                    mass += exp_below(y, y_max);
+                    if (!(y > -INFINITY)) gone |= 1u << i;  // (a quotient that overflowed)
+                }
             }
         }
         if (kFlags) {
             for (uint32_t bits = marked & here; bits; bits &= bits - 1) {
-                const float y = marked_value(__ffs(bits) - 1);
-                if (y > -INFINITY) mass += exp_below(y, y_max);
+                const int i = __ffs(bits) - 1;
+                const float y = marked_value(i);
+                if (y > -INFINITY) mass += exp_below(y, y_max); else gone |= 1u << i;
             }
         }
         raw_sum = warp_sum(raw_sum);
         mass = kProcessed ? warp_sum(mass) : raw_sum;
-        const uint32_t alive = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(here & ~banned));
+        const uint32_t alive = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(here & ~gone));
         const bool all_finite = __all_sync(0xFFFFFFFFu, finite);
         if (lane == 0) {
             SegmentStats s;

@@ -74,3 +74,16 @@ def test_slots_outside_the_row_beside_a_maximum_that_690_does_not_move():
     for settings in (dict(), dict(temperature=0.9, repetition_penalty=1.2)):
         cfg = ol.make_config(max_new_tokens=1, do_sample=True, **settings)
         gh.check_rows_against_oracle(logits, hist, np.arange(rows + 1, dtype=np.int64) * 4, cfg, np.arange(rows, dtype=np.uint64))
+
+
+@pytest.mark.parametrize("penalty", [1.0, 1.5])
+def test_quotients_that_fall_to_minus_infinity_are_not_alive(penalty):
+    # -1000 / 1e-36 is -inf (removed, as by the reference), the positive logits' quotients are finite
+    vocab, rows = 3001, 4
+    logits, hist = ol.synth_rows(np.arange(rows) + 77, vocab, 2.0, 0.7, 30)
+    logits[:, ::7] = -1000.0
+    logits[:, 1500] = 50.0
+    hist[:, 0], hist[:, 1] = 7, 1500
+    cfg = ol.make_config(max_new_tokens=1, do_sample=True, temperature=1e-36, repetition_penalty=penalty)
+    _, want = gh.check_rows_against_oracle(logits, hist, np.arange(rows + 1, dtype=np.int64) * 30, cfg, np.arange(rows, dtype=np.uint64))
+    assert (want["survivors"] < vocab).all()
