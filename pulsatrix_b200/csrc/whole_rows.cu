@@ -176,7 +176,26 @@ __global__ void __launch_bounds__(kThreads) draw_token_kernel(const __grid_const
     z = warp_sum(z);
     if (lane == 0) s_z[warp] = z;
     const RunningSum run = block_running_sum(mass, s_mass);
-    const double total = run.total, target = u * total;
+    if (!(y_max < INFINITY)) {
+        // A quotient overflowed: every probability of the reference is NaN then, and its walk (:140-152) ends at the last column.
+        if (p.diag) {
+            alive = __reduce_add_sync(0xFFFFFFFFu, alive);
+            if (lane == 0) atomicAdd(&s_alive, (int)alive);
+            __syncthreads();
+        }
+        if (tid == 0) {
+            double z_total = s_z[0];
+            for (int i = 1; i < kWarps; ++i) z_total += s_z[i];
+            p.row_status[row] = PSX_ROW_OK;
+            p.tokens[row] = p.vocab - 1;
+            p.log_probs[row] = (float)log(exp((double)p.logits[row * p.row_stride + p.vocab - 1] - (double)raw_max) / z_total);
+            if (p.diag) p.diag[row] = psx_row_diag{(int)p.vocab, s_alive, NAN, INFINITY};
+        }
+        return;
+    }
+    // (The maximum's own mass is 1, so the total is positive and some thread holds every target from 0 on; a uniform below
+    // 0 takes the first token that has mass, one that is not below 1 the last.)
+    const double total = run.total, target = u < 0.0 ? 0.0 : u * total;
     // ---- the segment that holds the crossing: the running sum rises above the target there (:140-152); if rounding
     // leaves none, the last that holds mass ----------------------------------------------------------------------------
     bool holds = run.before <= target && target < run.upto;

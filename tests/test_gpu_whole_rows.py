@@ -87,3 +87,25 @@ def test_quotients_that_fall_to_minus_infinity_are_not_alive(penalty):
     cfg = ol.make_config(max_new_tokens=1, do_sample=True, temperature=1e-36, repetition_penalty=penalty)
     _, want = gh.check_rows_against_oracle(logits, hist, np.arange(rows + 1, dtype=np.int64) * 30, cfg, np.arange(rows, dtype=np.uint64))
     assert (want["survivors"] < vocab).all()
+
+
+@pytest.mark.parametrize("settings", [dict(temperature=1e-38), dict(repetition_penalty=1e-38), dict(temperature=1e-38, repetition_penalty=1.5)], ids=str)
+def test_quotients_that_overflow(settings):
+    # every probability of the reference is NaN: its walk ends at the last column
+    vocab, rows = 3001, 4
+    logits, hist = ol.synth_rows(np.arange(rows) + 78, vocab, 2.0, 0.7, 30)
+    logits[:, 1500] = 6.0  # 6 / 1.5 / 1e-38 = 4e38, above the largest float (5 would give 3.33e38, below it)
+    hist[:, 0] = 1500
+    cfg = ol.make_config(max_new_tokens=1, do_sample=True, **settings)
+    (tokens, _, _, _), _ = gh.check_rows_against_oracle(logits, hist, np.arange(rows + 1, dtype=np.int64) * 30, cfg, np.arange(rows, dtype=np.uint64))
+    assert (tokens == vocab - 1).all()
+
+
+def test_uniforms_outside_the_unit_interval():
+    vocab = 5003
+    logits, _ = ol.synth_rows(np.arange(5) + 79, vocab, 2.0, 0.7, 4)
+    uniforms = np.array([-0.25, -1e300, 1.0, 7.5, np.nan])
+    for settings in (dict(), dict(temperature=0.8)):
+        cfg = ol.make_config(max_new_tokens=1, do_sample=True, **settings)
+        tokens, _, status, _ = gh.sample_on_gpu(logits, None, None, cfg, uniforms)
+        assert (status == 0).all() and tokens.tolist() == [0, 0, vocab - 1, vocab - 1, vocab - 1]
