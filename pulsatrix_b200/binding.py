@@ -152,6 +152,15 @@ def _stream_of(tensor):
     return _cuda_getCurrentRawStream(device)
 
 
+def _zeroed_word(device, stream):
+    """A one-element int32 tensor of its own, zeroed on the stream of the call that may set it."""
+    import torch
+    if stream is None:
+        return torch.zeros(1, dtype=torch.int32, device=device)
+    with torch.cuda.stream(torch.cuda.ExternalStream(stream, device=device)):
+        return torch.zeros(1, dtype=torch.int32, device=device)
+
+
 def _ptr(t):
     return None if t is None else t.data_ptr()
 
@@ -214,7 +223,6 @@ class Context:
         self._ctx = C.c_void_p()
         _check(self._lib.psx_b200_ctx_create(C.c_int(device), C.byref(self._ctx)))
         self._handle = self._ctx.value  # (what the native calls take)
-        self._zero_words = []
         self.device = device
 
     def close(self):
@@ -437,13 +445,6 @@ class Context:
                                    out.data_ptr(), indices.shape[0], table.shape[1]))
         return out
 
-    def _zero_word(self, device):
-        """A one-element int32 tensor that holds zero: the next of a block that was zeroed with one launch."""
-        if not self._zero_words or self._zero_words[-1].device != device:
-            import torch
-            self._zero_words = list(torch.zeros(256, dtype=torch.int32, device=device).split(1))
-        return self._zero_words.pop()
-
     def decode_attention(self, q, keys, values, cached, scale=None, causal=True, window=0, key_keep=None, stream=None):
         """Attention of the new positions over the KV cache (psx_b200_decode_attention).  q: cuda float32
         (batch, heads, q_len, head_dim); keys / values: the cache, (batch, kv_heads, max_len, head_dim), with
@@ -455,7 +456,7 @@ class Context:
         if scale is None:
             scale = 1.0 / float(np.sqrt(np.float32(head_dim)))
         context = torch.empty_like(q)
-        status = self._zero_word(q.device)
+        status = _zeroed_word(q.device, stream)
         _check(_native.decode_attention(self._handle, _stream_of(q) if stream is None else stream, q.data_ptr(), keys.data_ptr(),
                                         values.data_ptr(), _ptr(key_keep), context.data_ptr(), batch, heads, kv_heads, q_len, head_dim,
                                         cached, max_len, float(scale), int(bool(causal)), window, status.data_ptr()))

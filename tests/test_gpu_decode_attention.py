@@ -79,3 +79,57 @@ def test_bad_arguments_are_refused():
     with pytest.raises(psx.PsxError) as e:   # 64 query rows per kv head
         ctx.decode_attention(q, kv, kv, 8)
     assert e.value.status == psx.ERR_UNSUPPORTED
+
+
+def _small_call(ctx, **kw):
+    import torch
+    q = torch.zeros((1, 2, 1, 64), device="cuda")
+    kv = torch.zeros((1, 2, 16, 64), device="cuda")
+    return lambda: ctx.decode_attention(q, kv, kv, 7, **kw)[1]
+
+
+@pytest.mark.parametrize("explicit", [False, True])
+def test_status_words_belong_to_their_calls_stream(explicit):
+    # a call on one stream waits behind long work; a call on another stream must not depend on anything that waits there
+    import torch
+    ctx, a, b = psx.Context(0), torch.cuda.Stream(), torch.cuda.Stream()
+    _small_call(psx.Context(0))()  # (the kernel is loaded)
+    first, second = _small_call(ctx, stream=a.cuda_stream if explicit else None), _small_call(ctx, stream=b.cuda_stream if explicit else None)
+    with torch.cuda.stream(a):
+        stale = [torch.full((256,), -1, dtype=torch.int32, device="cuda") for _ in range(64)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        del stale  # (what this stream allocates next holds -1)
+        torch.cuda._sleep(400_000_000)  # some 0.2 s
+        mine = first()
+    with torch.cuda.stream(b):
+        other = second()
+    b.synchronize()
+    assert int(other.cpu()) == 0
+    other.fill_(1)
+    torch.cuda.synchronize()
+    assert int(mine.cpu()) == 0 and int(other.cpu()) == 1
+    assert mine.untyped_storage().data_ptr() != other.untyped_storage().data_ptr()
+
+
+def test_a_captured_call_zeroes_its_status_in_every_replay():
+    import torch
+    ctx = psx.Context(0)
+    call = _small_call(ctx)
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        status = call()
+    eager = call()  # (a word handed out after the capture)
+    for _ in range(2):
+        status.fill_(1)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert int(status.cpu()) == 0
+    assert int(eager.cpu()) == 0
+
+
+def test_status_on_the_default_stream_given_by_its_handle():
+    ctx = psx.Context(0)
+    assert int(_small_call(ctx, stream=0)().cpu()) == 0
