@@ -35,7 +35,7 @@ def _stale() -> bool:
     if not LIBRARY.exists() or not PYTHON_CALLS.exists():
         return True
     built = min(LIBRARY.stat().st_mtime, PYTHON_CALLS.stat().st_mtime)
-    deps = (list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list((PACKAGE / "host").glob("*.cpp")) +
+    deps = (list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.hpp")) + list((PACKAGE / "host").glob("*.cpp")) +
             list((PACKAGE.parent / "include").rglob("*.h*")))
     return any(p.stat().st_mtime > built for p in deps)
 

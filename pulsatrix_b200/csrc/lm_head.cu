@@ -296,12 +296,8 @@ template <int R, int G, int H, int KC, int S, int kCtas, int EM, bool kTokenMajo
 cudaError_t launch_one(HeadParams p, int sm_count, cudaStream_t stream) {
     typedef Head<R, G, H, KC, S, EM, kTokenMajor> K;
     const auto kernel = head_kernel<R, G, H, KC, S, kCtas, EM, kTokenMajor>;
-    static bool configured = false;  // (per instantiation; raising the limit twice is harmless)
-    if (!configured) {
-        const cudaError_t e = allow_all_dynamic_shared(kernel);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    static OncePerDevice configured;  // (per instantiation)
+    if (const cudaError_t e = allow_all_dynamic_shared_once(configured, kernel); e != cudaSuccess) return e;
     // Every CTA that the GPU holds at once takes whole tiles round after round; the rest goes round once, in the
     // smallest tiles with which it does.
     const int64_t lanes = 32 * H;  // entries of a CTA's tile per entry of a lane

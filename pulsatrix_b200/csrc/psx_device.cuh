@@ -9,6 +9,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include "once_per_device.hpp"
+
 namespace psx {
 
 // ---- geometry of the row pass ----------------------------------------------------------------
@@ -245,6 +247,14 @@ inline cudaError_t allow_all_dynamic_shared(Kernel kernel) {
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 most - (int)attributes.sharedSizeBytes);
+}
+
+// ... the first time it is asked for on the current device.  (The limit is the device's own; done: one per kernel.)
+template <class Kernel>
+inline cudaError_t allow_all_dynamic_shared_once(OncePerDevice& done, Kernel kernel) {
+    int device = 0;
+    if (const cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return e;
+    return done.run(device, [&] { return allow_all_dynamic_shared(kernel); });
 }
 
 // Launches `kernel` so that it may begin while the kernel before it in `stream` is still running

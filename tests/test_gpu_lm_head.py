@@ -103,3 +103,15 @@ def test_head_and_sampling_in_one_call_match_sampling_the_references_logits():
     assert (out["status"].cpu().numpy() == 0).all()
     assert out["tokens"].cpu().numpy().tolist() == want["token"].tolist()
     assert np.allclose(out["log_probs"].cpu().numpy(), want["log_prob"], rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("rows", [1, 4, 64])
+def test_a_second_device_of_the_process(rows):
+    # (more shared memory per block than the default limit, which is raised device by device)
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one GPU")
+    rng = np.random.RandomState(rows)
+    hidden, weight = rng.randn(rows, 64).astype(np.float32), rng.randn(500, 64).astype(np.float32)
+    got = [psx.Context(d).lm_head_logits(torch.from_numpy(hidden).to(f"cuda:{d}"), torch.from_numpy(weight).to(f"cuda:{d}")).cpu() for d in (0, 1)]
+    assert torch.equal(got[0], got[1])
