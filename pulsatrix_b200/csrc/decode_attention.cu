@@ -366,12 +366,8 @@ __global__ void join_attention_splits_kernel(const AttentionParams p) {
 
 template <int R, int C>
 cudaError_t launch_one(const AttentionParams& p, size_t shared, cudaStream_t stream) {
-    static bool configured = false;  // (per instantiation; raising the limit twice is harmless)
-    if (!configured) {
-        const cudaError_t e = allow_all_dynamic_shared(decode_attention_kernel<R, C>);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    static OncePerDevice configured;  // (per instantiation)
+    if (const cudaError_t e = allow_all_dynamic_shared_once(configured, decode_attention_kernel<R, C>); e != cudaSuccess) return e;
     decode_attention_kernel<R, C><<<dim3((unsigned)(p.batch * p.kv_heads), (unsigned)p.splits), kAttnWarps * 32, shared, stream>>>(p);
     return cudaGetLastError();
 }

@@ -133,3 +133,17 @@ def test_a_captured_call_zeroes_its_status_in_every_replay():
 def test_status_on_the_default_stream_given_by_its_handle():
     ctx = psx.Context(0)
     assert int(_small_call(ctx, stream=0)().cpu()) == 0
+
+
+def test_a_second_device_of_the_process():
+    # (more shared memory per block than the default limit, which is raised device by device)
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one GPU")
+    rng = np.random.RandomState(0)
+    q, kv = rng.randn(2, 4, 1, 128).astype(np.float32), rng.randn(2, 2, 2, 40, 128).astype(np.float32)
+    got = []
+    for d in (0, 1):
+        on = [torch.from_numpy(x).to(f"cuda:{d}") for x in (q, kv[0], kv[1])]
+        got.append(psx.Context(d).decode_attention(*on, 33)[0].cpu())
+    assert torch.equal(got[0], got[1])
