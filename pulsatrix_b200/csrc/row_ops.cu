@@ -6,7 +6,8 @@
 // softmax / logsumexp read every element once and (softmax) write it once:
 //   - a row of up to 32,768 columns belongs to as few warps as hold it with eight 128-bit vectors per lane (one warp up
 //     to 1024 columns, four up to 4096, 16 from 8192 on): all of a lane's loads are in flight at once, and few warps meet.
-//     Rows that do not start on a 16-byte boundary are taken as the aligned vectors they span;
+//     Rows that do not start on a 16-byte boundary are taken as the aligned vectors they span; a result that lies differently
+//     against the boundary is written element by element, and beyond 8190 columns or so takes the way below;
 //   - a longer row is a thread-block cluster's: up to eight CTAs of 16,384 columns (beyond 131,072 columns 32,768), so that two
 //     CTAs share an SM; the row's maximum and sum meet in distributed shared memory;
 //   - beyond 262,144 columns one CTA walks the row three times.
@@ -46,7 +47,8 @@ __device__ __forceinline__ float quotient(float e, float sum, float reciprocal) 
 // kWarps warps hold a row, kVecs vectors per lane; with one warp per row a CTA has eight rows.
 // HBM bound.  8192 x 4096 softmax: 16 warps with two vectors per lane took 58.6 us, four with eight take 43.5 (6.2 TB/s);
 // 65,536 x 128: 69.6 us with 32 scalar loads per lane, 12.3 now.
-template <bool kSoftmax, int kWarps, int kVecs>
+// kAlike: a row of the result lies against the boundary like the row of the input; else it is written element by element.
+template <bool kSoftmax, int kWarps, int kVecs, bool kAlike = true>
 __global__ void __launch_bounds__(kWarps == 1 ? 256 : kWarps * 32) few_warps_kernel(const float* __restrict__ in, float* out, size_t rows,
                                                                                     size_t cols) {
     constexpr int T = kWarps * 32;
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(kWarps == 1 ? 256 : kWarps * 32) few_warps_ker
             const int j = k * T + tid;
             if (j > last) continue;
             const float4 q = make_float4(quotient(v[k].x, s, r), quotient(v[k].y, s, r), quotient(v[k].z, s, r), quotient(v[k].w, s, r));
-            if ((j == 0 && before > 0) || (j == last && after > 0)) {
+            if (!kAlike || (j == 0 && before > 0) || (j == last && after > 0)) {
                 const float c[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -253,21 +255,24 @@ cudaError_t launch_rows(const float* in, float* out, size_t rows, size_t cols, c
     const bool on_boundaries = cols % 4 == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0;
     const bool alike = !kSoftmax || (reinterpret_cast<uintptr_t>(in) - reinterpret_cast<uintptr_t>(out)) % 16 == 0;
     const size_t most = on_boundaries ? cols / 4 : (cols + 6) / 4;  // vectors a row spans
-    if (alike && most <= (size_t)kCtaThreads * kCtaVecs) {
-        auto launch = [&](void (*kernel)(const float*, float*, size_t, size_t), int warps) {
+    // A result that lies differently against the boundary than the input is written element by element, up to where the cluster
+    // kernel's scalar reads and writes take over (65,536 x 128: 416 -> 18.6 us, 4000 x 6001: 53.3 -> 39.1; 2000 x 12,001
+    // would take 49.3 so and takes 45.1 there).
+    if (most <= (alike ? (size_t)kCtaThreads * kCtaVecs : (size_t)2048)) {
+        auto launch = [&](void (*like)(const float*, float*, size_t, size_t), void (*unlike)(const float*, float*, size_t, size_t), int warps) {
             const unsigned blocks = (unsigned)(warps == 1 ? (rows + 7) / 8 : rows);
-            kernel<<<blocks, warps == 1 ? 256 : warps * 32, 0, stream>>>(in, out, rows, cols);
+            (alike ? like : unlike)<<<blocks, warps == 1 ? 256 : warps * 32, 0, stream>>>(in, out, rows, cols);
             return cudaGetLastError();
         };
-        if (most <= 32) return launch(few_warps_kernel<kSoftmax, 1, 1>, 1);
-        if (most <= 64) return launch(few_warps_kernel<kSoftmax, 1, 2>, 1);
-        if (most <= 128) return launch(few_warps_kernel<kSoftmax, 1, 4>, 1);
-        if (most <= 256) return launch(few_warps_kernel<kSoftmax, 1, 8>, 1);
-        if (most <= 512) return launch(few_warps_kernel<kSoftmax, 4, 4>, 4);
-        if (most <= 1024) return launch(few_warps_kernel<kSoftmax, 4, 8>, 4);
-        if (most <= 2048) return launch(few_warps_kernel<kSoftmax, 8, 8>, 8);
-        if (most <= 4096) return launch(few_warps_kernel<kSoftmax, 16, 8>, 16);
-        return launch(few_warps_kernel<kSoftmax, 16, 16>, 16);
+        if (most <= 32) return launch(few_warps_kernel<kSoftmax, 1, 1>, few_warps_kernel<kSoftmax, 1, 1, !kSoftmax>, 1);
+        if (most <= 64) return launch(few_warps_kernel<kSoftmax, 1, 2>, few_warps_kernel<kSoftmax, 1, 2, !kSoftmax>, 1);
+        if (most <= 128) return launch(few_warps_kernel<kSoftmax, 1, 4>, few_warps_kernel<kSoftmax, 1, 4, !kSoftmax>, 1);
+        if (most <= 256) return launch(few_warps_kernel<kSoftmax, 1, 8>, few_warps_kernel<kSoftmax, 1, 8, !kSoftmax>, 1);
+        if (most <= 512) return launch(few_warps_kernel<kSoftmax, 4, 4>, few_warps_kernel<kSoftmax, 4, 4, !kSoftmax>, 4);
+        if (most <= 1024) return launch(few_warps_kernel<kSoftmax, 4, 8>, few_warps_kernel<kSoftmax, 4, 8, !kSoftmax>, 4);
+        if (most <= 2048) return launch(few_warps_kernel<kSoftmax, 8, 8>, few_warps_kernel<kSoftmax, 8, 8, !kSoftmax>, 8);
+        if (most <= 4096) return launch(few_warps_kernel<kSoftmax, 16, 8>, nullptr, 16);
+        return launch(few_warps_kernel<kSoftmax, 16, 16>, nullptr, 16);
     }
     if (cols > (size_t)kCtaCols * kMaxCluster) {
         long_rows_kernel<kSoftmax><<<(unsigned)rows, kCtaThreads, 0, stream>>>(in, out, rows, cols);

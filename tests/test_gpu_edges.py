@@ -89,3 +89,40 @@ def test_lists_of_every_length(vocab, settings):
     logits[6, -1] = logits[6].max() + 1.0              # the last column
     _check(logits, vocab, do_sample=True, **settings)
     _check(logits, vocab, do_sample=False)
+
+
+@pytest.mark.parametrize("cols", [1, 3, 126, 128, 254, 512, 1021, 1023, 1025, 2046, 4093, 4096, 8187, 8189, 8192])
+@pytest.mark.parametrize("shift,out_shift", [(0, 1), (0, 2), (1, 0), (2, 1), (3, 2), (1, 3)])
+def test_softmax_into_a_buffer_that_lies_differently(cols, shift, out_shift):
+    import torch
+    rows = 19
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(cols * 16 + shift * 4 + out_shift)
+    x = torch.randn((rows * cols + 8,), generator=gen, device="cuda")[shift: shift + rows * cols].view(rows, cols)
+    flat = torch.full((rows * cols + 8,), float("nan"), device="cuda")
+    out = flat[out_shift: out_shift + rows * cols].view(rows, cols)
+    gh.ctx().softmax_rows(x, out=out)
+    want = torch.softmax(x.double(), dim=1)
+    assert ((out.double() - want).abs() / want).max().item() < 4e-6  # (as above)
+    assert flat[:out_shift].isnan().all() and flat[out_shift + rows * cols:].isnan().all()
+
+
+def test_a_narrow_softmax_into_a_buffer_that_lies_differently_takes_a_warp_per_row():
+    # 512 threads for a row of 128 columns took 34 times as long as a warp does; a scalar write in place of a vector 1.5 times
+    import torch
+    x = torch.randn((65536 * 128 + 4,), device="cuda")
+    like, other = x[:-4].view(65536, 128), x[1:-3].view(65536, 128)
+    out = torch.empty_like(like)
+
+    def best(source):
+        times = []
+        for _ in range(20):
+            begin, end = torch.cuda.Event(True), torch.cuda.Event(True)
+            begin.record()
+            gh.ctx().softmax_rows(source, out=out)
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times)
+
+    assert best(other) < 6 * best(like)
