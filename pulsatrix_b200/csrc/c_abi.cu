@@ -103,7 +103,19 @@ psx_status reserve(Buffer& b, size_t bytes) {
     return PSX_OK;
 }
 
-// The same for page-locked host memory.  (Nothing is in flight in it: the host entry points end with a synchronisation.)
+// A host entry point from its first copy on.  The staged inputs are being copied in by transfers just enqueued, so no promise about
+// inputs holds meanwhile; and however the call ends, nothing is in flight in the staging memory afterwards.
+struct StagedCall {
+    psx_ctx* ctx;
+    bool promised, drained = false;
+    explicit StagedCall(psx_ctx* c) : ctx(c), promised(c->inputs_ready) { ctx->inputs_ready = false; }
+    ~StagedCall() {
+        ctx->inputs_ready = promised;
+        if (!drained) cudaStreamSynchronize(ctx->stream);  // (on the way out with an error)
+    }
+};
+
+// The same for page-locked host memory.  (Nothing is in flight in it: see StagedCall.)
 psx_status reserve_pinned(Buffer& b, size_t bytes) {
     if (bytes <= b.bytes) return PSX_OK;
     if (b.ptr) PSX_CUDA(cudaFreeHost(b.ptr));
@@ -596,15 +608,10 @@ psx_status psx_b200_process_logits_host(psx_ctx* ctx, float* logits, int64_t row
     if (psx_status s = reserve(ctx->h_results, (size_t)rows * sizeof(int32_t))) return s;
     if (psx_status s = reserve_pinned(ctx->pinned_results, (size_t)rows * sizeof(int32_t))) return s;
     float* const device_rows = static_cast<float*>(ctx->h_logits.ptr);
+    StagedCall staged(ctx);
     HostInputs in;
     if (psx_status s = upload_inputs(ctx, stream, rows, history_ids, history_offsets, nullptr, in)) return s;
     if (psx_status s = copy_rows(ctx, stream, device_rows, logits, rows, vocab, row_stride, /*to_device=*/true)) return s;
-    struct RestorePromise {  // the staged inputs are being copied in by the transfers just enqueued
-        psx_ctx* ctx;
-        bool saved;
-        ~RestorePromise() { ctx->inputs_ready = saved; }
-    } restore{ctx, ctx->inputs_ready};
-    ctx->inputs_ready = false;
     if (psx_status s = psx_b200_process_logits(ctx, stream, device_rows, rows, vocab, vocab, in.history, in.offsets, config,
                                                static_cast<int32_t*>(ctx->h_results.ptr))) {
         return s;
@@ -614,6 +621,7 @@ psx_status psx_b200_process_logits_host(psx_ctx* ctx, float* logits, int64_t row
     PSX_CUDA(cudaStreamSynchronize(stream));  // (the ring is free again)
     if (psx_status s = copy_rows(ctx, stream, device_rows, logits, rows, vocab, row_stride, /*to_device=*/false)) return s;
     PSX_CUDA(cudaStreamSynchronize(stream));
+    staged.drained = true;
     if (row_status) std::memcpy(row_status, out_status, (size_t)rows * sizeof(int32_t));
     for (int64_t r = 0; r < rows; ++r) {
         if (out_status[r] != PSX_ROW_OK && out_status[r] != PSX_ROW_ALL_REMOVED) {
@@ -692,24 +700,18 @@ psx_status psx_b200_sample_rows_host(psx_ctx* ctx, const float* logits, int64_t 
     if (psx_status s = reserve(ctx->h_results, result_bytes)) return s;
     if (psx_status s = reserve_pinned(ctx->pinned_results, result_bytes)) return s;
     float* const device_rows = reinterpret_cast<float*>(static_cast<char*>(ctx->h_logits.ptr) + kLeadBytes);
+    StagedCall staged(ctx);
     HostInputs in;
     size_t lead = 0;
-    const bool staged = !copy_engine_reaches(logits);
+    const bool through_ring = !copy_engine_reaches(logits);
     if (psx_status s = upload_inputs(ctx, stream, rows, history_ids, history_offsets, config->do_sample ? uniforms : nullptr, in, device_rows,
-                                     staged ? &lead : nullptr)) {
+                                     through_ring ? &lead : nullptr)) {
         return s;
     }
     if (psx_status s = copy_rows(ctx, stream, device_rows, const_cast<float*>(logits), rows, vocab, row_stride, /*to_device=*/true,
                                  ctx->pinned_inputs.ptr, lead)) {
         return s;
     }
-    // The staged inputs are being copied in by the transfers just enqueued: no promise holds for them.
-    struct RestorePromise {
-        psx_ctx* ctx;
-        bool saved;
-        ~RestorePromise() { ctx->inputs_ready = saved; }
-    } restore{ctx, ctx->inputs_ready};
-    ctx->inputs_ready = false;
     // A few results: the kernels write them to the page-locked host memory themselves (it has the same address on the device), which saves
     // a copy behind them.
     char* const arrived = static_cast<char*>(ctx->pinned_results.ptr);
@@ -726,6 +728,7 @@ psx_status psx_b200_sample_rows_host(psx_ctx* ctx, const float* logits, int64_t 
     }
     if (!in_place) PSX_CUDA(cudaMemcpyAsync(arrived, results, result_bytes, cudaMemcpyDeviceToHost, stream));
     PSX_CUDA(cudaStreamSynchronize(stream));
+    staged.drained = true;
     std::memcpy(tokens, tokens_in(arrived), 8 * n);
     std::memcpy(log_probs, log_probs_in(arrived), 4 * n);
     std::memcpy(row_status, status_in(arrived), 4 * n);
