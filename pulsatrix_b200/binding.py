@@ -165,6 +165,13 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
+def _host_array(a):
+    """A numpy array as it is (the native calls take its address), any other host array's address."""
+    if a is None or (isinstance(a, np.ndarray) and a.ndim > 0):
+        return a
+    return a.ctypes.data if hasattr(a, "ctypes") else a.data_ptr()
+
+
 def _check(status):
     if status != OK:
         raise PsxError(status, library().psx_b200_last_error().decode())
@@ -210,7 +217,7 @@ def sample_rows_static(logits, history_ids, history_offsets, config, uniforms, t
         library()
     status_code = _native.sample_rows_static(
         _stream_of(logits) if stream is None else stream, logits.data_ptr(), rows, vocab, logits.stride(0) if rows else vocab,
-        _ptr(history_ids), _ptr(history_offsets), config, _ptr(uniforms), _ptr(tokens), _ptr(log_probs), _ptr(status))
+        _ptr(history_ids), _ptr(history_offsets), C.addressof(config), _ptr(uniforms), _ptr(tokens), _ptr(log_probs), _ptr(status))
     if status_code:
         _check(status_code)
 
@@ -293,7 +300,7 @@ class Context:
         out = out or self.alloc_outputs(rows)
         status = _native.sample_rows(
             self._handle, _stream_of(logits) if stream is None else stream, logits.data_ptr(), rows, vocab,
-            row_stride if rows else vocab, _ptr(history_ids), _ptr(history_offsets), config, _ptr(uniforms),
+            row_stride if rows else vocab, _ptr(history_ids), _ptr(history_offsets), C.addressof(config), _ptr(uniforms),
             out["tokens"].data_ptr(), out["log_probs"].data_ptr(), out["status"].data_ptr(), _ptr(out["diag"]))
         if status:
             _check(status)
@@ -346,8 +353,8 @@ class Context:
         rows, vocab = logits.shape
         status = np.zeros(rows, dtype=np.int32)
 
-        _check(_native.process_logits_host(self._handle, logits, rows, vocab, logits.strides[0] // 4, history_ids, history_offsets,
-                                           config, status))
+        _check(_native.process_logits_host(self._handle, _host_array(logits), rows, vocab, logits.strides[0] // 4, _host_array(history_ids),
+                                           _host_array(history_offsets), C.addressof(config), status))
         return status
 
     def row_pass_only(self, logits, history_ids, history_offsets, config, stream=None, vocab=None):
@@ -378,11 +385,8 @@ class Context:
         status = np.zeros(rows, dtype=np.int32)
         diag = np.zeros(rows, dtype=ROW_DIAG_DTYPE)
 
-        def host(a):  # numpy arrays give their address themselves
-            return a.data_ptr() if hasattr(a, "data_ptr") else a
-
-        rc = _native.sample_rows_host(self._handle, host(logits), rows, vocab, row_stride, host(history_ids), host(history_offsets),
-                                      config, host(uniforms), tokens, logp, status, diag)
+        rc = _native.sample_rows_host(self._handle, _host_array(logits), rows, vocab, row_stride, _host_array(history_ids), _host_array(history_offsets),
+                                      C.addressof(config), _host_array(uniforms), tokens, logp, status, diag)
         if rc != OK and (rc != ERR_ROW_FAILED or raise_on_row_failure):
             _check(rc)
         return tokens, logp, status, diag
@@ -417,7 +421,7 @@ class Context:
         out = out or self.alloc_outputs(rows)
         _check(_native.lm_head_sample_rows(
             self._handle, _stream_of(hidden) if stream is None else stream, hidden.data_ptr(), rows, d, weight.data_ptr(), vocab,
-            0 if vocab_by_d else 1, _ptr(history_ids), _ptr(history_offsets), config, _ptr(uniforms), _ptr(out["tokens"]),
+            0 if vocab_by_d else 1, _ptr(history_ids), _ptr(history_offsets), C.addressof(config), _ptr(uniforms), _ptr(out["tokens"]),
             _ptr(out["log_probs"]), _ptr(out["status"]), _ptr(out["diag"])))
         return out
 
@@ -469,7 +473,7 @@ class Context:
     def shard_scan(self, shard_logits, shard_begin, vocab, history_ids, history_offsets, config, records, stream=None):
         rows, cols = shard_logits.shape
         _check(_native.shard_scan(self._handle, _stream_of(shard_logits) if stream is None else stream, shard_logits.data_ptr(), rows,
-                                  cols, shard_logits.stride(0), shard_begin, vocab, _ptr(history_ids), _ptr(history_offsets), config,
+                                  cols, shard_logits.stride(0), shard_begin, vocab, _ptr(history_ids), _ptr(history_offsets), C.addressof(config),
                                   _ptr(records)))
 
     def shard_merge(self, gathered, num_shards, rows, vocab, config, uniforms, out=None, stream=None, row_begin=0,
@@ -479,7 +483,7 @@ class Context:
         row_count = rows - row_begin if row_count is None else row_count
         out = out or self.alloc_outputs(row_count)
         _check(_native.shard_merge_rows(self._handle, _stream_of(gathered) if stream is None else stream, gathered.data_ptr(), num_shards,
-                                        rows, row_begin, row_count, vocab, config, _ptr(uniforms), _ptr(out["tokens"]),
+                                        rows, row_begin, row_count, vocab, C.addressof(config), _ptr(uniforms), _ptr(out["tokens"]),
                                         _ptr(out["log_probs"]), _ptr(out["status"]), _ptr(out.get("diag"))))
         return out
 
@@ -520,7 +524,7 @@ class Exchange:
         if rows != self.rows:
             raise ValueError(f"the exchange was created for {self.rows} rows, got {rows}")
         _check(_native.exchange_sample(self._ex.value, _stream_of(shard_logits) if stream is None else stream, shard_logits.data_ptr(),
-                                       cols, shard_logits.stride(0), shard_begin, vocab, _ptr(history_ids), _ptr(history_offsets), config,
+                                       cols, shard_logits.stride(0), shard_begin, vocab, _ptr(history_ids), _ptr(history_offsets), C.addressof(config),
                                        _ptr(uniforms)))
         return self.results(shard_logits.device)
 

@@ -2,7 +2,7 @@
 //
 // A decoding step's GPU work is of the order of ten microseconds, and a call of fourteen arguments through ctypes spends
 // half of that on converting them.  Here a call is one vectorcall into C: integers become pointers and sizes, None is a
-// null pointer, anything with a buffer (numpy arrays, ctypes structures) its address.  The functions return the
+// null pointer, and where the entry point takes an array of numbers an array is its own address.  The functions return the
 // psx_status; binding.py turns it into exceptions.  The library is the one that binding.py has loaded: load(path) looks
 // the entry points up there, so that both see the same one.
 #define PY_SSIZE_T_CLEAN
@@ -19,7 +19,9 @@
 
 namespace {
 
-// The address that a pointer argument stands for.
+// The address that a pointer argument stands for.  Handles, streams and settings (T is not a pointer to numbers or to
+// psx_row_diag) are integers; a numpy scalar, which has a buffer of its own, is neither an integer nor an array here.
+template <class T>
 bool address_of(PyObject* o, void** out) {
     if (o == Py_None) {
         *out = nullptr;
@@ -29,18 +31,23 @@ bool address_of(PyObject* o, void** out) {
         *out = PyLong_AsVoidPtr(o);
         return !PyErr_Occurred();
     }
-    Py_buffer view;
-    if (PyObject_GetBuffer(o, &view, PyBUF_STRIDES) != 0) return false;
-    *out = view.buf;  // (the caller's frame keeps the object, and with it the memory, for the length of the call)
-    PyBuffer_Release(&view);
-    return true;
+    if constexpr (std::is_arithmetic_v<std::remove_pointer_t<T>> || std::is_same_v<T, psx_row_diag*>) {
+        Py_buffer view;
+        if (PyObject_GetBuffer(o, &view, PyBUF_STRIDES) != 0) return false;
+        *out = view.buf;  // (the caller's frame keeps the object, and with it the memory, for the length of the call)
+        const int dimensions = view.ndim;
+        PyBuffer_Release(&view);
+        if (dimensions > 0) return true;
+    }
+    PyErr_Format(PyExc_TypeError, "%s where an address is expected", Py_TYPE(o)->tp_name);
+    return false;
 }
 
 template <class T>
 bool convert(PyObject* o, T* out) {
     if constexpr (std::is_pointer_v<T>) {
         void* p = nullptr;
-        if (!address_of(o, &p)) return false;
+        if (!address_of<T>(o, &p)) return false;
         *out = reinterpret_cast<T>(p);
     } else if constexpr (std::is_floating_point_v<T>) {
         *out = static_cast<T>(PyFloat_AsDouble(o));

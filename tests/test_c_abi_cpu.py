@@ -79,3 +79,40 @@ def test_exchange_entry_points_check_their_arguments_before_touching_a_gpu(lib):
     assert lib.psx_b200_exchange_results(None, None, None) == binding.ERR_BAD_ARGUMENT
     assert lib.psx_b200_exchange_test_wait(None, 0, 0) == binding.ERR_BAD_ARGUMENT
     lib.psx_b200_exchange_destroy(None)  # a null exchange is nothing to destroy
+
+
+def test_native_calls_take_addresses_and_arrays_of_numbers_only(lib):
+    native, row = binding._native, np.zeros(4, dtype=np.float32)
+    cfg = binding.SamplingConfig.make(do_sample=False)
+
+    def softmax(context=None, stream=0, x=row):
+        return native.softmax_rows(context, stream, x, x, 1, 4)
+
+    assert softmax() == binding.ERR_BAD_ARGUMENT and softmax(stream=None) == binding.ERR_BAD_ARGUMENT  # (no context)
+    assert softmax(x=row.ctypes.data) == binding.ERR_BAD_ARGUMENT
+    for refused in (dict(stream=np.int64(0)), dict(stream=np.uint64(0)), dict(stream=row), dict(context=row), dict(context=np.int64(0)),
+                    dict(stream=b"12345678"), dict(stream=0.0), dict(x=np.float32(1.0)), dict(x=1.5), dict(x="row")):
+        with pytest.raises(TypeError):
+            softmax(**refused)
+
+    def sample(config):
+        return native.sample_rows_static(0, None, 0, 4, 4, None, None, config, None, None, None, None)
+
+    assert sample(C.addressof(cfg)) == binding.OK  # (no rows)
+    for refused in (np.zeros(8, dtype=np.uint8), b"1234", np.int64(0), cfg):
+        with pytest.raises(TypeError):
+            sample(refused)
+
+
+def test_settings_are_a_ctypes_structure(lib):
+    # (as through ctypes: anything else is refused before its bytes are read)
+    class Rows:
+        shape = (0, 4)
+
+        def data_ptr(self):
+            return 0
+
+    for refused in (None, np.zeros(8, dtype=np.uint8), b"1234"):
+        with pytest.raises(TypeError):
+            psx.sample_rows_static(Rows(), None, None, refused, None, None, None, None, stream=0)
+    psx.sample_rows_static(Rows(), None, None, psx.SamplingConfig.make(do_sample=False), None, None, None, None, stream=0)
