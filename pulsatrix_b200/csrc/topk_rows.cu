@@ -718,18 +718,10 @@ cudaError_t launch_topk_rows(const float* in, float* values, float* indices, siz
     else if (held) kernel = largest ? topk_rows_kernel<true, true, kWidest> : topk_rows_kernel<false, true, kWidest>;
     const size_t shared = entries * 8 + (p.in_shared ? (size_t)p.slice * 4 + 32 : held ? (p.slice / 4 + threads - 1) / threads * threads * 16 + 32 : 0);
     if (rows * (size_t)p.cluster > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
-    if (shared > 48 * 1024) {
-        // Once per device and kernel (the call sets the same value every time, so two host threads
-        // that both find the flag clear do no harm).
-        static bool lifted[8][64] = {};
-        int device = 0;
-        if (cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return e;
-        bool& done = lifted[(largest ? 1 : 0) + (!held ? 0 : threads == 64 ? 2 : threads == 128 ? 4 : 6)][device & 63];
-        if (!done) {
-            if (const cudaError_t e = allow_all_dynamic_shared(kernel); e != cudaSuccess) return e;
-            done = true;
-        }
-    }
+    // (whatever the size: what a block may use without asking counts the kernel's own arrays as well)
+    static OncePerDevice lifted[8];
+    OncePerDevice& done = lifted[(largest ? 1 : 0) + (!held ? 0 : threads == 64 ? 2 : threads == 128 ? 4 : 6)];
+    if (const cudaError_t e = allow_all_dynamic_shared_once(done, kernel); e != cudaSuccess) return e;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)(rows * p.cluster));
     config.blockDim = dim3((unsigned)threads);

@@ -104,3 +104,33 @@ def test_argument_errors_use_the_reference_wording():
         assert err.value.status == 1 and "top_k: k must be in [1, 4]" in str(err.value)
     values, indices = gh.ctx().top_k_rows(torch.zeros((0, 4), device="cuda"), 2)
     assert values.shape == (0, 2)
+
+
+_SIZES_IN_A_FRESH_PROCESS = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import torch
+import pulsatrix_b200 as psx
+ctx, failed = psx.Context(0), []
+for k in (1, 16, 64, 300):
+    for largest in (True, False):
+        for cols in range(9000, 13000, 124):
+            x = torch.randn((3, cols), device="cuda")
+            try:
+                values, _ = ctx.top_k_rows(x, k, largest=largest)
+                if not torch.equal(values, torch.topk(x, k, largest=largest).values):
+                    failed.append((k, largest, cols, "values"))
+            except psx.PsxError as error:
+                failed.append((k, largest, cols, str(error)))
+assert not failed, (len(failed), failed[:4])
+"""
+
+
+def test_sizes_around_the_default_shared_memory_limit_in_a_fresh_process():
+    # A block may use 48 KB without asking, its kernel's own arrays included; the sizes ascend, so nothing has asked before.
+    import subprocess
+    import sys
+    from pathlib import Path
+    root = Path(psx.__file__).resolve().parent.parent
+    out = subprocess.run([sys.executable, "-c", _SIZES_IN_A_FRESH_PROCESS, str(root)], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
