@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
                 return;
             }
         }
-        if (tid == 0) s_listed = 0;
+        // (s_listed stays as it is: a warp that is late has yet to read it, and all have to come to the same verdict)
         for (int i = tid; i < 2 * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
         meet();  // (the cluster adds its histograms up)
     }

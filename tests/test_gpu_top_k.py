@@ -134,3 +134,24 @@ def test_sizes_around_the_default_shared_memory_limit_in_a_fresh_process():
     root = Path(psx.__file__).resolve().parent.parent
     out = subprocess.run([sys.executable, "-c", _SIZES_IN_A_FRESH_PROCESS, str(root)], capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stderr[-2000:]
+
+
+@pytest.mark.parametrize("largest", [True, False])
+def test_many_rows_whose_lists_overflow(largest):
+    # Thousands of rows of a few values each leave the short way at once, blocks beside blocks: every warp of a block has to.
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(12)
+    for rows, cols, k in ((8192, 1000, 8), (4096, 3001, 31), (2048, 9000, 16), (1024, 16384, 64), (512, 40000, 100)):
+        x = torch.randint(0, 3, (rows, cols), generator=gen, device="cuda").float()
+        x[::2] = 0.5
+        x[1::4] = -float("inf") if largest else float("inf")
+        x[1::4, 3] = 7.0
+        first = None
+        for _ in range(5):
+            values, indices = gh.ctx().top_k_rows(x, k, largest)
+            assert torch.equal(values, torch.topk(x, k, largest=largest).values)
+            # equal values by ascending column: a stable sort
+            want = torch.sort(x, dim=1, descending=largest, stable=True).indices[:, :k].float() if first is None else first
+            assert torch.equal(indices, want)
+            first = want
