@@ -10,7 +10,7 @@
 // 67.9 now; 8192 x 4096, k 16: 63.5 -> 34.8 us.  Sweep one notes every thread's best entry; the smallest over the warps of
 // the kp-th best of those (kp = ceil(k / 8)) is a bound that k entries of the slice reach.  Sweep
 // two lists what reaches the bound, usually k and a few; the list is put in rank order by
-// counting, and with several CTAs per row the best k of each meet in the first CTA's shared memory
+// counting (beyond 256 entries by sorting), and with several CTAs per row the best k of each meet in the first CTA's shared memory
 // (distributed shared memory, two cluster barriers), where each finds its place in the others' lists by bisection.
 //
 // The long way (larger k, or a list that overflowed: thousands of ties): the slice becomes keys in
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
     // ---- 0. the short way (k <= 256): two sweeps over the slice as floats, the second one out of L2.
     //      Sweep one notes every thread's best entry; a bound that k of those reach is a lower bound of
     //      the slice's k-th best.  Sweep two lists what reaches the bound, usually k and a few; the list
-    //      is put in rank order by counting, and the best k of every CTA meet in the first CTA. ----------
+    //      is put in rank order, and the best k of every CTA meet in the first CTA. ----------
     if (p.list_cap != 0) {  // uniform over the cluster
         __shared__ uint32_t s_warp_bound[kThreads / 32];
         constexpr int kBatch = 8;  // loads in flight per thread
@@ -379,35 +379,45 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
                     gathered0[place] = entry;
                 }
             };
-            // An entry's place by looking at all the others' keys, four at a time; neighbouring threads share an entry when there are
-            // threads left over.  Entries with equal keys find themselves at the same place: then (rare) the columns are looked at too.
-            uint32_t n_pad = 8;
-            while (n_pad < on_list && n_pad < (uint32_t)kThreads) n_pad <<= 1;
-            const uint32_t share = (uint32_t)kThreads / n_pad < 32u ? (uint32_t)kThreads / n_pad : 32u, slice = tid & (share - 1);
-            const uint32_t quads = (on_list + 3) / 4, per_round = (uint32_t)kThreads / share;  // (zeros behind the list)
-            bool tied = false;
-            for (uint32_t first = 0; first < on_list; first += per_round) {
-                const uint32_t i = first + (uint32_t)tid / share;
-                if (first + (uint32_t)(tid & ~31) / share >= on_list) break;  // (nothing for this warp)
-                const uint32_t key = i < on_list ? list_key[i] : ~0u;
-                uint32_t place = 0;
-#pragma unroll 4
-                for (uint32_t j = slice; j < quads; j += share) {
-                    const uint4 other = reinterpret_cast<const uint4*>(list_key)[j];
-                    place += (other.x > key ? 1u : 0u) + (other.y > key ? 1u : 0u) + (other.z > key ? 1u : 0u) + (other.w > key ? 1u : 0u);
-                }
-                for (uint32_t o = share >> 1; o > 0; o >>= 1) place += __shfl_xor_sync(0xFFFFFFFFu, place, o);
-                if (slice == 0 && i < on_list && place < best) {
-                    if (atomicAdd(&claimed[place], 1u) != 0) tied = true;
-                    place_entry(list[i], place);
-                }
-            }
-            if (__syncthreads_or(tied ? 1 : 0) != 0) {
-                for (uint32_t i = tid; i < on_list; i += kThreads) {
-                    const u64 entry = list[i];
+            if (!kHeld && on_list > (uint32_t)kWidest) {  // (held slices: k is at most 64, and a list holds 256)
+                // a long list: sorting it takes fewer steps than looking at all the others (4096 x 1000, k 256: 594 us so, 300 sorted)
+                uint32_t n_pad = 2 * kWidest;
+                while (n_pad < on_list) n_pad <<= 1;
+                for (uint32_t i = on_list + tid; i < n_pad; i += kThreads) list[i] = 0;
+                __syncthreads();
+                block_bitonic_sort(list, (int)n_pad, /*descending=*/true);
+                for (uint32_t i = tid; i < best; i += kThreads) place_entry(list[i], i);
+            } else {
+                // An entry's place by looking at all the others' keys, four at a time; neighbouring threads share an entry when there are
+                // threads left over.  Entries with equal keys find themselves at the same place: then (rare) the columns are looked at too.
+                uint32_t n_pad = 8;
+                while (n_pad < on_list && n_pad < (uint32_t)kThreads) n_pad <<= 1;
+                const uint32_t share = (uint32_t)kThreads / n_pad < 32u ? (uint32_t)kThreads / n_pad : 32u, slice = tid & (share - 1);
+                const uint32_t quads = (on_list + 3) / 4, per_round = (uint32_t)kThreads / share;  // (zeros behind the list)
+                bool tied = false;
+                for (uint32_t first = 0; first < on_list; first += per_round) {
+                    const uint32_t i = first + (uint32_t)tid / share;
+                    if (first + (uint32_t)(tid & ~31) / share >= on_list) break;  // (nothing for this warp)
+                    const uint32_t key = i < on_list ? list_key[i] : ~0u;
                     uint32_t place = 0;
-                    for (uint32_t j = 0; j < on_list; ++j) place += list[j] > entry ? 1u : 0u;
-                    place_entry(entry, place);
+#pragma unroll 4
+                    for (uint32_t j = slice; j < quads; j += share) {
+                        const uint4 other = reinterpret_cast<const uint4*>(list_key)[j];
+                        place += (other.x > key ? 1u : 0u) + (other.y > key ? 1u : 0u) + (other.z > key ? 1u : 0u) + (other.w > key ? 1u : 0u);
+                    }
+                    for (uint32_t o = share >> 1; o > 0; o >>= 1) place += __shfl_xor_sync(0xFFFFFFFFu, place, o);
+                    if (slice == 0 && i < on_list && place < best) {
+                        if (atomicAdd(&claimed[place], 1u) != 0) tied = true;
+                        place_entry(list[i], place);
+                    }
+                }
+                if (__syncthreads_or(tied ? 1 : 0) != 0) {
+                    for (uint32_t i = tid; i < on_list; i += kThreads) {
+                        const u64 entry = list[i];
+                        uint32_t place = 0;
+                        for (uint32_t j = 0; j < on_list; ++j) place += list[j] > entry ? 1u : 0u;
+                        place_entry(entry, place);
+                    }
                 }
             }
             if (ranks == 1) return;
@@ -710,7 +720,9 @@ cudaError_t launch_topk_rows(const float* in, float* values, float* indices, siz
     p.in_shared = p.list_cap == 0 && p.slice <= (uint32_t)kSliceMax &&
                   entries * 8 + (size_t)p.slice * 4 + 4096 <= 227 * 1024 ? 1 : 0;
     p.wait_limit_ns = kDefaultWaitLimitNs;
-    const bool held = p.list_cap != 0 && p.slice <= kHeldMax;
+    // Beyond k 64 the lists grow long and overflow more often, and a block that holds its slice has fewer beside it to hide the
+    // radix selection: 4096 x 16,384, k 256: 840 us with held slices, 548 without (k 100: 125 and 121; 4096 x 4096, k 128: 99 and 106).
+    const bool held = p.list_cap != 0 && p.slice <= kHeldMax && k <= 64;
     const int threads = !held || k > 32 ? kWidest : p.slice <= 4096 && k <= 32 ? 64 : 128;
     auto kernel = largest ? topk_rows_kernel<true, false, kWidest> : topk_rows_kernel<false, false, kWidest>;
     if (held && threads == 64) kernel = largest ? topk_rows_kernel<true, true, 64> : topk_rows_kernel<false, true, 64>;

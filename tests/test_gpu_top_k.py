@@ -155,3 +155,19 @@ def test_many_rows_whose_lists_overflow(largest):
             want = torch.sort(x, dim=1, descending=largest, stable=True).indices[:, :k].float() if first is None else first
             assert torch.equal(indices, want)
             first = want
+
+
+@pytest.mark.parametrize("cols", [300, 1000, 2047, 16384, 40000])
+@pytest.mark.parametrize("k", [64, 65, 100, 200, 256])
+def test_long_lists(k, cols):
+    # up to and beyond 256 entries on a list: exactly 257, all there are, ties at every place, one CTA and several
+    rng = np.random.RandomState(k + cols)
+    for largest in (True, False):
+        x = rng.randn(5, cols).astype(np.float32)
+        x[1, : cols // 2] = x[1, cols // 2: 2 * (cols // 2)]
+        x[2] = np.round(x[2] * 50)
+        x[3, rng.permutation(cols)[:257]] += 20.0 if largest else -20.0
+        x[4, rng.randint(cols, size=7)] = np.nan
+        values, indices = gpu_top_k(x, k, largest, shift=1)
+        want_values, want_indices = ol.top_k_rows("oracle", x, k, largest)
+        assert same_bits(values, want_values) and (indices == want_indices).all()
