@@ -151,6 +151,170 @@ __device__ __forceinline__ Found find_digit(cg::cluster_group& cluster, uint32_t
     return f;
 }
 
+// The long way (k > 256, or a list that overflowed: ties in the thousands), by the whole cluster over its slices.
+// held4: the slice from its first 16-byte boundary on as floats in shared memory, or null.
+template <bool kLargest, bool kHeld, int kThreads>
+__device__ __forceinline__ void select_row(const TopKParams& p, u64* collected, uint32_t* keys, const float4* held4) {
+    // histograms, used in turn by the passes; a pass clears the one before it once the cluster has met again (nobody reads it any more)
+    __shared__ __align__(16) uint32_t s_hist[2][256];
+    __shared__ uint32_t s_prefix, s_remaining, s_inside, s_collected;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), ranks = p.cluster;
+    const size_t row_index = blockIdx.x / (unsigned)p.cluster;
+    constexpr bool largest = kLargest;
+    const float* row = p.in + row_index * p.cols;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t n = (uint32_t)p.cols;
+    const uint32_t begin = min(n, (uint32_t)rank * p.slice), mine = min(n, begin + p.slice) - begin;
+    const bool in_shared = p.in_shared != 0;
+    const float* src = row + begin;
+    const uint32_t head = min(mine, (uint32_t)((4 - ((reinterpret_cast<uintptr_t>(src) >> 2) & 3)) & 3));
+    const uint32_t vectors = (mine - head) / 4;
+    const float4* src4 = reinterpret_cast<const float4*>(src + head);
+    float* out_v = p.values + row_index * p.k;
+    float* out_i = p.indices + row_index * p.k;
+    // The cluster's barrier costs about a microsecond; one CTA on its own meets with the block barrier.
+    auto meet = [&]() {
+        if (ranks > 1) cluster.sync(); else __syncthreads();
+    };
+    for (int i = tid; i < 2 * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
+    if (tid == 0) s_collected = 0;
+
+    // ---- 0. the slice as keys in shared memory, where it fits ------------------------------------------------
+    if (in_shared) {
+        // keys[head] on a 16-byte boundary, like src[head]: the array starts up to three words in
+        keys = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(keys) + 15) & ~uintptr_t(15)) + ((4 - head) & 3);
+        for (uint32_t i = tid; i < head; i += kThreads) keys[i] = rank_key(src[i], largest);
+        uint4* keys4 = reinterpret_cast<uint4*>(keys + head);
+        constexpr int kBatch = 8;  // loads in flight per thread
+        for (uint32_t v0 = tid; v0 < vectors; v0 += kBatch * kThreads) {
+            float4 d[kBatch];
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const uint32_t v = v0 + q * kThreads;
+                d[q] = v < vectors ? __ldg(src4 + v) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const uint32_t v = v0 + q * kThreads;
+                if (v < vectors) {
+                    keys4[v] = make_uint4(rank_key(d[q].x, largest), rank_key(d[q].y, largest), rank_key(d[q].z, largest),
+                                          rank_key(d[q].w, largest));
+                }
+            }
+        }
+        for (uint32_t i = head + 4 * vectors + tid; i < mine; i += kThreads) keys[i] = rank_key(src[i], largest);
+    }
+    __syncthreads();
+    auto slice_key = [&](uint32_t i) { return in_shared ? keys[i] : rank_key(src[i], largest); };
+
+    // visit(key, column) for every entry of the slice: four at a time where the slice lies in shared memory
+    auto each_entry = [&](auto visit) {
+        if (kHeld && held4 != nullptr) {
+            for (uint32_t i = tid; i < head; i += kThreads) visit(rank_key(src[i], largest), begin + i);
+            for (uint32_t v = tid; v < vectors; v += kThreads) {
+                const float4 d = held4[v];
+                const uint32_t col = begin + head + 4 * v;
+                visit(rank_key(d.x, largest), col);
+                visit(rank_key(d.y, largest), col + 1);
+                visit(rank_key(d.z, largest), col + 2);
+                visit(rank_key(d.w, largest), col + 3);
+            }
+            for (uint32_t i = head + 4 * vectors + tid; i < mine; i += kThreads) visit(rank_key(src[i], largest), begin + i);
+        } else {
+            for (uint32_t i = tid; i < mine; i += kThreads) visit(slice_key(i), begin + i);
+        }
+    };
+    const int first_rank = 0;
+
+    // ---- 1. radix select of the k-th key ---------------------------------------------------------------
+    uint32_t prefix = 0, mask = 0, remaining = (uint32_t)p.k, inside = 0;
+    for (int pass = 0; pass < 4; ++pass) {
+        const int shift = 24 - 8 * pass;
+        uint32_t* hist = s_hist[pass & 1];
+        each_entry([&](uint32_t key, uint32_t) {
+            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
+        });
+        meet();
+        if (pass > 0) {
+            for (int i = tid; i < 256; i += kThreads) s_hist[(pass - 1) & 1][i] = 0;
+        }
+        if (tid < 32) {
+            const Found f = find_digit(cluster, hist, first_rank, ranks, remaining, lane);
+            if (lane == 0) {
+                s_prefix = prefix | (f.digit << shift);
+                s_remaining = remaining - f.above;
+                s_inside = f.inside;
+            }
+        }
+        __syncthreads();
+        prefix = s_prefix;
+        remaining = s_remaining;
+        inside = s_inside;
+        mask |= 255u << shift;
+    }
+    const uint32_t kth = prefix;
+    const uint32_t ties_wanted = remaining;  // entries equal to the k-th key to take; `inside` entries equal it
+
+    // ---- 2. more ties than wanted: the column up to which they are taken ------------------------------------
+    uint32_t last_tie_column = 0xFFFFFFFFu;
+    if (inside > ties_wanted) {  // uniform over the cluster
+        uint32_t cprefix = 0, cmask = 0, cremaining = ties_wanted;
+        for (int pass = 0; pass < 3; ++pass) {
+            const int shift = 16 - 8 * pass;
+            uint32_t* hist = s_hist[pass & 1];  // the key's four passes left [0] cleared and [1] to clear
+            each_entry([&](uint32_t key, uint32_t col) {
+                const uint32_t inverted = ~col & 0x00FFFFFFu;  // lower columns rank higher; columns are below 2^24
+                if (key == kth && (inverted & cmask) == cprefix) atomicAdd(&hist[(inverted >> shift) & 255u], 1u);
+            });
+            meet();
+            for (int i = tid; i < 256; i += kThreads) s_hist[(pass + 1) & 1][i] = 0;
+            if (tid < 32) {
+                const Found f = find_digit(cluster, hist, first_rank, ranks, cremaining, lane);
+                if (lane == 0) {
+                    s_prefix = cprefix | (f.digit << shift);
+                    s_remaining = cremaining - f.above;
+                }
+            }
+            __syncthreads();
+            cprefix = s_prefix;
+            cremaining = s_remaining;
+            cmask |= 255u << shift;
+        }
+        last_tie_column = ~cprefix & 0x00FFFFFFu;
+    }
+
+    // ---- 3. collect in the first CTA, sort there, write -------------------------------------------------------
+    {
+        uint32_t* count0 = cluster.map_shared_rank(&s_collected, first_rank);
+        u64* collected0 = cluster.map_shared_rank(collected, first_rank);
+        each_entry([&](uint32_t key, uint32_t col) {
+            if (key > kth || (key == kth && col <= last_tie_column)) {
+                const uint32_t slot = atomicAdd(count0, 1u);
+                if (slot < p.k_pad) collected0[slot] = ((u64)key << 32) | (uint32_t)~col;
+            }
+        });
+    }
+    meet();  // nobody touches another CTA's shared memory after this
+    if (rank != 0) return;
+    const uint32_t taken = min(s_collected, (uint32_t)p.k);  // == k
+    for (uint32_t i = taken + tid; i < p.k_pad; i += kThreads) collected[i] = 0;
+    __syncthreads();
+    if (p.k_pad > 1) block_bitonic_sort(collected, (int)p.k_pad, /*descending=*/true);
+    for (uint32_t j = tid; j < taken; j += kThreads) {
+        const uint32_t col = ~(uint32_t)collected[j];
+        out_v[j] = row[col];
+        out_i[j] = (float)col;
+    }
+}
+
+// The same as a call, so that the short way of a held slice has the registers to itself (4096 x 16,384, k 64: 77.8 us with the long way
+// in line, 73.7 so); without a held slice the long way is the usual one and stays in line (k 256: 483 us, called 784).
+template <bool kLargest, int kThreads>
+__device__ __noinline__ void select_held_row(const TopKParams& p, u64* collected, uint32_t* keys, const float4* held4) {
+    select_row<kLargest, true, kThreads>(p, collected, keys, held4);
+}
+
 // kHeld: the short way keeps its slice (at most kHeldMax entries) in shared memory, where four bulk copies bring it, each on a barrier of its
 // own; the sweeps read it from there.
 // kThreads: most of a CTA's instructions are a warp's own (its bound, its entries, their places), whatever its share of the
@@ -166,10 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
     uint32_t* claimed = list_key + p.list_cap;                            // entries that found themselves at a place
     u64* gathered = reinterpret_cast<u64*>(claimed + p.list_cap);
     uint32_t* keys = reinterpret_cast<uint32_t*>(gathered + (size_t)p.k_pad * (p.cluster > 1 && p.list_cap != 0 ? p.cluster : 0));
-    // histograms of the long way, used in turn by its passes; a pass clears the one before it once the
-    // cluster has met again (nobody reads it any more)
-    __shared__ __align__(16) uint32_t s_hist[2][256];
-    __shared__ uint32_t s_prefix, s_remaining, s_inside, s_collected, s_listed, s_overflow;
+    __shared__ uint32_t s_listed, s_overflow;
 
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
@@ -181,7 +342,6 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
     const uint32_t n = (uint32_t)p.cols;
     const uint32_t begin = min(n, (uint32_t)rank * p.slice), end = min(n, begin + p.slice);
     const uint32_t mine = end - begin;
-    const bool in_shared = p.in_shared != 0;
     // the slice from its first 16-byte boundary on, as vectors; up to three entries before them and after them
     const float* src = row + begin;
     const uint32_t head = min(mine, (uint32_t)((4 - ((reinterpret_cast<uintptr_t>(src) >> 2) & 3)) & 3));
@@ -205,17 +365,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
         const float worst = kLargest ? -INFINITY : INFINITY;
         held4[(trips - 1) * kThreads + tid] = make_float4(worst, worst, worst, worst);
     }
-    // The cluster's barrier costs about a microsecond; one CTA on its own meets with the block barrier.
-    auto meet = [&]() {
-        if (ranks > 1) cluster.sync(); else __syncthreads();
-    };
-
     for (uint32_t i = tid; i < p.list_cap / 2; i += kThreads) reinterpret_cast<uint4*>(list_key)[i] = make_uint4(0, 0, 0, 0);  // (claimed, too)
-    if (p.list_cap == 0) {
-        for (int i = tid; i < 2 * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
-    }
     if (tid == 0) {
-        s_collected = 0;
         s_listed = 0;
         s_overflow = 0;
     }
@@ -223,6 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
     float* out_v = p.values + row_index * p.k;
     float* out_i = p.indices + row_index * p.k;
 
+    bool held_here = false;  // the slice lies in shared memory as floats
     // ---- 0. the short way (k <= 256): two sweeps over the slice as floats, the second one out of L2.
     //      Sweep one notes every thread's best entry; a bound that k of those reach is a lower bound of
     //      the slice's k-th best.  Sweep two lists what reaches the bound, usually k and a few; the list
@@ -291,6 +443,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
             for (uint32_t c = 0; c * kHeldChunk < vectors; ++c) barrier_wait_bounded(&s_bar[c], 0, p.wait_limit_ns);
             landed = false;
         }
+        held_here = kHeld && landed;
         const float edge = largest ? from_ordered_key(bound) : from_ordered_key(~bound);
         const bool everything = bound == 0 && landed, only_nan = edge != edge || !landed;  // (or only what no number lies below)
         auto reaches = [&](float x) { return largest ? !(x < edge) : x <= edge; };
@@ -363,7 +516,9 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
         }
         __syncthreads();
         const uint32_t on_list = s_listed;
-        const bool fits = on_list <= p.list_cap;
+        // (A list of the whole slice is a row of equal values, as a rule: the radix selection is faster than telling them apart.  16,384
+        // constant rows of 200, k 8: 310 us, 163 so.)
+        const bool fits = on_list <= p.list_cap && (everything || on_list < mine);
         const uint32_t best = min(on_list, (uint32_t)p.k);  // entries of this CTA that can be among the row's k best
         // Where the best entries go: straight out (one CTA), or into this CTA's k_pad slots of the
         // first CTA's array.  An entry's place is the number of entries that rank before it.
@@ -457,127 +612,9 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
             }
         }
         // (s_listed stays as it is: a warp that is late has yet to read it, and all have to come to the same verdict)
-        for (int i = tid; i < 2 * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
-        meet();  // (the cluster adds its histograms up)
     }
-
-    // ---- the slice as keys in shared memory, for the long way ----------------------------------------------
-    if (in_shared) {
-        // keys[head] on a 16-byte boundary, like src[head]: the array starts up to three words in
-        keys = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(keys) + 15) & ~uintptr_t(15)) + ((4 - head) & 3);
-        for (uint32_t i = tid; i < head; i += kThreads) keys[i] = rank_key(src[i], largest);
-        uint4* keys4 = reinterpret_cast<uint4*>(keys + head);
-        constexpr int kBatch = 8;  // loads in flight per thread
-        for (uint32_t v0 = tid; v0 < vectors; v0 += kBatch * kThreads) {
-            float4 d[kBatch];
-#pragma unroll
-            for (int q = 0; q < kBatch; ++q) {
-                const uint32_t v = v0 + q * kThreads;
-                d[q] = v < vectors ? __ldg(src4 + v) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-#pragma unroll
-            for (int q = 0; q < kBatch; ++q) {
-                const uint32_t v = v0 + q * kThreads;
-                if (v < vectors) {
-                    keys4[v] = make_uint4(rank_key(d[q].x, largest), rank_key(d[q].y, largest), rank_key(d[q].z, largest),
-                                          rank_key(d[q].w, largest));
-                }
-            }
-        }
-        for (uint32_t i = head + 4 * vectors + tid; i < mine; i += kThreads) keys[i] = rank_key(src[i], largest);
-    }
-    __syncthreads();
-    auto slice_key = [&](uint32_t i) { return in_shared ? keys[i] : rank_key(row[begin + i], largest); };
-
-    // ---- the long way (k > 256, keys not in shared memory, or a list that overflowed: ties in the thousands):
-    //      the whole cluster, over the slices ------------------------------------------------------------------
-    const uint32_t count = mine;
-    auto key_at = [&](uint32_t i) { return slice_key(i); };
-    auto col_at = [&](uint32_t i) { return begin + i; };
-    const int first_rank = 0;
-
-    // ---- 1. radix select of the k-th key ---------------------------------------------------------------
-    uint32_t prefix = 0, mask = 0, remaining = (uint32_t)p.k, inside = 0;
-    for (int pass = 0; pass < 4; ++pass) {
-        const int shift = 24 - 8 * pass;
-        uint32_t* hist = s_hist[pass & 1];
-        for (uint32_t i = tid; i < count; i += kThreads) {
-            const uint32_t key = key_at(i);
-            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-        }
-        meet();
-        if (pass > 0) {
-            for (int i = tid; i < 256; i += kThreads) s_hist[(pass - 1) & 1][i] = 0;
-        }
-        if (tid < 32) {
-            const Found f = find_digit(cluster, hist, first_rank, ranks, remaining, lane);
-            if (lane == 0) {
-                s_prefix = prefix | (f.digit << shift);
-                s_remaining = remaining - f.above;
-                s_inside = f.inside;
-            }
-        }
-        __syncthreads();
-        prefix = s_prefix;
-        remaining = s_remaining;
-        inside = s_inside;
-        mask |= 255u << shift;
-    }
-    const uint32_t kth = prefix;
-    const uint32_t ties_wanted = remaining;  // entries equal to the k-th key to take; `inside` entries equal it
-
-    // ---- 2. more ties than wanted: the column up to which they are taken ------------------------------------
-    uint32_t last_tie_column = 0xFFFFFFFFu;
-    if (inside > ties_wanted) {  // uniform over the cluster
-        uint32_t cprefix = 0, cmask = 0, cremaining = ties_wanted;
-        for (int pass = 0; pass < 3; ++pass) {
-            const int shift = 16 - 8 * pass;
-            uint32_t* hist = s_hist[pass & 1];  // the key's four passes left [0] cleared and [1] to clear
-            for (uint32_t i = tid; i < count; i += kThreads) {
-                if (key_at(i) != kth) continue;
-                const uint32_t inverted = ~col_at(i) & 0x00FFFFFFu;  // lower columns rank higher; columns are below 2^24
-                if ((inverted & cmask) == cprefix) atomicAdd(&hist[(inverted >> shift) & 255u], 1u);
-            }
-            meet();
-            for (int i = tid; i < 256; i += kThreads) s_hist[(pass + 1) & 1][i] = 0;
-            if (tid < 32) {
-                const Found f = find_digit(cluster, hist, first_rank, ranks, cremaining, lane);
-                if (lane == 0) {
-                    s_prefix = cprefix | (f.digit << shift);
-                    s_remaining = cremaining - f.above;
-                }
-            }
-            __syncthreads();
-            cprefix = s_prefix;
-            cremaining = s_remaining;
-            cmask |= 255u << shift;
-        }
-        last_tie_column = ~cprefix & 0x00FFFFFFu;
-    }
-
-    // ---- 3. collect in the first CTA, sort there, write -------------------------------------------------------
-    {
-        uint32_t* count0 = cluster.map_shared_rank(&s_collected, first_rank);
-        u64* collected0 = cluster.map_shared_rank(collected, first_rank);
-        for (uint32_t i = tid; i < count; i += kThreads) {
-            const uint32_t key = key_at(i), col = col_at(i);
-            if (key > kth || (key == kth && col <= last_tie_column)) {
-                const uint32_t slot = atomicAdd(count0, 1u);
-                if (slot < p.k_pad) collected0[slot] = ((u64)key << 32) | (uint32_t)~col;
-            }
-        }
-    }
-    meet();  // nobody touches another CTA's shared memory after this
-    if (rank != 0) return;
-    const uint32_t taken = min(s_collected, (uint32_t)p.k);  // == k
-    for (uint32_t i = taken + tid; i < p.k_pad; i += kThreads) collected[i] = 0;
-    __syncthreads();
-    if (p.k_pad > 1) block_bitonic_sort(collected, (int)p.k_pad, /*descending=*/true);
-    for (uint32_t j = tid; j < taken; j += kThreads) {
-        const uint32_t col = ~(uint32_t)collected[j];
-        out_v[j] = row[col];
-        out_i[j] = (float)col;
-    }
+    if (kHeld) select_held_row<kLargest, kThreads>(p, collected, keys, held_here ? held4 : nullptr);
+    else select_row<kLargest, false, kThreads>(p, collected, keys, nullptr);
 }
 
 // ---- k beyond what one CTA's shared memory sorts: the whole row is sorted in global memory -----------
@@ -721,7 +758,7 @@ cudaError_t launch_topk_rows(const float* in, float* values, float* indices, siz
                   entries * 8 + (size_t)p.slice * 4 + 4096 <= 227 * 1024 ? 1 : 0;
     p.wait_limit_ns = kDefaultWaitLimitNs;
     // Beyond k 64 the lists grow long and overflow more often, and a block that holds its slice has fewer beside it to hide the
-    // radix selection: 4096 x 16,384, k 256: 840 us with held slices, 548 without (k 100: 125 and 121; 4096 x 4096, k 128: 99 and 106).
+    // radix selection: 4096 x 16,384, k 256: 840 us with held slices, 483 without (k 100: 125 and 120; 4096 x 4096, k 128: 99 and 104).
     const bool held = p.list_cap != 0 && p.slice <= kHeldMax && k <= 64;
     const int threads = !held || k > 32 ? kWidest : p.slice <= 4096 && k <= 32 ? 64 : 128;
     auto kernel = largest ? topk_rows_kernel<true, false, kWidest> : topk_rows_kernel<false, false, kWidest>;
