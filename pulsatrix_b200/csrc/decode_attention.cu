@@ -57,6 +57,14 @@ __device__ __forceinline__ bool masked(const float* keep_row, int64_t i, int64_t
     return keep_row != nullptr && keep_row[j] == 0.0f;
 }
 
+// A query row whose scores are all -inf (products beyond the range of a float) ends with the masked value as its maximum, and all masked
+// positions weigh the same, those before the window that the sweep left out among them.  They are added here; by one thread per
+// column, and as far as `oldest` says they were left out.
+__device__ __forceinline__ void add_left_out(const float* values, int D, int d, int64_t oldest, float& l, float& acc) {
+    for (int64_t j = 0; j < oldest; ++j) acc += values[j * D + d];
+    l += (float)oldest;
+}
+
 // R: query rows answered together (group x L, padded to 1, 2, 4 or 8); C: float4 chunks of a
 // context row per lane (D <= 128 C).
 template <int R, int C>
@@ -106,7 +114,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(const
 
     // Positions before the oldest query's window are masked for every query, and a masked score's weight is exactly zero -- unless
     // a query has nothing left at all: then its weights are equal over all positions.  With key padding that is ruled out by a
-    // position that is kept and lies in every query's window.  (32 x 8 kv heads, 8001 positions, a window of 1024: 420 -> 64 us.)
+    // position that is kept and lies in every query's window; scores of -inf are looked after at the end.  (32 x 8 kv heads, 8001 positions, a window of 1024: 420 -> 64 us.)
     int64_t oldest = 0;
     if (p.causal != 0 && p.window > 0) {
         oldest = max((int64_t)0, p.offset - p.window + 1);
@@ -329,6 +337,10 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(const
         const int64_t head = kvh * p.group + r / p.q_len;
         const int64_t out_row = (n * p.heads + head) * p.q_len + r % p.q_len;
         if (p.splits == 1) {
+            if (oldest > 0 && !(m > kMasked)) {
+                add_left_out(values, D, d, oldest, l, acc);
+                any = true;
+            }
             p.context[out_row * D + d] = any ? __fdiv_rn(acc, l) : 0.0f;
         } else {  // unnormalised, with its maximum and sum, for the second kernel
             float* part = p.partial + ((out_row * p.splits + split) * (D + 2));
@@ -360,6 +372,13 @@ __global__ void join_attention_splits_kernel(const AttentionParams p) {
             l = __fmaf_rn(ls, f, l);
             acc = __fmaf_rn(part[s * (D + 2) + d], f, acc);
         }
+    }
+    if (p.causal != 0 && p.window > 0 && p.offset >= p.window && !(m > kMasked)) {
+        // (what the first kernel left out, and why: a kept position in every query's window)
+        const int64_t nh = row / p.q_len, n = nh / p.heads, kvh = n * p.kv_heads + nh % p.heads / p.group;
+        bool kept = p.key_keep == nullptr;
+        for (int64_t j = max((int64_t)0, p.offset + p.q_len - p.window); j <= p.offset && !kept; ++j) kept = p.key_keep[n * p.total + j] != 0.0f;
+        if (kept) add_left_out(p.values + kvh * p.max_len * D, D, d, p.offset - p.window + 1, l, acc);
     }
     p.context[i] = l > 0.0f ? __fdiv_rn(acc, l) : 0.0f;
 }

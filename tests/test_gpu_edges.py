@@ -126,3 +126,28 @@ def test_a_narrow_softmax_into_a_buffer_that_lies_differently_takes_a_warp_per_r
         return min(times)
 
     assert best(other) < 6 * best(like)
+
+
+@pytest.mark.parametrize("batch", [1, 200])
+@pytest.mark.parametrize("q_len,padding", [(1, False), (2, False), (2, True)])
+def test_scores_of_minus_infinity_in_a_window(batch, q_len, padding):
+    # Every product overflows to -inf: what the mask hides weighs more than what it shows, in the window and before it.
+    import torch
+    heads, kv_heads, d, cached, window = 2, 1, 64, 1500, 800
+    rng = np.random.RandomState(q_len)
+    total = cached + q_len
+    q = np.full((batch, heads, q_len, d), 1e30, dtype=np.float32)
+    keys = np.full((batch, kv_heads, total + 2, d), -1e30, dtype=np.float32)
+    values = rng.randn(batch, kv_heads, total + 2, d).astype(np.float32)
+    q[0, 1] = 1.0  # (a row of ordinary scores beside it)
+    keep = None
+    if padding:
+        keep = (rng.rand(batch, total) > 0.3).astype(np.float32)
+        keep[batch - 1] = 0.0
+    few = slice(0, 3) if batch > 3 else slice(None)
+    want = ol.decode_attention("oracle", q[few], keys[few], values[few], cached, 1.0, True, window, None if keep is None else keep[few])
+    got, status = gh.ctx().decode_attention(*(torch.from_numpy(x).cuda() for x in (q, keys, values)), cached, scale=1.0, window=window,
+                                            key_keep=None if keep is None else torch.from_numpy(keep).cuda())
+    assert int(status[0]) == 0
+    # 1500 terms, each weight and each sum rounded: 1e-4 as the other cases
+    assert np.abs(got[few].cpu().numpy() - want).max() < 1e-4
