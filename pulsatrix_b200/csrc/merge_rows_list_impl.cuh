@@ -122,9 +122,10 @@ __device__ __forceinline__ bool join_parts(const RowView& v, PartsJoined& j) {
     return (j.bad & 4u) == 0;
 }
 
-// true: the row has a non-finite logit, a copy that did not arrive, or nothing left; its status is written
-__device__ __forceinline__ bool settle_bad_row(const RowView& v, const PartsJoined& j) {
-    if (j.bad == 0 && j.y_max > -INFINITY) return false;
+// true: the row has a non-finite logit, a copy that did not arrive, or nothing left (top: its largest processed value; -inf
+// also when every quotient by the temperature overflows); its status is written
+__device__ __forceinline__ bool settle_bad_row(const RowView& v, const PartsJoined& j, const float top) {
+    if (j.bad == 0 && top > -INFINITY) return false;
     if (threadIdx.x == 0) {
         *v.token = -1;
         *v.log_prob = 0.0f;
@@ -196,7 +197,7 @@ __device__ __forceinline__ bool list_greedy(const MergeParams& p, const RowView&
     load_parts(p, v, j);
     walk.fetch(c, where);
     if (!join_parts(v, j)) return false;
-    if (settle_bad_row(v, j)) return true;
+    if (settle_bad_row(v, j, j.y_max)) return true;
     PSX_MERGE_STAGE(3);
     const float keep_from = fmaxf(j.y_max, -FLT_MAX);
     RawSum z(j.raw_max);
@@ -275,7 +276,8 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
     const double u = v.u ? *v.u : 0.5;
     __syncthreads();
     if (!join_parts(v, j)) return false;
-    if (settle_bad_row(v, j)) return true;
+    const float x_max = temper(j.y_max, apply_t, p.temperature);
+    if (settle_bad_row(v, j, x_max)) return true;
     PSX_MERGE_STAGE(3);
     // ---- 1. what reaches the largest part threshold (that part alone has k logits which reach it), and its histogram -------
     const float keep_from = relax_threshold(j.thr, apply_t, p.temperature);
@@ -343,7 +345,6 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
         const uint32_t reached = __ballot_sync(0xFFFFFFFFu, (int64_t)incl >= p.top_k);
         if (reached != 0) cut = __ffs(reached) - 1;
     }
-    const float x_max = temper(j.y_max, apply_t, p.temperature);
     if (!(fabsf(x_max) < INFINITY)) return false;  // (quotients that overflow tie: merge_row's business)
     for (int first = warp * 32; first < wide; first += kMergeThreads) {
         const int e = first + lane;
@@ -566,11 +567,11 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
     const double u = v.u ? *v.u : 0.5;
     __syncthreads();
     if (!join_parts(v, j)) return false;
-    if (settle_bad_row(v, j)) return true;
+    const float x_max = temper(j.y_max, apply_t, p.temperature);
+    if (settle_bad_row(v, j, x_max)) return true;
     PSX_MERGE_STAGE(3);
     // ---- 1. candidates at or above the largest part threshold into shared memory, their masses by value; what lies below it
     // belongs to the rest of the vocabulary, which the candidates do not cover ---------------------------------------------------
-    const float x_max = temper(j.y_max, apply_t, p.temperature);
     if (!(fabsf(x_max) < INFINITY)) return false;  // (quotients that overflow tie: merge_row's business)
     const float keep_from = relax_threshold(j.thr, apply_t, p.temperature);
     const float x_low = temper(keep_from, apply_t, p.temperature);

@@ -34,3 +34,22 @@ def test_rows_handed_on_whole(vocab, settings):
             continue
         cfg = ol.make_config(max_new_tokens=2, do_sample=True, **settings, **extra)
         gh.check_rows_against_oracle(logits.astype(np.float32), hist, np.arange(11, dtype=np.int64) * 12, cfg, np.arange(10, dtype=np.uint64) + vocab)
+
+
+@pytest.mark.parametrize("vocab", [1, 2, 33, 700, 1024, 1025, 20000])
+@pytest.mark.parametrize("settings", [dict(top_k=30), dict(top_p=0.9), dict(min_p=0.1)], ids=str)
+def test_quotients_that_overflow_on_lists(vocab, settings):
+    # T = 1e-36: below -340 a quotient is -inf and the token removed, alone or with all the others
+    if settings.get("top_k", 0) >= vocab:
+        settings = dict(top_p=0.5)
+    rng = np.random.RandomState(vocab)
+    logits = rng.randn(5, vocab) * 3.0
+    logits[1] -= 1000.0
+    logits[2, ::3] = -1000.0
+    logits[3] = -400.0
+    logits[4] *= 20.0  # (up to 300: 3e38 after the divide, still a float)
+    hist = np.zeros((5, 1), dtype=np.int64)
+    cfg = ol.make_config(max_new_tokens=1, do_sample=True, temperature=1e-36, **settings)
+    (_, _, status, _), _ = gh.check_rows_against_oracle(logits.astype(np.float32), hist, np.arange(6, dtype=np.int64), cfg,
+                                                        np.arange(5, dtype=np.uint64), expect_ok=False)
+    assert status[1] == status[3] == 5 and status[0] == 0
