@@ -110,13 +110,25 @@ __device__ __forceinline__ void load_parts(const MergeParams& p, const RowView& 
     }
 }
 
-// false: the row is not for this way (a list that ran out of slots)
-__device__ __forceinline__ bool join_parts(const RowView& v, PartsJoined& j) {
+// false: the row is not for this way (a list that ran out of slots).  A part that lies below the threshold of another as a whole, and so
+// far below the row's maxima that all its logits together weigh less than 1e-38 of them, is left aside instead: the parts of a row in
+// which all but a few logits are masked by a number (one row of 50,000 with 50 left, top-k 1: 484 us decided from the row, 10 so).
+__device__ __forceinline__ bool join_parts(const MergeParams& p, const RowView& v, PartsJoined& j) {
     j.count = min(j.count, (uint32_t)v.cap);
     j.raw_max = warp_max(j.mine.raw_max);
     j.y_max = warp_max(j.mine.y_max);
     j.thr = warp_max(j.mine.thr);
     j.bad = __reduce_or_sync(0xFFFFFFFFu, (j.mine.nonfinite & 3u) | (j.mine.overflow ? 4u : 0u));
+    if ((j.bad & 4u) != 0) {
+        const bool apply_t = p.apply_temperature != 0;
+        const bool aside = j.mine.raw_max < j.raw_max - 100.0f && j.mine.y_max < relax_threshold(j.thr, apply_t, p.temperature) &&
+                           temper(j.mine.y_max, apply_t, p.temperature) < temper(j.y_max, apply_t, p.temperature) - 100.0f;
+        if (j.mine.overflow && aside) {
+            j.count = 0;
+            j.mine.alive_tail = 1;  // (some of it is outside the lists, however many)
+        }
+        j.bad = (j.bad & 3u) | (__any_sync(0xFFFFFFFFu, j.mine.overflow && !aside) ? 4u : 0u);
+    }
     j.tail_alive = __reduce_add_sync(0xFFFFFFFFu, j.mine.alive_tail);
     j.longest = __reduce_max_sync(0xFFFFFFFFu, j.count);
     return (j.bad & 4u) == 0;
@@ -196,7 +208,7 @@ __device__ __forceinline__ bool list_greedy(const MergeParams& p, const RowView&
     ready();
     load_parts(p, v, j);
     walk.fetch(c, where);
-    if (!join_parts(v, j)) return false;
+    if (!join_parts(p, v, j)) return false;
     if (settle_bad_row(v, j, j.y_max)) return true;
     PSX_MERGE_STAGE(3);
     const float keep_from = fmaxf(j.y_max, -FLT_MAX);
@@ -275,7 +287,7 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
     walk.fetch(c, where);
     const double u = v.u ? *v.u : 0.5;
     __syncthreads();
-    if (!join_parts(v, j)) return false;
+    if (!join_parts(p, v, j)) return false;
     const float x_max = temper(j.y_max, apply_t, p.temperature);
     if (settle_bad_row(v, j, x_max)) return true;
     PSX_MERGE_STAGE(3);
@@ -566,7 +578,7 @@ __device__ __forceinline__ bool list_nucleus(const MergeParams& p, const int64_t
     walk.fetch(c, where);
     const double u = v.u ? *v.u : 0.5;
     __syncthreads();
-    if (!join_parts(v, j)) return false;
+    if (!join_parts(p, v, j)) return false;
     const float x_max = temper(j.y_max, apply_t, p.temperature);
     if (settle_bad_row(v, j, x_max)) return true;
     PSX_MERGE_STAGE(3);

@@ -1,6 +1,8 @@
-"""Rows that are handed on whole (up to 1024 logits, no threshold): the survivor stage's lists cut them by ranges of a fixed width.
+"""Rows that the survivor stage's lists held only after a look at what they are made of.
+
+Rows that are handed on whole (up to 1024 logits, no threshold): the survivor stage's lists cut them by ranges of a fixed width.
 Logits whose spread is a fraction of a range, a few ranges or far beyond the last, ties, masked entries --
-token ids, survivor counts and statuses as the checker's, log-probs within 1e-5."""
+token ids, survivor counts and statuses as the checker's, log-probs within 1e-5.  Rows masked by a number: whole parts of them are equal."""
 import numpy as np
 import pytest
 
@@ -53,3 +55,44 @@ def test_quotients_that_overflow_on_lists(vocab, settings):
     (_, _, status, _), _ = gh.check_rows_against_oracle(logits.astype(np.float32), hist, np.arange(6, dtype=np.int64), cfg,
                                                         np.arange(5, dtype=np.uint64), expect_ok=False)
     assert status[1] == status[3] == 5 and status[0] == 0
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 50000), (3, 128256), (40, 151936)])
+@pytest.mark.parametrize("settings", [
+    dict(do_sample=False), dict(top_k=1), dict(top_k=5, temperature=0.8, top_p=0.9), dict(top_p=0.95), dict(min_p=0.05, temperature=1.5),
+    dict(top_p=0.9, temperature=1000.0),  # (at 1e7 a token of probability exp(-65504) is drawn, whose log-probability is -inf on both sides)
+], ids=str)
+def test_rows_masked_by_a_number(rows, vocab, settings):
+    rng = np.random.RandomState(vocab)
+    logits = rng.randn(rows, vocab) * 2.5
+    for r in range(rows):
+        mask = np.ones(vocab, dtype=bool)
+        mask[rng.randint(vocab, size=rng.choice([1, 7, 60]))] = False
+        logits[r, mask] = [-1e9, -65504.0, -200.0][r % 3]
+    hist = rng.randint(0, vocab, size=(rows, 8)).astype(np.int64)
+    for penalty in (1.0, 1.3, 0.7):
+        cfg = ol.make_config(max_new_tokens=1, **{"do_sample": True, "repetition_penalty": penalty, **settings})
+        gh.check_rows_against_oracle(logits.astype(np.float32), hist, np.arange(rows + 1, dtype=np.int64) * 8, cfg, np.arange(rows, dtype=np.uint64))
+
+
+@pytest.mark.parametrize("settings", [dict(do_sample=False), dict(do_sample=True, top_k=1)], ids=str)
+def test_a_masked_row_takes_no_longer_than_others(settings):
+    # (7 and 33 times as long when the parts without a live logit left their lists)
+    import torch
+    plain = torch.randn((1, 50000), device="cuda")
+    masked = torch.full_like(plain, -1e9)
+    masked[0, :50] = plain[0, :50]
+    uniforms, config = torch.rand(1, dtype=torch.float64, device="cuda"), gh.psx_config(ol.make_config(max_new_tokens=1, **settings))
+
+    def best(x):
+        out, times = gh.ctx().alloc_outputs(1), []
+        for _ in range(30):
+            begin, end = torch.cuda.Event(True), torch.cuda.Event(True)
+            begin.record()
+            gh.ctx().sample_rows(x, None, None, config, uniforms, out=out)
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times)
+
+    assert best(masked) < 3 * best(plain)
