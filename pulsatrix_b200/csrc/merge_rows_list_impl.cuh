@@ -25,12 +25,12 @@ namespace survivor {
 
 constexpr int kListWarps = kMergeThreads / 32;
 constexpr int kListCap = 512;        // entries that look at one another
-constexpr int kWideCap = 2048;       // candidates at or above the threshold, before the cut (top-k)
+constexpr int kWideLeast = 2048;     // room for candidates at or above the threshold, before the cut (top-k): at least
 constexpr int kNucleusCap = 4096;    // the same without a top-k
 constexpr double kDoubt = 1e-11;     // of the whole mass: well above 512 units of 2^-52
 constexpr double kNucleusDoubt = 4e-9;  // the same for kNucleusCap units of 2^-40
 constexpr uint32_t kRemoved = 0x80000000u;
-constexpr int kTopKArena = kListCap * (16 + 8 + 4) + kWideCap * 12;
+constexpr int kTopKArena = kListCap * (16 + 8 + 4) + kWideLeast * 12;
 constexpr int kNucleusArena = kListCap * (16 + 4) + kNucleusCap * 20 + 4 * 256 * 4;
 
 // Where one row's inputs lie and where its results go.
@@ -267,7 +267,9 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
     uint32_t* const s_by_column = s_by_value + kListCap;                          // entry, kRemoved
     float* const s_raw = reinterpret_cast<float*>(s_by_column + kListCap);
     u64* const s_wide = reinterpret_cast<u64*>(s_raw + kListCap);        // raw logit, column | flags
-    float* const s_wide_y = reinterpret_cast<float*>(s_wide + kWideCap);
+    // as many candidates as the launch has shared memory for: 3670 and more (64 rows of 151,936, top-k 200: 80 us with 2048, 58 so)
+    const int wide_cap = (p.dyn_bytes - kListCap * (16 + 8 + 4)) / 12;
+    float* const s_wide_y = reinterpret_cast<float*>(s_wide + wide_cap);
     __shared__ uint32_t s_hist[32];
     __shared__ u64 s_z[kListWarps];
     __shared__ double s_log_z;
@@ -329,7 +331,7 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int mine = at + __popc(votes[q] & below);
-                if (((votes[q] >> lane) & 1u) && mine < kWideCap) {
+                if (((votes[q] >> lane) & 1u) && mine < wide_cap) {
                     s_wide[mine] = ((u64)c[q].x << 32) | c[q].y;
                     s_wide_y[mine] = y[q];
                 }
@@ -342,7 +344,7 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
     __syncthreads();
     PSX_MERGE_STAGE(4);
     const int wide = s_wide_n;
-    if (wide > kWideCap) return false;
+    if (wide > wide_cap) return false;
     // ---- 2. the list: down to the bin in which the count reaches k.  The place in the histogram is by the value before the
     // temperature; a candidate is listed by the bin of its value raised by what the divide can merge (twice
     // relax_threshold's margin), so one that is not listed lies below k others after the divide as well -------------------------

@@ -96,3 +96,14 @@ def test_a_masked_row_takes_no_longer_than_others(settings):
         return min(times)
 
     assert best(masked) < 3 * best(plain)
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 50000), (20, 151936)])
+@pytest.mark.parametrize("k", [100, 180, 200, 256])
+def test_more_candidates_than_2048_at_the_threshold(rows, vocab, k):
+    # (a k of some 200 from every part)
+    logits, hist = ol.synth_rows(np.arange(rows) + k, vocab, 2.5, 0.0, 20)
+    logits[0] = np.round(logits[0] * 8) / 8
+    for settings in (dict(), dict(top_p=0.9, temperature=0.7, repetition_penalty=1.2)):
+        cfg = ol.make_config(max_new_tokens=1, do_sample=True, top_k=k, **settings)
+        gh.check_rows_against_oracle(logits, hist, np.arange(rows + 1, dtype=np.int64) * 20, cfg, np.arange(rows, dtype=np.uint64))
