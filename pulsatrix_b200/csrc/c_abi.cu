@@ -1078,11 +1078,12 @@ psx_status psx_b200_decode_attention(psx_ctx* ctx, void* stream_ptr, const float
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     psx::AttentionParams p{};
     p.q = q; p.keys = keys; p.values = values; p.key_keep = key_keep; p.context = context; p.status = status;
-    p.batch = batch; p.total = total; p.max_len = max_len; p.offset = cached; p.window = window;
+    p.batch = batch; p.total = total; p.max_len = max_len; p.offset = cached;
+    p.window = std::min(window, total);  // (a wider one hides nothing more, and sums with it stay in range)
     p.heads = (int32_t)heads; p.kv_heads = (int32_t)kv_heads; p.group = (int32_t)group; p.q_len = (int32_t)q_len;
     p.head_dim = (int32_t)head_dim; p.causal = causal ? 1 : 0; p.scale = scale;
     p.wait_limit_ns = ctx->wait_limit_ns;
-    const int64_t seen = causal && window > 0 ? std::min(total, window + q_len - 1) : total;  // what lies before the window is not read
+    const int64_t seen = causal && window > 0 ? std::min(total, p.window + q_len - 1) : total;  // what lies before the window is not read
     p.splits = psx::attention_splits(batch * kv_heads, seen, ctx->sm_count, (int)head_dim);
     if (p.splits > 1) {
         if (psx_status s = reserve(ctx->attention_partial, psx::attention_partial_bytes(p))) return s;

@@ -147,3 +147,14 @@ def test_a_second_device_of_the_process():
         on = [torch.from_numpy(x).to(f"cuda:{d}") for x in (q, kv[0], kv[1])]
         got.append(psx.Context(d).decode_attention(*on, 33)[0].cpu())
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("window", [2001, 2002, 2**31, 2**62, 2**63 - 1])
+def test_a_window_wider_than_the_cache_is_none(window):
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    q = torch.randn((2, 4, 1, 64), generator=gen, device="cuda")
+    keys, values = (torch.randn((2, 2, 2010, 64), generator=gen, device="cuda") for _ in range(2))
+    got, want = (gh.ctx().decode_attention(q, keys, values, 2000, window=w)[0] for w in (window, 0))
+    assert torch.equal(got, want)
