@@ -37,6 +37,7 @@ psx_status fail(psx_status code, std::string message) {
     do {                                                                                                 \
         const cudaError_t psx_cuda_result = (call);                                                      \
         if (psx_cuda_result != cudaSuccess) {                                                            \
+            cudaGetLastError(); /* (said here; the next launch's check is not to find it again) */       \
             return fail(PSX_ERR_CUDA, std::string("CUDA error: ") + cudaGetErrorString(psx_cuda_result) + \
                                           " at " __FILE__ ":" + std::to_string(__LINE__));               \
         }                                                                                                \

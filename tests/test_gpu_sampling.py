@@ -379,3 +379,16 @@ def test_a_prepared_call_enqueues_the_same_call_again():
     torch.cuda.synchronize()
     expect = ol.rows("oracle", other, hist.ravel(), offsets, cfg, seeds)
     assert out["tokens"].cpu().numpy().tolist() == expect["token"].tolist()
+
+
+def test_a_failed_allocation_is_reported_once():
+    # (40 TB of records: refused by the allocation, before any launch)
+    import torch
+    ctx = psx.Context(0)
+    x = torch.randn((4, 4000), device="cuda")
+    out, config = ctx.alloc_outputs(4), psx.SamplingConfig.make(do_sample=False)
+    status = psx.binding._native.sample_rows(ctx._handle, 0, x.data_ptr(), 1 << 40, 4000, 4000, None, None, psx.binding.C.addressof(config), None,
+                                             out["tokens"].data_ptr(), out["log_probs"].data_ptr(), out["status"].data_ptr(), None)
+    assert status == psx.ERR_CUDA
+    got = ctx.softmax_rows(x)  # (whose check of its launch found the allocation's error)
+    assert torch.allclose(got, torch.softmax(x, 1), atol=1e-6)
