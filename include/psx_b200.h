@@ -322,8 +322,10 @@ PSX_API psx_status psx_b200_lm_head_sample_rows(psx_ctx* ctx, void* stream, cons
  * cache, (batch, kv_heads, max_len, head_dim), holding positions 0 .. cached + q_len - 1 (the new keys and
  * values already appended, :554-559); query head h reads kv head h / (heads / kv_heads) in place;
  * key_keep: (batch, cached + q_len) or null.  All device pointers, stream-asynchronous.  status (device,
- * may be null): bit 0 is set if a bounded device-side wait for a copy ran out.  Float sums in another
- * order than the reference's loops: within its 1e-4 CPU/GPU equivalence tolerance, not bit for bit.
+ * may be null, the caller's to zero): bit 0 is set if a bounded device-side wait for a copy ran out, nothing
+ * is ever cleared.  Positions before the windows of all new positions are not read (a value there that is
+ * not finite is not seen).  Float sums in another order than the reference's loops: within its 1e-4
+ * CPU/GPU equivalence tolerance, not bit for bit.
  * Limits: (heads / kv_heads) * q_len <= 8, head_dim a multiple of 4 up to 256 (else PSX_ERR_UNSUPPORTED). */
 PSX_API psx_status psx_b200_decode_attention(psx_ctx* ctx, void* stream, const float* q, const float* keys, const float* values,
                                              const float* key_keep, float* context, int64_t batch, int64_t heads,

@@ -24,7 +24,7 @@
 //     positions, the tile's probabilities go to shared memory;
 //   - lane c accumulates floats 4c .. 4c+3 of the context rows from the V rows (one contiguous run per
 //     tile, one bulk copy, asked for when the tile starts: it lands while the scores are formed).
-// 64 x 8 kv heads of 128, four query rows each, 4001 positions: 420 us so, 363 now (5.8 TB/s).
+// 64 x 8 kv heads of 128, four query rows each, 4001 positions: 420 us so, 361 to 385 now from box to box (5.4 to 5.8 TB/s).
 // One K tile and one V tile per warp (33 KB for a head dimension of 128) leave room for six warps per SM.
 // The warps' partial results (maximum, sum, unnormalised context) meet in shared memory; with several
 // slices per (batch, kv head) they go to scratch and a second kernel joins them.

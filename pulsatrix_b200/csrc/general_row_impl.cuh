@@ -1,8 +1,8 @@
 // general_row: one row of src/generation.cpp:55-156 decided from the row itself, by one CTA.
 //
 // The survivor stage normally works on the few candidates the row pass hands on.  Some rows do not
-// fit that scheme: sampling with no filter at all (every token survives), a top-p or min-p whose
-// kept set is wider than the candidate lists, a top-k beyond what a part can bound, thousands of
+// fit that scheme: sampling with no filter at all through the allocation-free entry point (elsewhere whole_rows.cu
+// has it), a top-p or min-p whose kept set is wider than the candidate lists, a top-k beyond what a part can bound, thousands of
 // exact ties at a cut.  The reference answers all of them, so this path does too: the CTA walks
 // the whole row again (it has just been read, so mostly out of L2), a dozen or so times, and
 // replays the reference with block-wide primitives --
@@ -18,7 +18,8 @@
 // order of the additions: the same input gives the same bits.  They differ from the reference's
 // sequential double sums by at most about vocab * 3e-14; a decision closer than that to its
 // boundary may differ from the reference's, and the distances are reported per row (draw_margin,
-// top_p_margin) so that a caller can tell.  Slow (a hundred microseconds or so per row) and rare.
+// top_p_margin) so that a caller can tell.  Slow (about a
+// millisecond per row of 50,000 columns: one CTA, a dozen sweeps) and rare.
 #pragma once
 
 #include "merge_rows_impl.cuh"

@@ -511,7 +511,8 @@ __device__ __forceinline__ bool list_top_k(const MergeParams& p, const int64_t r
 }
 
 // ---- sampling without a top-k ----------------------------------------------------------------------------------------------
-// Masses by range: 256 sums of units of 2^-40, as 20 low and 21 high bits in two words (4096 of either fit 32 bits).
+// Masses by range: 256 sums of units of 2^-40, as 20 low and 21 high bits in two words.  (4096 of either fit 32 bits, but for 4096 entries that all weigh
+// 2^40: their sum reads zero, no range is found and the row is replayed.)
 __device__ __forceinline__ void add_units(uint32_t* hist, uint32_t bin, u64 units) {
     atomicAdd(&hist[bin], (uint32_t)units & 0xFFFFFu);
     atomicAdd(&hist[256 + bin], (uint32_t)(units >> 20));

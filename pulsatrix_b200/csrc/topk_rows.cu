@@ -14,7 +14,7 @@
 // (distributed shared memory, two cluster barriers), where each finds its place in the others' lists by bisection.
 //
 // The long way (larger k, or a list that overflowed: thousands of ties): the slice becomes keys in
-// shared memory (or is swept from global memory when it does not fit), and
+// shared memory (or is swept where the short way holds it, or from global memory when it does not fit), and
 //   1. a 4 x 8-bit radix select finds the k-th key: every CTA counts its slice's digits into a
 //      histogram of its own, the cluster meets, and every CTA adds the cluster's histograms up
 //      through distributed shared memory for itself;

@@ -447,8 +447,8 @@ __global__ void __launch_bounds__(kThreads, 8) weigh_segments_kernel(const __gri
 cudaError_t launch_whole_rows(const WholeRowParams& p, cudaStream_t stream) {
     if (p.rows <= 0) return cudaSuccess;
     if (p.rows > 65535ll * 65535ll || p.rows > 0x7FFFFFFFll) return cudaErrorInvalidConfiguration;
-    // One segment per warp while that leaves the GPU short of warps; up to four, which share a CTA's table and
-    // bitmap, once there are some six thousand warps' worth (148 SMs x 40 warps).
+    // One segment per warp up to 24,000 segments (some five rounds of the 148 SMs x 32 warps that are resident); from there on up to
+    // four, one after the other, which share a CTA's bitmap.
     WholeRowParams q = p;
     q.segments_per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(kMostPerWarp, p.rows * p.segments / 12000));
     const int64_t per_cta = (int64_t)kWarps * q.segments_per_warp;

@@ -1,9 +1,7 @@
-"""The survivor stage with one warp per row (greedy, and sampling under a top-k of at most 64) and the
-hand-over of the rows it leaves to the block-per-row kernel: many ties at the k-th value, ties at the
-maximum, every filter at once, EOS bans, penalties on either side of one, a top-k of 64 (the longer
-list), batches that do not fill the last CTA.  Everything against the CPU checker: token ids equal,
-log-probs within 1e-5 relative, survivor counts equal.  (Launches of fewer than 256 rows stay with the
-block-per-row kernel, so the batches here are larger.)"""
+"""The survivor stage's lists over batches of some 256 rows (greedy, and sampling under a top-k of at most 64) and the
+rows they leave to the replay: many ties at the k-th value, ties at the
+maximum, every filter at once, EOS bans, penalties on either side of one, a top-k of 64, odd batch sizes.  Everything against the CPU checker: token ids equal,
+log-probs within 1e-5 relative, survivor counts equal."""
 import numpy as np
 import pytest
 
@@ -28,12 +26,12 @@ def _rows(rows, vocab, seed, sigma=2.5, zeta=1.0, hlen=40):
     dict(do_sample=False, repetition_penalty=1.3),
     dict(do_sample=False),
 ])
-def test_short_lists_by_warp(rows, settings):
+def test_short_lists(rows, settings):
     logits, hist, offsets, seeds = _rows(rows, 20011, 900 + rows)
     gh.check_rows_against_oracle(logits, hist, offsets, ol.make_config(max_new_tokens=1, **settings), seeds)
 
 
-def test_rows_with_more_ties_than_a_warps_list_go_to_the_block_kernel():
+def test_rows_with_hundreds_of_ties():
     # every third row: 300 logits tie at the k-th value (all stay, src/generation.cpp:85); every fifth: 90 tie at the top
     logits, hist, offsets, seeds = _rows(259, 30011, 4242)
     rng = np.random.RandomState(3)
@@ -50,10 +48,10 @@ def test_rows_with_more_ties_than_a_warps_list_go_to_the_block_kernel():
         cfg = ol.make_config(max_new_tokens=1, **settings)
         (_, _, status, diag), want = gh.check_rows_against_oracle(logits, hist, offsets, cfg, seeds)
         if settings["do_sample"]:
-            assert diag["survivors"].max() > 128  # the block kernel's rows are among them
+            assert diag["survivors"].max() > 128
 
 
-def test_eos_bans_and_unaligned_rows_by_warp():
+def test_eos_bans_and_unaligned_rows():
     logits, hist, offsets, seeds = _rows(263, 32003, 55)
     eos = [int(np.argmax(logits[r])) for r in range(6)]
     for sample in (True, False):
@@ -64,9 +62,8 @@ def test_eos_bans_and_unaligned_rows_by_warp():
 
 
 @pytest.mark.parametrize("seed", range(5000, 5012))
-def test_randomised_settings_by_warp(seed):
-    """Random vocabularies, scales, ties on a grid, histories with ids out of range, every filter, bans: 256
-    rows or more, so the launch goes by warps (and by blocks for what the warps leave)."""
+def test_randomised_settings(seed):
+    """Random vocabularies, scales, ties on a grid, histories with ids out of range, every filter, bans; 256 rows or more."""
     rng = np.random.RandomState(seed)
     vocab = int(rng.choice([257, 1025, 4097, 16385, 20000, 33000]))
     rows = int(rng.choice([256, 261, 300]))

@@ -7,7 +7,7 @@ import pytest
 CPP = Path(__file__).resolve().parent / "cpp"
 
 
-@pytest.mark.parametrize("name", ["once_per_device_test"])
+@pytest.mark.parametrize("name", ["once_per_device_test", "exp_of_gap_test"])
 def test_unit(name, tmp_path):
     binary = tmp_path / name
     subprocess.run(["g++", "-std=c++17", "-O1", "-ffp-contract=off", str(CPP / (name + ".cpp")), "-o", str(binary)], check=True)

@@ -138,9 +138,8 @@ def test_static_entry_point_bans_eos_ids_and_forgets_them_again():
     del rng
 
 
-def test_static_entry_point_with_enough_rows_for_the_survivor_stage_by_warps():
-    # 300 rows of one part each: the launch goes through the warp-per-row survivor kernel and the block
-    # kernel behind it; some rows tie 200 logits at the k-th value, more than a warp's list holds.
+def test_static_entry_point_with_hundreds_of_rows_and_ties():
+    # 300 rows of one part each; some rows tie 200 logits at the k-th value.
     logits, hist = ol.synth_rows(np.arange(300) + 6000, 15001, 2.5, 1.0, 24)
     offsets = np.arange(301, dtype=np.int64) * 24
     seeds = np.arange(300, dtype=np.uint64) + 6000
