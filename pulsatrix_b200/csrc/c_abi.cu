@@ -410,7 +410,7 @@ namespace {
 // Argument checks, plan, scratch and parameters shared by the sampling entry points.
 psx_status plan_row_pass(psx_ctx* ctx, cudaStream_t stream, const float* logits, int64_t rows, int64_t vocab,
                          int64_t row_stride, const int64_t* history_ids, const int64_t* history_offsets,
-                         const psx_sampling_config* config, Plan& plan, psx::ScanParams& sp, bool alternate = false) {
+                         const psx_sampling_config* config, Plan& plan, psx::ScanParams& sp, int alternate_set = -1) {
     PSX_CUDA(cudaSetDevice(ctx->device));
     plan = psx::make_plan(logits, rows, vocab, row_stride, vocab, config, ctx->sm_count);
     sp = psx::ScanParams{};
@@ -423,12 +423,12 @@ psx_status plan_row_pass(psx_ctx* ctx, cudaStream_t stream, const float* logits,
     sp.history_ids = history_ids;
     sp.history_offsets = history_offsets;
     if (psx_status s = prepare_scan(ctx, stream, config, plan, sp)) return s;
-    if (!alternate) return reserve_scan_scratch(ctx, rows, plan, sp);
+    if (alternate_set < 0) return reserve_scan_scratch(ctx, rows, plan, sp);
     // A row pass followed by a survivor stage, call after call on one stream: this call's scratch is the set
     // that the call before it did not use, and only the row pass's last CTA waits for the kernel before it.
-    ctx->scratch_set ^= 1;
+    // (The caller notes the change once nothing can refuse the call any more: a call that launches nothing uses no set.)
     sp.wait_before_writes = 0;
-    return reserve_scan_scratch(ctx, rows, plan, sp, ctx->scratch_set);
+    return reserve_scan_scratch(ctx, rows, plan, sp, alternate_set);
 }
 
 }  // namespace
@@ -467,8 +467,9 @@ psx_status psx_b200_sample_rows(psx_ctx* ctx, void* stream_ptr, const float* log
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     Plan plan;
     psx::ScanParams sp;
+    const int set = ctx->scratch_set ^ 1;
     if (psx_status s = plan_row_pass(ctx, stream, logits, rows, vocab, row_stride, history_ids, history_offsets, config,
-                                     plan, sp, /*alternate=*/true)) {
+                                     plan, sp, set)) {
         return s;
     }
     cudaEvent_t marks[3] = {nullptr, nullptr, nullptr};
@@ -491,8 +492,9 @@ psx_status psx_b200_sample_rows(psx_ctx* ctx, void* stream_ptr, const float* log
         wp.temperature = sp.temperature;
         wp.segments = (int32_t)psx::whole_row_segments(vocab);
         wp.inputs_ready = sp.inputs_ready;
-        Buffer& records = ctx->stats[ctx->scratch_set];
+        Buffer& records = ctx->stats[set];
         if (psx_status s = reserve(records, (size_t)rows * wp.segments * sizeof(psx::SegmentStats))) return s;
+        ctx->scratch_set = set;
         wp.stats = static_cast<psx::SegmentStats*>(records.ptr);
         wp.uniforms = uniforms;
         wp.tokens = tokens;
@@ -509,6 +511,7 @@ psx_status psx_b200_sample_rows(psx_ctx* ctx, void* stream_ptr, const float* log
         return PSX_OK;
     }
     if (psx_status s = configure_merge(ctx, plan, plan.parts)) return s;
+    ctx->scratch_set = set;
 
     psx::MergeParams mp{};
     psx::fill_merge_params(mp, sp, plan, config, rows, vocab, uniforms, tokens, log_probs, row_status, diag, logits, row_stride);

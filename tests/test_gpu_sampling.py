@@ -392,3 +392,31 @@ def test_a_failed_allocation_is_reported_once():
     assert status == psx.ERR_CUDA
     got = ctx.softmax_rows(x)  # (whose check of its launch found the allocation's error)
     assert torch.allclose(got, torch.softmax(x, 1), atol=1e-6)
+
+
+def test_a_call_that_is_refused_for_its_size_leaves_the_scratch_sets_in_turn():
+    # Successive calls alternate between two sets of scratch, because a row pass may start under the stage before it.  A call whose scratch
+    # cannot be had launches nothing and must not count: the next one still takes the set that the last one did not use.
+    import torch
+    ctx = psx.Context(0)
+    rows, vocab = 600, 40000
+    logits = torch.randn((rows, vocab), device="cuda")
+    uniforms = torch.rand(rows, dtype=torch.float64, device="cuda")
+    config = psx.SamplingConfig.make(do_sample=True, top_k=20)
+    out = ctx.alloc_outputs(rows)
+
+    def used_by(call):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        call()
+        torch.cuda.synchronize()
+        return before - torch.cuda.mem_get_info()[0]
+
+    ctx.sample_rows(logits, None, None, config, uniforms, out=out)
+    first = out["tokens"].clone()
+    status = psx.binding._native.sample_rows(ctx._handle, 0, logits.data_ptr(), 1 << 40, vocab, vocab, None, None, psx.binding.C.addressof(config),
+                                             uniforms.data_ptr(), out["tokens"].data_ptr(), out["log_probs"].data_ptr(), out["status"].data_ptr(), None)
+    assert status == psx.ERR_CUDA  # (40 TB of records: refused by the allocation, before any launch)
+    # 600 rows x 3 parts x 1024 slots of 8 bytes: the second set is made by the second call that runs
+    assert used_by(lambda: ctx.sample_rows(logits, None, None, config, uniforms, out=out)) >= 600 * 3 * 1024 * 8
+    assert torch.equal(out["tokens"], first)
