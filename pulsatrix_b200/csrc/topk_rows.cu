@@ -10,7 +10,7 @@
 // 67.9 now; 8192 x 4096, k 16: 63.5 -> 34.8 us.  Sweep one notes every thread's best entry; the smallest over the warps of
 // the kp-th best of those (kp = ceil(k / 8)) is a bound that k entries of the slice reach.  Sweep
 // two lists what reaches the bound, usually k and a few; the list is put in rank order by
-// counting (beyond 256 entries by sorting), and with several CTAs per row the best k of each meet in the first CTA's shared memory
+// counting (a long one by sorting), and with several CTAs per row the best k of each meet in the first CTA's shared memory
 // (distributed shared memory, two cluster barriers), where each finds its place in the others' lists by bisection.
 //
 // The long way (larger k, or a list that overflowed: thousands of ties): the slice becomes keys in
@@ -42,6 +42,9 @@ namespace {
 using u64 = unsigned long long;
 constexpr int kWidest = 256;  // threads of a CTA at most
 constexpr int kSliceMax = 48 * 1024;  // keys one CTA keeps in shared memory (192 KB)
+// A list from which sorting it takes fewer steps than looking at all the others for each entry (4096 x 500, k 128: 175 us counted, 149
+// sorted; 1000 x 300, k 65: 25 and 39).
+constexpr uint32_t kSortedFrom = 448;
 constexpr uint32_t kHeldMax = 16 * 1024;  // entries the short way keeps in shared memory: 64 KB, three CTAs per SM
 constexpr uint32_t kHeldCopies = 4, kHeldChunk = kHeldMax / 4 / kHeldCopies;  // bulk copies, vectors of each
 
@@ -319,7 +322,9 @@ __device__ __noinline__ void select_held_row(const TopKParams& p, u64* collected
 // own; the sweeps read it from there.
 // kThreads: most of a CTA's instructions are a warp's own (its bound, its entries, their places), whatever its share of the
 // slice: few warps where each still has at most 32 vectors per lane and k is at most half of the threads.
-template <bool kLargest, bool kHeld, int kThreads>
+// kSorts: lists may be long (k above 64, where a list holds 512 entries and more) and are sorted then; a kernel of its own, since the code
+// for it costs the others 2.5 %.
+template <bool kLargest, bool kHeld, int kThreads, bool kSorts>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(const __grid_constant__ TopKParams p) {
     extern __shared__ __align__(16) unsigned char dyn[];
     // layout: [k_pad collected entries][list_cap listed entries][cluster * k_pad gathered entries], 8 bytes
@@ -534,9 +539,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) topk_rows_kernel(co
                     gathered0[place] = entry;
                 }
             };
-            if (!kHeld && on_list > (uint32_t)kWidest) {  // (held slices: k is at most 64, and a list holds 256)
-                // a long list: sorting it takes fewer steps than looking at all the others (4096 x 1000, k 256: 594 us so, 300 sorted)
-                uint32_t n_pad = 2 * kWidest;
+            if (kSorts && on_list > kSortedFrom) {
+                uint32_t n_pad = 512;
                 while (n_pad < on_list) n_pad <<= 1;
                 for (uint32_t i = on_list + tid; i < n_pad; i += kThreads) list[i] = 0;
                 __syncthreads();
@@ -757,19 +761,21 @@ cudaError_t launch_topk_rows(const float* in, float* values, float* indices, siz
     p.in_shared = p.list_cap == 0 && p.slice <= (uint32_t)kSliceMax &&
                   entries * 8 + (size_t)p.slice * 4 + 4096 <= 227 * 1024 ? 1 : 0;
     p.wait_limit_ns = kDefaultWaitLimitNs;
-    // Beyond k 64 the lists grow long and overflow more often, and a block that holds its slice has fewer beside it to hide the
-    // radix selection: 4096 x 16,384, k 256: 840 us with held slices, 483 without (k 100: 125 and 120; 4096 x 4096, k 128: 99 and 104).
-    const bool held = p.list_cap != 0 && p.slice <= kHeldMax && k <= 64;
+    // Beyond k 128 lists overflow more often than not, and a block that holds its slice has fewer beside it to hide the radix
+    // selection: 4096 x 16,384, k 256: 840 us with held slices, 483 without (k 100: 115 and 120).  Where all blocks are resident at once,
+    // three on each of 148 SMs, it does not matter: 64 x 16,384, k 200: 23 to 34 us held (as lists overflow), 37 not.
+    const bool held = p.list_cap != 0 && p.slice <= kHeldMax && (k <= 128 || rows * p.cluster <= 3 * 148);
     const int threads = !held || k > 32 ? kWidest : p.slice <= 4096 && k <= 32 ? 64 : 128;
-    auto kernel = largest ? topk_rows_kernel<true, false, kWidest> : topk_rows_kernel<false, false, kWidest>;
-    if (held && threads == 64) kernel = largest ? topk_rows_kernel<true, true, 64> : topk_rows_kernel<false, true, 64>;
-    else if (held && threads == 128) kernel = largest ? topk_rows_kernel<true, true, 128> : topk_rows_kernel<false, true, 128>;
-    else if (held) kernel = largest ? topk_rows_kernel<true, true, kWidest> : topk_rows_kernel<false, true, kWidest>;
+    auto kernel = largest ? topk_rows_kernel<true, false, kWidest, true> : topk_rows_kernel<false, false, kWidest, true>;
+    if (held && threads == 64) kernel = largest ? topk_rows_kernel<true, true, 64, false> : topk_rows_kernel<false, true, 64, false>;
+    else if (held && threads == 128) kernel = largest ? topk_rows_kernel<true, true, 128, false> : topk_rows_kernel<false, true, 128, false>;
+    else if (held && k <= 64) kernel = largest ? topk_rows_kernel<true, true, kWidest, false> : topk_rows_kernel<false, true, kWidest, false>;
+    else if (held) kernel = largest ? topk_rows_kernel<true, true, kWidest, true> : topk_rows_kernel<false, true, kWidest, true>;
     const size_t shared = entries * 8 + (p.in_shared ? (size_t)p.slice * 4 + 32 : held ? (p.slice / 4 + threads - 1) / threads * threads * 16 + 32 : 0);
     if (rows * (size_t)p.cluster > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
     // (whatever the size: what a block may use without asking counts the kernel's own arrays as well)
-    static OncePerDevice lifted[8];
-    OncePerDevice& done = lifted[(largest ? 1 : 0) + (!held ? 0 : threads == 64 ? 2 : threads == 128 ? 4 : 6)];
+    static OncePerDevice lifted[10];
+    OncePerDevice& done = lifted[(largest ? 1 : 0) + (!held ? 0 : threads == 64 ? 2 : threads == 128 ? 4 : k <= 64 ? 6 : 8)];
     if (const cudaError_t e = allow_all_dynamic_shared_once(done, kernel); e != cudaSuccess) return e;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)(rows * p.cluster));
