@@ -38,6 +38,40 @@ namespace psx {
 
 namespace {
 
+constexpr int kSmCount = 148;
+
+// What the lists of a row do not decide, by the whole block.
+__device__ __forceinline__ void replay_row(const MergeParams& p, const int64_t row, unsigned long long* dyn) {
+    if (p.general != 2) survivor::merge_row(p, row, dyn);  // too many for the list, or a decision too close to its level
+    if (p.general != 0 && p.logits != nullptr) {
+        // A row the candidate lists could not decide is decided from the row itself.
+        __syncthreads();
+        if (p.general == 2 || p.row_status[row] == PSX_ROW_TOO_WIDE) survivor::general_row(p, row, dyn);
+    }
+}
+
+// Greedy, a warp per row and eight rows per block.  A greedy row has a few candidates per part: latency bound, a trip to memory and two
+// exponentials, for which eight warps are seven too many once there are more rows than blocks fit the GPU at once.  1024 x 49,152, the whole
+// call: 44.9 us with a block per row (2.3 rounds of them), 41.1 so; 4000 x 8000: 59 and 41 us.
+__global__ void __launch_bounds__(kMergeThreads, 3) merge_greedy_rows_kernel(const __grid_constant__ MergeParams p) {
+    extern __shared__ __align__(16) unsigned long long dyn[];
+    __shared__ uint32_t s_left;  // rows that their warps could not decide
+    const int warp = threadIdx.x >> 5;
+    const int64_t first = (int64_t)blockIdx.x * survivor::kListWarps;
+    if (threadIdx.x == 0) s_left = 0;
+    __syncthreads();
+    grid_dependency_wait();        // everything this kernel reads was written by the kernel before it
+    grid_dependents_may_launch();  // a row pass that follows reads none of this kernel's results
+    if (first + warp < p.rows && !survivor::list_greedy_by_warp(p, survivor::view_of_row(p, p.row_begin + first + warp))) {
+        if ((threadIdx.x & 31) == 0) atomicOr(&s_left, 1u << warp);
+    }
+    __syncthreads();
+    for (uint32_t left = s_left; left; left &= left - 1) {
+        replay_row(p, p.row_begin + first + __ffs(left) - 1, dyn);
+        __syncthreads();
+    }
+}
+
 template <int kKind>
 __global__ void __launch_bounds__(kMergeThreads, kKind == survivor::kListNucleus ? 2 : 3) merge_rows_kernel(const __grid_constant__ MergeParams p) {
     extern __shared__ __align__(16) unsigned long long dyn[];
@@ -70,12 +104,7 @@ __global__ void __launch_bounds__(kMergeThreads, kKind == survivor::kListNucleus
         }
     } else if (p.general == 2 || !survivor::list_row<kKind>(p, row, survivor::view_of_row(p, row), dyn, ready)) {
         __syncthreads();
-        if (p.general != 2) survivor::merge_row(p, row, dyn);  // too many for the list, or a decision too close to its level
-        if (p.general != 0 && p.logits != nullptr) {
-            // A row the candidate lists could not decide is decided from the row itself.
-            __syncthreads();
-            if (p.general == 2 || p.row_status[row] == PSX_ROW_TOO_WIDE) survivor::general_row(p, row, dyn);
-        }
+        replay_row(p, row, dyn);
     }
     if (p.arrivals != nullptr) {
         __syncthreads();
@@ -120,6 +149,7 @@ int merge_slot_shift(int parts, int part_cap, int expected) {
 
 cudaError_t configure_merge_rows() {
     cudaError_t e = allow_all_dynamic_shared(merge_rows_kernel<survivor::kListGreedy>);
+    if (e == cudaSuccess) e = allow_all_dynamic_shared(merge_greedy_rows_kernel);
     if (e == cudaSuccess) e = allow_all_dynamic_shared(merge_rows_kernel<survivor::kListTopK>);
     if (e == cudaSuccess) e = allow_all_dynamic_shared(merge_rows_kernel<survivor::kListNucleus>);
     return e;
@@ -140,6 +170,12 @@ cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_
     MergeParams with_size = p;
     with_size.dyn_bytes = (int32_t)shared;
     if (launched != nullptr) ++*launched;
+    // A warp per greedy row where a block each would take a second round (three to an SM), on lists of few slots.  (500 x 49,152: 24.9 us by blocks, 22.9
+    // by warps; 400 rows: 18.3 and 18.0, one row: 6.7 and 7.8.  16 parts, 500 x 262,144: 92.7 and 93.9; rows that are handed on whole, 1024 x 600: 19 and 26.)
+    if (!p.do_sample && p.rows > 3 * kSmCount && p.parts <= 8 && p.whole_rows == 0 && p.arrivals == nullptr && p.survivor_cols == nullptr) {
+        const unsigned blocks = (unsigned)((p.rows + survivor::kListWarps - 1) / survivor::kListWarps);
+        return launch_overlapping(merge_greedy_rows_kernel, dim3(blocks), dim3(kMergeThreads), shared, stream, with_size);
+    }
     return launch_overlapping(kernel_for(p), dim3((unsigned)p.rows), dim3(kMergeThreads), shared, stream, with_size);
 }
 

@@ -22,6 +22,7 @@ struct MergeParams {
     int32_t part_cap;            // slots of a part's list
     int32_t slot_shift;          // 2^slot_shift slots of every list are fetched before the counts are known;
                                  // parts << slot_shift <= 16 * kMergeThreads
+    int32_t whole_rows;          // the lists hold their rows whole (no threshold)
     int64_t rows;                // rows this launch decides: row_begin .. row_begin + rows - 1
     int64_t row_begin;           // (every array below and above is indexed by the absolute row)
     int64_t vocab;               // global vocabulary size

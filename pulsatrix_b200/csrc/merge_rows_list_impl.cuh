@@ -134,16 +134,18 @@ __device__ __forceinline__ bool join_parts(const MergeParams& p, const RowView& 
     return (j.bad & 4u) == 0;
 }
 
+__device__ __forceinline__ void report_bad_row(const RowView& v, const PartsJoined& j) {  // (by one thread)
+    *v.token = -1;
+    *v.log_prob = 0.0f;
+    *v.status = (j.bad & 2u) ? PSX_ROW_DEVICE_TIMEOUT : (j.bad & 1u) ? PSX_ROW_NON_FINITE : PSX_ROW_ALL_REMOVED;
+    if (v.diag) *v.diag = psx_row_diag{0, 0, INFINITY, INFINITY};
+}
+
 // true: the row has a non-finite logit, a copy that did not arrive, or nothing left (top: its largest processed value; -inf
 // also when every quotient by the temperature overflows); its status is written
 __device__ __forceinline__ bool settle_bad_row(const RowView& v, const PartsJoined& j, const float top) {
     if (j.bad == 0 && top > -INFINITY) return false;
-    if (threadIdx.x == 0) {
-        *v.token = -1;
-        *v.log_prob = 0.0f;
-        *v.status = (j.bad & 2u) ? PSX_ROW_DEVICE_TIMEOUT : (j.bad & 1u) ? PSX_ROW_NON_FINITE : PSX_ROW_ALL_REMOVED;
-        if (v.diag) *v.diag = psx_row_diag{0, 0, INFINITY, INFINITY};
-    }
+    if (threadIdx.x == 0) report_bad_row(v, j);
     return true;
 }
 
@@ -256,6 +258,59 @@ __device__ __forceinline__ bool list_greedy(const MergeParams& p, const RowView&
         if (v.diag) *v.diag = psx_row_diag{1, 1, INFINITY, INFINITY};
     }
     PSX_MERGE_STAGE(9);
+    return true;
+}
+
+// The same by one warp, for many rows: a greedy row has a handful of candidates, and what a block does for it is mostly to meet.
+__device__ __forceinline__ bool list_greedy_by_warp(const MergeParams& p, const RowView& v) {
+    const int lane = threadIdx.x & 31;
+    PartsJoined j;
+    uint2 c[4];
+    // 32 slots of four parts' lists at a time (slots beyond a list's count are fetched as well, and not looked at)
+    auto fetch = [&](uint32_t slot, int part) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            c[q] = part + q < p.parts && slot < (uint32_t)v.cap ? reinterpret_cast<const uint2*>(v.lists + (part + q) * v.list_stride)[slot] : make_uint2(0, 0);
+        }
+    };
+    load_parts(p, v, j);
+    fetch(lane, 0);
+    if (!join_parts(p, v, j)) return false;
+    if (j.bad != 0 || !(j.y_max > -INFINITY)) {
+        if (lane == 0) report_bad_row(v, j);
+        return true;
+    }
+    const float keep_from = fmaxf(j.y_max, -FLT_MAX);
+    RawSum z(j.raw_max);
+    u64 best = 0;  // the maximum's lowest column, as ~column above the raw logit
+    for (uint32_t first = 0; first < j.longest; first += 32) {
+        for (int part = 0; part < p.parts; part += 4) {
+            if (first + (uint32_t)part > 0) fetch(first + lane, part);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t here = __shfl_sync(0xFFFFFFFFu, j.count, (part + q) & 31);
+                if (part + q >= p.parts || first + lane >= here) continue;
+                const float l = __uint_as_float(c[q].x);
+                if (processed_before_temperature(l, c[q].y, p.penalty) >= keep_from) {
+                    z.high += exp_below(l, j.raw_max);
+                    const u64 key = ((u64)~(c[q].y & kColumnMask) << 32) | c[q].x;
+                    best = key > best ? key : best;
+                } else {
+                    z.add_low(l);
+                }
+            }
+            __syncwarp();
+        }
+    }
+    const double tails = tails_of_parts(j);
+    const u64 sum = z.of_warp();
+    const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(best >> 32));
+    if ((uint32_t)(best >> 32) == top && (top != 0 || lane == 0)) {  // (columns differ: one lane)
+        *v.status = PSX_ROW_OK;
+        *v.token = (int64_t)(uint32_t)~top;
+        *v.log_prob = (float)(((double)__uint_as_float((uint32_t)best) - (double)j.raw_max) - log((double)sum * 0x1p-40 + tails));  // src/generation.cpp:156
+        if (v.diag) *v.diag = psx_row_diag{1, 1, INFINITY, INFINITY};
+    }
     return true;
 }
 

@@ -108,6 +108,7 @@ inline void fill_merge_params(MergeParams& mp, const ScanParams& sp, const Plan&
     mp.parts = plan.parts;
     mp.part_cap = kPartCap;
     mp.slot_shift = plan.slot_shift;
+    mp.whole_rows = plan.k_need >= kPartCap ? 1 : 0;
     mp.stats_part_stride = sizeof(PartStats);
     mp.stats_row_stride = mp.stats_part_stride * plan.parts;
     mp.count_part_stride = sizeof(uint32_t);
