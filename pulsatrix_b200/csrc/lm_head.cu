@@ -22,8 +22,8 @@
 //     every x, zeros of either sign among them), with the -0.0 from the kernel's arguments: a mul.rn.f32x2 ahead of an
 //     add.rn.f32x2 is contracted into one fused operation by the compiler whatever its rounding suffix says.
 //   - an empty last round.  The CTAs are as many as the GPU holds, each works through whole tiles of 128 entries a
-//     warp, and what is left after the last full round is handed out in tiles of 32, 64, 96 or 128 entries a warp,
-//     whichever is the smallest that goes round once (151,936 entries are 2.005 rounds of 256 x 296: a third round of
+//     warp (256 in the layouts of eight entries per lane), and what is left after the last full round is handed out in tiles of 32 entries
+//     a warp or a multiple of it, the smallest that goes round once (151,936 entries are 2.005 rounds of 256 x 296: a third round of
 //     whole tiles would take half as long again); see Head::kBalanced for one and two rows.
 // The weights arrive by cp.async, S chunks of features deep; the hidden states of a chunk come with them,
 // 4 bytes at a time, transposed on the way ([feature][row]), so that a pair of rows is one 64-bit operand.
@@ -230,9 +230,12 @@ struct Head {
                     for (int f = 0; f < KC; ++f) {
                         if (f < kc) {
                             float w[E];
-                            if (E == 4) {
-                                const float4 v = *reinterpret_cast<const float4*>(mine + f * 32 * E * H);
-                                w[0] = v.x; w[1 % E] = v.y; w[2 % E] = v.z; w[3 % E] = v.w;
+                            if (E % 4 == 0) {
+#pragma unroll
+                                for (int e = 0; e + 3 < E; e += 4) {
+                                    const float4 v = *reinterpret_cast<const float4*>(mine + f * 32 * E * H + e);
+                                    w[e] = v.x; w[e + 1] = v.y; w[e + 2] = v.z; w[e + 3] = v.w;
+                                }
                             } else {
 #pragma unroll
                                 for (int e = 0; e < E; ++e) w[e] = mine[f * 32 * E * H + e];
@@ -267,6 +270,15 @@ struct Head {
     }
 };
 
+// The tiles of the last round: E to EM entries per lane, as many as it says.
+template <class K, int E, int EM>
+__device__ __forceinline__ void last_tiles(const HeadParams& p, float* shared, int64_t j0) {
+    if constexpr (E < EM) {
+        if (p.last_entries > E) return last_tiles<K, E + 1, EM>(p, shared, j0);
+    }
+    K::template tiles<E>(p, shared, j0, 0, 1);
+}
+
 template <int R, int G, int H, int KC, int S, int kCtas, int EM, bool kTokenMajor>
 __global__ void __launch_bounds__(32 * G * H, kCtas) head_kernel(const __grid_constant__ HeadParams p) {
     typedef Head<R, G, H, KC, S, EM, kTokenMajor> K;
@@ -286,10 +298,7 @@ __global__ void __launch_bounds__(32 * G * H, kCtas) head_kernel(const __grid_co
     if (p.full_rounds > 0) K::template tiles<EM>(p, head_shared, (int64_t)blockIdx.x * K::kTile, round, p.full_rounds);
     const int64_t j0 = p.full_rounds * round + (int64_t)blockIdx.x * 32 * p.last_entries * H;
     if (p.last_entries == 0 || j0 >= p.vocab) return;
-    if (EM == 1 || p.last_entries == 1) K::template tiles<1>(p, head_shared, j0, 0, 1);
-    else if (EM == 2 || p.last_entries == 2) K::template tiles<EM < 2 ? EM : 2>(p, head_shared, j0, 0, 1);
-    else if (p.last_entries == 3) K::template tiles<EM < 3 ? EM : 3>(p, head_shared, j0, 0, 1);
-    else K::template tiles<EM < 4 ? EM : 4>(p, head_shared, j0, 0, 1);
+    last_tiles<K, 1, EM>(p, head_shared, j0);
 }
 
 template <int R, int G, int H, int KC, int S, int kCtas, int EM, bool kTokenMajor>
@@ -319,19 +328,27 @@ cudaError_t launch_one(HeadParams p, int sm_count, cudaStream_t stream) {
 template <bool kTokenMajor>
 cudaError_t launch_group(const HeadParams& p, int sm_count, cudaStream_t stream) {
     // Rows per thread, row groups, warps along the vocabulary; features per chunk, chunks; CTAs per SM; entries per lane.
-    // The fastest of the layouts that were timed on 151,936 x 2048 (the whole call with its sampling step, us, token-major /
-    // feature-major; the version of one entry per thread beside it):
-    //   1 row    215 / 212   (266 / 1039)      8 rows    323 / 328   (478 / 641)
-    //   2 rows   222 / 249   (284 / 604)      16 rows    463 / 479   (708 / 944)
-    //   4 rows   270 / 324   (337 / 559)      32 rows    862 / 905   (1256 / 1756)      64 rows   1536 / 1607   (2731 / 2894)
+    // The fastest of the layouts that were timed (the logits alone, us; token-major / feature-major of 151,936 x 2048, then of 32,000 x 4096;
+    // behind the bar the next wider layout, which these rows had before there was one for them):
+    //    1 row    204 / 201                                        8 rows   295 / 306    206 / 250
+    //    6 rows   288 / 304    150 / 248  |  293 / 304   203 / 248     12 rows   392 / 428    207 / 300  |  459 / 438   293 / 334
+    //   16 rows   447 / 443    246 / 354                          24 rows   641 / 658    383 / 373  |  806 / 877   448 / 475
+    //   32 rows   786 / 898    441 / 504                          48 rows  1207 / 1203   586 / 576  | 1479 / 1457  819 / 846
+    //   64 rows  1512 / 1504   824 / 861
     // Up to two rows a lane takes one entry, which leaves room for longer runs of an entry's features per chunk (256 bytes:
-    // HBM serves 5.9 TB/s in runs of 256 bytes, 5.0 in runs of 128); from four rows on the reads of the hidden states weigh, so four.
+    // HBM serves 5.9 TB/s in runs of 256 bytes, 5.0 in runs of 128); from four rows on the reads of the hidden states weigh, so four, or eight
+    // where the rows leave the registers for it.  Token-major, up to 16 rows, chunks of 32 features gain for the same reason (16 rows: 463 us and
+    // 308 with 16 features); feature-major a chunk of 32 is more rows of the matrix and no longer a run (9 to 12 rows: 537 us for 428).
     if (p.rows <= 1) return kTokenMajor ? launch_one<1, 1, 4, 64, 2, 3, 1, true>(p, sm_count, stream) : launch_one<1, 1, 4, 32, 4, 3, 1, false>(p, sm_count, stream);
     if (p.rows <= 2) return kTokenMajor ? launch_one<2, 1, 4, 64, 2, 3, 1, true>(p, sm_count, stream) : launch_one<2, 1, 4, 32, 3, 3, 1, false>(p, sm_count, stream);
     if (p.rows <= 4) return launch_one<2, 2, 2, 32, 2, 3, 4, kTokenMajor>(p, sm_count, stream);
+    if (kTokenMajor && p.rows <= 6) return launch_one<2, 3, 2, 32, 2, 3, 4, true>(p, sm_count, stream);
     if (p.rows <= 8) return launch_one<4, 2, 2, 16, 2, 4, 4, kTokenMajor>(p, sm_count, stream);
-    if (p.rows <= 16) return launch_one<8, 2, 2, 16, 2, 4, 4, kTokenMajor>(p, sm_count, stream);
-    if (p.rows <= 32) return launch_one<8, 4, 2, 16, 3, 2, 4, kTokenMajor>(p, sm_count, stream);
+    if (p.rows <= 12) return kTokenMajor ? launch_one<4, 3, 2, 32, 2, 2, 4, true>(p, sm_count, stream) : launch_one<4, 3, 2, 16, 2, 4, 4, false>(p, sm_count, stream);
+    if (p.rows <= 16) return kTokenMajor ? launch_one<8, 2, 2, 32, 2, 2, 4, true>(p, sm_count, stream) : launch_one<8, 2, 2, 16, 2, 4, 4, false>(p, sm_count, stream);
+    if (p.rows <= 24) return launch_one<4, 6, 2, 16, 2, 2, 8, kTokenMajor>(p, sm_count, stream);
+    if (p.rows <= 32) return kTokenMajor ? launch_one<16, 2, 2, 16, 2, 2, 8, true>(p, sm_count, stream) : launch_one<8, 4, 2, 16, 3, 2, 4, false>(p, sm_count, stream);
+    if (p.rows <= 48) return launch_one<8, 6, 2, 16, 2, 1, 8, kTokenMajor>(p, sm_count, stream);
     return launch_one<16, 4, 2, 16, 3, 2, 4, kTokenMajor>(p, sm_count, stream);
 }
 

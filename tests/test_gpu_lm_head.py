@@ -84,6 +84,22 @@ def test_rounds_of_whole_tiles_and_the_tiles_after_them(rows, d, vocab, vocab_by
     test_head_equals_the_references_loop_bit_for_bit(rows, d, vocab, vocab_by_d)
 
 
+@pytest.mark.parametrize("rows", [5, 6, 9, 12, 13, 16, 24, 32, 33, 48, 49])
+@pytest.mark.parametrize("vocab_by_d", [True, False])
+def test_every_layout_of_rows(rows, vocab_by_d):
+    """The smallest and the largest row count of every layout, on a size with a short last chunk and copies of four bytes, and one without."""
+    test_head_equals_the_references_loop_bit_for_bit(rows, 71, 1503, vocab_by_d)
+    test_head_equals_the_references_loop_bit_for_bit(rows, 64, 640, vocab_by_d)
+
+
+@pytest.mark.parametrize("rows", [24, 32, 48])
+@pytest.mark.parametrize("rest", [1, 2, 3, 4, 5, 6, 7, 8])
+def test_the_last_round_takes_any_number_of_entries(rows, rest):
+    """Layouts of eight entries per lane: 296 CTAs of 64 entries per entry of a lane (148 for 48 rows), a last round of `rest` of them."""
+    round_of_one = (148 if rows == 48 else 296) * 64
+    test_head_equals_the_references_loop_bit_for_bit(rows, 9, round_of_one * rest - 5, rest % 2 == 0)
+
+
 def test_head_and_sampling_in_one_call_match_sampling_the_references_logits():
     import torch
     rng = np.random.RandomState(4)
