@@ -171,8 +171,9 @@ cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_
     with_size.dyn_bytes = (int32_t)shared;
     if (launched != nullptr) ++*launched;
     // A warp per greedy row where a block each would take a second round (three to an SM), on lists of few slots.  (500 x 49,152: 24.9 us by blocks, 22.9
-    // by warps; 400 rows: 18.3 and 18.0, one row: 6.7 and 7.8.  16 parts, 500 x 262,144: 92.7 and 93.9; rows that are handed on whole, 1024 x 600: 19 and 26.)
-    if (!p.do_sample && p.rows > 3 * kSmCount && p.parts <= 8 && p.whole_rows == 0 && p.arrivals == nullptr && p.survivor_cols == nullptr) {
+    // by warps; 400 rows: 18.3 and 18.0, one row: 6.7 and 7.8.  Up to four
+    // parts, which one look takes; 16 parts, 500 x 262,144: 92.7 and 93.9; rows that are handed on whole, 1024 x 600: 19 and 26.)
+    if (!p.do_sample && p.rows > 3 * kSmCount && p.parts <= 4 && p.whole_rows == 0 && p.arrivals == nullptr && p.survivor_cols == nullptr) {
         const unsigned blocks = (unsigned)((p.rows + survivor::kListWarps - 1) / survivor::kListWarps);
         return launch_overlapping(merge_greedy_rows_kernel, dim3(blocks), dim3(kMergeThreads), shared, stream, with_size);
     }
