@@ -88,14 +88,15 @@ __device__ __forceinline__ void sweep_row(const float* x, int n, Visit visit) {
 }
 
 // hist[digit] += units over the lanes that take part (at least one), by the whole warp.  Neighbouring columns share the high digits of their number, and the
-// logits of a row the high digits of their keys: additions to one 64-bit counter queue up, so lanes of one digit are added up first (units below
-// 2^59 / 32), as long as four or more share the digit of the first one left.
+// logits of a row the high digits of their keys: additions to one 64-bit counter queue up, so lanes of one digit are added up first,
+// as long as four or more share the digit of the first one left.  What the two 32-bit reductions do not hold -- the units of a mass that is no
+// number, 2^63 -- goes to the counter by itself.
 __device__ __forceinline__ void add_by_digit(u64* hist, uint32_t digit, u64 units, bool takes_part) {
     const int lane = threadIdx.x & 31;
-    for (uint32_t left = __ballot_sync(0xFFFFFFFFu, takes_part); left != 0;) {
+    for (uint32_t left = __ballot_sync(0xFFFFFFFFu, takes_part && (units >> 59) == 0); left != 0;) {
         const int leader = __ffs(left) - 1;
         const uint32_t theirs = __shfl_sync(0xFFFFFFFFu, digit, leader);
-        const bool same = takes_part && digit == theirs;
+        const bool same = ((left >> lane) & 1u) && digit == theirs;
         const uint32_t group = __ballot_sync(0xFFFFFFFFu, same);
         if (__popc(group) < 4) break;
         const u64 lo = __reduce_add_sync(0xFFFFFFFFu, same ? (uint32_t)units & 0x7FFFFFFu : 0u);

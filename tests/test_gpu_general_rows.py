@@ -83,3 +83,20 @@ def test_process_logits_on_wide_rows_is_bit_exact(name):
         assert rc == 0
         differ = np.nonzero(got[r].view(np.uint32) != want.view(np.uint32))[0]
         assert differ.size == 0, (name, r, differ[:8], got[r][differ[:8]], want[differ[:8]])
+
+
+def test_process_logits_with_infinite_logits_side_by_side():
+    """Every probability is NaN then and the top-p walk removes nothing; masses that are no number must reach the histograms one by one
+    (five neighbours of one digit and a sixth elsewhere: an even number of 2^63 is nothing, the sixth alone is not)."""
+    vocab = 30011
+    logits = np.random.RandomState(5).randn(2, vocab).astype(np.float32)
+    logits[0, [0, 1, 2, 3, 4, 1000]] = np.inf
+    logits[1, 20000:20032] = np.inf
+    cfg = ol.make_config(max_new_tokens=1, do_sample=True, top_k=1000, top_p=0.7)
+    got = logits.copy()
+    status = gh.ctx().process_logits_host(got, np.zeros(2, dtype=np.int64), np.arange(3, dtype=np.int64), gh.psx_config(cfg))
+    assert (status == 0).all()
+    for r in range(2):
+        rc, want = ol.process_logits("oracle", logits[r], np.zeros(1, dtype=np.int64), 0, cfg)
+        assert rc == 0 and np.isfinite(want).sum() > 900
+        assert (got[r] == want).all(), (r, np.nonzero(got[r] != want)[0][:8])
