@@ -19,8 +19,8 @@
 // sequential double sums by at most about vocab * 3e-14; a decision closer than that to its
 // boundary may differ from the reference's, and the distances are reported per row (draw_margin,
 // top_p_margin) so that a caller can tell.  Slow (one CTA, a dozen
-// sweeps, each a chain of loads out of L2 and of double-precision exponentials) and rare.  One row of 50,021, top-p 0.95 on normal logits: 1544 us one
-// column at a time per thread, 1022 now; 148 rows 2530 and 1264; 300 rows of 128,256 with a history: 16.7 and 7.2 ms (14.0 with the columns batched alone).
+// sweeps, each a chain of loads out of L2 and of double-precision exponentials) and rare.  One row of 50,257, top-p 0.95 on normal logits with a history: 1409 us one
+// column at a time per thread, 992 now; 148 rows 1536 and 1206; 300 rows of 128,256: 9.5 and 5.6 ms.
 #pragma once
 
 #include "merge_rows_impl.cuh"
@@ -64,30 +64,58 @@ __device__ __forceinline__ double block_mass_sum(u64 units, double* scratch) {
     return (double)block_sum_u64(units, scratch) / kMassUnit;
 }
 
-// visit(column, logit, whether the row has it) for every column of a row, by whole warps.  A sweep is a chain of loads out of L2 and of exponentials, one per column and thread:
-// eight of each side by side.
-template <class Visit>
-__device__ __forceinline__ void sweep_row_by_warps(const float* x, int n, Visit visit) {
-    constexpr int kBatch = 8;
-    const int lane = threadIdx.x & 31;
-#pragma unroll 1
-    for (int first = threadIdx.x - lane; first < n; first += kBatch * kMergeThreads) {
-        float l[kBatch];
-#pragma unroll
-        for (int q = 0; q < kBatch; ++q) l[q] = first + lane + q * kMergeThreads < n ? x[first + lane + q * kMergeThreads] : 0.0f;
-#pragma unroll
-        for (int q = 0; q < kBatch; ++q) visit(first + lane + q * kMergeThreads, l[q], first + lane + q * kMergeThreads < n);
-    }
-}
-// ... that it has.
+// What a sweep over a row waits for is its loads out of L2: those of eight columns go out together.
+constexpr int kSweepBatch = 8;
+
+// visit(column, logit) for every column of a row.
 template <class Visit>
 __device__ __forceinline__ void sweep_row(const float* x, int n, Visit visit) {
-    sweep_row_by_warps(x, n, [&](int i, float l, bool there) {
-        if (there) visit(i, l);
-    });
+#pragma unroll 1
+    for (int first = threadIdx.x; first < n; first += kSweepBatch * kMergeThreads) {
+        float l[kSweepBatch];
+#pragma unroll
+        for (int q = 0; q < kSweepBatch; ++q) l[q] = first + q * kMergeThreads < n ? x[first + q * kMergeThreads] : 0.0f;
+#pragma unroll
+        for (int q = 0; q < kSweepBatch; ++q) {
+            if (first + q * kMergeThreads < n) visit(first + q * kMergeThreads, l[q]);
+        }
+    }
 }
 
-// hist[digit] += units over the lanes that take part (at least one), by the whole warp.  Neighbouring columns share the high digits of their number, and the
+// take(column, logit, units, whether there is such a column) for the columns that are wanted, by whole warps; mass_of(column, logit): below 0 takes the column
+// out after all.  A lane notes its wanted columns of a batch, and the warp weighs every lane's next one as long as there are any: a sweep pays for what is left
+// of the row.  (Weighing a column of all lanes wherever one of them wants it, in eight copies of the code: 444 rows of 8000, top-k 400 and top-p
+// 0.9, 516 us and 235 so; a single row of 50,257, top-p 0.95, 1117 and 992; two or four columns of a lane side by side gain nothing: 1012 and more.)
+template <class Wanted, class MassOf, class Take>
+__device__ __forceinline__ void weigh_row(const float* x, int n, Wanted wanted, MassOf mass_of, Take take) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int first = threadIdx.x - lane; first < n; first += kSweepBatch * kMergeThreads) {
+        float l[kSweepBatch];
+        uint32_t noted = 0;
+#pragma unroll
+        for (int q = 0; q < kSweepBatch; ++q) l[q] = first + lane + q * kMergeThreads < n ? x[first + lane + q * kMergeThreads] : 0.0f;
+#pragma unroll
+        for (int q = 0; q < kSweepBatch; ++q) {
+            if (first + lane + q * kMergeThreads < n && wanted(first + lane + q * kMergeThreads, l[q])) noted |= 1u << q;
+        }
+#pragma unroll 1
+        while (__any_sync(0xFFFFFFFFu, noted != 0)) {
+            const int at = __ffs(noted) - 1;
+            const bool mine = noted != 0;
+            noted &= noted - 1;
+            const int i = mine ? first + lane + at * kMergeThreads : 0;
+            float of = l[0];
+#pragma unroll
+            for (int q = 1; q < kSweepBatch; ++q) of = at == q ? l[q] : of;
+            const double mass = mine ? mass_of(i, of) : -1.0;
+            const bool on = mine && !(mass < 0.0);
+            take(i, of, on ? (u64)__double2ull_rn(mass * kMassUnit) : 0ull, on);
+        }
+    }
+}
+
+// hist[digit] += units over the lanes that take part, by the whole warp.  Neighbouring columns share the high digits of their number, and the
 // logits of a row the high digits of their keys: additions to one 64-bit counter queue up, so lanes of one digit are added up first,
 // as long as four or more share the digit of the first one left.  What the two 32-bit reductions do not hold -- the units of a mass that is no
 // number, 2^63 -- goes to the counter by itself.
@@ -121,13 +149,8 @@ __device__ inline void row_mass_select(const float* x, KeyOf key_of, InPlay in_p
 #pragma unroll 1
     for (int shift = top_shift; shift >= 0; shift -= 8) {
         u64* h = hist + 256 * (shift >> 3);
-        sweep_row_by_warps(x, n, [&](int i, float l, bool there) {
-            const uint32_t key = there ? key_of(i, l) : 0u;
-            const bool on = there && (key & mask) == prefix && in_play(i, l);
-            if (!__any_sync(0xFFFFFFFFu, on)) return;
-            const u64 units = on ? (u64)__double2ull_rn(mass_of(i, l) * kMassUnit) : 0;
-            add_by_digit(h, (key >> shift) & 255u, units, on);
-        });
+        weigh_row(x, n, [&](int i, float l) { return (key_of(i, l) & mask) == prefix && in_play(i, l); }, mass_of,
+                  [&](int i, float l, u64 units, bool on) { add_by_digit(h, (key_of(i, l) >> shift) & 255u, units, on); });
         __syncthreads();
         u64 run[8];  // lane L owns bins 8L .. 8L+7, ascending
         u64 local = 0;
@@ -272,7 +295,6 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
         return;
     }
     auto ex_of = [&](int i, float l) { return exp((double)processed(i, l) - (double)x_top); };  // (:46; -inf gives 0)
-    auto units_of = [&](double mass) { return (u64)__double2ull_rn(mass * kMassUnit); };
 
     // ---- top-k: the k-th largest of the processed row, ties kept (:80-88) ----
     uint32_t kth_key = 0;
@@ -288,9 +310,7 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
     if (sample && p.top_p < 1.0f) {
         const double limit = 1.0 - (double)p.top_p;
         u64 units = 0;
-        sweep_row(x, V, [&](int i, float l) {
-            if (key_of(i, l) >= kth_key) units += units_of(ex_of(i, l));
-        });
+        weigh_row(x, V, [&](int i, float l) { return key_of(i, l) >= kth_key; }, ex_of, [&](int, float, u64 u, bool) { units += u; });
         const double sum = block_mass_sum(units, s_scratch);
         clear_hist();
         double mass_below, mass_at;
@@ -334,21 +354,23 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
     const bool min_p_on = sample && p.min_p > 0.0f;
     if (min_p_on) {
         u64 units = 0;
-        sweep_row(x, V, [&](int i, float l) {
-            if (alive_p(i, l)) units += units_of(ex_of(i, l));
-        });
+        weigh_row(x, V, alive_p, ex_of, [&](int, float, u64 u, bool) { units += u; });
         min_p_sum = block_mass_sum(units, s_scratch);
     }
-    auto alive = [&](int i, float l) {
-        if (!alive_p(i, l)) return false;
+    auto lives = [&](int i, double mass) {
         if (!min_p_on || i == best_col) return true;
-        return !(ex_of(i, l) / min_p_sum < (double)p.min_p * (1.0 / min_p_sum));  // the maximum has exp(0) = 1
+        return !(mass / min_p_sum < (double)p.min_p * (1.0 / min_p_sum));  // the maximum has exp(0) = 1
+    };
+    // what a column that top-k and top-p leave weighs, or -1
+    auto mass_alive = [&](int i, float l) {
+        const double mass = ex_of(i, l);
+        return lives(i, mass) ? mass : -1.0;
     };
 
     if (process) {  // ProcessLogits: the row as the filters leave it, in place
         float* out = p.process_out + row * p.logits_row_stride;
         for (int i = tid; i < V; i += kMergeThreads) {
-            const float l = x[i], value = alive(i, l) ? processed(i, l) : -INFINITY;  // (reads column i before it writes it)
+            const float l = x[i], value = alive_p(i, l) && lives(i, min_p_on ? ex_of(i, l) : 0.0) ? processed(i, l) : -INFINITY;  // (reads column i before it writes it)
             out[i] = value;
         }
         if (tid == 0) p.row_status[row] = kRowDoneInPlace;
@@ -360,11 +382,9 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
     if (sample) {
         u64 units = 0;
         int count = 0;
-        sweep_row(x, V, [&](int i, float l) {
-            if (alive(i, l)) {
-                units += units_of(ex_of(i, l));
-                ++count;
-            }
+        weigh_row(x, V, alive_p, mass_alive, [&](int, float, u64 u, bool on) {
+            units += u;
+            count += on ? 1 : 0;
         });
         const double sum = block_mass_sum(units, s_scratch);
         survivors = (int)block_sum_u64((u64)count, s_scratch);
@@ -373,8 +393,7 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
         uint32_t hit;
         double mass_before, mass_at;
         const int column_shift = V <= (1 << 16) ? 8 : V <= (1 << 24) ? 16 : 24;
-        row_mass_select(x, [&](int i, float) { return (uint32_t)i; }, [&](int i, float l) { return alive(i, l) && ex_of(i, l) / sum != 0.0; }, ex_of, V,
-                        column_shift, u * sum, reinterpret_cast<u64*>(hist), hit, mass_before, mass_at);
+        row_mass_select(x, [&](int i, float) { return (uint32_t)i; }, alive_p, mass_alive, V, column_shift, u * sum, reinterpret_cast<u64*>(hist), hit, mass_before, mass_at);
         __syncthreads();
         const double before = mass_before / sum, upto = (mass_before + mass_at) / sum;
         draw_margin = before == 0.0 ? fabs(u - upto) : fmin(fabs(u - before), fabs(u - upto));
@@ -384,7 +403,8 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
     double z = 0.0;
     {
         u64 units = 0;
-        sweep_row(x, V, [&](int, float l) { units += units_of(exp((double)l - (double)raw_max)); });
+        weigh_row(x, V, [](int, float) { return true; }, [&](int, float l) { return exp((double)l - (double)raw_max); },
+                  [&](int, float, u64 u, bool) { units += u; });
         z = block_mass_sum(units, s_scratch);
     }
     if (tid == 0) {

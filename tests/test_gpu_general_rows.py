@@ -100,3 +100,11 @@ def test_process_logits_with_infinite_logits_side_by_side():
         rc, want = ol.process_logits("oracle", logits[r], np.zeros(1, dtype=np.int64), 0, cfg)
         assert rc == 0 and np.isfinite(want).sum() > 900
         assert (got[r] == want).all(), (r, np.nonzero(got[r] != want)[0][:8])
+
+
+@pytest.mark.parametrize("vocab", [1028, 2047, 2048, 2049, 2081, 4095, 6145])
+@pytest.mark.parametrize("name", ["top_k 1000", "top_k 300 + min_p"])
+def test_edges_of_a_sweep(vocab, name):
+    """A block looks at 2048 columns at a time, eight per lane."""
+    logits, hist, offsets, seeds = _rows(7, vocab, vocab)
+    _check(logits, hist, offsets, seeds, ol.make_config(max_new_tokens=1, **SETTINGS[name]), pad_columns=vocab % 3, shift=vocab % 2)
