@@ -199,6 +199,43 @@ __device__ inline void row_mass_select(const float* x, KeyOf key_of, InPlay in_p
     at = (double)at_units / kMassUnit;
 }
 
+constexpr int kHistWords = 4 * 256 * 2;
+__device__ __forceinline__ int bitmap_words(int columns) { return ((columns + 31) / 32 + 3) & ~3; }
+// Whether the whole row is on this GPU and its bitmap fits beside the histograms.
+__device__ __forceinline__ bool row_fits(const MergeParams& p) {
+    return (size_t)(bitmap_words((int)p.vocab) + kHistWords) * 4 <= (size_t)p.dyn_bytes && p.logits_col_begin == 0;
+}
+__device__ __forceinline__ bool row_has_flags(const MergeParams& p) { return (p.history_ids != nullptr && p.penalty != 1.0f) || p.num_banned > 0; }
+
+// The columns that the history (src/generation.cpp:62) or the EOS ban names, as a bitmap over the row; by the whole block.
+__device__ __forceinline__ void mark_flagged(const MergeParams& p, const int64_t row, uint32_t* bits) {
+    const int tid = threadIdx.x, words = bitmap_words((int)p.vocab);
+    for (int i = tid; i < words; i += kMergeThreads) bits[i] = 0;
+    __syncthreads();
+    if (p.history_ids != nullptr && p.penalty != 1.0f) {
+        for (int64_t i = p.history_offsets[row] + tid; i < p.history_offsets[row + 1]; i += kMergeThreads) {
+            const int64_t id = p.history_ids[i];
+            if (id >= 0 && id < p.vocab) atomicOr(&bits[id >> 5], 1u << (id & 31));
+        }
+    }
+    for (int i = tid; i < p.num_banned; i += kMergeThreads) {
+        const int64_t id = p.banned_ids[i];
+        if (id >= 0 && id < p.vocab) atomicOr(&bits[id >> 5], 1u << (id & 31));
+    }
+    __syncthreads();
+}
+
+// Column i's logit after the penalty and the ban (src/generation.cpp:59-73).
+__device__ __forceinline__ float flagged_logit(const MergeParams& p, const uint32_t* bits, int i, float l) {
+    if (!((bits[i >> 5] >> (i & 31)) & 1u)) return l;
+    bool banned = false;
+    for (int b = 0; b < p.num_banned; ++b) banned |= p.banned_ids[b] == (int64_t)i;
+    return banned ? -INFINITY : penalize(l, p.penalty);
+}
+
+// A raw logit's term of the sum below the log-probability (src/generation.cpp:133).
+__device__ __forceinline__ u64 raw_units(float l, float raw_max) { return (u64)__double2ull_rn(exp((double)l - (double)raw_max) * kMassUnit); }
+
 // (MergeParams by value: the copy is made where the call is, not on entry to the kernel.)
 __device__ __noinline__ void general_row(const MergeParams p, const int64_t row, u64* dyn) {
     __shared__ double s_scratch[kMergeThreads / 32];
@@ -207,16 +244,13 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
     const float* x = p.logits + row * p.logits_row_stride;
     const bool sample = p.do_sample != 0, apply_t = p.apply_temperature != 0;
     const bool top_k_on = sample && p.top_k > 0 && p.top_k < p.vocab;
-    const bool penalise = p.history_ids != nullptr && p.penalty != 1.0f;
-    const bool use_flags = penalise || p.num_banned > 0;
+    const bool use_flags = row_has_flags(p);
     const bool process = p.process_out != nullptr;
 
     // shared memory: the history bitmap, then the histograms of one selection at a time (1024 counters
     // of 32 bits, or 4 x 256 masses of 64)
-    const int words = ((V + 31) / 32 + 3) & ~3;
     uint32_t* bits = reinterpret_cast<uint32_t*>(dyn);
-    uint32_t* hist = bits + words;
-    constexpr int kHistWords = 4 * 256 * 2;
+    uint32_t* hist = bits + bitmap_words(V);
     auto give_up = [&](int status) {
         if (tid == 0) {
             p.row_status[row] = status;
@@ -227,7 +261,7 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
             if (p.diag) p.diag[row] = psx_row_diag{V, 0, INFINITY, INFINITY};
         }
     };
-    if ((size_t)(words + kHistWords) * 4 > (size_t)p.dyn_bytes || p.logits_col_begin != 0) {
+    if (!row_fits(p)) {
         give_up(PSX_ROW_TOO_WIDE);  // a vocabulary whose bitmap does not fit beside the histograms
         return;
     }
@@ -236,29 +270,10 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
         for (int i = tid; i < kHistWords; i += kMergeThreads) hist[i] = 0;
         __syncthreads();
     };
-    if (use_flags) {
-        for (int i = tid; i < words; i += kMergeThreads) bits[i] = 0;
-        __syncthreads();
-        if (penalise) {
-            for (int64_t i = p.history_offsets[row] + tid; i < p.history_offsets[row + 1]; i += kMergeThreads) {
-                const int64_t id = p.history_ids[i];
-                if (id >= 0 && id < p.vocab) atomicOr(&bits[id >> 5], 1u << (id & 31));  // src/generation.cpp:62
-            }
-        }
-        for (int i = tid; i < p.num_banned; i += kMergeThreads) {
-            const int64_t id = p.banned_ids[i];
-            if (id >= 0 && id < p.vocab) atomicOr(&bits[id >> 5], 1u << (id & 31));
-        }
-        __syncthreads();
-    }
+    if (use_flags) mark_flagged(p, row, bits);
     // the processed logit of column i (src/generation.cpp:59-79)
     auto processed = [&](int i, float l) {
-        float y = l;
-        if (use_flags && ((bits[i >> 5] >> (i & 31)) & 1u)) {
-            bool banned = false;
-            for (int b = 0; b < p.num_banned; ++b) banned |= p.banned_ids[b] == (int64_t)i;
-            y = banned ? -INFINITY : penalize(y, p.penalty);
-        }
+        const float y = use_flags ? flagged_logit(p, bits, i, l) : l;
         return sample ? temper(y, apply_t, p.temperature) : y;
     };
     auto key_of = [&](int i, float l) { return ordered_key(processed(i, l)); };
@@ -403,8 +418,7 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
     double z = 0.0;
     {
         u64 units = 0;
-        weigh_row(x, V, [](int, float) { return true; }, [&](int, float l) { return exp((double)l - (double)raw_max); },
-                  [&](int, float, u64 u, bool) { units += u; });
+        sweep_row(x, V, [&](int, float l) { units += raw_units(l, raw_max); });
         z = block_mass_sum(units, s_scratch);
     }
     if (tid == 0) {
@@ -412,6 +426,32 @@ __device__ __noinline__ void general_row(const MergeParams p, const int64_t row,
         p.tokens[row] = chosen;
         p.log_probs[row] = (float)log(exp((double)x[chosen] - (double)raw_max) / z);
         if (p.diag) p.diag[row] = psx_row_diag{V, survivors, draw_margin, top_p_margin};
+    }
+}
+
+// A greedy row whose lists ran over (a constant row, thousands of ties at the maximum).  The row pass knows the maxima, so one sweep gives the first column
+// of the processed one (:135) and the sum below the log-probability (:133,156), with general_row's terms.  (One constant row among 1024 x 49,152: the call
+// takes 122 us through merge_row and general_row, 90 so, 41 without such a row.)
+__device__ __noinline__ void greedy_row(const MergeParams p, const int64_t row, const float raw_max, const float y_max, u64* dyn) {
+    __shared__ double s_scratch[kMergeThreads / 32];
+    const int V = (int)p.vocab;
+    const float* x = p.logits + row * p.logits_row_stride;
+    const bool use_flags = row_has_flags(p);
+    uint32_t* bits = reinterpret_cast<uint32_t*>(dyn);
+    if (use_flags) mark_flagged(p, row, bits);
+    u64 units = 0;
+    uint32_t first = (uint32_t)V - 1u;
+    sweep_row(x, V, [&](int i, float l) {
+        if ((use_flags ? flagged_logit(p, bits, i, l) : l) == y_max) first = min(first, (uint32_t)i);
+        units += raw_units(l, raw_max);
+    });
+    const double z = block_mass_sum(units, s_scratch);
+    const uint32_t chosen = block_min_u32(first, s_scratch);
+    if (threadIdx.x == 0) {
+        p.row_status[row] = PSX_ROW_OK;
+        p.tokens[row] = (int64_t)chosen;
+        p.log_probs[row] = (float)log(exp((double)x[chosen] - (double)raw_max) / z);
+        if (p.diag) p.diag[row] = psx_row_diag{V, 1, INFINITY, INFINITY};
     }
 }
 

@@ -34,14 +34,25 @@ __device__ unsigned long long g_merge_times[1024 * 4];
 #include "merge_rows_list_impl.cuh"
 #include "peer_exchange.cuh"
 
+#include <algorithm>
+
 namespace psx {
 
 namespace {
 
 constexpr int kSmCount = 148;
 
-// What the lists of a row do not decide, by the whole block.
+// What the lists of a row do not decide, by the whole block: of a greedy row the parts' maxima are known all the same.
 __device__ __forceinline__ void replay_row(const MergeParams& p, const int64_t row, unsigned long long* dyn) {
+    if (!p.do_sample && p.general == 1 && p.parts <= 32 && survivor::row_fits(p)) {
+        const survivor::RowView v = survivor::view_of_row(p, row);
+        survivor::PartsJoined j;
+        survivor::load_parts(p, v, j);
+        survivor::join_parts(p, v, j);
+        j.bad &= 3u;  // (that a list ran over is known)
+        if (!survivor::settle_bad_row(v, j, j.y_max)) survivor::greedy_row(p, row, j.raw_max, j.y_max, dyn);
+        return;
+    }
     if (p.general != 2) survivor::merge_row(p, row, dyn);  // too many for the list, or a decision too close to its level
     if (p.general != 0 && p.logits != nullptr) {
         // A row the candidate lists could not decide is decided from the row itself.
@@ -50,24 +61,28 @@ __device__ __forceinline__ void replay_row(const MergeParams& p, const int64_t r
     }
 }
 
-// Greedy, a warp per row and eight rows per block.  A greedy row has a few candidates per part: latency bound, a trip to memory and two
+// Greedy, a warp per row and up to eight rows per block.  A greedy row has a few candidates per part: latency bound, a trip to memory and two
 // exponentials, for which eight warps are seven too many once there are more rows than blocks fit the GPU at once.  1024 x 49,152, the whole
-// call: 44.9 us with a block per row (2.3 rounds of them), 41.1 so; 4000 x 8000: 59 and 41 us.
+// call: 45.2 us with a block per row (2.3 rounds of them), 40.8 so; 4000 x 8000: 59 and 41 us.
+// A row that its warp cannot decide is left to its block, the block's rows one after another.  Such rows lie side by side (padding) or a power of two
+// apart, so a block's rows lie an odd number of blocks apart, and as many blocks share the rows as the GPU holds.  1024 x 49,152 with 64 constant
+// rows side by side: 183 us by blocks, 583 with eight neighbours to a block, 102 so; every fourth row constant: 223, 252, 140; a quarter at random: 223, 415, 221;
+// all: 593, 756, 318.
 __global__ void __launch_bounds__(kMergeThreads, 3) merge_greedy_rows_kernel(const __grid_constant__ MergeParams p) {
     extern __shared__ __align__(16) unsigned long long dyn[];
     __shared__ uint32_t s_left;  // rows that their warps could not decide
     const int warp = threadIdx.x >> 5;
-    const int64_t first = (int64_t)blockIdx.x * survivor::kListWarps;
+    const int64_t mine = blockIdx.x + (int64_t)gridDim.x * warp;
     if (threadIdx.x == 0) s_left = 0;
     __syncthreads();
     grid_dependency_wait();        // everything this kernel reads was written by the kernel before it
     grid_dependents_may_launch();  // a row pass that follows reads none of this kernel's results
-    if (first + warp < p.rows && !survivor::list_greedy_by_warp(p, survivor::view_of_row(p, p.row_begin + first + warp))) {
+    if (mine < p.rows && !survivor::list_greedy_by_warp(p, survivor::view_of_row(p, p.row_begin + mine))) {
         if ((threadIdx.x & 31) == 0) atomicOr(&s_left, 1u << warp);
     }
     __syncthreads();
     for (uint32_t left = s_left; left; left &= left - 1) {
-        replay_row(p, p.row_begin + first + __ffs(left) - 1, dyn);
+        replay_row(p, p.row_begin + blockIdx.x + (int64_t)gridDim.x * (__ffs(left) - 1), dyn);
         __syncthreads();
     }
 }
@@ -174,7 +189,7 @@ cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_
     // by warps; 400 rows: 18.3 and 18.0, one row: 6.7 and 7.8.  Up to four
     // parts, which one look takes; 16 parts, 500 x 262,144: 92.7 and 93.9; rows that are handed on whole, 1024 x 600: 19 and 26.)
     if (!p.do_sample && p.rows > 3 * kSmCount && p.parts <= 4 && p.whole_rows == 0 && p.arrivals == nullptr && p.survivor_cols == nullptr) {
-        const unsigned blocks = (unsigned)((p.rows + survivor::kListWarps - 1) / survivor::kListWarps);
+        const unsigned blocks = (unsigned)std::max<int64_t>(3 * kSmCount - 1, (p.rows + survivor::kListWarps - 1) / survivor::kListWarps) | 1u;
         return launch_overlapping(merge_greedy_rows_kernel, dim3(blocks), dim3(kMergeThreads), shared, stream, with_size);
     }
     return launch_overlapping(kernel_for(p), dim3((unsigned)p.rows), dim3(kMergeThreads), shared, stream, with_size);

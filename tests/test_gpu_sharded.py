@@ -102,3 +102,29 @@ def test_a_shard_scan_may_be_the_first_call_of_a_process():
                            f"{Path(__file__).resolve()}::test_c5_in_eight_shards_matches_the_reference_fixture"],
                           capture_output=True, text=True, timeout=600)
     assert done.returncode == 0, done.stdout[-2000:] + done.stderr[-2000:]
+
+
+@pytest.mark.parametrize("world", [2, 3, 4])
+@pytest.mark.parametrize("rows", [444, 445, 450])
+def test_many_greedy_rows_over_few_shards(world, rows):
+    """More rows than the survivor stage has blocks for, records of 64 slots; a record that overflows is reported, as it is with fewer rows."""
+    rng = np.random.RandomState(rows + world)
+    vocab = 6000
+    logits = (rng.randn(rows, vocab) * 3).astype(np.float32)
+    logits[5, [11, 3000, 5999]] = logits[5].max() + 2.0  # ties across shards: lowest column wins
+    logits[rows - 1, [4500, 100]] = logits[rows - 1].max() + 1.0
+    logits[200:212] = 1.0                                # constant: no record holds their ties
+    logits[300, 5000] = np.nan
+    hist = rng.randint(0, vocab, size=(rows, 10)).astype(np.int64)
+    offsets = np.arange(rows + 1, dtype=np.int64) * 10
+    seeds = np.arange(rows, dtype=np.uint64)
+    cfg = ol.make_config(max_new_tokens=1, repetition_penalty=1.3)
+    want = ol.rows("oracle", logits, hist.ravel(), offsets, cfg, seeds)
+    tokens, logp, status = run_sharded(logits, hist.ravel(), offsets, cfg, None, world)
+    few_tokens, few_logp, few_status = run_sharded(logits, hist.ravel(), offsets, cfg, None, world, merge_blocks=3)
+    assert (tokens == few_tokens).all() and (status == few_status).all() and np.abs(logp - few_logp).max() <= 1e-6
+    ok = np.ones(rows, dtype=bool)
+    ok[200:212] = ok[300] = False
+    assert (status[ok] == 0).all() and status[300] == psx.ROW_NON_FINITE and (status[200:212] == psx.ROW_TOO_WIDE).all()
+    assert tokens[ok].tolist() == want["token"][ok].tolist()
+    assert (np.abs(logp[ok] - want["log_prob"][ok]) <= 1e-5 * np.abs(want["log_prob"][ok]) + 1e-9).all()
