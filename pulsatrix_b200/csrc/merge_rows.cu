@@ -185,10 +185,11 @@ cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_
     MergeParams with_size = p;
     with_size.dyn_bytes = (int32_t)shared;
     if (launched != nullptr) ++*launched;
-    // A warp per greedy row where a block each would take a second round (three to an SM), on lists of few slots.  (500 x 49,152: 24.9 us by blocks, 22.9
-    // by warps; 400 rows: 18.3 and 18.0, one row: 6.7 and 7.8.  Up to four
-    // parts, which one look takes; 16 parts, 500 x 262,144: 92.7 and 93.9; rows that are handed on whole, 1024 x 600: 19 and 26.)
-    if (!p.do_sample && p.rows > 3 * kSmCount && p.parts <= 4 && p.whole_rows == 0 && p.arrivals == nullptr && p.survivor_cols == nullptr) {
+    // A warp per greedy row where a block each would take a second round (three to an SM), up to eight parts.  The whole call by blocks and by warps, us:
+    // three parts, 49,152 columns: 400 rows 18.3 and 18.0, 500 25.2 and 23.0, 1024 45.2 and 40.8; five parts, 81,920: 450 rows 33.6 and 33.2, 1024 66.1 and
+    // 62.5 (65,537, up to 512 rows: 32.1 and 32.9); eight parts, 128,256: 450 rows 47.6 and 47.1, 1024 97.2 and 93.6; sixteen, 262,144: 500 rows 92.7 and 93.9.
+    // Rows that are handed on whole, 1024 x 600: 19 and 26.
+    if (!p.do_sample && p.rows > 3 * kSmCount && p.parts <= 8 && p.whole_rows == 0 && p.arrivals == nullptr && p.survivor_cols == nullptr) {
         const unsigned blocks = (unsigned)std::max<int64_t>(3 * kSmCount - 1, (p.rows + survivor::kListWarps - 1) / survivor::kListWarps) | 1u;
         return launch_overlapping(merge_greedy_rows_kernel, dim3(blocks), dim3(kMergeThreads), shared, stream, with_size);
     }

@@ -104,7 +104,7 @@ def test_a_shard_scan_may_be_the_first_call_of_a_process():
     assert done.returncode == 0, done.stdout[-2000:] + done.stderr[-2000:]
 
 
-@pytest.mark.parametrize("world", [2, 3, 4])
+@pytest.mark.parametrize("world", [2, 4, 5, 8, 9])
 @pytest.mark.parametrize("rows", [444, 445, 450])
 def test_many_greedy_rows_over_few_shards(world, rows):
     """More rows than the survivor stage has blocks for, records of 64 slots; a record that overflows is reported, as it is with fewer rows."""
