@@ -271,10 +271,16 @@ struct Head {
 };
 
 // The tiles of the last round: E to EM entries per lane, as many as it says.
-template <class K, int E, int EM>
+template <class K, int E, int EM, bool kTokenMajor>
 __device__ __forceinline__ void last_tiles(const HeadParams& p, float* shared, int64_t j0) {
     if constexpr (E < EM) {
-        if (p.last_entries > E) return last_tiles<K, E + 1, EM>(p, shared, j0);
+        if (p.last_entries > E) return last_tiles<K, E + 1, EM, kTokenMajor>(p, shared, j0);
+    }
+    if constexpr (EM == 8 && !kTokenMajor) {
+        // A last tile that is not whole would come in 4 bytes at a time, and the wider it is the longer the others would wait for it: it is moved back,
+        // onto entries that its neighbour forms as well, bit for bit.  (48 rows of 65,536 x 2048, feature-major: 874 and 480 us.)
+        constexpr int kWidth = K::kTile / EM * E;
+        if (p.vector_ok && p.vocab >= kWidth) j0 = min(j0, p.vocab - kWidth);
     }
     K::template tiles<E>(p, shared, j0, 0, 1);
 }
@@ -298,7 +304,7 @@ __global__ void __launch_bounds__(32 * G * H, kCtas) head_kernel(const __grid_co
     if (p.full_rounds > 0) K::template tiles<EM>(p, head_shared, (int64_t)blockIdx.x * K::kTile, round, p.full_rounds);
     const int64_t j0 = p.full_rounds * round + (int64_t)blockIdx.x * 32 * p.last_entries * H;
     if (p.last_entries == 0 || j0 >= p.vocab) return;
-    last_tiles<K, 1, EM>(p, head_shared, j0);
+    last_tiles<K, 1, EM, kTokenMajor>(p, head_shared, j0);
 }
 
 template <int R, int G, int H, int KC, int S, int kCtas, int EM, bool kTokenMajor>
@@ -339,15 +345,27 @@ cudaError_t launch_group(const HeadParams& p, int sm_count, cudaStream_t stream)
     // HBM serves 5.9 TB/s in runs of 256 bytes, 5.0 in runs of 128); from four rows on the reads of the hidden states weigh, so four, or eight
     // where the rows leave the registers for it.  Token-major, up to 16 rows, chunks of 32 features gain for the same reason (16 rows: 463 us and
     // 308 with 16 features); feature-major a chunk of 32 is more rows of the matrix and no longer a run (9 to 12 rows: 537 us for 428).
+    // groups: what an SM has of the vocabulary, in the 64 entries that a CTA takes per entry of a lane.  Where the next wider layout fills its rounds better it
+    // is the faster one all the same (2048 features, us, the layout of the row count and the wider one): token-major, 16 rows, 100,000 entries (11 groups) 338 and 325;
+    // 32 rows, 16,000 (2) 175 and 165, 80,000 (9) 469 and 452, 151,552 (16) 788 and 778, 227,328 of 1024 features (24) 683 and 587, but 100,000 (11) 574 and 626;
+    // feature-major, 12 rows, 90,000 (10) 441 and 430; 24 rows, 80,000 (9) 502 and 481, and where the copies are of 4 bytes 75,777 (9) 760 and 617, 90,001 (10) 887
+    // and 736, 130,001 (14) 1180 and 1087, but 100,001 (11) 825 and 879.
+    const int64_t lanes = 64 * (int64_t)sm_count, groups = (p.vocab + lanes - 1) / lanes;
     if (p.rows <= 1) return kTokenMajor ? launch_one<1, 1, 4, 64, 2, 3, 1, true>(p, sm_count, stream) : launch_one<1, 1, 4, 32, 4, 3, 1, false>(p, sm_count, stream);
     if (p.rows <= 2) return kTokenMajor ? launch_one<2, 1, 4, 64, 2, 3, 1, true>(p, sm_count, stream) : launch_one<2, 1, 4, 32, 3, 3, 1, false>(p, sm_count, stream);
     if (p.rows <= 4) return launch_one<2, 2, 2, 32, 2, 3, 4, kTokenMajor>(p, sm_count, stream);
     if (kTokenMajor && p.rows <= 6) return launch_one<2, 3, 2, 32, 2, 3, 4, true>(p, sm_count, stream);
     if (p.rows <= 8) return launch_one<4, 2, 2, 16, 2, 4, 4, kTokenMajor>(p, sm_count, stream);
-    if (p.rows <= 12) return kTokenMajor ? launch_one<4, 3, 2, 32, 2, 2, 4, true>(p, sm_count, stream) : launch_one<4, 3, 2, 16, 2, 4, 4, false>(p, sm_count, stream);
-    if (p.rows <= 16) return kTokenMajor ? launch_one<8, 2, 2, 32, 2, 2, 4, true>(p, sm_count, stream) : launch_one<8, 2, 2, 16, 2, 4, 4, false>(p, sm_count, stream);
-    if (p.rows <= 24) return launch_one<4, 6, 2, 16, 2, 2, 8, kTokenMajor>(p, sm_count, stream);
-    if (p.rows <= 32) return kTokenMajor ? launch_one<16, 2, 2, 16, 2, 2, 8, true>(p, sm_count, stream) : launch_one<8, 4, 2, 16, 3, 2, 4, false>(p, sm_count, stream);
+    if (p.rows <= 12 && kTokenMajor) return launch_one<4, 3, 2, 32, 2, 2, 4, true>(p, sm_count, stream);
+    if (p.rows <= 12 && !(groups >= 9 && groups <= 12)) return launch_one<4, 3, 2, 16, 2, 4, 4, false>(p, sm_count, stream);
+    if (p.rows <= 16) return kTokenMajor && groups != 11 && groups != 12 ? launch_one<8, 2, 2, 32, 2, 2, 4, true>(p, sm_count, stream)
+                                                                                        : launch_one<8, 2, 2, 16, 2, 4, 4, kTokenMajor>(p, sm_count, stream);
+    const bool wider_24 = !kTokenMajor && (groups == 9 || (!p.vector_ok && (groups == 10 || groups == 14)));
+    if (p.rows <= 24 && !wider_24) return launch_one<4, 6, 2, 16, 2, 2, 8, kTokenMajor>(p, sm_count, stream);
+    if (p.rows <= 32) {
+        const bool eight = kTokenMajor && p.rows > 24 && ((groups >= 3 && groups <= 6) || (groups >= 10 && groups <= 14) || (groups >= 17 && groups <= 22));
+        return eight ? launch_one<16, 2, 2, 16, 2, 2, 8, true>(p, sm_count, stream) : launch_one<8, 4, 2, 16, 3, 2, 4, kTokenMajor>(p, sm_count, stream);
+    }
     if (p.rows <= 48) return launch_one<8, 6, 2, 16, 2, 1, 8, kTokenMajor>(p, sm_count, stream);
     return launch_one<16, 4, 2, 16, 3, 2, 4, kTokenMajor>(p, sm_count, stream);
 }

@@ -131,3 +131,28 @@ def test_a_second_device_of_the_process(rows):
     hidden, weight = rng.randn(rows, 64).astype(np.float32), rng.randn(500, 64).astype(np.float32)
     got = [psx.Context(d).lm_head_logits(torch.from_numpy(hidden).to(f"cuda:{d}"), torch.from_numpy(weight).to(f"cuda:{d}")).cpu() for d in (0, 1)]
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("rows,vocab,vocab_by_d", [
+    # two full rounds and a rest, at the largest row count of every layout from 5 rows on
+    (6, 2 * 113_664 + 30_000, True), (8, 2 * 151_552 + 44, True), (12, 2 * 75_776 + 40_000, True), (16, 2 * 75_776 + 60_000, True),
+    (24, 2 * 151_552 + 30_000, True), (32, 2 * 75_776 + 20_000, True), (48, 2 * 75_776 + 40_000, True), (64, 2 * 75_776 + 20_000, True),
+    (8, 2 * 151_552 + 44, False), (12, 2 * 151_552 + 40_000, False), (16, 2 * 151_552 + 4, False), (24, 2 * 151_552 + 30_004, False),
+    (32, 2 * 75_776 + 20_004, False), (48, 2 * 75_776 + 40_004, False), (64, 2 * 75_776 + 100, False),
+    # five, six and seven entries per lane, and a last tile that is four entries wide
+    (24, 90_004, True), (24, 90_004, False), (24, 113_604, False), (24, 130_004, False), (48, 45_060, True), (48, 45_060, False), (48, 66_308, False),
+])
+def test_whole_chunks_over_several_tiles(rows, vocab, vocab_by_d):
+    """Features enough for several chunks and a shorter last one, copies of 16 bytes; against the same loop as elementwise torch operations on the GPU."""
+    import torch
+    d = 68
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows + vocab)
+    hidden = torch.randn((rows, d), generator=gen, device="cuda")
+    weight = torch.randn((d, vocab), generator=gen, device="cuda").mul_(0.05)
+    hidden[0, 0] = -0.0
+    want = torch.zeros((rows, vocab), device="cuda")
+    for p in range(d):
+        want.add_(hidden[:, p:p + 1] * weight[p])  # (the product and the sum are operations of their own: both rounded)
+    got = gh.ctx().lm_head_logits(hidden, weight.T.contiguous() if vocab_by_d else weight, vocab_by_d=vocab_by_d)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
