@@ -520,7 +520,7 @@ psx_status psx_b200_sample_rows(psx_ctx* ctx, void* stream_ptr, const float* log
         ++ctx->launches;
     }
     if (ctx->timing) PSX_CUDA(cudaEventRecord(marks[1], stream));
-    PSX_CUDA(psx::launch_merge_rows(mp, stream, &ctx->launches));
+    PSX_CUDA(psx::launch_merge_rows(mp, ctx->sm_count, stream, &ctx->launches));
     if (ctx->timing) {
         PSX_CUDA(cudaEventRecord(marks[2], stream));
         ctx->timing_events.insert(ctx->timing_events.end(), marks, marks + 3);
@@ -585,7 +585,7 @@ psx_status psx_b200_process_logits(psx_ctx* ctx, void* stream_ptr, float* logits
         mp.survivor_vals = static_cast<float*>(ctx->surv_vals.ptr);
         mp.survivor_counts = static_cast<uint32_t*>(ctx->surv_counts.ptr);
         mp.survivor_cap = plan.sort_capacity;
-        PSX_CUDA(psx::launch_merge_rows(mp, stream));
+        PSX_CUDA(psx::launch_merge_rows(mp, ctx->sm_count, stream));
         ++ctx->launches;
         pp.survivor_cols = mp.survivor_cols;
         pp.survivor_vals = mp.survivor_vals;
@@ -895,7 +895,7 @@ psx_status shard_merge_impl(psx_ctx* ctx, cudaStream_t stream, const char* base,
         mp.publish = 1;
         mp.peers = *publish_to;
     }
-    PSX_CUDA(psx::launch_merge_rows(mp, stream, &ctx->launches));
+    PSX_CUDA(psx::launch_merge_rows(mp, ctx->sm_count, stream, &ctx->launches));
     return PSX_OK;
 }
 }  // namespace
@@ -964,7 +964,7 @@ psx_status psx_b200_top_k_rows(psx_ctx* ctx, void* stream_ptr, const float* in, 
         ctx->launches += (rows + batch - 1) / batch;
         return PSX_OK;
     }
-    PSX_CUDA(psx::launch_topk_rows(in, values, indices, rows, cols, k, largest != 0, stream));
+    PSX_CUDA(psx::launch_topk_rows(in, values, indices, rows, cols, k, largest != 0, ctx->sm_count, stream));
     ++ctx->launches;
     return PSX_OK;
 }

@@ -1,4 +1,4 @@
-// The survivor stage: one CTA per row turns the row pass's candidates into a token.
+// The survivor stage: a CTA per row -- a warp per row for many greedy rows -- turns the row pass's candidates into a token.
 //
 // Input per row: for each part its raw max / tail sum-exp and a few dozen candidates (raw logit,
 // column, flags).  The stage
@@ -40,18 +40,19 @@ namespace psx {
 
 namespace {
 
-constexpr int kSmCount = 148;
-
 // What the lists of a row do not decide, by the whole block: of a greedy row the parts' maxima are known all the same.
+template <bool kGreedy>
 __device__ __forceinline__ void replay_row(const MergeParams& p, const int64_t row, unsigned long long* dyn) {
-    if (!p.do_sample && p.general == 1 && p.parts <= 32 && survivor::row_fits(p)) {
-        const survivor::RowView v = survivor::view_of_row(p, row);
-        survivor::PartsJoined j;
-        survivor::load_parts(p, v, j);
-        survivor::join_parts(p, v, j);
-        j.bad &= 3u;  // (that a list ran over is known)
-        if (!survivor::settle_bad_row(v, j, j.y_max)) survivor::greedy_row(p, row, j.raw_max, j.y_max, dyn);
-        return;
+    if constexpr (kGreedy) {
+        if (p.general == 1 && p.parts <= 32 && survivor::row_fits(p)) {
+            const survivor::RowView v = survivor::view_of_row(p, row);
+            survivor::PartsJoined j;
+            survivor::load_parts(p, v, j);
+            survivor::join_parts(p, v, j);
+            j.bad &= 3u;  // (that a list ran over is known)
+            if (!survivor::settle_bad_row(v, j, j.y_max)) survivor::greedy_row(p, row, j.raw_max, j.y_max, dyn);
+            return;
+        }
     }
     if (p.general != 2) survivor::merge_row(p, row, dyn);  // too many for the list, or a decision too close to its level
     if (p.general != 0 && p.logits != nullptr) {
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_greedy_rows_kernel(con
     }
     __syncthreads();
     for (uint32_t left = s_left; left; left &= left - 1) {
-        replay_row(p, p.row_begin + blockIdx.x + (int64_t)gridDim.x * (__ffs(left) - 1), dyn);
+        replay_row<true>(p, p.row_begin + blockIdx.x + (int64_t)gridDim.x * (__ffs(left) - 1), dyn);
         __syncthreads();
     }
 }
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(kMergeThreads, kKind == survivor::kListNucleus
         }
     } else if (p.general == 2 || !survivor::list_row<kKind>(p, row, survivor::view_of_row(p, row), dyn, ready)) {
         __syncthreads();
-        replay_row(p, row, dyn);
+        replay_row<kKind == survivor::kListGreedy>(p, row, dyn);
     }
     if (p.arrivals != nullptr) {
         __syncthreads();
@@ -177,7 +178,7 @@ auto kernel_for(const MergeParams& p) {
 }
 }  // namespace
 
-cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_t* launched) {
+cudaError_t launch_merge_rows(const MergeParams& p, int sm_count, cudaStream_t stream, uint64_t* launched) {
     if (p.rows <= 0) return cudaSuccess;
     // The same condition as the kernel's: the overlaid layout is for plans without a top-k.
     const bool overlay = p.overlay != 0 && p.logits != nullptr && !(p.do_sample && p.top_k > 0 && p.top_k < p.vocab);
@@ -189,8 +190,8 @@ cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_
     // three parts, 49,152 columns: 400 rows 18.3 and 18.0, 500 25.2 and 23.0, 1024 45.2 and 40.8; five parts, 81,920: 450 rows 33.6 and 33.2, 1024 66.1 and
     // 62.5 (65,537, up to 512 rows: 32.1 and 32.9); eight parts, 128,256: 450 rows 47.6 and 47.1, 1024 97.2 and 93.6; sixteen, 262,144: 500 rows 92.7 and 93.9.
     // Rows that are handed on whole, 1024 x 600: 19 and 26.
-    if (!p.do_sample && p.rows > 3 * kSmCount && p.parts <= 8 && p.whole_rows == 0 && p.arrivals == nullptr && p.survivor_cols == nullptr) {
-        const unsigned blocks = (unsigned)std::max<int64_t>(3 * kSmCount - 1, (p.rows + survivor::kListWarps - 1) / survivor::kListWarps) | 1u;
+    if (!p.do_sample && p.rows > 3 * sm_count && p.parts <= 8 && p.whole_rows == 0 && p.arrivals == nullptr && p.survivor_cols == nullptr) {
+        const unsigned blocks = (unsigned)std::max<int64_t>(3 * sm_count - 1, (p.rows + survivor::kListWarps - 1) / survivor::kListWarps) | 1u;
         return launch_overlapping(merge_greedy_rows_kernel, dim3(blocks), dim3(kMergeThreads), shared, stream, with_size);
     }
     return launch_overlapping(kernel_for(p), dim3((unsigned)p.rows), dim3(kMergeThreads), shared, stream, with_size);

@@ -87,7 +87,7 @@ size_t merge_rows_shared_bytes(int sort_capacity, int gather_capacity, bool over
 // The slot_shift for lists that usually hold about `expected` candidates, within the fetch budget.
 int merge_slot_shift(int parts, int part_cap, int expected);
 cudaError_t configure_merge_rows();  // once per device: lifts the kernel's dynamic shared-memory limit to the device's
-// launched (optional): how many kernels the call launched, added to what is there.
-cudaError_t launch_merge_rows(const MergeParams& p, cudaStream_t stream, uint64_t* launched = nullptr);
+// sm_count: the device's.  launched (optional): how many kernels the call launched, added to what is there.
+cudaError_t launch_merge_rows(const MergeParams& p, int sm_count, cudaStream_t stream, uint64_t* launched = nullptr);
 
 }  // namespace psx

@@ -168,7 +168,8 @@ struct RawSum {
     }
     __device__ __forceinline__ void add_low(float l) { low += ex2_approx(__fmaf_rn(l, kLog2e, -c_l2)); }
     // The warp's sum, in units of 2^-40 of the largest term: integer reductions, a fraction of the time of five additions in double
-    // one after another.  (A lane has at most a few dozen terms of at most one.)
+    // one after another.  (A lane has up to 128 terms of at most one, 256 where a warp has a row of eight full lists to itself, as a rule a few: their
+    // float sum differs from another order's by a rounding of the float log-probability, the units stay below 2^49.)
     __device__ __forceinline__ u64 of_warp() const { return warp_sum_units((u64)__double2ull_rn((high + (double)low * exp2_of_minus_small(c_res)) * 0x1p40)); }
 };
 

@@ -51,6 +51,7 @@ static __device__ __align__(256) unsigned char g_scratch[sizeof(StaticScratch)];
 struct DeviceSetup {
     bool done = false;
     StaticScratch* scratch = nullptr;
+    int sm_count = 0;
 };
 DeviceSetup g_setup[kMaxDevices];
 std::mutex g_setup_mutex;
@@ -114,6 +115,7 @@ extern "C" psx_status psx_b200_sample_rows_static(void* stream_ptr, const float*
     PSX_STATIC_CUDA(cudaGetDevice(&device));
     if (device < 0 || device >= kMaxDevices) return set_error(PSX_ERR_UNSUPPORTED, "psx_b200: device index too large");
     StaticScratch* scratch = nullptr;
+    int sm_count = 0;
     {
         std::lock_guard<std::mutex> lock(g_setup_mutex);
         DeviceSetup& setup = g_setup[device];
@@ -124,10 +126,12 @@ extern "C" psx_status psx_b200_sample_rows_static(void* stream_ptr, const float*
             // once, and nobody lowers them again.
             PSX_STATIC_CUDA(psx::configure_scan_rows());
             PSX_STATIC_CUDA(psx::configure_merge_rows());
+            PSX_STATIC_CUDA(cudaDeviceGetAttribute(&setup.sm_count, cudaDevAttrMultiProcessorCount, device));
             setup.scratch = static_cast<StaticScratch*>(address);
             setup.done = true;
         }
         scratch = setup.scratch;
+        sm_count = setup.sm_count;
     }
     cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
 
@@ -167,6 +171,6 @@ extern "C" psx_status psx_b200_sample_rows_static(void* stream_ptr, const float*
 
     psx::MergeParams mp{};
     psx::fill_merge_params(mp, sp, plan, c, rows, vocab, uniforms, tokens, log_probs, row_status, nullptr, logits, row_stride);
-    PSX_STATIC_CUDA(psx::launch_merge_rows(mp, stream));
+    PSX_STATIC_CUDA(psx::launch_merge_rows(mp, sm_count, stream));
     return PSX_OK;
 }

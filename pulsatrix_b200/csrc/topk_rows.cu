@@ -741,7 +741,7 @@ cudaError_t launch_sort_rows(const float* in, float* values, float* indices, siz
 }
 
 cudaError_t launch_topk_rows(const float* in, float* values, float* indices, size_t rows, size_t cols, size_t k,
-                             bool largest, cudaStream_t stream) {
+                             bool largest, int sm_count, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
     TopKParams p;
     p.in = in;
@@ -763,8 +763,8 @@ cudaError_t launch_topk_rows(const float* in, float* values, float* indices, siz
     p.wait_limit_ns = kDefaultWaitLimitNs;
     // Beyond k 128 lists overflow more often than not, and a block that holds its slice has fewer beside it to hide the radix
     // selection: 4096 x 16,384, k 256: 840 us with held slices, 483 without (k 100: 115 and 120).  Where all blocks are resident at once,
-    // three on each of 148 SMs, it does not matter: 64 x 16,384, k 200: 23 to 34 us held (as lists overflow), 37 not.
-    const bool held = p.list_cap != 0 && p.slice <= kHeldMax && (k <= 128 || rows * p.cluster <= 3 * 148);
+    // three on each SM, it does not matter: 64 x 16,384, k 200: 23 to 34 us held (as lists overflow), 37 not.
+    const bool held = p.list_cap != 0 && p.slice <= kHeldMax && (k <= 128 || rows * p.cluster <= 3 * (size_t)sm_count);
     const int threads = !held || k > 32 ? kWidest : p.slice <= 4096 && k <= 32 ? 64 : 128;
     auto kernel = largest ? topk_rows_kernel<true, false, kWidest, true> : topk_rows_kernel<false, false, kWidest, true>;
     if (held && threads == 64) kernel = largest ? topk_rows_kernel<true, true, 64, false> : topk_rows_kernel<false, true, 64, false>;

@@ -9,7 +9,7 @@ constexpr int kTopKMax = 4096;  // largest k the shared-memory sorter of one CTA
 
 // k <= kTopKMax: selection, then a sort of the k winners in shared memory.
 cudaError_t launch_topk_rows(const float* in, float* values, float* indices, size_t rows, size_t cols, size_t k,
-                             bool largest, cudaStream_t stream);
+                             bool largest, int sm_count, cudaStream_t stream);
 // Any k: the whole row is sorted in `scratch` (sort_rows_scratch_bytes bytes; the rows go through it
 // in launches of *rows_per_launch rows).
 size_t sort_rows_scratch_bytes(size_t rows, size_t cols, size_t* rows_per_launch);
