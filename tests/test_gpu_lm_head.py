@@ -139,6 +139,9 @@ def test_a_second_device_of_the_process(rows):
     (24, 2 * 151_552 + 30_000, True), (32, 2 * 75_776 + 20_000, True), (48, 2 * 75_776 + 40_000, True), (64, 2 * 75_776 + 20_000, True),
     (8, 2 * 151_552 + 44, False), (12, 2 * 151_552 + 40_000, False), (16, 2 * 151_552 + 4, False), (24, 2 * 151_552 + 30_004, False),
     (32, 2 * 75_776 + 20_004, False), (48, 2 * 75_776 + 40_004, False), (64, 2 * 75_776 + 100, False),
+    # vocabularies at which the next wider layout is taken
+    (16, 110_004, True), (32, 18_900, True), (32, 70_000, True), (32, 227_328, True), (12, 90_004, False), (24, 80_004, False), (20, 90_001, False),
+    (24, 130_001, False),
     # five, six and seven entries per lane, and a last tile that is four entries wide
     (24, 90_004, True), (24, 90_004, False), (24, 113_604, False), (24, 130_004, False), (48, 45_060, True), (48, 45_060, False), (48, 66_308, False),
 ])
